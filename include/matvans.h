@@ -195,27 +195,28 @@ typedef struct mv_q8_view {
                                  or of the global table                      */
 } mv_q8_view;
 
-/* y = W x for any batch >= 1 (passes of up to 16 vectors share one decode). */
+/* y = W x for any batch >= 1 (passes of up to 64 vectors share one decode). */
 mv_status mv_q8_matvec(const mv_q8_view *m, const int8_t *x_dev, int batch, int32_t *y_dev,
                        const float *row_scales_dev, float *y_scaled_dev, void *stream);
 
 /* Launch parameters of the persistent Q8 kernel (0 = library default).
- *   warps        warps per CTA (default 8; 16 for the float forward on
- *                the CUDA cores): up to 16, except 8 for the float backward
- *                and the float form on the tensor cores
+ * The integer product runs one CTA per SM: `warps` is the number of its decode
+ * warps (default: as many as fit, up to 16), `parts` as below, and the others
+ * only have to fit shared memory (MV_ERR_UNSUPPORTED if they do not).
+ *   warps        float form: warps per CTA (default 8; 16 for the forward on the
+ *                CUDA cores): up to 16, except 8 for the backward and for
+ *                the tensor cores
  *   ilp          independent segments decoded per warp (1 or 2, default 2;
  *                1 for the float form)
- *   depth        shared-memory stream buffers per warp (1 or 2, default 1):
- *                2 keeps the next work item's bulk copies in flight
+ *   depth        shared-memory stream buffers per warp (1 or 2, default 1)
  *   ctas_per_sm  cap on resident CTAs per SM (default: occupancy limit)
  *   parts        work items per 32-row stripe (its segments split in `parts`
  *                ranges; default: whole stripes in stacks, enough parts to
  *                fill the GPU for a single matrix)
- *   engine       int8 product of 3..16 vectors: 0 = tensor cores
- *                (tcgen05.mma kind::i8, TMEM accumulators, always 16
- *                vectors wide with the missing ones zero; ilp is then 1),
- *                1 = CUDA cores (dp4a).  One or two vectors always use
- *                dp4a. */
+ *   engine       int8 product of 3 or more vectors: 0 = tensor cores
+ *                (tcgen05.mma kind::i8, TMEM accumulators, up to 64 vectors
+ *                per decode), 1 = CUDA cores (dp4a, up to 16).  One or two
+ *                vectors always use dp4a. */
 #define MV_ENGINE_AUTO 0
 #define MV_ENGINE_DP4A 1
 /* Smallest integer batch that engine 0 (MV_ENGINE_AUTO) runs on the tensor
@@ -253,8 +254,8 @@ typedef struct mv_q8_job {
     int8_t *x_tiles;
 } mv_q8_job;
 
-/* Bytes of the x_tiles scratch of a job on matrix m: one 2 KB tile (16
- * vectors x 128 columns) per 32 quads of every segment. */
+/* Bytes of an x_tiles scratch of a job on matrix m (2 KB per 32 quads of every
+ * segment), for callers that still provide one. */
 size_t mv_q8_x_tiles_bytes(const mv_q8_view *m);
 
 typedef struct mv_q8_stack_info {

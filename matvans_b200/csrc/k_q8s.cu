@@ -47,11 +47,10 @@
 #include <cuda_bf16.h>
 
 #include "mv_device.cuh"
+#include "q8w.cuh"
 #include "umma.cuh"
 
 namespace mv {
-
-typedef mv_q8_job Q8Job;
 
 // Shared-memory layout of q8s_kernel (byte offsets; see q8s_layout).
 constexpr uint32_t kStageOffs = 40;  // u32 per staging area: 33 relative offsets, [36] valid, [37] first entry
@@ -229,42 +228,6 @@ __device__ __forceinline__ void issue_step(const Q8SLaunch &L, const StepCursor 
     }
 }
 
-// x loads: plain (coherent, L1-cached) global loads rather than the read-only path.  In a chained
-// launch x was written earlier by other CTAs; the acquire load and CTA barrier of chain_wait order these
-// loads after those writes, which the read-only path would not guarantee.
-__device__ __forceinline__ uint4 ldx_u4(const void *p) { return *reinterpret_cast<const uint4 *>(p); }
-__device__ __forceinline__ uint32_t ldx_u32(const void *p) { return *reinterpret_cast<const uint32_t *>(p); }
-
-template <int NV>
-__device__ __forceinline__ void load_x(const int8_t *x, int cols, int q, uint32_t (&xv)[NV]) {
-#pragma unroll
-    for (int v = 0; v < NV; v++) xv[v] = ldx_u32(reinterpret_cast<const uint32_t *>(x + (size_t)v * cols) + q);
-}
-
-// Four consecutive quads of x (16 bytes) per vector; q % 4 == 0.
-template <int NV>
-__device__ __forceinline__ void load_x4(const int8_t *x, int cols, int q, uint4 (&xv)[NV]) {
-#pragma unroll
-    for (int v = 0; v < NV; v++) xv[v] = ldx_u4(x + (size_t)v * cols + 4 * q);
-}
-
-// The chained pipeline's epilogue of one output: job j's int8 result, the reference's fp32
-// requantisation (ans-warp-rows-kernel.cu:212-220), stored as the next job's x.
-__device__ __forceinline__ void chain_emit(const Q8SLaunch &L, const Q8Job &J, int j, int v, int row, int sum) {
-    const int r = __float2int_rn((float)sum * __ldg(L.chain_scales + j));
-    int8_t *o = j + 1 < L.njobs ? const_cast<int8_t *>(L.jobs[j + 1].x) : L.chain_out8;
-    o[(size_t)v * J.m.rows + row] = (int8_t)max(-128, min(127, r));
-}
-
-template <int NV>
-__device__ __forceinline__ void dot4(uint32_t w, const uint4 (&xv)[NV], int j, int (&acc)[NV]) {
-#pragma unroll
-    for (int v = 0; v < NV; v++) {
-        const uint32_t xw = j == 0 ? xv[v].x : j == 1 ? xv[v].y : j == 2 ? xv[v].z : xv[v].w;
-        acc[v] = __dp4a((int)w, (int)xw, acc[v]);
-    }
-}
-
 // Refill of one stream.  koff is the byte offset (from the start of shared memory) of the lane's next word:
 // it is read every step, and taken when the high half of the state is empty; the offset then moves one
 // 128-byte word-row on, never past kend (the row after the block), so a corrupt stream rereads that row and
@@ -326,41 +289,14 @@ __device__ __forceinline__ uint32_t q8_step_wide(uint32_t &lo, uint32_t &hi, uin
     return __byte_perm(__byte_perm(e0.x, e1.x, 0x0062), __byte_perm(e2.x, e3.x, 0x0062), 0x5410);
 }
 
-// The narrow step over 4-byte entries at a 256-byte pitch: entry (q, lane) at byte q*256 + lane*4 from the
-// start of shared memory, so that one byte permute forms each address as in the wide layout (the other 128
-// bytes of each 256-byte row belong to the consumer).
-__device__ __forceinline__ uint32_t q8_step_n256(uint32_t &lo, uint32_t &hi, uint32_t &koff, const uint32_t kend,
-                                                 const unsigned char *lut_b, uint32_t lane4, uint32_t &P) {
-    q8_refill(lo, hi, koff, kend, lut_b);
-    const uint32_t e0 = *reinterpret_cast<const uint32_t *>(lut_b + __byte_perm(lo, lane4, 0x5504));
-    const uint32_t e1 = *reinterpret_cast<const uint32_t *>(lut_b + __byte_perm(lo, lane4, 0x5514));
-    const uint32_t e2 = *reinterpret_cast<const uint32_t *>(lut_b + __byte_perm(lo, lane4, 0x5524));
-    const uint32_t e3 = *reinterpret_cast<const uint32_t *>(lut_b + __byte_perm(lo, lane4, 0x5534));
-    // entry = f | sym << 16 | r << 24 (byte 1 zero, so the low half-word is exactly f)
-    const uint32_t r0 = __umulhi(e0, 256u), r1 = __umulhi(e1, 256u);
-    const uint32_t r2 = e2 >> 24, r3 = e3 >> 24;
-    const uint32_t u01 = __dp2a_lo(r1, e0, r0);     // r0 + f0*r1
-    const uint32_t t2 = __dp2a_lo(r3, e2, r2);      // r2 + f2*r3
-    const uint32_t p01 = __dp2a_lo(e1, e0, 0u);     // f1*f0
-    const uint32_t p23 = __dp2a_lo(e3, e2, 0u);     // f3*f2
-    P = p01 * p23;
-    const uint32_t t0 = u01 + p01 * t2;             // r0 + f0 r1 + f0 f1 (r2 + f2 r3) < P
-    const unsigned long long st = (unsigned long long)hi * P + t0;
-    lo = (uint32_t)st;
-    hi = (uint32_t)(st >> 32);
-    return __byte_perm(__byte_perm(e0, e1, 0x0062), __byte_perm(e2, e3, 0x0062), 0x5410);
-}
-
 // One step through whichever table layout the consumer uses; sm is the start of shared memory (where the
 // wide and the 256-byte-pitch narrow tables sit), lut the lane's column of the 128-byte-pitch narrow table.
-template <bool kWide, bool k256 = false>
+template <bool kWide>
 __device__ __forceinline__ uint32_t q8_step_t(uint32_t &lo, uint32_t &hi, uint32_t &koff, const uint32_t kend,
                                               const unsigned char *sm, const uint32_t *lut, uint32_t stride, int lane,
                                               uint32_t &P) {
     if constexpr (kWide)
         return q8_step_wide(lo, hi, koff, kend, sm, (uint32_t)lane << 3, P);
-    else if constexpr (k256)
-        return q8_step_n256(lo, hi, koff, kend, sm, (uint32_t)lane << 2, P);
     else
         return q8_step(lo, hi, koff, kend, sm, lut, stride, P);
 }
@@ -386,78 +322,6 @@ struct SegStream {
 // the kernel's output.  Per item it is set up (begin_item), fed groups of four
 // quads (load_group / use) and single tail quads (single), and closes the item
 // (finish_item, which may synchronise the CTA).
-
-// y = W x, int8 x, exact int32 y (+ optional fp32 s*y).
-template <int NV>
-struct IntCons {
-    static constexpr int kNV = NV;
-    static constexpr int kRedNV = NV;
-    static constexpr int kRedBufs = 2;          // alternating reduction areas: one CTA barrier per item
-    static constexpr bool kFinishSyncs = true;  // finish_item holds a CTA barrier
-    static constexpr int kMinCtas = 1;
-    static constexpr int kMaxThreads = 512;  // up to 16 warps per CTA
-    static constexpr int kTmemCols = 0;
-    static constexpr bool kWideLut = true;
-    static constexpr bool kLut256 = false;
-    static __host__ __device__ constexpr size_t extra_bytes(int) { return 0; }
-    static __host__ __device__ constexpr size_t tbl_alias_bytes(int) { return 0; }
-    __device__ __forceinline__ void init(const Q8SLaunch &, unsigned char *, uint32_t, int, int, int) {}
-    __device__ __forceinline__ void drain(const Q8SLaunch &) {}
-    template <int ILP>
-    __device__ __forceinline__ void run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int W,
-                                             const uint32_t (&rows_now)[ILP], const unsigned char *sm,
-                                             uint32_t soff, const uint32_t *lut_l, int lane);
-    const int8_t *x;
-    int cols, job_idx;
-    int acc[NV];
-    struct Group {
-        uint4 xv[NV];
-    };
-    __device__ __forceinline__ void begin_item(const Q8SLaunch &L, const Q8Job &J, int, int, int job) {
-        x = J.x;
-        cols = J.m.cols;
-        job_idx = job;
-#pragma unroll
-        for (int v = 0; v < NV; v++) acc[v] = 0;
-    }
-    __device__ __forceinline__ void load_group(Group &g, int q) const { load_x4<NV>(x, cols, q, g.xv); }
-    __device__ __forceinline__ void use(const Group &g, int j, int, uint32_t wq, int) { dot4<NV>(wq, g.xv, j, acc); }
-    __device__ __forceinline__ void single(int q, uint32_t wq, int) {
-        uint32_t xv[NV];
-        load_x<NV>(x, cols, q, xv);
-#pragma unroll
-        for (int v = 0; v < NV; v++) acc[v] = __dp4a((int)wq, (int)xv[v], acc[v]);
-    }
-    // The CTA barrier here is the only one of an item without a table rebuild: `red` alternates between two
-    // areas, so the next item's partial sums never meet this item's readers.  Every warp has finished its
-    // decode at the barrier, so the decode table may be rebuilt right after it.
-    __device__ __forceinline__ void finish_item(const Q8SLaunch &L, const Q8Job &J, int stripe, int warp, int lane,
-                                                int W, void *red_smem) {
-        int *red = reinterpret_cast<int *>(red_smem);
-#pragma unroll
-        for (int v = 0; v < NV; v++) red[(warp * NV + v) * 32 + lane] = acc[v];
-        __syncthreads();
-        const mv_q8_view &m = J.m;
-        for (int t = threadIdx.x; t < NV * 32; t += blockDim.x) {
-            const int v = t >> 5, l = t & 31;
-            int sum = 0;
-            for (int w = 0; w < W; w++) sum += red[(w * NV + v) * 32 + l];
-            const int row = stripe * 32 + l;
-            if (row < m.rows && v < L.batch) {
-                int32_t *dst = J.y + (size_t)v * m.rows + row;
-                if (J.atomic) {
-                    atomicAdd(dst, sum);
-                } else {
-                    *dst = sum;
-                    if (J.ys) J.ys[(size_t)v * m.rows + row] = (float)sum * J.scales[row];
-                    if (L.chain_scales) chain_emit(L, J, job_idx, v, row, sum);
-                }
-            }
-        }
-        // a chain counts the item as done (thread 0, next) only after every output of it is stored
-        if (L.chain_scales) __syncthreads();
-    }
-};
 
 // four int8 weights (packed) -> fp32: the bytes biased by 128 are the low
 // mantissa bits of 2^23, so each conversion is one byte permute and one add
@@ -733,13 +597,6 @@ __device__ __forceinline__ void decode_step(const Q8SLaunch &L, const mv_q8_view
 
 template <int NV>
 template <int ILP>
-__device__ __forceinline__ void IntCons<NV>::run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int W,
-                                                      const uint32_t (&rows_now)[ILP], const unsigned char *sm,
-                                                      uint32_t soff, const uint32_t *lut_l, int lane) {
-    decode_step<IntCons<NV>, ILP>(L, m, seg0, W, rows_now, sm, soff, lut_l, lane, *this);
-}
-template <int NV>
-template <int ILP>
 __device__ __forceinline__ void FwdCons<NV>::run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int W,
                                                       const uint32_t (&rows_now)[ILP], const unsigned char *sm,
                                                       uint32_t soff, const uint32_t *lut_l, int lane) {
@@ -752,313 +609,6 @@ __device__ __forceinline__ void BwdCons<NV>::run_step(const Q8SLaunch &L, const 
                                                       uint32_t soff, const uint32_t *lut_l, int lane) {
     decode_step<BwdCons<NV>, ILP>(L, m, seg0, W, rows_now, sm, soff, lut_l, lane, *this);
 }
-
-// y = W x for 8..16 int8 vectors on the tensor cores.  Every 16 decoded quads
-// the 32 lanes of a warp (= the 32 rows of the stripe) hold a 32 x 64 int8
-// tile of W, one row per lane: each lane writes its row straight from
-// registers into its own TMEM lane (tcgen05.st, 8 quads at a time), and one
-// lane issues two tcgen05.mma.kind::i8 (K = 32 each) with A = that tile in
-// TMEM (M = 128: the warp's lane quarter holds its 32 rows, the other lanes
-// are never written and their results never read), B = the x tile in shared
-// memory (N = 16 vectors, K-major core matrices of 8 rows x 16 bytes),
-// accumulating exactly in int32 in the warp's own 16 TMEM columns.  Each warp
-// owns 32 TMEM columns: D [0,16) and the A tile [16,32).  One tcgen05.commit
-// per 16 quads arrives on the warp's mbarrier; the A tile is rewritten only
-// after the previous pair of MMAs completed (issued a whole 16-quad decode
-// earlier, so the wait is normally already over).  x moves through a
-// 128-column window (4 x 32 columns x 16 vectors, 2 KB per warp); the next
-// window is loaded while the current one is in use.  ILP 1 only.
-//
-// Shared memory: the decode table takes 4-byte entries at a 256-byte pitch
-// (entry (q, lane) at byte q*256 + lane*4, one byte permute per address), and
-// the x tiles of warps 0..7 live in the other half of each 256-byte row: 256
-// holes of 128 bytes, one core matrix each, 32 per warp (two tiles of 16).
-// Core matrix c = t*16 + p*4 + n*2 + k ((n, k) of piece p of tile t) sits at
-// base + c * stride: stride 256 B in the holes (LBO, K direction, 256 B; SBO,
-// N direction, 512 B), 128 B for warps 8..15, whose tiles are contiguous
-// behind the table (LBO 128, SBO 256).  64 KB hold table and eight warps' x
-// tiles, as much as the 32 KB table with separate x tiles, so two 8-warp CTAs
-// still fit an SM.  The tiles also take the cross-warp reduction.
-struct MmaCons {
-    static constexpr int kNV = 16;
-    static constexpr int kRedNV = 0;      // reduction area: the x tiles
-    static constexpr int kRedBufs = 1;
-    static constexpr bool kFinishSyncs = true;
-    static constexpr int kMinCtas = 1;    // with up to 16 warps: at most 128 registers per thread
-    static constexpr int kMaxThreads = 512;  // 2 x 8 warps per SM (stacks) or 1 x 16 (chains)
-    static constexpr int kTmemCols = 1;   // > 0: the kernel allocates TMEM
-    static constexpr bool kWideLut = false;
-    static constexpr bool kLut256 = true;  // 4-byte entries at a 256-byte pitch, x tiles in between
-    static constexpr int kXChunks = 4;    // x tile: 4 pieces of 32 columns x 16 vectors (512 B each)
-    static constexpr int kXBytes = kXChunks * 512;
-    static constexpr uint32_t kHoles = kXBytes / 128;  // core matrices per tile
-    // x tiles of warps 8..15 (4 KB each) at the start of the consumer region
-    static __host__ __device__ constexpr size_t xr_bytes(int W) { return W > 8 ? (size_t)(W - 8) * 2 * kXBytes : 0; }
-    static __host__ __device__ constexpr size_t extra_bytes(int W) {
-        // those x tiles, three mbarriers per warp (MMA commits, x copies into tile 0 / 1), TMEM address slot
-        // (the last 128 bytes); a multiple of 128 bytes, so the stream buffers that follow stay 16-byte
-        // aligned
-        return ((xr_bytes(W) + (size_t)W * 24 + 128) + 127) / 128 * 128;
-    }
-    static __host__ __device__ constexpr size_t tbl_alias_bytes(int) { return 0; }
-    static __host__ __device__ constexpr uint32_t tmem_cols(int W) {
-        return W <= 1 ? 32 : W <= 2 ? 64 : W <= 4 ? 128 : W <= 8 ? 256 : 512;
-    }
-    // warp w's core matrix 0 of tile 0 (byte offset from the start of shared memory) and core-matrix stride
-    static __device__ __forceinline__ uint32_t tile_base(const Q8SLaunch &L, int w) {
-        return w < 8 ? (uint32_t)w * (2u * kHoles) * 256u + 128u : L.lay.extra + (uint32_t)(w - 8) * 2u * kXBytes;
-    }
-    static __device__ __forceinline__ uint32_t tile_stride(int w) { return w < 8 ? 256u : 128u; }
-    uint32_t xt, d_tmem, st_addr, ld_addr, ncommit, xcur, xcnt0, xcnt1, xb, cst;
-    uint64_t b_desc0;
-    uint32_t mbar, xbar;  // shared-memory addresses: the MMA barrier, the two x-window barriers (8 bytes apart)
-    unsigned char *sm0;  // start of shared memory (table and holes)
-    const int8_t *x;
-    const int8_t *tiles;  // x laid out per (segment, window) by q8s_build_x_tiles, or null
-    int cols, batch, job_idx, nwin;
-    bool any;
-
-    __device__ __forceinline__ void init(const Q8SLaunch &L, unsigned char *extra, uint32_t tmem_base, int,
-                                         int lane, int W) {
-        // the warp index through a shuffle from lane 0 is known warp-uniform to the compiler, so the MMA
-        // operands derived from it stay in uniform registers
-        const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
-        sm0 = extra - L.lay.extra;  // the table (and its holes) starts shared memory
-        xb = tile_base(L, warp);
-        cst = tile_stride(warp);
-        xt = smem_u32(sm0) + xb;  // tile 0, core matrix 0
-        uint64_t *mb = reinterpret_cast<uint64_t *>(extra + xr_bytes(W)) + warp;
-        uint64_t *xbp = reinterpret_cast<uint64_t *>(extra + xr_bytes(W) + (size_t)W * 8) + 2 * warp;
-        if (lane == 0) {
-            mbar_init(mb, 1);
-            mbar_init(&xbp[0], 32);  // x windows: one arrival per lane (x_copy)
-            mbar_init(&xbp[1], 32);
-        }
-        mbar = smem_u32(mb);
-        xbar = smem_u32(xbp);
-        fence_mbar_init();
-        __syncwarp();
-        // TMEM addresses: lane in bits [16,32), column in [0,16); a warp may touch only the 32 lanes of its
-        // quarter (warp % 4) with tcgen05.ld/st, while an MMA with M = 128 addresses lanes from 0
-        const uint32_t quarter = ((uint32_t)(warp & 3) * 32u) << 16;
-        d_tmem = tmem_base + 32u * (uint32_t)warp;
-        st_addr = d_tmem + 16u + quarter;
-        ld_addr = d_tmem + quarter;
-        b_desc0 = umma_smem_desc(xt, cst, 2u * cst);
-        ncommit = 0;
-        xcur = 1;  // the x tile of the latest window; a segment's first window goes to the other one
-        xcnt0 = xcnt1 = 0;
-    }
-    __device__ __forceinline__ void begin_item(const Q8SLaunch &L, const Q8Job &J, int, int, int job) {
-        x = J.x;
-        cols = J.m.cols;
-        batch = L.batch;
-        any = false;
-        job_idx = job;
-        tiles = J.x_tiles;
-        nwin = (J.m.seg_quads + 31) / 32;
-    }
-    // Asynchronous copies of x window w of segment seg (2 KB, contiguous in the x tiles) into tile t: lane l
-    // copies the 16-byte rows l, l + 32, l + 64, l + 96 (row k = row k % 8 of core matrix k / 8, which sits in
-    // its own hole) and then arrives on the tile's barrier once its copies have landed.  Every lane counts
-    // the window.  The tile's previous readers (MMAs) are done.  Per-lane 16-byte copies rather than one
-    // 128-byte bulk copy per core matrix: bulk copies take warp-uniform operands, so sixteen lanes each
-    // issuing one compiled to a loop over the lanes that cost about 8 instructions per decode step.
-    __device__ __forceinline__ void x_copy(int t, int seg, int w, int lane) {
-        const int8_t *src = tiles + ((size_t)seg * nwin + w) * kXBytes;
-        const uint32_t dst = xt + (uint32_t)t * kHoles * cst;
-#pragma unroll
-        for (uint32_t i = 0; i < kXBytes / 512; i++) {
-            const uint32_t k = (uint32_t)lane + 32u * i;
-            cp_async_16(dst + (k >> 3) * cst + (k & 7u) * 16u, src + (size_t)k * 16);
-        }
-        cp_async_mbar_arrive_noinc(xbar + 8u * (uint32_t)t);
-        if (t) xcnt1++;
-        else xcnt0++;
-    }
-    // The window's copies (generic proxy) are visible to every lane once the barrier phase completes; the
-    // proxy fence orders them before the tensor core's reads of the tile (async proxy).
-    __device__ __forceinline__ void x_wait(const Q8SLaunch &L, int t) {
-        const uint32_t n = t ? xcnt1 : xcnt0;
-        // on a timeout (flagged) wait once more, bounded, so that no copy is left in flight
-        const uint32_t bar = xbar + 8u * (uint32_t)t;
-        if (!mbar_wait_bounded(bar, (n - 1) & 1, L.status, L.spin_limit))
-            mbar_wait_bounded(bar, (n - 1) & 1, nullptr, L.spin_limit);
-        fence_proxy_async_smem();
-    }
-    // wait until every MMA issued so far completed (the latest commit covers all earlier MMAs)
-    __device__ __forceinline__ bool wait_mma(const Q8SLaunch &L) {
-        if (ncommit == 0) return true;
-        return mbar_wait_bounded(mbar, (ncommit - 1) & 1, L.status, L.spin_limit);
-    }
-    __device__ __forceinline__ void issue(int piece, bool two) {
-        tcgen05_fence_before();
-        __syncwarp();
-        if (elect_one()) {
-            tcgen05_fence_after();
-            // B descriptor start addresses are in 16-byte units: tile xcur is 16 core matrices in, piece p 4
-            const uint32_t idesc = umma_idesc_i8(128, 16);
-            const uint64_t bd = b_desc0 + (uint64_t)(xcur * cst + (uint32_t)piece * (cst / 4u));
-            umma_i8_ts(d_tmem, d_tmem + 16u, bd, idesc, any ? 1u : 0u);
-            if (two) umma_i8_ts(d_tmem, d_tmem + 24u, bd + cst / 4u, idesc, 1u);  // the next piece
-            umma_commit(mbar);
-        }
-        __syncwarp();
-        any = true;
-        ncommit++;
-    }
-    // lane (b, h) holds 16 bytes (column half h) of vector b for each 32-column piece of a window
-    __device__ __forceinline__ void load_window(uint4 (&xr)[kXChunks], const int8_t *xrow, bool xok, int colbase,
-                                                int pbase, int npieces) const {
-        if (xok && pbase + kXChunks <= npieces && colbase + 32 * (pbase + kXChunks - 1) < cols) {
-            // a full window inside the row: plain loads, no per-piece checks
-#pragma unroll
-            for (int i = 0; i < kXChunks; i++) xr[i] = ldx_u4(xrow + 32 * (pbase + i));
-            return;
-        }
-#pragma unroll
-        for (int i = 0; i < kXChunks; i++) {
-            const int c = pbase + i;
-            xr[i] = make_uint4(0, 0, 0, 0);
-            // cols % 16 == 0, so a 16-byte piece that starts inside the row ends inside it
-            if (xok && c < npieces && colbase + 32 * c < cols) xr[i] = ldx_u4(xrow + 32 * c);
-        }
-    }
-    template <int ILP>
-    __device__ __forceinline__ void run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int,
-                                             const uint32_t (&rows_now)[ILP], const unsigned char *sm,
-                                             uint32_t soff, const uint32_t *lut_l, int lane) {
-        const int qtot = (m.cols + 3) >> 2;
-        const int q0 = seg0 * m.seg_quads;
-        const int nq = rows_now[0] ? min(m.seg_quads, qtot - q0) : 0;
-        if (nq <= 0) return;
-        const int npieces = (nq + 7) >> 3;  // 32-column pieces (8 quads each)
-        const int b = lane >> 1, h = lane & 1;
-        const bool xok = b < batch;
-        const int colbase = 4 * q0 + 16 * h;
-        const int8_t *xrow = x + (size_t)(xok ? b : 0) * cols + colbase;
-        // core matrix (n, k) = (b / 8, h) of piece i is core matrix 4 i + 2 n + k of tile 0, row b % 8
-        const uint32_t xdst = xt + ((uint32_t)(b >> 3) * 2u + (uint32_t)h) * cst + (uint32_t)(b & 7) * 16u;
-        uint4 xr[kXChunks];
-        // with x tiles: the first window goes to the tile the latest window did not use (its MMAs completed
-        // before the latest window started); without: windows pass through registers into tile 0
-        int xnext = xcur ^ 1u;
-        if (tiles) {
-            x_copy(xnext, seg0, 0, lane);
-        } else {
-            xcur = 0;
-            load_window(xr, xrow, xok, colbase, 0, npieces);
-        }
-        SegStream S(sm, soff, rows_now[0], lane);
-        // pieces in pairs: piece p = 2 * pair (+1); a window holds 2 pairs.  A pair of two full pieces (16
-        // quads) takes the body without the tail tests; the segment's last pair may be partial.
-        auto pair = [&](const int p, auto full) {
-            constexpr bool kFull = decltype(full)::value;
-            uint32_t w[8];
-            const int qc = 8 * p;
-            if (kFull || qc + 8 <= nq) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) w[j] = q8_step_t<kWideLut, kLut256>(S.lo, S.hi, S.koff, S.kend, sm, lut_l, L.lut_stride, lane, S.P);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    w[j] = (qc + j < nq) ? q8_step_t<kWideLut, kLut256>(S.lo, S.hi, S.koff, S.kend, sm, lut_l, L.lut_stride, lane, S.P) : 0u;
-            }
-            // the previous pair of MMAs is done with the A tile (and, at a window start, with the x tile)
-            wait_mma(L);
-            const int pw = p & (kXChunks - 1);  // piece within the window
-            if (pw == 0 && tiles) {
-                // this window's copy has landed (it was the only one in flight); the next goes to the other
-                // tile, whose MMAs are done (above)
-                x_wait(L, xnext);
-                xcur = xnext;
-                if (p + kXChunks < npieces) {
-                    xnext = xcur ^ 1u;
-                    x_copy(xnext, seg0, (p + kXChunks) / kXChunks, lane);
-                }
-            } else if (pw == 0) {
-                // the whole window is stored (pieces past the segment hold zeros or stale x, and are never
-                // multiplied: the MMAs of a pair read only the pieces that exist)
-#pragma unroll
-                for (int i = 0; i < kXChunks; i++)
-                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(xdst + (uint32_t)i * 4u * cst),
-                                 "r"(xr[i].x), "r"(xr[i].y), "r"(xr[i].z), "r"(xr[i].w)
-                                 : "memory");
-                fence_proxy_async_smem();  // the x tile is read by the tensor core (async proxy)
-                if (p + kXChunks < npieces) load_window(xr, xrow, xok, colbase, p + kXChunks, npieces);
-            }
-            tcgen05_fence_after();
-            tmem_st_32x32b_x8_nowait(st_addr, w);
-            const bool two = kFull || p + 1 < npieces;
-            if (two) {
-                const int qc2 = qc + 8;
-                if (kFull || qc2 + 8 <= nq) {
-#pragma unroll
-                    for (int j = 0; j < 8; j++) w[j] = q8_step_t<kWideLut, kLut256>(S.lo, S.hi, S.koff, S.kend, sm, lut_l, L.lut_stride, lane, S.P);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        w[j] = (qc2 + j < nq) ? q8_step_t<kWideLut, kLut256>(S.lo, S.hi, S.koff, S.kend, sm, lut_l, L.lut_stride, lane, S.P) : 0u;
-                }
-                tmem_st_32x32b_x8_nowait(st_addr + 8u, w);
-            }
-            tmem_wait_st();
-            issue(pw, two);
-        };
-        const int pfull = (nq >> 4) << 1;  // pieces covered by full pairs
-        for (int p = 0; p < pfull; p += 2) pair(p, std::true_type{});
-        if (pfull < npieces) pair(pfull, std::false_type{});
-        if (!S.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
-    }
-    __device__ __forceinline__ void finish_item(const Q8SLaunch &L, const Q8Job &J, int stripe, int warp, int lane,
-                                                int W, void *) {
-        uint32_t r[16];
-        if (any) {
-            wait_mma(L);
-            tcgen05_fence_after();
-            tmem_ld_32x32b_x16(ld_addr, r);  // lane = stripe row, r[v] = vector v
-        } else {
-#pragma unroll
-            for (int v = 0; v < 16; v++) r[v] = 0;
-        }
-        // this warp's MMAs (and x copies) are complete, so its own x tiles take its partial sums: vector v
-        // of stripe row l in core matrix v of tile 0, word l
-#pragma unroll
-        for (int v = 0; v < 16; v++) *reinterpret_cast<int *>(sm0 + xb + (uint32_t)v * cst + 4 * lane) = (int)r[v];
-        tcgen05_fence_before();
-        __syncthreads();
-        const mv_q8_view &m = J.m;
-        const int W8 = min(W, 8);
-        for (int t = threadIdx.x; t < 16 * 32; t += blockDim.x) {
-            const int v = t >> 5, l = t & 31;
-            int sum = 0;
-            // warps 0..7: tile 0 at hole 32 w (byte 8192 w + 128), core matrix v one 256-byte row further
-            const unsigned char *h = sm0 + 128u + (uint32_t)v * 256u + 4u * (uint32_t)l;
-#pragma unroll
-            for (int w = 0; w < 8; w++)
-                if (w < W8) sum += *reinterpret_cast<const int *>(h + (uint32_t)w * 2u * kHoles * 256u);
-            for (int w = 8; w < W; w++)
-                sum += *reinterpret_cast<const int *>(sm0 + tile_base(L, w) + (uint32_t)v * tile_stride(w) + 4 * l);
-            const int row = stripe * 32 + l;
-            if (row < m.rows && v < L.batch) {
-                int32_t *dst = J.y + (size_t)v * m.rows + row;
-                if (J.atomic) {
-                    atomicAdd(dst, sum);
-                } else {
-                    *dst = sum;
-                    if (J.ys) J.ys[(size_t)v * m.rows + row] = (float)sum * J.scales[row];
-                    if (L.chain_scales) chain_emit(L, J, job_idx, v, row, sum);
-                }
-            }
-        }
-        fence_proxy_async_smem();  // these generic accesses come before the tensor core's later reads of the tiles
-        __syncthreads();  // the x tiles are written again (tables, x) by the next item
-    }
-    __device__ __forceinline__ void drain(const Q8SLaunch &L) {
-        wait_mma(L);
-        cp_async_wait_all();  // no x copy is left writing shared memory after the CTA exits
-    }
-};
 
 // four int8 weights (packed) -> four bf16 (exact: |w| <= 127 needs 7 significand bits), as two bf16x2
 // words in column order: lo = (w0, w1), hi = (w2, w3)
@@ -1668,6 +1218,8 @@ __device__ __forceinline__ void build_table(const Q8SLaunch &L, const mv_q8_view
     }
 }
 
+__host__ __device__ constexpr uint32_t tmem_cols(int W) { return W <= 1 ? 32 : W <= 2 ? 64 : W <= 4 ? 128 : W <= 8 ? 256 : 512; }
+
 template <class Cons, int ILP, int DEPTH>
 __global__ void __launch_bounds__(Cons::kMaxThreads, Cons::kMinCtas) q8s_kernel(const Q8SLaunch L) {
     constexpr int NV = Cons::kRedNV;
@@ -1693,7 +1245,7 @@ __global__ void __launch_bounds__(Cons::kMaxThreads, Cons::kMinCtas) q8s_kernel(
     uint32_t tmem_base = 0;
     if (Cons::kTmemCols) {
         uint32_t *slot = reinterpret_cast<uint32_t *>(extra + Cons::extra_bytes(W) - 128);
-        if (warp == 0) tmem_alloc(slot, MmaCons::tmem_cols(W));
+        if (warp == 0) tmem_alloc(slot, tmem_cols(W));
         tcgen05_fence_before();
         __syncthreads();
         tcgen05_fence_after();
@@ -1865,37 +1417,13 @@ __global__ void __launch_bounds__(Cons::kMaxThreads, Cons::kMinCtas) q8s_kernel(
         cons.drain(L);
         tcgen05_fence_before();
         __syncthreads();
-        if (warp == 0) tmem_dealloc(tmem_base, MmaCons::tmem_cols(W));
+        if (warp == 0) tmem_dealloc(tmem_base, tmem_cols(W));
     }
 }
 
 }  // namespace mv
 
 namespace mv {
-
-// x of every job with x_tiles, laid out per (segment, 32-quad window) in the tensor-core consumer's x tile
-// layout: 2 KB per tile = 4 pieces of 32 columns; piece = 2 groups of 8 vectors (256 B); group = 2 column
-// halves (128 B); half = 8 vectors x 16 bytes.  Vectors past the batch and columns past the row are zero.
-__global__ void q8s_build_x_tiles(const Q8Job *jobs, int njobs, int batch) {
-    for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
-        const Q8Job &J = jobs[j];
-        if (!J.x_tiles) continue;
-        const mv_q8_view &m = J.m;
-        const int nwin = (m.seg_quads + 31) / 32;
-        const size_t units = (size_t)m.nseg * nwin * 128;  // 16-byte units
-        for (size_t u = blockIdx.x * (size_t)blockDim.x + threadIdx.x; u < units; u += (size_t)gridDim.x * blockDim.x) {
-            const size_t tile = u >> 7;
-            const int o = (int)(u & 127);
-            const int sg = (int)(tile / nwin), w = (int)(tile % nwin);
-            const int i = o >> 5, g = (o >> 4) & 1, h = (o >> 3) & 1, r = o & 7;
-            const int v = 8 * g + r;
-            const int col = 4 * sg * m.seg_quads + 128 * w + 32 * i + 16 * h;  // a multiple of 16
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (v < batch && col < m.cols) val = *reinterpret_cast<const uint4 *>(J.x + (size_t)v * m.cols + col);
-            *reinterpret_cast<uint4 *>(J.x_tiles + tile * 2048 + (size_t)o * 16) = val;
-        }
-    }
-}
 
 __global__ void q8s_zero_atomic_y(const Q8Job *jobs, int njobs, int batch) {
     for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
@@ -1963,7 +1491,7 @@ mv_status launch_q8s_t(const Q8SLaunch &L0, int W, int ctas_per_sm, cudaStream_t
         rc = resident_ctas((const void *)kern, smem, 32 * W, &bps);
         if (rc) return rc;
         if (ctas_per_sm > 0) bps = std::min(bps, ctas_per_sm);
-        bps = std::max(1, std::min<int>(bps, 512 / MmaCons::tmem_cols(W)));
+        bps = std::max(1, std::min<int>(bps, 512 / tmem_cols(W)));
     }
     if (L.chain_scales) {
         // the chained pipeline waits across CTAs: a cooperative launch guarantees that they are all resident.
@@ -2001,22 +1529,9 @@ mv_status launch_q8s_c(const Q8SLaunch &L, const mv_q8_tuning &t, cudaStream_t s
     }
 }
 
-// Integer batches of at least this many vectors (rounded up to 4, 8 or 16) go to the tensor-core consumer
-// (engine 0), which always multiplies 16 vectors, the missing ones zero: its cost hardly depends on the batch
-// (the 224-matrix stack: 3.86 ms at 8 vectors, 3.88 ms at 16), while the dp4a consumer's grows with it (4.25
-// ms at 4 vectors, 2.91 ms at 1).
+// Integer batches of at least this many vectors go to the tensor-core consumer (engine 0), whose cost hardly depends
+// on the batch, while the dp4a consumer's grows with it.
 constexpr int kMmaMinVectors = MV_MMA_MIN_VECTORS;
-
-mv_status launch_q8s(const Q8SLaunch &L, int nv, const mv_q8_tuning &t, cudaStream_t st) {
-    if (nv >= kMmaMinVectors && t.engine == MV_ENGINE_AUTO) return launch_q8s_c<MmaCons>(L, t, st);
-    switch (nv) {
-        case 1: return launch_q8s_c<IntCons<1>>(L, t, st);
-        case 2: return launch_q8s_c<IntCons<2>>(L, t, st);
-        case 4: return launch_q8s_c<IntCons<4>>(L, t, st);
-        case 8: return launch_q8s_c<IntCons<8>>(L, t, st);
-        default: return launch_q8s_c<IntCons<16>>(L, t, st);
-    }
-}
 
 // mode 1: float forward, mode 2: float backward (transposed); nv in {1,2,4,8}
 // float form: batches of at least this many vectors go to the tensor-core consumers (engine 0)
@@ -2070,6 +1585,8 @@ mv_q8_tuning resolve(const mv_q8_tuning *t) {
 // parts = 0: whole stripes (stacks); otherwise split each stripe's segments into `parts`
 void plan_job(Q8Job &J, const mv_q8_tuning &t, uint32_t &item, int parts) {
     J.ngroups = std::max(1, std::min(parts > 0 ? parts : 1, J.m.nseg));
+    const int spp = (J.m.nseg + J.ngroups - 1) / J.ngroups;
+    J.ngroups = (J.m.nseg + spp - 1) / spp;  // no empty part
     J.atomic = J.ngroups > 1;
     J.item0 = item;
     J.pad = 0;  // work-queue counter (job 0 of a stack) or item counter (chains)
@@ -2081,7 +1598,7 @@ void plan_job(Q8Job &J, const mv_q8_tuning &t, uint32_t &item, int parts) {
 // Work items per stripe for a single matrix: enough items for ~4 per SM, but no more than it takes
 // to give each of the CTA's sg = warps x ilp segment slots one segment per item (ceil, so that the
 // items of a stripe are as even as its segment count allows)
-int default_parts(int nseg, int sg, int stripes) {
+int fill_parts(int nseg, int sg, int stripes) {
     const int fill = (4 * sm_count() + stripes - 1) / stripes;
     const int even = (nseg + sg - 1) / sg;
     return std::max(1, std::min(fill, even));
@@ -2110,27 +1627,64 @@ bool q8s_supports(const mv_q8_view *m, const int8_t *x) {
     return (m->cols & 15) == 0 && ((uintptr_t)x & 15) == 0 && (m->seg_quads & 3) == 0;
 }
 
-// Single matrix through the persistent kernel (one inline job).
+// The launch shape a caller asks for (or the default one) has to fit shared memory with a decode table of 64 KB and
+// `warps` x ilp x depth stream slots, whatever shape the kernel then runs in.
+mv_status check_shape(const mv_q8_tuning &t, bool mma, int nv, int max_blk_rows, uint32_t tbl_stripe_max) {
+    const int ilp = mma ? 1 : t.ilp;
+    const size_t slots = (size_t)t.warps * ilp * t.depth;
+    const size_t need = 65536 + slots * (size_t)(max_blk_rows + 1) * 128 + 2 * ((size_t)tbl_stripe_max + 8) +
+                        (mma ? (size_t)std::max(0, t.warps - 8) * 4096 + (size_t)t.warps * 24 + 128
+                             : (size_t)2 * t.warps * nv * 128) + 1024;
+    if (need > (size_t)max_smem_optin())
+        return fail(MV_ERR_UNSUPPORTED, "Q8 launch: %d warps x %d segments x %d buffers need %zu B of shared memory (max %d)",
+                    t.warps, ilp, t.depth, need, max_smem_optin());
+    return MV_OK;
+}
+
+// Parts per stripe of a single matrix, from the time of the busiest CTA: its units in rounds of kDecodeWarps (a step
+// of a lone warp takes ~70 cycles, of a full CTA ~9 per warp), no less than its table builds (~2500 cycles each),
+// plus, with more than one part, the zeroing of y and the atomics (~5000 cycles).
+int default_parts(int nseg, int seg_quads, int stripes) {
+    constexpr long long kDecodeWarps = 15, kBuild = 6000, kAtomics = 5000;
+    const long long G = sm_count();
+    int best = 1;
+    long long best_cost = -1;
+    for (int p = 1; p <= 64 && p <= nseg; p++) {
+        const long long items = ((long long)stripes * p + G - 1) / G, units = items * ((nseg + p - 1) / p);
+        const long long rounds = (units + kDecodeWarps - 1) / kDecodeWarps;
+        const long long cost =
+            std::max(seg_quads * std::max(rounds * 70, units * 9), items * kBuild) + (p > 1 ? kAtomics : 0);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = p;
+        }
+    }
+    return best;
+}
+
+// Single matrix through the persistent kernel (one inline job): passes of up to 64 vectors on the tensor cores, of
+// up to 16 on the CUDA cores.
 mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y, const float *scales, float *ys,
                      const mv_q8_tuning *tuning, cudaStream_t st) {
     mv_status rc;
     uint32_t *status = device_status_word(&rc);
     if (rc) return rc;
     const mv_q8_tuning t = resolve(tuning);
-    for (int v0 = 0; v0 < batch; v0 += 16) {
-        const int nb = std::min(16, batch - v0);
-        Q8SLaunch L{};
+    const int pass = t.engine == MV_ENGINE_AUTO ? 64 : 16;
+    for (int v0 = 0; v0 < batch; v0 += pass) {
+        const int nb = std::min(pass, batch - v0);
+        const bool mma = t.engine == MV_ENGINE_AUTO && nb >= kMmaMinVectors;
+        rc = check_shape(t, mma, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
+        if (rc) return rc;
+        Q8WLaunch L{};
         L.job0.m = *m;
         L.job0.x = x + (size_t)v0 * m->cols;
         L.job0.y = y + (size_t)v0 * m->rows;
         L.job0.scales = scales;
         L.job0.ys = ys ? ys + (size_t)v0 * m->rows : nullptr;
         uint32_t items = 0;
-        // a single matrix: split stripes so that every warp slot of the GPU gets work
         const int stripes = (m->rows + 31) / 32;
-        const int sg = t.warps * t.ilp;
-        int parts = t.parts > 0 ? t.parts : default_parts(m->nseg, sg, stripes);
-        plan_job(L.job0, t, items, parts);
+        plan_job(L.job0, t, items, t.parts > 0 ? t.parts : default_parts(m->nseg, m->seg_quads, stripes));
         if (L.job0.atomic) L.job0.ys = nullptr;
         L.jobs = nullptr;
         L.njobs = 1;
@@ -2139,12 +1693,14 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.status = status;
         L.spin_limit = wait_spin_limit();
         L.drop_copy = inject_drop_copy();
-        L.buf_words = (m->max_blk_rows + 1) * 32;
+        L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
-        L.lut_stride = 32;
         if (L.job0.atomic)
             MV_CUDA_TRY(cudaMemsetAsync(L.job0.y, 0, sizeof(int32_t) * (size_t)nb * m->rows, st), "cudaMemsetAsync(y)");
-        rc = launch_q8s(L, nv_round(nb), t, st);
+        const int spp = (m->nseg + L.job0.ngroups - 1) / L.job0.ngroups;
+        const long long per_cta = ((long long)items + sm_count() - 1) / sm_count() * spp;
+        rc = q8w_launch_int(L, nv_round(nb), mma, tuning && tuning->warps > 0 ? t.warps : 0,
+                            (int)std::min<long long>(per_cta, 1 << 20), st);
         if (rc) return rc;
         if (ys && L.job0.atomic) {
             const int n = nb * m->rows;
@@ -2182,7 +1738,7 @@ mv_status q8f_run(const mv_q8_view *m, int mode, const uint16_t *in, int batch, 
         int parts = 1;
         if (mode == 2) {
             const int stripes = (m->rows + 31) / 32, sg = t.warps * t.ilp;
-            parts = t.parts > 0 ? t.parts : mma ? default_parts(m->nseg, sg, stripes) : bwd_parts(m->nseg, sg, stripes);
+            parts = t.parts > 0 ? t.parts : mma ? fill_parts(m->nseg, sg, stripes) : bwd_parts(m->nseg, sg, stripes);
         }
         plan_job(L.job0, t, items, parts);
         if (mode == 1 && L.job0.atomic) return fail(MV_ERR_ARG, "float forward needs whole stripes (parts = 1)");
@@ -2312,7 +1868,7 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
         return mv::fail(MV_ERR_ARG, "mv_q8_chain_matvec: tuning differs from the one the jobs were planned with");
     cudaStream_t st = (cudaStream_t)stream;
     mv_status rc;
-    mv::Q8SLaunch L{};
+    mv::Q8WLaunch L{};
     L.status = mv::device_status_word(&rc);
     if (rc) return rc;
     L.jobs = jobs_dev;
@@ -2321,14 +1877,17 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
     L.batch = batch;
     L.spin_limit = mv::wait_spin_limit();
     L.drop_copy = mv::inject_drop_copy();
-    L.buf_words = (info->max_blk_rows + 1) * 32;
+    L.slot_bytes = (uint32_t)(info->max_blk_rows + 1) * 128u;
     L.tbl_stage = (int)((info->tbl_stripe_max + 7) & ~7u);
-    L.lut_stride = 32;
     L.chain_scales = chain_scales_dev;
     L.chain_out8 = out8_dev;
+    const int nv = mv::nv_round(batch);
+    const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
+    rc = mv::check_shape(t, mma, nv, info->max_blk_rows, info->tbl_stripe_max);
+    if (rc) return rc;
     mv::q8s_chain_reset<<<(njobs + 255) / 256, 256, 0, st>>>(reinterpret_cast<mv::Q8Job *>(jobs_dev), njobs);
     MV_CUDA_TRY(cudaGetLastError(), "q8s_chain_reset launch");
-    return mv::launch_q8s(L, mv::nv_round(batch), t, st);
+    return mv::q8w_launch_int(L, nv, mma, tuning && tuning->warps > 0 ? t.warps : 0, 1 << 20, st);
 }
 
 mv_status mv_q8_stack_matvec(const mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_info *info, int batch,
@@ -2340,7 +1899,7 @@ mv_status mv_q8_stack_matvec(const mv_q8_job *jobs_dev, int njobs, const mv_q8_s
         return mv::fail(MV_ERR_ARG, "mv_q8_stack_matvec: tuning differs from the one the jobs were planned with");
     cudaStream_t st = (cudaStream_t)stream;
     mv_status rc;
-    mv::Q8SLaunch L{};
+    mv::Q8WLaunch L{};
     L.status = mv::device_status_word(&rc);
     if (rc) return rc;
     L.jobs = jobs_dev;
@@ -2349,21 +1908,20 @@ mv_status mv_q8_stack_matvec(const mv_q8_job *jobs_dev, int njobs, const mv_q8_s
     L.batch = batch;
     L.spin_limit = mv::wait_spin_limit();
     L.drop_copy = mv::inject_drop_copy();
-    L.buf_words = (info->max_blk_rows + 1) * 32;
+    L.slot_bytes = (uint32_t)(info->max_blk_rows + 1) * 128u;
     L.tbl_stage = (int)((info->tbl_stripe_max + 7) & ~7u);
-    L.lut_stride = 32;
     // work queue: jobs_dev[0].pad, zero after planning and after every completed launch
     if (info->nitems < 0x7FFFFFFFu) L.queue = const_cast<uint32_t *>(&jobs_dev[0].pad);
+    const int nv = mv::nv_round(batch);
+    const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
+    rc = mv::check_shape(t, mma, nv, info->max_blk_rows, info->tbl_stripe_max);
+    if (rc) return rc;
     dim3 zg(64, std::min(njobs, 1024));
     if (info->atomic_jobs > 0) {
         mv::q8s_zero_atomic_y<<<zg, 256, 0, st>>>(jobs_dev, njobs, batch);
         MV_CUDA_TRY(cudaGetLastError(), "q8s_zero_atomic_y launch");
     }
-    if (mv::nv_round(batch) >= mv::kMmaMinVectors && t.engine == MV_ENGINE_AUTO) {  // the tensor-core consumer reads x tiles
-        mv::q8s_build_x_tiles<<<zg, 256, 0, st>>>(jobs_dev, njobs, batch);
-        MV_CUDA_TRY(cudaGetLastError(), "q8s_build_x_tiles launch");
-    }
-    rc = mv::launch_q8s(L, mv::nv_round(batch), t, st);
+    rc = mv::q8w_launch_int(L, nv, mma, tuning && tuning->warps > 0 ? t.warps : 0, 1 << 20, st);
     if (rc) return rc;
     if (info->atomic_jobs > 0) {
         mv::q8s_scale_atomic_y<<<zg, 256, 0, st>>>(jobs_dev, njobs, batch);

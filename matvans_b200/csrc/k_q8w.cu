@@ -1,0 +1,1187 @@
+// Decode + int8 product over a list of Q8-stripe matrices ("jobs": one matrix
+// with its x and y each) in one launch, for sm_100a: a persistent,
+// warp-specialised kernel, one CTA per SM.
+//
+//   unit   one segment of one stripe (32 rows x seg_quads quads): what a decode
+//          warp takes at a time
+//   item   one stripe, or one of `parts` ranges of its segments: the units
+//          that share a decode table and are summed together
+//
+// Roles within a CTA (warps run on their own; nothing is synchronised CTA-wide
+// between the start and the end of a launch):
+//   * producer (1 warp): takes items (work queue, or every G-th one), publishes
+//     their records in a ring, and keeps a ring of stream slots filled with the
+//     units' blocks, in unit order, by 1-D bulk copies (cp.async.bulk, no
+//     multicast) that complete on the slot's mbarrier;
+//   * stager (1 warp): copies an item's symbol tables to shared memory, one item
+//     ahead of its decode;
+//   * table warps (4): expand them into one of two decode tables while the decode
+//     warps work from the other, and write an item's outputs once its units are
+//     decoded (with MMA consumers from tensor memory, one warp per lane quarter);
+//   * decode warps (W): each takes the CTA's next unit, waits for its slot and
+//     its item's table, decodes, and counts the unit as done.
+// One CTA-wide barrier per item, a table build and a cross-warp sum between the
+// items of the form this replaced left the SM idle for a third of a launch: the
+// seven matrices of a 7B layer took 139 us there with one vector and take 74 us,
+// with 16 vectors 136 and 109 us; 64 vectors of 11008x4096, 197 and 69 us.
+//
+// Decode table: entry (q, lane) = f | sym << 16 | r << 24 (frequency of the
+// symbol that owns quantile q, the symbol, r = q - cum), 4 bytes at byte
+// q*256 + lane*4 of a 64 KB region; the second table sits in the other half of
+// each 256-byte row.  One byte permute of the state forms a lookup address:
+// the quantile byte lands in bits 8..15, the lane's byte and the table's half
+// in bits 0..7.  A warp's lookup is one conflict-free wavefront.  (8-byte
+// entries save two permutes a step but take two wavefronts a lookup, and the
+// second table would not fit.)
+//
+// Decode step (per lane, per quad of 4 symbols):
+//   refill:   if (hi == 0) { hi = lo; lo = next word; load the word after it },
+//             predicated; the stream position moves one 128-byte word-row on and
+//             is clamped every 4 steps to the row after the block
+//   update:   r0 + f0 r1 = dp4a of e0 with (r1, 0, 0, 1), one byte permute of e1;
+//             f0 f1 by dp2a of the entries; (hi:lo) = hi*P + t0, one 32x32->64
+//             multiply-add
+//
+// What bounds it: issue and the ALU pipe.  A step takes 29 instructions (9 byte
+// permutes at half rate) and 5 shared-memory wavefronts; a loop of steps alone
+// runs at 9.2 SM cycles a step with 16 warps (a single warp's step takes 80), and
+// the kernel at 11 on a 7B layer (one vector).
+#include <algorithm>
+
+#include "mv_device.cuh"
+#include "q8w.cuh"
+#include "umma.cuh"
+
+namespace mv {
+
+constexpr int kRing = 8;       // items in flight (records, partial sums, counters)
+constexpr int kTableWarps = 4; // warps 0..3: one per TMEM lane quarter
+constexpr int kProducer = 4;   // the producer warp
+constexpr int kStager = 5;     // the warp that stages table data
+constexpr int kFirstDecode = 6;
+constexpr uint32_t kTdone = 1u << 16;  // arrivals of an item's `tdone`: its units, and the producer for the rest
+constexpr int kStages = 2;     // staging areas for table data
+constexpr uint32_t kLutBytes = 65536;
+constexpr uint32_t kStageOffs = 40;  // u32: 33 relative offsets, [37] where the first entry landed
+constexpr uint32_t kStagePad = 16;   // entries: copies start and end on 8-entry boundaries
+
+// One unit as the producer publishes it with its slot.
+struct alignas(16) UnitDesc {
+    int32_t item;  // running index of its item in this CTA, or -1: no more units
+    uint32_t unit;  // its running number
+    int32_t seg;
+    uint32_t rows;  // word-rows of its block (0: rejected, nothing to decode)
+};
+
+// MMA consumers: the warps that hold a part of an item's sums in their first and second accumulator.
+struct alignas(8) ItemState {
+    uint32_t acc[2];
+};
+
+// An item as the producer records it, with what the other warps need of its job (the job table is in global memory:
+// a read of it takes longer than an item's epilogue).
+struct alignas(16) ItemRec {
+    int32_t it, job, stripe, tab;  // it < 0: no more items; tab: decode table
+    int32_t gen;        // number of its table's build in this CTA
+    int32_t build;      // 1: the table is built for this item
+    int32_t area_item;  // the item whose build must be over before this one's data is staged (-1: none)
+    int32_t sb;         // first segment
+    uint32_t n;         // number of units
+    int32_t rows, cols, seg_quads, atomic, local;
+    float chain_scale;
+    const int8_t *x;
+    int32_t *y;
+    const float *scales;
+    float *ys;
+    int8_t *chain_out;  // a chain's int8 output, or nullptr
+};
+
+namespace {
+
+__device__ __forceinline__ const Q8Job &job_at(const Q8WLaunch &L, int j) { return L.jobs ? L.jobs[j] : L.job0; }
+
+// mbarriers, in the order they are laid out
+struct Bars {
+    uint32_t base;  // shared-memory address
+    int S, W;
+    static constexpr int kFixed = 4 * kRing + kStages;
+    __device__ __forceinline__ uint32_t at(int i) const { return base + 8u * (uint32_t)i; }
+    __device__ __forceinline__ uint32_t rfull(int k) const { return at(k); }              // item record written
+    __device__ __forceinline__ uint32_t tfull(int k) const { return at(kRing + k); }      // decode table ready
+    __device__ __forceinline__ uint32_t tdone(int k) const { return at(2 * kRing + k); }  // item decoded
+    __device__ __forceinline__ uint32_t idone(int k) const { return at(3 * kRing + k); }  // item's outputs written
+    __device__ __forceinline__ uint32_t staged(int g) const { return at(4 * kRing + g); } // table data in shared memory
+    __device__ __forceinline__ uint32_t sfull(int s) const { return at(kFixed + s); }
+    __device__ __forceinline__ uint32_t sempty(int s) const { return at(kFixed + S + s); }
+    __device__ __forceinline__ uint32_t mma(int w) const { return at(kFixed + 2 * S + w); }
+    __device__ __forceinline__ uint32_t dempty(int w, int b) const { return at(kFixed + 2 * S + W + 2 * w + b); }
+    static __host__ __device__ constexpr int count(int S, int W, bool mma) { return kFixed + 2 * S + (mma ? 3 * W : 0); }
+    // arrivals that complete barrier i's phase
+    __device__ __forceinline__ int arrivals(int i) const {
+        if (i >= 2 * kRing && i < 3 * kRing) return (int)kTdone;
+        if (i >= 4 * kRing && i < kFixed) return 33;  // the stager's lanes, and once for the offsets
+        return i >= kFixed + 2 * S + W ? kTableWarps : 1;  // dempty: every table warp has read the sums
+    }
+};
+
+// Bounded wait.  A wait that runs out raises MV_DEV_WAIT_TIMEOUT and the CTA's failure flag; every later wait of
+// the CTA then gives up within a few polls, and every role leaves its loop.
+__device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, uint32_t *status, uint32_t limit,
+                                       volatile uint32_t *failed) {
+    for (uint32_t it = 0; it < limit; it++) {
+        __nanosleep(40);  // a polling warp takes issue slots from the decoding ones
+        if (mbar_try_wait(bar, parity)) return true;
+        if (*failed) return false;
+    }
+    atomicOr(status, MV_DEV_WAIT_TIMEOUT);
+    *failed = 1u;
+    return false;
+}
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, const Q8WLaunch &L, volatile uint32_t *failed) {
+    if (mbar_try_wait(bar, parity)) return true;
+    return wait_slow(bar, parity, L.status, L.spin_limit, failed);
+}
+
+// One poll without suspension.
+__device__ __forceinline__ bool test_bar(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+__device__ __forceinline__ void arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void arrive_n(uint32_t bar, uint32_t n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
+__device__ __forceinline__ void arrive_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_in(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// Barrier of the four table warps; true if every one of them passes true.
+__device__ __forceinline__ bool table_vote(bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)ok)
+        : "memory");
+    return r != 0;
+}
+
+// CUDA-core consumers: whether the slots hold their segments' x (segments of up to kXQuads quads, not in a chain)
+constexpr int kXQuads = 64;
+__device__ __forceinline__ bool x_in_slot(const Q8WLaunch &L, int seg_quads) {
+    return L.x_off != 0 && seg_quads <= kXQuads;
+}
+
+// ---------------------------------------------------------------- work items
+
+__device__ __forceinline__ void item_segs(const mv_q8_view &m, int ngroups, int group, int &sb, int &se) {
+    const int spp = (m.nseg + ngroups - 1) / ngroups;
+    sb = group * spp;
+    se = min(m.nseg, sb + spp);
+}
+
+// Item number -> job, stripe and segment range.  Each CTA takes its items in increasing order, so the job search
+// runs forward from the previous item's job: one comparison in the common case, a binary search otherwise.
+__device__ __forceinline__ void locate(const Q8WLaunch &L, uint32_t it, int &job, int &stripe, int &sb, int &se) {
+    uint32_t rel = it;
+    int ng = L.job0.ngroups;
+    if (L.jobs) {
+        if (job + 1 < L.njobs && __ldg(&L.jobs[job + 1].item0) <= it) {
+            int lo = job + 1, hi = L.njobs - 1;
+            while (lo < hi) {  // last job with item0 <= it
+                const int mid = (lo + hi + 1) >> 1;
+                if (__ldg(&L.jobs[mid].item0) <= it) lo = mid;
+                else hi = mid - 1;
+            }
+            job = lo;
+        }
+        rel = it - __ldg(&L.jobs[job].item0);
+        ng = __ldg(&L.jobs[job].ngroups);
+    }
+    stripe = (int)(rel / (uint32_t)ng);
+    item_segs(job_at(L, job).m, ng, (int)(rel % (uint32_t)ng), sb, se);
+}
+
+// The chained pipeline's int8 output: the reference's fp32 requantisation (ans-warp-rows-kernel.cu:212-220).
+__device__ __forceinline__ int8_t chain_q(const ItemRec &I, int sum) {
+    return (int8_t)max(-128, min(127, __float2int_rn((float)sum * I.chain_scale)));
+}
+
+// One output: y (exact int32), its scaled form, and the chain's int8.
+__device__ __forceinline__ void emit(const ItemRec &I, int v, int row, int sum) {
+    const size_t i = (size_t)v * I.rows + row;
+    if (I.atomic) {
+        atomicAdd(I.y + i, sum);
+        return;
+    }
+    I.y[i] = sum;
+    if (I.ys) I.ys[i] = (float)sum * __ldg(I.scales + row);
+    if (I.chain_out) I.chain_out[i] = chain_q(I, sum);
+}
+
+// ------------------------------------------------------------------- producer
+
+// Table data of item r into staging area r.gen % kStages: offsets relative to the first entry by plain loads, the
+// entries by 16-byte asynchronous copies (zero-filled past the readable end), both counted on the area's barrier.
+__device__ __forceinline__ void stage_table(const Q8WLaunch &L, const ItemRec &r, unsigned char *sm, const Bars &B, int lane) {
+    const mv_q8_view &m = job_at(L, r.job).m;
+    const int area = r.gen % kStages;
+    uint32_t *so = reinterpret_cast<uint32_t *>(sm + L.lay.stage_o) + area * kStageOffs;
+    const uint32_t r0 = m.local ? (uint32_t)r.stripe * 32u : 0u;
+    const uint32_t nt = m.local ? 32u : 1u;
+    const uint32_t o = (uint32_t)lane <= nt ? __ldg(m.tbl_off + r0 + lane) : 0u;
+    const uint32_t te = __ldg(m.tbl_off + r0 + nt);
+    const uint32_t tb = __shfl_sync(0xffffffffu, o, 0);
+    const bool ok = te >= tb && te <= m.tbl_len && te - tb <= (uint32_t)L.tbl_stage;
+    if ((uint32_t)lane <= nt) so[lane] = (ok && o >= tb && o <= te) ? o - tb : 0u;
+    if (lane == 0) {
+        if (nt == 32u) so[32] = ok ? te - tb : 0u;
+        so[37] = tb & 7u;
+        if (!ok) atomicOr(L.status, MV_DEV_BAD_TABLE);
+    }
+    if (ok) {
+        const uint32_t a = tb & ~7u, n = te - a;
+        unsigned char *se = sm + L.lay.stage_e + (uint32_t)area * ((uint32_t)L.tbl_stage + kStagePad) * 2u;
+        if (((uintptr_t)m.tbl & 15) == 0) {
+            const uint32_t dst = smem_u32(se);
+            for (uint32_t c = lane; 8 * c < n; c += 32) {
+                const uint32_t avail = min(8u, m.tbl_len - (a + 8 * c));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16u * c), "l"(m.tbl + a + 8 * c),
+                             "r"(2u * avail)
+                             : "memory");
+            }
+        } else {
+            uint16_t *d = reinterpret_cast<uint16_t *>(se);
+            for (uint32_t e = lane; e < n; e += 32) d[e] = __ldg(m.tbl + a + e);
+        }
+    }
+    cp_async_mbar_arrive_noinc(B.staged(area));
+    __syncwarp();
+    if (lane == 0) arrive(B.staged(area));
+}
+
+// The stager warp: the table data of every item that needs a build, as soon as its record is written.
+__device__ __forceinline__ void stage_tables(const Q8WLaunch &L, unsigned char *sm, const Bars &B, volatile uint32_t *failed) {
+    const int lane = threadIdx.x & 31;
+    const ItemRec *ring = reinterpret_cast<const ItemRec *>(sm + L.lay.ring);
+    for (int k = 0;; k++) {
+        if (!__all_sync(0xffffffffu, wait_bar(B.rfull(k % kRing), (uint32_t)(k / kRing) & 1u, L, failed))) break;
+        const ItemRec &r = ring[k % kRing];
+        if (r.it < 0) break;
+        if (!r.build) continue;
+        if (r.area_item >= 0 && r.area_item > k - kRing) {  // (earlier items are done)
+            const bool built = wait_bar(B.tfull(r.area_item % kRing), (uint32_t)(r.area_item / kRing) & 1u, L, failed);
+            if (!__all_sync(0xffffffffu, built)) break;
+        }
+        stage_table(L, r, sm, B, lane);
+    }
+    cp_async_wait_all();
+}
+
+__device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, const Bars &B, volatile uint32_t *failed) {
+    const int lane = threadIdx.x & 31;
+    ItemRec *ring = reinterpret_cast<ItemRec *>(sm + L.lay.ring);
+    UnitDesc *desc = reinterpret_cast<UnitDesc *>(sm + L.lay.desc);
+    const uint32_t slots = smem_u32(sm) + L.lay.slots;
+    const uint32_t S = (uint32_t)L.S, W = (uint32_t)L.W;
+    uint32_t u = 0;              // units published
+    uint32_t next = blockIdx.x;  // the CTA's latest item number; its first one is static
+    uint32_t grabbed = 0;        // lane 0: the queue's answer for the item after it
+    int job = 0, tjob = -1, tstripe = -1, gen = -1;
+    int fb1 = -1, fb2 = -1;  // first items of the two latest table builds (fb1 the latest)
+    bool ok = true;
+
+    // Writes item k's record (its number is in `next`) and takes the number after it, so that the queue's latency
+    // passes while units go out.
+    auto record = [&](int k) {
+        if (k >= kRing && ok) ok = wait_bar(B.idone(k % kRing), (uint32_t)(k / kRing - 1) & 1u, L, failed);
+        ItemRec r{};
+        const bool end = next >= L.nitems;
+        r.it = end ? -1 : (int32_t)next;
+        r.n = W;  // one end mark per decode warp
+        r.area_item = -1;
+        if (!end) {
+            int se = 0;
+            locate(L, next, job, r.stripe, r.sb, se);
+            if (L.queue && lane == 0) grabbed = atomicAdd(L.queue, 1u);
+            r.job = job;
+            r.n = (uint32_t)max(0, se - r.sb);
+            const Q8Job &J = job_at(L, job);
+            r.rows = J.m.rows;
+            r.cols = J.m.cols;
+            r.seg_quads = J.m.seg_quads;
+            r.local = J.m.local;
+            r.atomic = J.atomic;
+            r.x = J.x;
+            r.y = J.y;
+            r.scales = J.scales;
+            r.ys = J.ys;
+            if (L.chain_scales) {
+                r.chain_scale = __ldg(L.chain_scales + job);
+                r.chain_out = job + 1 < L.njobs ? const_cast<int8_t *>(L.jobs[job + 1].x) : L.chain_out8;
+            }
+            r.build = job != tjob || (r.local && r.stripe != tstripe);
+            if (r.build) {
+                // two tables and two staging areas: build g overwrites those of build g - 2
+                gen++;
+                r.area_item = gen >= 2 ? fb2 : -1;
+                fb2 = fb1;
+                fb1 = k;
+                tjob = job;
+                tstripe = r.stripe;
+            }
+            r.gen = gen;
+            r.tab = gen & 1;
+        }
+        if (ok && lane == 0) {
+            ring[k % kRing] = r;
+            if (!end) arrive_n(B.tdone(k % kRing), kTdone - r.n);  // the units' arrivals are left
+            arrive(B.rfull(k % kRing));
+        }
+        __syncwarp();
+        return r;
+    };
+    ItemRec r = record(0);
+    for (int k = 0; ok; k++) {
+        const bool end = r.it < 0;
+        const mv_q8_view &m = job_at(L, r.job).m;
+        // The next item's record goes ahead of this item's last units, so that its table is built while this item
+        // decodes.
+        ItemRec rn{};
+        bool ahead = end;
+        auto look_ahead = [&]() {
+            next = L.queue ? __shfl_sync(0xffffffffu, grabbed, 0) + gridDim.x : next + gridDim.x;
+            // the counter is reset by whoever makes the launch's last grab
+            if (L.queue && lane == 0 && next == L.nitems + gridDim.x - 1) atomicExch(L.queue, 0u);
+            rn = record(k + 1);
+            ahead = true;
+        };
+        for (uint32_t base = 0; base < r.n && ok; base += 32) {
+            const uint32_t i = base + (uint32_t)lane;
+            uint32_t o0 = 0, rows = 0;
+            if (!end && i < r.n) {
+                const int b = r.stripe * m.nseg + r.sb + (int)i;
+                o0 = __ldg(m.blk_off + b);
+                const uint32_t o1 = __ldg(m.blk_off + b + 1);
+                rows = o1 - o0;
+                if (o1 < o0 || o1 > m.blocks_rows || rows < 2 || (rows + 1) * 128u > L.block_bytes) {
+                    atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
+                    rows = 0;
+                }
+            }
+            const uint32_t cnt = min(32u, r.n - base);
+            const uint32_t ui = u + (uint32_t)lane, slot = ui % S, turn = ui / S;
+            // the slots become free in unit order: publish the leading run of free ones, then wait for the next
+            for (uint32_t pos = 0, it = 0; pos < cnt;) {
+                const bool mine = (uint32_t)lane >= pos && (uint32_t)lane < cnt;
+                const bool free_ = mine && (turn == 0 || test_bar(B.sempty((int)slot), (turn - 1) & 1u));
+                const uint32_t ball = __ballot_sync(0xffffffffu, free_) >> pos;
+                const uint32_t run = ~ball ? (uint32_t)__ffs((int)~ball) - 1u : 32u;
+                if (run) {
+                    if (mine && (uint32_t)lane < pos + run) {
+                        UnitDesc d;
+                        d.item = end ? -1 : k;
+                        d.unit = ui;
+                        d.seg = r.sb + (int)i;
+                        d.rows = rows;
+                        desc[slot] = d;
+                        const uint32_t dst = slots + slot * L.slot_bytes, bar = B.sfull((int)slot);
+                        // the block, and behind it (CUDA-core consumers) the segment's x of every vector
+                        const int q = (r.sb + (int)i) * m.seg_quads;
+                        const uint32_t xb =
+                            x_in_slot(L, m.seg_quads) && rows ? 4u * (uint32_t)max(0, min(m.seg_quads, (m.cols >> 2) - q)) : 0u;
+                        arrive_tx(bar, rows * 128u + xb * (uint32_t)L.batch);
+                        if (rows && !L.drop_copy) {
+                            bulk_in(dst, m.blocks + (size_t)o0 * 32, rows * 128u, bar);
+                            const int8_t *x = r.x + 4 * (size_t)q;
+                            if (xb)
+                                for (int v = 0; v < L.batch; v++)
+                                    bulk_in(dst + L.x_off + 4u * (uint32_t)(v * m.seg_quads), x + (size_t)v * m.cols, xb, bar);
+                        }
+                    }
+                    __syncwarp();
+                    pos += run;
+                    it = 0;
+                    continue;
+                }
+                if (!ahead) {
+                    look_ahead();
+                    if (!ok) break;
+                    continue;
+                }
+                const uint32_t us = u + pos;
+                if (mbar_try_wait(B.sempty((int)(us % S)), (us / S - 1) & 1u)) continue;
+                __nanosleep(40);
+                if (++it >= L.spin_limit || *failed) {
+                    if (it >= L.spin_limit && lane == 0) atomicOr(L.status, MV_DEV_WAIT_TIMEOUT);
+                    *failed = 1u;
+                    ok = false;
+                    break;
+                }
+            }
+            u += cnt;
+        }
+        if (end) break;
+        if (ok && !ahead) look_ahead();
+        r = rn;
+    }
+    if (!ok) {
+        // a failed launch still leaves the queue at zero: take (and drop) items until one grab fails
+        if (L.queue && lane == 0 && next < L.nitems) {
+            next = grabbed + gridDim.x;
+            for (;;) {
+                if (next == L.nitems + gridDim.x - 1) atomicExch(L.queue, 0u);
+                if (next >= L.nitems) break;
+                next = atomicAdd(L.queue, 1u) + gridDim.x;
+            }
+        }
+        // no copy may be left writing the shared memory of a CTA that has exited: wait (bounded) for each slot's
+        // latest one
+        const uint32_t live = min(u, S);
+        for (uint32_t i = lane; i < live; i += 32) {
+            const uint32_t ui = u - 1 - i;
+            for (uint32_t it = 0; it < L.spin_limit; it++)
+                if (mbar_try_wait(B.sfull((int)(ui % S)), (ui / S) & 1u)) break;
+        }
+        __syncwarp();
+    }
+}
+
+// --------------------------------------------------------------- table warps
+
+__device__ __forceinline__ uint32_t table_entry(uint32_t ent) {  // r = 0; ent: symbol | f << 8
+    return (ent >> 8) | (ent & 0xFFu) << 16;
+}
+
+// Decode table from the staged data: warp s fills quantiles [64 s, 64 s + 64), lane l its row's column, with no
+// divergence: the column is cleared, each symbol's entry (r = 0) goes to its first quantile, and one pass then
+// carries the entries forward, r growing by one per quantile.  (A walk that stores quantile by quantile and moves
+// to the next symbol by a branch took 3.2 us a table with the decode warps at work.)
+__device__ __forceinline__ void build_table(const Q8WLaunch &L, int local, unsigned char *lut,
+                                            const uint32_t *so, const uint16_t *tsm) {
+    const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = local ? lane : 0;
+    const uint32_t o1 = max(so[t + 1], so[t]);
+    const uint32_t qlo = 64u * (uint32_t)s, qhi = qlo + 64u;
+    uint32_t k = so[t], cum = 0;
+    unsigned char *rows = lut + 256u * qlo;
+    {  // clear: lane l the 16 bytes 16 (l % 8) of rows l / 8, l / 8 + 4, ...
+        unsigned char *z = rows + 256u * (uint32_t)(lane >> 3) + 16u * (uint32_t)(lane & 7);
+#pragma unroll
+        for (int i = 0; i < 16; i++) *reinterpret_cast<uint4 *>(z + 1024 * i) = make_uint4(0, 0, 0, 0);
+    }
+    // symbols that end at or before qlo, four at a time (independent loads)
+    while (k + 4 <= o1) {
+        const uint32_t c4 = cum + ((uint32_t)tsm[k] >> 8) + ((uint32_t)tsm[k + 1] >> 8) +
+                            ((uint32_t)tsm[k + 2] >> 8) + ((uint32_t)tsm[k + 3] >> 8);
+        if (c4 > qlo) break;
+        cum = c4;
+        k += 4;
+    }
+    uint32_t ent = k < o1 ? (uint32_t)tsm[k] : 0u;
+    while (k < o1 && cum + (ent >> 8) <= qlo) {
+        cum += ent >> 8;
+        k++;
+        ent = k < o1 ? (uint32_t)tsm[k] : 0u;
+    }
+    // the symbol that holds qlo starts the pass; e is one step (r) behind
+    bool bad = k >= o1;
+    constexpr uint32_t kR = 1u << 24;  // one step of r
+    uint32_t e = table_entry(ent) + (qlo - cum - 1u) * kR;
+    cum += ent >> 8;
+    __syncwarp();
+    unsigned char *col = rows + 4u * (uint32_t)lane;
+    while (cum < qhi) {
+        k++;
+        if (k >= o1) {  // the table ends early
+            bad = true;
+            break;
+        }
+        ent = tsm[k];
+        if ((ent >> 8) == 0) bad = true;
+        *reinterpret_cast<uint32_t *>(col + 256u * (cum - qlo)) = table_entry(ent);
+        cum += ent >> 8;
+    }
+    __syncwarp();
+    if (__any_sync(0xffffffffu, bad)) {
+        // not a valid table: entries of one quantile each keep the decode in bounds
+        atomicOr(L.status, MV_DEV_BAD_TABLE);
+        for (int q = 0; q < 64; q++) *reinterpret_cast<uint32_t *>(col + 256 * q) = 1u;
+        return;
+    }
+#pragma unroll 16
+    for (int q = 0; q < 64; q++) {
+        const uint32_t v = *reinterpret_cast<const uint32_t *>(col + 256 * q);
+        e = v ? v : e + kR;
+        *reinterpret_cast<uint32_t *>(col + 256 * q) = e;
+    }
+}
+
+// Chained pipeline: wait (thread 0, bounded) until every work item of job j is counted.  Items are numbered in job
+// order, each CTA takes its items in increasing order and the launch is cooperative, so the items waited for are
+// always making progress.
+__device__ __forceinline__ void chain_wait(const Q8WLaunch &L, int j, volatile uint32_t *failed) {
+    const uint32_t need = (j + 1 < L.njobs ? L.jobs[j + 1].item0 : L.nitems) - L.jobs[j].item0;
+    const uint32_t *cnt = &L.jobs[j].pad;
+    for (uint32_t it = 0;; it++) {
+        uint32_t done;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(done) : "l"(cnt) : "memory");
+        if (done >= need) break;
+        if (it >= L.spin_limit) {
+            atomicOr(L.status, MV_DEV_WAIT_TIMEOUT);
+            *failed = 1u;
+            break;
+        }
+        __nanosleep(32);
+    }
+}
+
+// --------------------------------------------------------------------- decode
+
+// One stream: the lane's 64-bit state, its next refill word (already loaded), the offset of the one after that and
+// the bound on that offset (the row after the block).
+struct Stream {
+    uint32_t lo, hi, nw, koff, kend, P;
+    __device__ __forceinline__ Stream(const unsigned char *sm, uint32_t soff, uint32_t rows, int lane) {
+        const uint32_t a = smem_u32(sm) + soff + (uint32_t)lane * 4u;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(lo) : "r"(a) : "memory");
+        asm volatile("ld.shared.u32 %0, [%1+128];" : "=r"(hi) : "r"(a) : "memory");
+        asm volatile("ld.shared.u32 %0, [%1+256];" : "=r"(nw) : "r"(a) : "memory");
+        koff = a + 384u;
+        kend = a + rows * 128u;
+        P = 0;
+    }
+    // the encoder starts every segment from the last quad's frequency product, so the decoder ends there
+    __device__ __forceinline__ bool ok() const { return hi == 0 && lo == P; }
+    // A corrupt stream stays within 4 word-rows of its block: called every 4 steps.
+    __device__ __forceinline__ void clamp() { koff = min(koff, kend); }
+    // Refill (predicated: a branch-free `select` form of it takes 4 instructions more) and the four table entries.
+    __device__ __forceinline__ void step(const unsigned char *sm, uint32_t lw, uint32_t (&e)[4]) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.eq.u32 p, %1, 0;\n\t"
+            "@p mov.u32 %1, %0;\n\t"
+            "@p mov.u32 %0, %2;\n\t"
+            "@p ld.shared.u32 %2, [%3];\n\t"
+            "@p add.u32 %3, %3, 128;\n\t}"
+            : "+r"(lo), "+r"(hi), "+r"(nw), "+r"(koff)::"memory");
+        e[0] = *reinterpret_cast<const uint32_t *>(sm + __byte_perm(lo, lw, 0x7604));
+        e[1] = *reinterpret_cast<const uint32_t *>(sm + __byte_perm(lo, lw, 0x7614));
+        e[2] = *reinterpret_cast<const uint32_t *>(sm + __byte_perm(lo, lw, 0x7624));
+        e[3] = *reinterpret_cast<const uint32_t *>(sm + __byte_perm(lo, lw, 0x7634));
+    }
+    // (hi:lo) = hi * p01 p23 + u01 + p01 u23 (written as the two halves of one wide multiply-add: the 64-bit C form
+    // costs register moves)
+    __device__ __forceinline__ void update(uint32_t u01, uint32_t p01, uint32_t u23, uint32_t p23) {
+        P = p01 * p23;
+        const uint32_t t = u01 + p01 * u23;
+        uint32_t h;
+        asm("{\n\tmad.lo.cc.u32 %0, %2, %3, %4;\n\tmadc.hi.u32 %1, %2, %3, 0;\n\t}"
+            : "=&r"(lo), "=r"(h)
+            : "r"(hi), "r"(P), "r"(t));
+        hi = h;
+    }
+    // one step; returns the four packed int8 symbols
+    __device__ __forceinline__ uint32_t step_i8(const unsigned char *sm, uint32_t lw) {
+        uint32_t e[4];
+        step(sm, lw, e);
+        // entry bytes (f, 0, sym, r): r0 + f0 r1 = e0 . (r1, 0, 0, 1); f0 f1 = dp2a of e1's low half with e0's f
+        const uint32_t u01 = __dp4a(e[0], __byte_perm(e[1], 1u, 0x4553), 0u);
+        const uint32_t u23 = __dp4a(e[2], __byte_perm(e[3], 1u, 0x4553), 0u);
+        const uint32_t p01 = __dp2a_lo(e[1], e[0], 0u), p23 = __dp2a_lo(e[3], e[2], 0u);
+        update(u01, p01, u23, p23);
+        return __byte_perm(__byte_perm(e[0], e[1], 0x0062), __byte_perm(e[2], e[3], 0x0062), 0x5410);
+    }
+};
+
+// x is read with plain (coherent) loads: in a chain it was written earlier in the same launch.
+__device__ __forceinline__ uint4 ldx_u4(const void *p) { return *reinterpret_cast<const uint4 *>(p); }
+
+// CUDA-core consumer: NV int8 vectors, dp4a.  The lane's partial sums go to the item's area in shared memory
+// (exact integer atomics); the warp that counts the item's last part writes the outputs.
+template <int NV>
+struct DotCons {
+    static constexpr bool kMma = false;
+    static constexpr int kRed = NV * 32;  // ints of an item's partial sums
+    static constexpr int kMaxDecode = NV <= 2 ? 16 : NV <= 4 ? 14 : NV <= 8 ? 10 : 6;
+    const int8_t *x;
+    int cols, seg_quads, qtot;
+    bool in_slot;
+    static constexpr int kUnroll = NV <= 2 ? 4 : 1;
+    int acc[NV];
+    __device__ __forceinline__ void init(const Q8WLaunch &, unsigned char *, const Bars &, uint32_t, int) {
+#pragma unroll
+        for (int v = 0; v < NV; v++) acc[v] = 0;
+    }
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I) {
+        in_slot = x_in_slot(L, I.seg_quads);
+        x = I.x;
+        cols = I.cols;
+        seg_quads = I.seg_quads;
+        qtot = cols >> 2;
+    }
+    __device__ __forceinline__ void group(Stream &s, const unsigned char *sm, uint32_t lw, const uint4 (&xv)[NV]) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t w = s.step_i8(sm, lw);
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                const uint32_t xw = j == 0 ? xv[v].x : j == 1 ? xv[v].y : j == 2 ? xv[v].z : xv[v].w;
+                acc[v] = __dp4a((int)w, (int)xw, acc[v]);
+            }
+        }
+        s.clamp();
+    }
+    __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
+                                         uint32_t lw, int lane, volatile uint32_t *) {
+        const int q0 = d.seg * seg_quads;
+        const int nq = min(seg_quads, qtot - q0);
+        Stream s(sm, soff, d.rows, lane);
+        if (in_slot) {  // x came with the block and lies behind it
+            const unsigned char *xs = sm + soff + L.x_off;
+            // unrolled: the loop's back edge costs register moves (4 instructions a step without)
+#pragma unroll kUnroll
+            for (int i = 0; i < nq; i += 4, xs += 16) {  // segments are whole groups of 4 quads (cols % 16 == 0)
+                uint4 xv[NV];
+#pragma unroll
+                for (int v = 0; v < NV; v++) xv[v] = *reinterpret_cast<const uint4 *>(xs + 4 * v * seg_quads);
+                group(s, sm, lw, xv);
+            }
+        } else {  // x from global memory, one group ahead: long segments, and chains, whose x is not there any earlier
+            const int8_t *xp = x + 4 * q0;
+            uint4 xn[NV];
+#pragma unroll
+            for (int v = 0; v < NV; v++) xn[v] = ldx_u4(xp + (size_t)v * cols);
+            for (int i = 0; i < nq; i += 4) {
+                uint4 xv[NV];
+                xp += i + 4 < nq ? 16 : 0;
+#pragma unroll
+                for (int v = 0; v < NV; v++) {
+                    xv[v] = xn[v];
+                    xn[v] = ldx_u4(xp + (size_t)v * cols);
+                }
+                group(s, sm, lw, xv);
+            }
+        }
+        if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
+    }
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, unsigned char *sm, const Bars &B, int lane,
+                                             volatile uint32_t *) {
+        int *red = reinterpret_cast<int *>(sm + L.lay.red) + (size_t)(k % kRing) * NV * 32 + lane;
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            atomicAdd(red + v * 32, acc[v]);
+            acc[v] = 0;
+        }
+        __syncwarp();
+        if (lane == 0) arrive(B.tdone(k % kRing));
+    }
+    // Table warps: the item's sums, one vector per warp at a time, lane = stripe row.
+    static __device__ __forceinline__ void epilogue(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm,
+                                                    const Bars &, uint32_t) {
+        const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        volatile int *red = reinterpret_cast<volatile int *>(sm + L.lay.red) + (size_t)(k % kRing) * NV * 32 + lane;
+        const int row = I.stripe * 32 + lane;
+        for (int v = q; v < NV; v += kTableWarps) {
+            const int sum = red[v * 32];
+            red[v * 32] = 0;
+            if (row < I.rows && v < L.batch) emit(I, v, row, sum);
+        }
+    }
+    __device__ __forceinline__ void drain(const Q8WLaunch &) {}
+};
+
+// Tensor-core consumer, up to 64 int8 vectors: D[vector][row] += x tile . W tile^T, kind::i8, exact int32.
+//   A = x: M = 64 vectors (rows past xrows read whatever follows and only reach lanes that are never read), K-major
+//       core matrices (8 vectors x 16 bytes), 64 columns at a time, brought in by the warp's own cp.async;
+//   B = W: the 32 rows of the stripe, each lane storing its row's 16-byte pieces (K-major, conflict-free);
+//   D: 32 TMEM columns per decode warp, vector v in lane 32 (v / 16) + v % 16.
+// Per 16 quads: two MMAs (K = 32) and one commit.  The previous pair's MMAs are waited for after the first 4 quads
+// of the next one are decoded, when W tile and x tile are rewritten; the x copies land during the other 12.
+//
+// kOwn (up to 16 vectors): the A operand starts 16 rows per lane quarter early, so that the vectors land in the warp's
+// own quarter; the warp reads its sums itself after each unit and adds them to the item's in shared memory.  With more
+// vectors the sums stay in TMEM for the item, the table warps read every warp's (one lane quarter each), and items
+// alternate between two accumulators, the second in the 16 lanes of each quarter that M = 64 leaves free.
+template <bool kOwn>
+struct MmaCons {
+    static constexpr bool kMma = true;
+    static constexpr int kPitch = 33;  // words per vector of the item's sums: lanes (vectors) hit distinct banks
+    static constexpr int kRed = kOwn ? 16 * kPitch : 0;
+    static constexpr int kMaxDecode = 16;
+    static constexpr uint32_t kWTile = 2048;  // 32 rows x 64 columns
+    static __host__ __device__ constexpr uint32_t x_tile(int xrows) { return 64u * (uint32_t)xrows; }
+    static __host__ __device__ constexpr uint32_t tile_bytes(int xrows) { return kWTile + x_tile(xrows); }
+    const int8_t *x;
+    int cols, seg_quads, qtot;
+    uint32_t wt, xt, d_tmem, lbo, nmma, ndp;  // nmma: commits so far, ndp: earlier items this warp has had a part in
+    uint32_t mbar, dempty;                    // dempty: of the first accumulator; the second's follows
+    uint64_t a_desc, b_desc;
+    int warp;
+    bool any;
+    __device__ __forceinline__ void init(const Q8WLaunch &L, unsigned char *sm, const Bars &B, uint32_t tmem, int w) {
+        warp = w;
+        wt = smem_u32(sm) + L.lay.tiles + (uint32_t)w * tile_bytes(L.xrows);
+        xt = wt + kWTile;
+        lbo = 16u * (uint32_t)L.xrows;
+        const uint32_t quarter = (uint32_t)(w + kFirstDecode) & 3u;  // of TMEM lanes, by the warp's number in the CTA
+        d_tmem = tmem + 32u * (uint32_t)w;
+        a_desc = umma_smem_desc(kOwn ? xt - 256u * quarter : xt, lbo, 128u);
+        b_desc = umma_smem_desc(wt, 512u, 128u);
+        mbar = B.mma(w);
+        dempty = B.dempty(w, 0);
+        nmma = ndp = 0;
+        any = false;
+    }
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I) {
+        if (!kOwn) {
+            if (any) ndp++;  // the sums of the item before stay where they are until a table warp has read them
+            any = false;
+        }
+        x = I.x;
+        cols = I.cols;
+        seg_quads = I.seg_quads;
+        qtot = cols >> 2;
+    }
+    // the accumulator of the current item (they alternate) is free: its sums of two items ago are read
+    __device__ __forceinline__ void wait_acc(const Q8WLaunch &L, volatile uint32_t *failed) const {
+        if (!kOwn && ndp >= 2) wait_bar(dempty + 8u * (ndp & 1u), (ndp / 2u - 1u) & 1u, L, failed);
+    }
+    // 64 columns from col on of every vector: lane (r, c) copies chunk c (16 bytes) of vectors r, r + 8, ....  What
+    // is not there (vectors past the batch, columns past the row) is left as it is: it meets zero weights, or ends
+    // up in accumulator lanes that are never read.
+    __device__ __forceinline__ void copy_x(const Q8WLaunch &L, int col, int lane) const {
+        const int r = lane & 7, c = col + 16 * (lane >> 3);
+        const int8_t *src = x + (size_t)r * cols + c;
+        uint32_t dst = xt + (uint32_t)(lane >> 3) * lbo + (uint32_t)r * 16u;
+        const int n = c < cols ? L.batch - r : 0;
+        if constexpr (kOwn) {
+            if (n > 0) cp_async_16(dst, src);
+            if (n > 8) cp_async_16(dst + 128u, src + 8 * (size_t)cols);
+        } else {
+#pragma unroll 2
+            for (int v = 0; v < n; v += 8) {
+                cp_async_16(dst, src);
+                src += 8 * (size_t)cols;
+                dst += 128u;
+            }
+        }
+    }
+    // four quads (16 columns) of the lane's row: piece c of the 64-column tile
+    __device__ __forceinline__ void store_w(uint32_t c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int lane) const {
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(wt + c * 512u + (uint32_t)lane * 16u), "r"(w0), "r"(w1),
+                     "r"(w2), "r"(w3)
+                     : "memory");
+    }
+    // the previous MMAs are done with both tiles; the x copies have the rest of the decode to land in
+    __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, int lane, volatile uint32_t *failed) const {
+        if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
+        copy_x(L, col, lane);
+    }
+    // the MMAs of a tile: two K steps of 32 columns, or one
+    __device__ __forceinline__ void issue(const Q8WLaunch &L, bool two, int lane, volatile uint32_t *failed) {
+        if (!any) wait_acc(L, failed);
+        cp_async_wait_all();
+        fence_proxy_async_smem();  // both tiles are read by the tensor core (async proxy)
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            tcgen05_fence_after();
+            const uint32_t idesc = umma_idesc_i8(64, 32);
+            const uint32_t d = kOwn ? d_tmem : d_tmem + ((ndp & 1u) << 20);  // the second accumulator: 16 lanes further
+            umma_i8(d, a_desc, b_desc, idesc, any ? 1u : 0u);
+            if (two) umma_i8(d, a_desc + (lbo >> 3), b_desc + 64u, idesc, 1u);
+            umma_commit(mbar);
+        }
+        __syncwarp();
+        any = true;
+        nmma++;
+    }
+    __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
+                                         uint32_t lw, int lane, volatile uint32_t *failed) {
+        const int q0 = d.seg * seg_quads;
+        const int nq = min(seg_quads, qtot - q0);
+        Stream s(sm, soff, d.rows, lane);
+        int q = 0;
+        for (; q + 16 <= nq; q += 16) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const uint32_t w0 = s.step_i8(sm, lw), w1 = s.step_i8(sm, lw), w2 = s.step_i8(sm, lw), w3 = s.step_i8(sm, lw);
+                s.clamp();
+                if (c == 0) refill_tiles(L, 4 * (q0 + q), lane, failed);
+                store_w((uint32_t)c, w0, w1, w2, w3, lane);
+            }
+            issue(L, true, lane, failed);
+        }
+        if (q < nq) {  // the segment's last 4, 8 or 12 quads (segments are whole groups of 4: cols % 16 == 0)
+            const int n = (nq - q) >> 2;
+#pragma unroll 1
+            for (int c = 0; c < n; c++) {
+                const uint32_t w0 = s.step_i8(sm, lw), w1 = s.step_i8(sm, lw), w2 = s.step_i8(sm, lw), w3 = s.step_i8(sm, lw);
+                s.clamp();
+                if (c == 0) refill_tiles(L, 4 * (q0 + q), lane, failed);
+                store_w((uint32_t)c, w0, w1, w2, w3, lane);
+            }
+            if (n & 1) store_w((uint32_t)n, 0u, 0u, 0u, 0u, lane);  // a K step is two pieces
+            issue(L, n > 2, lane, failed);
+        }
+        if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
+    }
+    // Counts the unit once its MMAs are complete, so that whoever sees the item's last unit counted may read the sums.
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, unsigned char *sm, const Bars &B, int lane,
+                                             volatile uint32_t *failed) {
+        if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
+        if (kOwn && any) {
+            tcgen05_fence_after();
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(d_tmem + (((uint32_t)(warp + kFirstDecode) & 3u) << 21), r);  // lane = vector, r[j] = row j
+            if (lane < L.batch) {
+                int *red = reinterpret_cast<int *>(sm + L.lay.red) + (size_t)(k % kRing) * kRed + lane * kPitch;
+#pragma unroll
+                for (int j = 0; j < 32; j++) atomicAdd(red + j, (int)r[j]);
+            }
+            any = false;
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            if (!kOwn && any) {
+                ItemState *st = reinterpret_cast<ItemState *>(sm + L.lay.cnt) + k % kRing;
+                atomicOr(&st->acc[ndp & 1u], 1u << warp);
+            }
+            arrive(B.tdone(k % kRing));
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ void drain(const Q8WLaunch &L) {
+        cp_async_wait_all();
+        if (nmma)
+            for (uint32_t it = 0; it < L.spin_limit; it++)
+                if (mbar_try_wait(mbar, (nmma - 1) & 1u)) break;
+    }
+    // Table warps: the sums of item I.  kOwn: from shared memory, one vector per warp at a time, lane = stripe row.
+    // Otherwise from the accumulators of the warps that took its units: warp q reads lane quarter q (vectors 16 q ..
+    // 16 q + 15, in the lower or upper 16 lanes by accumulator), 32 stripe rows per lane.
+    static __device__ __forceinline__ void epilogue(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm,
+                                                    const Bars &B, uint32_t tmem) {
+        const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if constexpr (kOwn) {
+            volatile int *red = reinterpret_cast<volatile int *>(sm + L.lay.red) + (size_t)(k % kRing) * kRed + lane;
+            const int row = I.stripe * 32 + lane;
+            for (int v = q; v < L.batch; v += kTableWarps) {
+                const int sum = red[v * kPitch];
+                red[v * kPitch] = 0;
+                if (row < I.rows) emit(I, v, row, sum);
+            }
+        } else {
+            tcgen05_fence_after();
+            ItemState *st = reinterpret_cast<ItemState *>(sm + L.lay.cnt) + k % kRing;
+            const uint32_t m0 = *reinterpret_cast<volatile uint32_t *>(&st->acc[0]);
+            const uint32_t m1 = *reinterpret_cast<volatile uint32_t *>(&st->acc[1]);
+            int sum[32];
+#pragma unroll
+            for (int r = 0; r < 32; r++) sum[r] = 0;
+            const bool active = 16 * q < L.batch;
+            for (uint32_t left = m0 | m1; left; left &= left - 1u) {
+                const int w = __ffs((int)left) - 1;
+                if (active) {
+                    uint32_t r[32];
+                    tmem_ld_32x32b_x32(tmem + 32u * (uint32_t)w + (((uint32_t)q * 32u) << 16), r);
+                    const bool mine = (lane < 16 ? m0 : m1) >> w & 1u;  // the accumulator's half of the quarter's lanes
+#pragma unroll
+                    for (int j = 0; j < 32; j++) sum[j] += mine ? (int)r[j] : 0;
+                    tcgen05_fence_before();
+                }
+                __syncwarp();
+                if (lane == 0) arrive(B.dempty(w, (int)(m1 >> w & 1u)));
+            }
+            uint32_t base = 0;
+            if (!m0) base = 16;  // every warp was at its second accumulator
+            else if (m1)         // some at the first, some at the second: lane l + 16 to lane l
+#pragma unroll
+                for (int j = 0; j < 32; j++) sum[j] += __shfl_down_sync(0xffffffffu, sum[j], 16);
+            const int v = 16 * q + lane - (int)base, row0 = I.stripe * 32;
+            if (active && (uint32_t)lane >= base && (uint32_t)lane < base + 16u && v < L.batch) {
+                if (!I.atomic && row0 + 32 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.y & 15) == 0) {
+                    int4 *dst = reinterpret_cast<int4 *>(I.y + (size_t)v * I.rows + row0);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) dst[j] = make_int4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+                    if (I.ys)
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            I.ys[(size_t)v * I.rows + row0 + j] = (float)sum[j] * __ldg(I.scales + row0 + j);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (row0 + j < I.rows) emit(I, v, row0 + j, sum[j]);
+                }
+            }
+            table_vote(true);  // every warp has read the masks
+            if (threadIdx.x == 0) st->acc[0] = st->acc[1] = 0;
+        }
+    }
+};
+
+// An item's outputs, once all its units are decoded (table warps).
+template <class Cons>
+__device__ __forceinline__ bool finish_item(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm, const Bars &B,
+                                            uint32_t tmem, volatile uint32_t *failed) {
+    // one warp polls, the others wait at the barrier (no issue slots taken from the decode warps)
+    if (!table_vote(threadIdx.x >= 32 || wait_bar(B.tdone(k % kRing), (uint32_t)(k / kRing) & 1u, L, failed))) return false;
+    Cons::epilogue(L, I, k, sm, B, tmem);
+    table_vote(true);
+    if (threadIdx.x == 0) {
+        if (L.chain_scales) {
+            __threadfence();  // this item's outputs are visible before it is counted
+            atomicAdd(const_cast<uint32_t *>(&L.jobs[I.job].pad), 1u);
+        }
+        arrive(B.idone(k % kRing));
+    }
+    return true;
+}
+
+template <class Cons>
+__device__ __forceinline__ void serve_tables(const Q8WLaunch &L, unsigned char *sm, const Bars &B, uint32_t tmem,
+                                             volatile uint32_t *failed) {
+    const ItemRec *ring = reinterpret_cast<const ItemRec *>(sm + L.lay.ring);
+    int done = 0;  // items whose epilogue is done
+    const bool poll = threadIdx.x < 32;
+    // Warp 0 waits, then all four vote: they leave together when a wait gives up, and the other three take no issue
+    // slots from the decode warps meanwhile.
+    for (int k = 0;; k++) {
+        if (!table_vote(!poll || wait_bar(B.rfull(k % kRing), (uint32_t)(k / kRing) & 1u, L, failed))) return;
+        const ItemRec &I = ring[k % kRing];
+        if (I.it < 0) {
+            for (; done < k; done++)
+                if (!finish_item<Cons>(L, ring[done % kRing], done, sm, B, tmem, failed)) return;
+            return;
+        }
+        if (I.build) {
+            const int area = I.gen % kStages;
+            bool ok = !poll || wait_bar(B.staged(area), (uint32_t)(I.gen / kStages) & 1u, L, failed);
+            // (the table's previous users are done: they are among the items finished above)
+            if (!table_vote(ok)) return;
+            const uint32_t *so = reinterpret_cast<const uint32_t *>(sm + L.lay.stage_o) + area * kStageOffs;
+            const uint16_t *se = reinterpret_cast<const uint16_t *>(
+                sm + L.lay.stage_e + (uint32_t)area * ((uint32_t)L.tbl_stage + kStagePad) * 2u);
+            build_table(L, I.local, sm + 128 * I.tab, so, se + so[37]);
+        }
+        if (L.chain_scales && I.job > 0) {
+            for (; done < k; done++)
+                if (!finish_item<Cons>(L, ring[done % kRing], done, sm, B, tmem, failed)) return;
+            if (threadIdx.x == 0) chain_wait(L, I.job - 1, failed);
+        }
+        if (!table_vote(true)) return;
+        if (threadIdx.x == 0) arrive(B.tfull(k % kRing));
+        // The previous item's outputs, before the next record is waited for: this item's decode may need its
+        // accumulators and, when it has more units than there are slots, holds that record up.
+        for (; done < k; done++)
+            if (!finish_item<Cons>(L, ring[done % kRing], done, sm, B, tmem, failed)) return;
+    }
+}
+
+template <class Cons>
+__device__ __forceinline__ void decode_units(const Q8WLaunch &L, unsigned char *sm, const Bars &B, uint32_t tmem,
+                                             volatile uint32_t *failed) {
+    const int lane = threadIdx.x & 31;
+    const int w = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5) - kFirstDecode, 0);
+    const ItemRec *ring = reinterpret_cast<const ItemRec *>(sm + L.lay.ring);
+    const UnitDesc *desc = reinterpret_cast<const UnitDesc *>(sm + L.lay.desc);
+    Cons cons;
+    cons.init(L, sm, B, tmem, w);
+    uint32_t *unext = reinterpret_cast<uint32_t *>(sm + L.lay.misc) + 2;
+    const uint32_t S = (uint32_t)L.S;
+    int cur = -1;
+    uint32_t lw = 0, taken = 0;
+    if (lane == 0) taken = atomicAdd(unext, 1u);
+    for (;;) {
+        // units are taken as the warps get to them: their pace differs with the other warps of their scheduler
+        const uint32_t u = __shfl_sync(0xffffffffu, taken, 0);
+        const uint32_t turn = S == 1u ? u : __umulhi(u, L.S_inv), slot = u - turn * S, ph = turn & 1u;
+        // A slot passes from warp to warp, so its barrier may still be a phase behind, where the parity test would
+        // pass too early: the unit number in the slot tells, and the copy is waited for again once it is right.
+        bool ok = wait_bar(B.sfull((int)slot), ph, L, failed);
+        const volatile uint32_t *un = &desc[slot].unit;
+        for (uint32_t it = 0; ok && *un != u; it++) ok = it < L.spin_limit && !*failed;
+        __syncwarp();
+        ok = ok && wait_bar(B.sfull((int)slot), ph, L, failed);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        const UnitDesc d = desc[slot];
+        if (d.item < 0) break;
+        if (d.item != cur) {
+            cur = d.item;
+            if (!__all_sync(0xffffffffu, wait_bar(B.tfull(cur % kRing), (uint32_t)(cur / kRing) & 1u, L, failed))) break;
+            const ItemRec &I = ring[cur % kRing];
+            cons.begin_item(L, I);
+            lw = (uint32_t)lane * 4u | (uint32_t)I.tab << 7;
+        }
+        if (d.rows) cons.unit(L, d, sm, L.lay.slots + slot * L.slot_bytes, lw, lane, failed);
+        if (lane == 0) taken = atomicAdd(unext, 1u);  // (its latency passes while this unit is closed)
+        __syncwarp();
+        if (lane == 0) arrive(B.sempty((int)slot));
+        cons.end_unit(L, cur, sm, B, lane, failed);
+    }
+    cons.drain(L);
+}
+
+__device__ __forceinline__ uint32_t tmem_cols(int W) { return W <= 1 ? 32u : W <= 2 ? 64u : W <= 4 ? 128u : W <= 8 ? 256u : 512u; }
+
+template <class Cons>
+__global__ void __launch_bounds__(32 * (kFirstDecode + Cons::kMaxDecode), 1) q8w_kernel(const __grid_constant__ Q8WLaunch L) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int warp = threadIdx.x >> 5;
+    Bars B{smem_u32(smem) + L.lay.bars, L.S, L.W};
+    uint32_t *misc = reinterpret_cast<uint32_t *>(smem + L.lay.misc);  // [0] failure flag, [1] TMEM address, [2] next unit
+    volatile uint32_t *failed = misc;
+    if (threadIdx.x == 0) misc[0] = misc[2] = 0;
+    {
+        const int n = Bars::count(L.S, L.W, Cons::kMma);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(B.at(i)), "r"(B.arrivals(i)) : "memory");
+        }
+        uint32_t *z = reinterpret_cast<uint32_t *>(smem + L.lay.cnt);
+        for (int i = threadIdx.x; i < kRing * 2; i += blockDim.x) z[i] = 0;
+        UnitDesc *desc = reinterpret_cast<UnitDesc *>(smem + L.lay.desc);
+        for (int i = threadIdx.x; i < L.S; i += blockDim.x) desc[i].unit = 0xFFFFFFFFu;
+        uint32_t *red = reinterpret_cast<uint32_t *>(smem + L.lay.red);
+        for (int i = threadIdx.x; i < kRing * Cons::kRed; i += blockDim.x) red[i] = 0;
+    }
+    fence_mbar_init();
+    uint32_t tmem = 0;
+    if (Cons::kMma) {
+        if (warp == 0) tmem_alloc(misc + 1, tmem_cols(L.W));
+        tcgen05_fence_before();
+    }
+    __syncthreads();
+    if (Cons::kMma) {
+        tcgen05_fence_after();
+        tmem = misc[1];
+    }
+    if (warp < kTableWarps) serve_tables<Cons>(L, smem, B, tmem, failed);
+    else if (warp == kProducer) produce(L, smem, B, failed);
+    else if (warp == kStager) stage_tables(L, smem, B, failed);
+    else if (warp < kFirstDecode + L.W) decode_units<Cons>(L, smem, B, tmem, failed);
+    if (Cons::kMma) {
+        tcgen05_fence_before();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(tmem, tmem_cols(L.W));
+    } else {
+        __syncthreads();
+    }
+}
+
+// Shared-memory layout for W decode warps and S slots.
+template <class Cons>
+Q8WLayout layout(const Q8WLaunch &L, int W, int S) {
+    Q8WLayout o{};
+    auto up = [](uint32_t p) { return (p + 127u) & ~127u; };
+    uint32_t p = kLutBytes;
+    o.tiles = p;
+    if constexpr (Cons::kMma) p += (uint32_t)W * Cons::tile_bytes(L.xrows);
+    o.slots = p = up(p);
+    p += (uint32_t)S * L.slot_bytes;
+    o.red = p;
+    p += (uint32_t)(kRing * Cons::kRed) * 4u;
+    o.bars = p;
+    p += 8u * (uint32_t)Bars::count(S, W, Cons::kMma);
+    p = (p + 15u) & ~15u;
+    o.desc = p;
+    p += (uint32_t)S * (uint32_t)sizeof(UnitDesc);
+    o.ring = p;
+    p += (uint32_t)(kRing * sizeof(ItemRec));
+    o.cnt = p;
+    p += (uint32_t)(kRing * sizeof(ItemState));
+    o.misc = p;
+    p += 16u;
+    o.stage_o = p;
+    p += kStages * kStageOffs * 4u;
+    o.stage_e = p = (p + 15u) & ~15u;
+    p += kStages * ((uint32_t)L.tbl_stage + kStagePad) * 2u;
+    // an x tile is read as 64 vectors, however many it holds: up to 1 KB past the last tile
+    o.total = Cons::kMma ? std::max(p, o.slots + 1024u) : p;
+    return o;
+}
+
+template <class Cons>
+mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
+    Q8WLaunch L = L0;
+    const uint32_t limit = (uint32_t)max_smem_optin();
+    // CUDA-core consumers: x of a segment behind its block, but for chains
+    L.block_bytes = L.slot_bytes;
+    if (!Cons::kMma && !L.chain_scales) {
+        L.x_off = L.slot_bytes;
+        L.slot_bytes += (uint32_t)(4 * L.batch * kXQuads);
+    }
+    // Decode warps: as many as asked for (or the consumer's most), no more than a CTA has units for.  The slots
+    // beyond one per warp hold the units that the warps take next: without any, a warp would wait for its copy
+    // at every unit, so fewer warps with spare slots come before more warps without.
+    int W = std::min(warps > 0 ? warps : Cons::kMaxDecode, Cons::kMaxDecode);
+    W = std::max(1, std::min(W, units));
+    int S = 0;
+    for (; W >= 1; W--) {
+        const int spare = W >= 4 ? W / 4 : 1;
+        for (S = std::min(2 * W + 4, std::max(units, W)); S >= W; S--)
+            if (layout<Cons>(L, W, S).total <= limit) break;
+        if (S >= W + spare || (S >= W && (W == 1 || S >= units))) break;
+        S = 0;
+    }
+    if (!S) {
+        const uint32_t need = layout<Cons>(L, 1, 1).total;
+        return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %u B of shared memory (max %u)", need, limit);
+    }
+    L.W = W;
+    L.S = S;
+    L.S_inv = (uint32_t)((0x100000000ull + (uint32_t)S - 1) / (uint32_t)S);
+    L.lay = layout<Cons>(L, W, S);
+    auto kern = q8w_kernel<Cons>;
+    mv_status rc = prepare_kernel((const void *)kern, L.lay.total, 32 * (kFirstDecode + W), nullptr);
+    if (rc) return rc;
+    const unsigned grid = (unsigned)std::max(1LL, std::min<long long>(L.nitems, sm_count()));
+    const dim3 block(32 * (kFirstDecode + W));
+    if (L.chain_scales) {
+        // the chained pipeline waits across CTAs: a cooperative launch guarantees that they are all resident
+        void *args[] = {&L};
+        MV_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), block, args, L.lay.total, st),
+                    "q8 chain cooperative launch");
+        return MV_OK;
+    }
+    kern<<<grid, block, L.lay.total, st>>>(L);
+    MV_CUDA_TRY(cudaGetLastError(), "q8 kernel launch");
+    return MV_OK;
+}
+
+}  // namespace
+
+mv_status q8w_launch_int(const Q8WLaunch &L0, int nv, bool mma, int warps, int units, cudaStream_t st) {
+    Q8WLaunch L = L0;
+    if (mma) {
+        L.xrows = (L.batch + 7) & ~7;
+        return L.batch <= 16 ? launch_t<MmaCons<true>>(L, warps, units, st) : launch_t<MmaCons<false>>(L, warps, units, st);
+    }
+    switch (nv) {
+        case 1: return launch_t<DotCons<1>>(L, warps, units, st);
+        case 2: return launch_t<DotCons<2>>(L, warps, units, st);
+        case 4: return launch_t<DotCons<4>>(L, warps, units, st);
+        case 8: return launch_t<DotCons<8>>(L, warps, units, st);
+        default: return launch_t<DotCons<16>>(L, warps, units, st);
+    }
+}
+
+}  // namespace mv

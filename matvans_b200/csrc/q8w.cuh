@@ -1,0 +1,44 @@
+// Launch record of the warp-specialised Q8 kernel (k_q8w.cu), shared with the
+// code that plans launches (k_q8s.cu).
+#pragma once
+
+#include "mv_device.cuh"
+
+namespace mv {
+
+typedef mv_q8_job Q8Job;
+
+struct Q8WLayout {  // byte offsets in shared memory
+    uint32_t tiles, slots, red, bars, desc, ring, cnt, stage_o, stage_e, misc, total;
+};
+
+struct Q8WLaunch {
+    Q8Job job0;         // the only job when jobs == nullptr
+    const Q8Job *jobs;  // device array of njobs jobs, or nullptr
+    int njobs;
+    uint32_t nitems;
+    int batch;  // valid vectors
+    uint32_t *status;
+    uint32_t spin_limit;
+    int drop_copy;
+    uint32_t slot_bytes;  // one stream slot: the largest block and the row after it
+    int tbl_stage;        // staged table entries
+    // chained pipeline (mv_q8_chain_matvec): job j's int8 output clamp(rn(y * chain_scales[j])) is job j+1's x
+    // (the last job's goes to chain_out8); jobs[j].pad counts job j's finished work items
+    const float *chain_scales;
+    int8_t *chain_out8;
+    uint32_t *queue;  // work queue of a stack (jobs[0].pad of the job table), or nullptr: static round robin
+    // set by the launcher
+    int W, S;              // decode warps, stream slots
+    uint32_t S_inv;        // ceil(2^32 / S): unit / S by multiplication
+    uint32_t block_bytes;  // of a slot, its block's part
+    uint32_t x_off;        // where a slot holds its segment's x (0: nowhere)
+    int xrows;  // MMA consumers: rows of the x tile (batch rounded up to 8)
+    Q8WLayout lay;
+};
+
+// Integer product of L.batch vectors: on the tensor cores (up to 64 vectors) or, with dp4a, nv >= batch vectors
+// (1, 2, 4, 8 or 16).  warps: decode warps per CTA (0: as many as fit); units: the most units a CTA can get.
+mv_status q8w_launch_int(const Q8WLaunch &L, int nv, bool mma, int warps, int units, cudaStream_t st);
+
+}  // namespace mv

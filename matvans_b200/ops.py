@@ -11,7 +11,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import MMA_MIN_BATCH, Q8Job, Q8StackInfo, Q8Tuning, Q8View, check, lib
+from ._lib import Q8Job, Q8StackInfo, Q8Tuning, Q8View, check, lib
 
 _STATUS_BITS = {1: "stream overrun", 2: "final coder state mismatch", 4: "wait timeout", 8: "bad table"}
 
@@ -299,11 +299,6 @@ class Q8Stack:
                     for M in self.matrices] if scales is not None else None
         n = len(self.matrices)
         jobs = (Q8Job * n)()
-        # 3..16 vectors run on the tensor cores (engine 0): x is laid out in tiles first (device scratch per
-        # matrix)
-        self._tiled = self.batch >= MMA_MIN_BATCH and self.tuning.engine == 0
-        use_tiles = self._tiled
-        self.x_tiles = []
         for i, M in enumerate(self.matrices):
             x = self.xs[i]
             if x.dtype != torch.int8 or tuple(x.shape) != (self.batch, M.cols) or not x.is_contiguous():
@@ -311,11 +306,6 @@ class Q8Stack:
             jobs[i].m = M.view()
             jobs[i].x = x.data_ptr()
             jobs[i].y = self.ys[i].data_ptr()
-            if use_tiles:
-                nb = lib().mv_q8_x_tiles_bytes(ctypes.byref(jobs[i].m))
-                t = torch.empty(nb, dtype=torch.uint8, device=self.device)
-                self.x_tiles.append(t)
-                jobs[i].x_tiles = t.data_ptr()
             if scales is not None:
                 jobs[i].scales = scales[i].data_ptr()
                 jobs[i].ys = self.yss[i].data_ptr()
@@ -331,9 +321,9 @@ class Q8Stack:
 
     @property
     def launches_per_run(self):
-        """Kernels one run() launches: the persistent decode, the x-tile layout pass when the tensor-core
-        consumer reads x tiles, and the zero/scale passes when any job accumulates atomically."""
-        return 1 + (1 if self._tiled else 0) + (2 if self.info.atomic_jobs else 0)
+        """Kernels one run() launches: the persistent decode, and the zero/scale passes when any job accumulates
+        atomically."""
+        return 1 + (2 if self.info.atomic_jobs else 0)
 
     def run(self):
         check(lib().mv_q8_stack_matvec(_p(self.jobs_dev), len(self.matrices), ctypes.byref(self.info), self.batch,

@@ -1,0 +1,51 @@
+"""Warp-specialised Q8 kernel: unit, slot and table hand-over at the sizes where they change, bit-exact against the
+CPU oracle.  (Tiny segments pass a stream slot from warp to warp within one decode; segments beyond 64 quads read x
+from global memory; fewer units than warps and single-segment stripes leave warps idle; batches cross the 16-vector
+lane groups and the 64-vector pass.)"""
+import numpy as np
+import pytest
+
+from conftest import cuda_ok
+import oracle
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not cuda_ok(), reason="needs a CUDA device")]
+
+if cuda_ok():
+    import torch
+    from matvans_b200 import ops
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads,local", [
+    (33, 16, 0, True), (5000, 64, 4, True), (257, 1040, 4, False), (96, 2048, 68, True), (64, 8192, 128, False),
+    (9600, 272, 0, True)])
+def test_units_and_batches(rows, cols, seg_quads, local):
+    rng = np.random.default_rng(rows + cols + seg_quads)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, local=local, seg_quads=seg_quads)
+    s = rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)
+    for B in (1, 2, 3, 17, 33, 64, 66):
+        x = rng.integers(-128, 128, size=(B, cols)).astype(np.int8)
+        y, ys = M.matvec(torch.from_numpy(x), scales=s)
+        ref = oracle.matvec_i8(W, x)
+        assert np.array_equal(y.cpu().numpy(), ref), B
+        assert np.array_equal(ys.cpu().numpy(), (ref.astype(np.float32) * s[None, :]).astype(np.float32)), B
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("B", [1, 2, 5, 16])
+def test_stack_of_uneven_items_runs_repeatedly(B):
+    # more items than CTAs, items of 1 to 40 units, tables shared and not: the work queue, the table hand-over and
+    # the accumulators over several launches of one plan
+    rng = np.random.default_rng(B)
+    shapes = [(4096, 64, 4), (640, 2560, 64), (3000, 160, 8), (64, 16, 0), (1504, 1024, 0)]
+    Ws = [np.clip(np.round(rng.normal(0, 3.0, size=sh[:2])), -127, 127).astype(np.int8) for sh in shapes]
+    Ms = [ops.Q8Matrix.encode(W, local=i % 2 == 0, seg_quads=sh[2]) for i, (W, sh) in enumerate(zip(Ws, shapes))]
+    S = ops.Q8Stack(Ms, batch=B)
+    for _ in range(3):
+        for M, xd in zip(Ms, S.xs):
+            xd.copy_(torch.from_numpy(rng.integers(-127, 128, size=(B, M.cols)).astype(np.int8)))
+        S.y_flat.fill_(-1)
+        S.run()
+        for W, xd, y in zip(Ws, S.xs, S.ys):
+            assert np.array_equal(y.cpu().numpy(), oracle.matvec_i8(W, xd.cpu().numpy())), W.shape
+    assert ops.device_status() == 0
