@@ -333,95 +333,6 @@ __device__ __forceinline__ void i8x4_to_f32(uint32_t wq, float (&f)[4]) {
     f[3] = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653)) - 8388736.0f;
 }
 
-__device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
-__device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
-
-// Y = diag(s) W X with X bf16 [NV][cols], fp32 accumulation, fp32 Y [NV][rows] (J.ys).
-template <int NV>
-struct FwdCons {
-    static constexpr int kNV = NV;
-    static constexpr int kRedNV = NV;
-    static constexpr int kRedBufs = 1;
-    static constexpr bool kFinishSyncs = true;
-    static constexpr int kMinCtas = 1;
-    static constexpr int kMaxThreads = 512;  // 16 warps: a stripe's segments over more warps (few stripes)
-    static constexpr int kTmemCols = 0;
-    static constexpr bool kWideLut = true;
-    static constexpr bool kLut256 = false;
-    static __host__ __device__ constexpr size_t extra_bytes(int) { return 0; }
-    static __host__ __device__ constexpr size_t tbl_alias_bytes(int) { return 0; }
-    __device__ __forceinline__ void init(const Q8SLaunch &, unsigned char *, uint32_t, int, int, int) {}
-    __device__ __forceinline__ void drain(const Q8SLaunch &) {}
-    template <int ILP>
-    __device__ __forceinline__ void run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int W,
-                                             const uint32_t (&rows_now)[ILP], const unsigned char *sm,
-                                             uint32_t soff, const uint32_t *lut_l, int lane);
-    const uint16_t *x;
-    int cols;
-    float acc[NV];
-    struct Group {
-        uint4 xv[NV][2];  // 16 bf16 = 4 quads
-    };
-    __device__ __forceinline__ void begin_item(const Q8SLaunch &, const Q8Job &J, int, int, int) {
-        x = reinterpret_cast<const uint16_t *>(J.x);
-        cols = J.m.cols;
-#pragma unroll
-        for (int v = 0; v < NV; v++) acc[v] = 0.f;
-    }
-    __device__ __forceinline__ void load_group(Group &g, int q) const {
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-            const uint4 *p = reinterpret_cast<const uint4 *>(x + (size_t)v * cols + 4 * q);
-            g.xv[v][0] = __ldg(p);
-            g.xv[v][1] = __ldg(p + 1);
-        }
-    }
-    __device__ __forceinline__ void fma4(uint32_t wq, uint32_t xa, uint32_t xb, float &a) {
-        float w[4];
-        i8x4_to_f32(wq, w);
-        a = fmaf(w[0], bf16_lo(xa), a);
-        a = fmaf(w[1], bf16_hi(xa), a);
-        a = fmaf(w[2], bf16_lo(xb), a);
-        a = fmaf(w[3], bf16_hi(xb), a);
-    }
-    __device__ __forceinline__ void use(const Group &g, int j, int, uint32_t wq, int) {
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-            const uint4 &h = g.xv[v][j >> 1];
-            const uint32_t xa = (j & 1) ? h.z : h.x, xb = (j & 1) ? h.w : h.y;
-            fma4(wq, xa, xb, acc[v]);
-        }
-    }
-    __device__ __forceinline__ void single(int q, uint32_t wq, int) {
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-            const uint2 xv = __ldg(reinterpret_cast<const uint2 *>(x + (size_t)v * cols + 4 * q));
-            fma4(wq, xv.x, xv.y, acc[v]);
-        }
-    }
-    __device__ __forceinline__ void finish_item(const Q8SLaunch &L, const Q8Job &J, int stripe, int warp, int lane,
-                                                int W, void *red_smem) {
-        float *red = reinterpret_cast<float *>(red_smem);
-#pragma unroll
-        for (int v = 0; v < NV; v++) red[(warp * NV + v) * 32 + lane] = acc[v];
-        __syncthreads();
-        const mv_q8_view &m = J.m;
-        for (int t = threadIdx.x; t < NV * 32; t += blockDim.x) {
-            const int v = t >> 5, l = t & 31;
-            float sum = 0.f;
-            for (int w = 0; w < W; w++) sum += red[(w * NV + v) * 32 + l];  // fixed order: deterministic
-            const int row = stripe * 32 + l;
-            if (row < m.rows && v < L.batch) {
-                float *dst = J.ys + (size_t)v * m.rows + row;
-                const float val = sum * J.scales[row];
-                if (J.atomic) atomicAdd(dst, val);
-                else *dst = val;
-            }
-        }
-        __syncthreads();
-    }
-};
-
 // dX = W^T (s . dY): dY bf16 [NV][rows] (J.x), dX fp32 [NV][cols] (J.ys, zeroed,
 // accumulated with fp32 atomics across stripes).  The 32 lanes of a warp are
 // the 32 rows of the stripe, so the four column contributions of a quad are
@@ -597,13 +508,6 @@ __device__ __forceinline__ void decode_step(const Q8SLaunch &L, const mv_q8_view
 
 template <int NV>
 template <int ILP>
-__device__ __forceinline__ void FwdCons<NV>::run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int W,
-                                                      const uint32_t (&rows_now)[ILP], const unsigned char *sm,
-                                                      uint32_t soff, const uint32_t *lut_l, int lane) {
-    decode_step<FwdCons<NV>, ILP>(L, m, seg0, W, rows_now, sm, soff, lut_l, lane, *this);
-}
-template <int NV>
-template <int ILP>
 __device__ __forceinline__ void BwdCons<NV>::run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int W,
                                                       const uint32_t (&rows_now)[ILP], const unsigned char *sm,
                                                       uint32_t soff, const uint32_t *lut_l, int lane) {
@@ -632,178 +536,6 @@ __device__ __forceinline__ void decode_piece(int qc, int nq, SegStream &S, const
             w[j] = (qc + j < nq) ? q8_step_t<kWide>(S.lo, S.hi, S.koff, S.kend, sm, lut_l, stride, lane, S.P) : 0u;
     }
 }
-
-// Float forward on the tensor cores: Y = diag(s) W X for up to 16 bf16 vectors,
-// fp32 accumulation (kind::f16 MMAs, bf16 A and B: the int8 weights and the bf16
-// inputs are exact in bf16, every product is exact in fp32).  Per 8 decoded
-// quads each lane converts its 32 weights to bf16 and stores them into its
-// TMEM lane (A, 16 columns); one lane issues two MMAs (K = 16 each) against the
-// x tile (B: 16 vectors x 32 columns of bf16, K-major core matrices, 1 KB) into
-// the warp's 16 fp32 D columns.  x moves through a 2-piece window (2 KB per
-// warp) loaded into registers ahead of use.  The x tiles hold the cross-warp
-// reduction (fixed order) at the end of a stripe and stage the decode tables.
-struct FwdMma {
-    static constexpr int kNV = 16;
-    static constexpr int kRedNV = 0;
-    static constexpr int kRedBufs = 1;
-    static constexpr bool kFinishSyncs = true;
-    static constexpr int kMinCtas = 2;
-    static constexpr int kMaxThreads = 256;
-    static constexpr int kTmemCols = 1;
-    static constexpr bool kWideLut = false;
-    static constexpr bool kLut256 = false;
-    static constexpr int kXPieces = 2;
-    static constexpr int kXBytes = kXPieces * 1024;
-    static __host__ __device__ constexpr size_t extra_bytes(int W) {
-        return (((size_t)W * kXBytes + (size_t)W * 8 + 128) + 127) / 128 * 128;
-    }
-    static __host__ __device__ constexpr size_t tbl_alias_bytes(int W) { return (size_t)W * kXBytes; }
-    uint32_t xt, d_tmem, st_addr, ld_addr, ncommit;
-    uint64_t b_desc0;
-    uint64_t *mbar;
-    float *xbase;
-    const uint16_t *x;
-    int cols, batch;
-    bool any;
-
-    __device__ __forceinline__ void init(const Q8SLaunch &, unsigned char *extra, uint32_t tmem_base, int, int lane,
-                                         int W) {
-        const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
-        const uint32_t base = smem_u32(extra);
-        xbase = reinterpret_cast<float *>(extra);
-        xt = base + (uint32_t)warp * (uint32_t)kXBytes;
-        mbar = reinterpret_cast<uint64_t *>(extra + (size_t)W * kXBytes) + warp;
-        if (lane == 0) mbar_init(mbar, 1);
-        fence_mbar_init();
-        __syncwarp();
-        const uint32_t quarter = ((uint32_t)(warp & 3) * 32u) << 16;
-        d_tmem = tmem_base + 32u * (uint32_t)warp;
-        st_addr = d_tmem + 16u + quarter;
-        ld_addr = d_tmem + quarter;
-        b_desc0 = umma_smem_desc(xt, 128u, 256u);
-        ncommit = 0;
-    }
-    __device__ __forceinline__ void begin_item(const Q8SLaunch &L, const Q8Job &J, int, int, int) {
-        x = reinterpret_cast<const uint16_t *>(J.x);
-        cols = J.m.cols;
-        batch = L.batch;
-        any = false;
-    }
-    __device__ __forceinline__ bool wait_mma(const Q8SLaunch &L) {
-        if (ncommit == 0) return true;
-        return mbar_wait_bounded(mbar, (ncommit - 1) & 1, L.status, L.spin_limit);
-    }
-    // lane (b, hh) moves vector b's 8-column chunks 2*hh and 2*hh+1 of each 32-column piece of a window
-    __device__ __forceinline__ void load_window(uint4 (&xr)[2 * kXPieces], const uint16_t *xrow, bool xok,
-                                                int colbase, int pbase, int npieces) const {
-#pragma unroll
-        for (int i = 0; i < kXPieces; i++) {
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const int p = pbase + i;
-                const int off = 32 * p + 8 * j;  // columns from xrow
-                xr[2 * i + j] = make_uint4(0, 0, 0, 0);
-                // cols % 16 == 0: an 8-column chunk that starts inside the row ends inside it
-                if (xok && p < npieces && colbase + off < cols)
-                    xr[2 * i + j] = __ldg(reinterpret_cast<const uint4 *>(xrow + off));
-            }
-        }
-    }
-    template <int ILP>
-    __device__ __forceinline__ void run_step(const Q8SLaunch &L, const mv_q8_view &m, int seg0, int,
-                                             const uint32_t (&rows_now)[ILP], const unsigned char *sm,
-                                             uint32_t soff, const uint32_t *lut_l, int lane) {
-        const int qtot = (m.cols + 3) >> 2;
-        const int q0 = seg0 * m.seg_quads;
-        const int nq = rows_now[0] ? min(m.seg_quads, qtot - q0) : 0;
-        if (nq <= 0) return;
-        const int npieces = (nq + 7) >> 3;
-        const int b = lane >> 1, hh = lane & 1;
-        const bool xok = b < batch;
-        const int colbase = 4 * q0 + 16 * hh;
-        const uint16_t *xrow = x + (size_t)(xok ? b : 0) * cols + colbase;
-        // chunk c8 = 2 hh + j of a piece: K step c8 >> 1 (512 B), K half c8 & 1 (128 B)
-        const uint32_t xdst = xt + (uint32_t)hh * 512u + (uint32_t)(b >> 3) * 256u + (uint32_t)(b & 7) * 16u;
-        uint4 xr[2 * kXPieces];
-        load_window(xr, xrow, xok, colbase, 0, npieces);
-        SegStream S(sm, soff, rows_now[0], lane);
-        for (int p = 0; p < npieces; p++) {
-            uint32_t w[8];
-            decode_piece<kWideLut>(8 * p, nq, S, sm, lut_l, L.lut_stride, lane, w);
-            uint32_t a[16];
-#pragma unroll
-            for (int j = 0; j < 8; j++) i8x4_to_bf16x4(w[j], a[2 * j], a[2 * j + 1]);
-            wait_mma(L);  // the previous MMAs are done with the A columns (and the x tile)
-            const int pw = p & (kXPieces - 1);
-            if (pw == 0) {
-                const int cn = min(kXPieces, npieces - p);
-#pragma unroll
-                for (int i = 0; i < kXPieces; i++)
-                    if (i < cn) {
-#pragma unroll
-                        for (int j = 0; j < 2; j++) {
-                            const uint4 v = xr[2 * i + j];
-                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(
-                                             xdst + (uint32_t)i * 1024u + (uint32_t)j * 128u),
-                                         "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-                                         : "memory");
-                        }
-                    }
-                fence_proxy_async_smem();
-                if (p + kXPieces < npieces) load_window(xr, xrow, xok, colbase, p + kXPieces, npieces);
-            }
-            tcgen05_fence_after();
-            tmem_st_32x32b_x16_nowait(st_addr, a);
-            tmem_wait_st();
-            tcgen05_fence_before();
-            __syncwarp();
-            if (elect_one()) {
-                tcgen05_fence_after();
-                const uint32_t idesc = umma_idesc_bf16(128, 16, 0, 0);
-                const uint64_t bd = b_desc0 + (uint64_t)(pw * 64);  // 1 KB per piece, in 16-byte units
-                umma_f16_ts(d_tmem, d_tmem + 16u, bd, idesc, any ? 1u : 0u);
-                umma_f16_ts(d_tmem, d_tmem + 24u, bd + 32u, idesc, 1u);
-                umma_commit(mbar);
-            }
-            __syncwarp();
-            any = true;
-            ncommit++;
-        }
-        if (!S.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
-    }
-    __device__ __forceinline__ void finish_item(const Q8SLaunch &L, const Q8Job &J, int stripe, int warp, int lane,
-                                                int W, void *) {
-        uint32_t r[16];
-        if (any) {
-            wait_mma(L);
-            tcgen05_fence_after();
-            tmem_ld_32x32b_x16(ld_addr, r);  // lane = stripe row, r[v] = vector v (fp32 bits)
-        } else {
-#pragma unroll
-            for (int v = 0; v < 16; v++) r[v] = 0;
-        }
-        float *red = xbase + warp * (kXBytes / 4);
-#pragma unroll
-        for (int v = 0; v < 16; v++) red[v * 32 + lane] = __uint_as_float(r[v]);
-        tcgen05_fence_before();
-        __syncthreads();
-        const mv_q8_view &m = J.m;
-        for (int t = threadIdx.x; t < 16 * 32; t += blockDim.x) {
-            const int v = t >> 5, l = t & 31;
-            float sum = 0.f;
-            for (int w = 0; w < W; w++) sum += xbase[w * (kXBytes / 4) + t];  // fixed order: deterministic
-            const int row = stripe * 32 + l;
-            if (row < m.rows && v < L.batch) {
-                float *dst = J.ys + (size_t)v * m.rows + row;
-                const float val = sum * J.scales[row];
-                if (J.atomic) atomicAdd(dst, val);
-                else *dst = val;
-            }
-        }
-        __syncthreads();
-    }
-    __device__ __forceinline__ void drain(const Q8SLaunch &L) { wait_mma(L); }
-};
 
 // Float backward on the tensor cores: dX = W^T (s . dY) for up to 32 bf16
 // vectors.  Per stripe the CTA builds G = s . dY for its 32 rows as a pair of
@@ -1533,26 +1265,16 @@ mv_status launch_q8s_c(const Q8SLaunch &L, const mv_q8_tuning &t, cudaStream_t s
 // on the batch, while the dp4a consumer's grows with it.
 constexpr int kMmaMinVectors = MV_MMA_MIN_VECTORS;
 
-// mode 1: float forward, mode 2: float backward (transposed); nv in {1,2,4,8}
-// float form: batches of at least this many vectors go to the tensor-core consumers (engine 0)
+// float backward: batches of at least this many vectors go to the tensor-core consumer (engine 0)
 constexpr int kFloatMmaMinBatch = 2;
 
-// vectors per pass of the float form: the tensor-core consumers take 16 (forward) / 32 (backward)
-int q8f_pass(int mode, int batch, const mv_q8_tuning &t) {
-    if (t.engine == MV_ENGINE_AUTO && batch >= kFloatMmaMinBatch) return mode == 1 ? FwdMma::kNV : BwdMma::kNV;
-    return 8;
+// vectors per pass of the float backward: the tensor-core consumer takes 32
+int q8b_pass(int batch, const mv_q8_tuning &t) {
+    return t.engine == MV_ENGINE_AUTO && batch >= kFloatMmaMinBatch ? BwdMma::kNV : 8;
 }
 
-mv_status launch_q8f(const Q8SLaunch &L, int mode, int nv, const mv_q8_tuning &t, bool mma, cudaStream_t st) {
-    if (mma) return mode == 1 ? launch_q8s_c<FwdMma>(L, t, st) : launch_q8s_c<BwdMma>(L, t, st);
-    if (mode == 1) {
-        switch (nv) {
-            case 1: return launch_q8s_c<FwdCons<1>>(L, t, st);
-            case 2: return launch_q8s_c<FwdCons<2>>(L, t, st);
-            case 4: return launch_q8s_c<FwdCons<4>>(L, t, st);
-            default: return launch_q8s_c<FwdCons<8>>(L, t, st);
-        }
-    }
+mv_status launch_q8b(const Q8SLaunch &L, int nv, const mv_q8_tuning &t, bool mma, cudaStream_t st) {
+    if (mma) return launch_q8s_c<BwdMma>(L, t, st);
     switch (nv) {
         case 1: return launch_q8s_c<BwdCons<1>>(L, t, st);
         case 2: return launch_q8s_c<BwdCons<2>>(L, t, st);
@@ -1712,36 +1434,66 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
     return MV_OK;
 }
 
-// Float forward / transposed product through the persistent kernel.
-mv_status q8f_run(const mv_q8_view *m, int mode, const uint16_t *in, int batch, const float *scales, float *out,
-                  const mv_q8_tuning *tuning, cudaStream_t st) {
+// Float forward: passes of up to 64 vectors through the warp-specialised kernel, whole stripes per work item.
+mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float *scales, float *y,
+                 const mv_q8_tuning *tuning, cudaStream_t st) {
+    mv_status rc;
+    uint32_t *status = device_status_word(&rc);
+    if (rc) return rc;
+    const mv_q8_tuning t = resolve(tuning);
+    const bool asked = tuning && tuning->warps > 0;
+    if (asked && t.warps > 8 && t.engine == MV_ENGINE_AUTO && batch >= 2)
+        return fail(MV_ERR_ARG, "Q8 launch: %d warps per CTA; the float form on the tensor cores takes at most 8", t.warps);
+    const size_t need = 32768 + (size_t)t.warps * t.depth * ((size_t)(m->max_blk_rows + 1) * 128 + 2056) +
+                        2 * ((size_t)m->tbl_stripe_max + 8) + 1024;
+    if (need > (size_t)max_smem_optin())
+        return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
+    for (int v0 = 0; v0 < batch; v0 += 64) {
+        Q8WLaunch L{};
+        L.job0.m = *m;
+        L.job0.x = reinterpret_cast<const int8_t *>(x + (size_t)v0 * m->cols);
+        L.job0.scales = scales;
+        L.job0.ys = y + (size_t)v0 * m->rows;
+        uint32_t items = 0;
+        plan_job(L.job0, t, items, 1);
+        L.njobs = 1;
+        L.nitems = items;
+        L.batch = std::min(64, batch - v0);
+        L.status = status;
+        L.spin_limit = wait_spin_limit();
+        L.drop_copy = inject_drop_copy();
+        L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
+        L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
+        const long long per_cta = ((long long)items + sm_count() - 1) / sm_count() * m->nseg;
+        rc = q8w_launch_fwd(L, asked ? t.warps : 0, (int)std::min<long long>(per_cta, 1 << 20), st);
+        if (rc) return rc;
+    }
+    return MV_OK;
+}
+
+// Transposed product through the persistent kernel.
+mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float *scales, float *dx,
+                 const mv_q8_tuning *tuning, cudaStream_t st) {
     mv_status rc;
     uint32_t *status = device_status_word(&rc);
     if (rc) return rc;
     mv_q8_tuning t = resolve(tuning);
     if (!tuning || (tuning->ilp != 1 && tuning->ilp != 2)) t.ilp = 1;  // the float form's default
-    const int in_len = mode == 1 ? m->cols : m->rows;   // elements per vector in
-    const int out_len = mode == 1 ? m->rows : m->cols;  // elements per vector out
-    if (mode == 2) MV_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)batch * out_len, st), "memset(dx)");
-    const int pass = q8f_pass(mode, batch, t);
+    MV_CUDA_TRY(cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)batch * m->cols, st), "memset(dx)");
+    const int pass = q8b_pass(batch, t);
     const bool mma = pass > 8;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         const int nb = std::min(pass, batch - v0);
         Q8SLaunch L{};
         L.job0.m = *m;
-        L.job0.x = reinterpret_cast<const int8_t *>(in + (size_t)v0 * in_len);
-        L.job0.y = nullptr;
+        L.job0.x = reinterpret_cast<const int8_t *>(dy + (size_t)v0 * m->rows);
         L.job0.scales = scales;
-        L.job0.ys = out + (size_t)v0 * out_len;
+        L.job0.ys = dx + (size_t)v0 * m->cols;
         uint32_t items = 0;
-        // forward: whole stripes (deterministic sums); backward: atomics anyway, so split for parallelism
-        int parts = 1;
-        if (mode == 2) {
-            const int stripes = (m->rows + 31) / 32, sg = t.warps * t.ilp;
-            parts = t.parts > 0 ? t.parts : mma ? fill_parts(m->nseg, sg, stripes) : bwd_parts(m->nseg, sg, stripes);
-        }
-        plan_job(L.job0, t, items, parts);
-        if (mode == 1 && L.job0.atomic) return fail(MV_ERR_ARG, "float forward needs whole stripes (parts = 1)");
+        // atomics anyway, so stripes are split for parallelism
+        const int stripes = (m->rows + 31) / 32, sg = t.warps * t.ilp;
+        plan_job(L.job0, t, items,
+                 t.parts > 0 ? t.parts : mma ? fill_parts(m->nseg, sg, stripes) : bwd_parts(m->nseg, sg, stripes));
         L.jobs = nullptr;
         L.njobs = 1;
         L.nitems = items;
@@ -1752,7 +1504,7 @@ mv_status q8f_run(const mv_q8_view *m, int mode, const uint16_t *in, int batch, 
         L.buf_words = (m->max_blk_rows + 1) * 32;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
         L.lut_stride = 32;
-        rc = launch_q8f(L, mode, nv_round(nb), t, mma, st);
+        rc = launch_q8b(L, nv_round(nb), t, mma, st);
         if (rc) return rc;
     }
     return MV_OK;
@@ -1768,15 +1520,7 @@ mv_status mv_q8_matvec_bf16(const mv_q8_view *m, const uint16_t *x_dev, int batc
         return mv::fail(MV_ERR_ARG, "mv_q8_matvec_bf16: bad arguments");
     if ((m->cols & 15) || ((uintptr_t)x_dev & 15) || (m->seg_quads & 3))
         return mv::fail(MV_ERR_ARG, "mv_q8_matvec_bf16: needs cols %% 16 == 0, seg_quads %% 4 == 0, 16-byte aligned x");
-    mv_q8_tuning t = mv::resolve(tuning);
-    t.parts = 1;
-    if (!tuning || (tuning->ilp != 1 && tuning->ilp != 2)) t.ilp = 1;  // the float form's default
-    // the forward keeps whole stripes per item (a fixed-order reduction): with fewer stripes than SMs, the
-    // CUDA-core consumer takes 16-warp CTAs so that each stripe's segments spread over more warps
-    // (4096x11008, one vector: 35.0 against 43.2 us; with 344 stripes 8 warps stay faster, 43.2 against 47.3)
-    if ((!tuning || tuning->warps <= 0) && mv::q8f_pass(1, batch, t) <= 8 && (m->rows + 31) / 32 < mv::sm_count())
-        t.warps = 16;
-    return mv::q8f_run(m, 1, x_dev, batch, row_scales_dev, y_dev, &t, (cudaStream_t)stream);
+    return mv::q8_fwd(m, x_dev, batch, row_scales_dev, y_dev, tuning, (cudaStream_t)stream);
 }
 
 mv_status mv_q8_matvec_t_bf16(const mv_q8_view *m, const uint16_t *dy_dev, int batch, const float *row_scales_dev,
@@ -1785,7 +1529,7 @@ mv_status mv_q8_matvec_t_bf16(const mv_q8_view *m, const uint16_t *dy_dev, int b
         return mv::fail(MV_ERR_ARG, "mv_q8_matvec_t_bf16: bad arguments");
     if ((m->cols & 15) || (m->seg_quads & 3))
         return mv::fail(MV_ERR_ARG, "mv_q8_matvec_t_bf16: needs cols %% 16 == 0 and seg_quads %% 4 == 0");
-    return mv::q8f_run(m, 2, dy_dev, batch, row_scales_dev, dx_dev, tuning, (cudaStream_t)stream);
+    return mv::q8_bwd(m, dy_dev, batch, row_scales_dev, dx_dev, tuning, (cudaStream_t)stream);
 }
 
 mv_status mv_q8_stack_plan(mv_q8_job *jobs, int njobs, const mv_q8_tuning *tuning, mv_q8_stack_info *info) {

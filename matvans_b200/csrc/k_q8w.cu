@@ -48,6 +48,8 @@
 // the kernel at 11 on a 7B layer (one vector).
 #include <algorithm>
 
+#include <cuda_bf16.h>
+
 #include "mv_device.cuh"
 #include "q8w.cuh"
 #include "umma.cuh"
@@ -86,7 +88,7 @@ struct alignas(16) ItemRec {
     int32_t build;      // 1: the table is built for this item
     int32_t area_item;  // the item whose build must be over before this one's data is staged (-1: none)
     int32_t sb;         // first segment
-    uint32_t n;         // number of units
+    uint32_t n, u0;     // number of units, and the first one's running number
     int32_t rows, cols, seg_quads, atomic, local;
     float chain_scale;
     const int8_t *x;
@@ -301,7 +303,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
     UnitDesc *desc = reinterpret_cast<UnitDesc *>(sm + L.lay.desc);
     const uint32_t slots = smem_u32(sm) + L.lay.slots;
     const uint32_t S = (uint32_t)L.S, W = (uint32_t)L.W;
-    uint32_t u = 0;              // units published
+    uint32_t u = 0, recorded = 0;  // units published, units of the items recorded
     uint32_t next = blockIdx.x;  // the CTA's latest item number; its first one is static
     uint32_t grabbed = 0;        // lane 0: the queue's answer for the item after it
     int job = 0, tjob = -1, tstripe = -1, gen = -1;
@@ -316,6 +318,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
         const bool end = next >= L.nitems;
         r.it = end ? -1 : (int32_t)next;
         r.n = W;  // one end mark per decode warp
+        r.u0 = recorded;
         r.area_item = -1;
         if (!end) {
             int se = 0;
@@ -350,6 +353,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
             r.gen = gen;
             r.tab = gen & 1;
         }
+        recorded += r.n;
         if (ok && lane == 0) {
             ring[k % kRing] = r;
             if (!end) arrive_n(B.tdone(k % kRing), kTdone - r.n);  // the units' arrivals are left
@@ -405,15 +409,16 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
                         const uint32_t dst = slots + slot * L.slot_bytes, bar = B.sfull((int)slot);
                         // the block, and behind it (CUDA-core consumers) the segment's x of every vector
                         const int q = (r.sb + (int)i) * m.seg_quads;
-                        const uint32_t xb =
-                            x_in_slot(L, m.seg_quads) && rows ? 4u * (uint32_t)max(0, min(m.seg_quads, (m.cols >> 2) - q)) : 0u;
+                        const uint32_t xb = x_in_slot(L, m.seg_quads) && rows
+                                                ? L.x_quad * (uint32_t)max(0, min(m.seg_quads, (m.cols >> 2) - q))
+                                                : 0u;
                         arrive_tx(bar, rows * 128u + xb * (uint32_t)L.batch);
                         if (rows && !L.drop_copy) {
                             bulk_in(dst, m.blocks + (size_t)o0 * 32, rows * 128u, bar);
-                            const int8_t *x = r.x + 4 * (size_t)q;
+                            const int8_t *x = r.x + (size_t)L.x_quad * q;
                             if (xb)
                                 for (int v = 0; v < L.batch; v++)
-                                    bulk_in(dst + L.x_off + 4u * (uint32_t)(v * m.seg_quads), x + (size_t)v * m.cols, xb, bar);
+                                    bulk_in(dst + L.x_off + 4u * (uint32_t)(v * m.seg_quads), x + (size_t)v * m.cols, xb, bar);  // (float: one vector)
                         }
                     }
                     __syncwarp();
@@ -466,14 +471,21 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
 
 // --------------------------------------------------------------- table warps
 
+// Table entries: of the integer consumers f | sym << 16 | r << 24, of the float ones f | r << 8 | bf16(sym) << 16.
+template <bool kFloat>
 __device__ __forceinline__ uint32_t table_entry(uint32_t ent) {  // r = 0; ent: symbol | f << 8
-    return (ent >> 8) | (ent & 0xFFu) << 16;
+    if constexpr (kFloat)
+        return (ent >> 8) |
+               (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn((float)(int8_t)(uint8_t)(ent & 0xFFu))) << 16;
+    else
+        return (ent >> 8) | (ent & 0xFFu) << 16;
 }
 
 // Decode table from the staged data: warp s fills quantiles [64 s, 64 s + 64), lane l its row's column, with no
 // divergence: the column is cleared, each symbol's entry (r = 0) goes to its first quantile, and one pass then
 // carries the entries forward, r growing by one per quantile.  (A walk that stores quantile by quantile and moves
 // to the next symbol by a branch took 3.2 us a table with the decode warps at work.)
+template <bool kFloat>
 __device__ __forceinline__ void build_table(const Q8WLaunch &L, int local, unsigned char *lut,
                                             const uint32_t *so, const uint16_t *tsm) {
     const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -503,8 +515,8 @@ __device__ __forceinline__ void build_table(const Q8WLaunch &L, int local, unsig
     }
     // the symbol that holds qlo starts the pass; e is one step (r) behind
     bool bad = k >= o1;
-    constexpr uint32_t kR = 1u << 24;  // one step of r
-    uint32_t e = table_entry(ent) + (qlo - cum - 1u) * kR;
+    constexpr uint32_t kR = kFloat ? 1u << 8 : 1u << 24;  // one step of r
+    uint32_t e = table_entry<kFloat>(ent) + (qlo - cum - 1u) * kR;
     cum += ent >> 8;
     __syncwarp();
     unsigned char *col = rows + 4u * (uint32_t)lane;
@@ -516,7 +528,7 @@ __device__ __forceinline__ void build_table(const Q8WLaunch &L, int local, unsig
         }
         ent = tsm[k];
         if ((ent >> 8) == 0) bad = true;
-        *reinterpret_cast<uint32_t *>(col + 256u * (cum - qlo)) = table_entry(ent);
+        *reinterpret_cast<uint32_t *>(col + 256u * (cum - qlo)) = table_entry<kFloat>(ent);
         cum += ent >> 8;
     }
     __syncwarp();
@@ -609,6 +621,22 @@ struct Stream {
         update(u01, p01, u23, p23);
         return __byte_perm(__byte_perm(e[0], e[1], 0x0062), __byte_perm(e[2], e[3], 0x0062), 0x5410);
     }
+    // one step over the float consumers' table: the four entries, whose upper halves are the bf16 symbols
+    __device__ __forceinline__ void step_f(const unsigned char *sm, uint32_t lw, uint32_t (&e)[4]) {
+        step(sm, lw, e);
+        // entry bytes (f, r, bf16): r0 + f0 r1 = e0 . (r1, 1, 0, 0), f0 f1 = e0 . (f1, 0, 0, 0)
+        const uint32_t u01 = __dp4a(e[0], __byte_perm(e[1], 1u, 0x5541), 0u);
+        const uint32_t u23 = __dp4a(e[2], __byte_perm(e[3], 1u, 0x5541), 0u);
+        const uint32_t p01 = __dp4a(e[0], e[1] & 0xFFu, 0u), p23 = __dp4a(e[2], e[3] & 0xFFu, 0u);
+        update(u01, p01, u23, p23);
+    }
+    // the four symbols as two bf16 pairs
+    __device__ __forceinline__ void step_bf16(const unsigned char *sm, uint32_t lw, uint32_t &w01, uint32_t &w23) {
+        uint32_t e[4];
+        step_f(sm, lw, e);
+        w01 = __byte_perm(e[0], e[1], 0x7632);
+        w23 = __byte_perm(e[2], e[3], 0x7632);
+    }
 };
 
 // x is read with plain (coherent) loads: in a chain it was written earlier in the same launch.
@@ -618,7 +646,7 @@ __device__ __forceinline__ uint4 ldx_u4(const void *p) { return *reinterpret_cas
 // (exact integer atomics); the warp that counts the item's last part writes the outputs.
 template <int NV>
 struct DotCons {
-    static constexpr bool kMma = false;
+    static constexpr bool kMma = false, kFloat = false, kStatic = false;
     static constexpr int kRed = NV * 32;  // ints of an item's partial sums
     static constexpr int kMaxDecode = NV <= 2 ? 16 : NV <= 4 ? 14 : NV <= 8 ? 10 : 6;
     const int8_t *x;
@@ -682,7 +710,7 @@ struct DotCons {
         }
         if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
     }
-    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, unsigned char *sm, const Bars &B, int lane,
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool, unsigned char *sm, const Bars &B, int lane,
                                              volatile uint32_t *) {
         int *red = reinterpret_cast<int *>(sm + L.lay.red) + (size_t)(k % kRing) * NV * 32 + lane;
 #pragma unroll
@@ -722,7 +750,7 @@ struct DotCons {
 // alternate between two accumulators, the second in the 16 lanes of each quarter that M = 64 leaves free.
 template <bool kOwn>
 struct MmaCons {
-    static constexpr bool kMma = true;
+    static constexpr bool kMma = true, kFloat = false, kStatic = false;
     static constexpr int kPitch = 33;  // words per vector of the item's sums: lanes (vectors) hit distinct banks
     static constexpr int kRed = kOwn ? 16 * kPitch : 0;
     static constexpr int kMaxDecode = 16;
@@ -845,7 +873,7 @@ struct MmaCons {
         if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
     }
     // Counts the unit once its MMAs are complete, so that whoever sees the item's last unit counted may read the sums.
-    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, unsigned char *sm, const Bars &B, int lane,
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool, unsigned char *sm, const Bars &B, int lane,
                                              volatile uint32_t *failed) {
         if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
         if (kOwn && any) {
@@ -895,47 +923,329 @@ struct MmaCons {
             ItemState *st = reinterpret_cast<ItemState *>(sm + L.lay.cnt) + k % kRing;
             const uint32_t m0 = *reinterpret_cast<volatile uint32_t *>(&st->acc[0]);
             const uint32_t m1 = *reinterpret_cast<volatile uint32_t *>(&st->acc[1]);
-            int sum[32];
-#pragma unroll
-            for (int r = 0; r < 32; r++) sum[r] = 0;
             const bool active = 16 * q < L.batch;
-            for (uint32_t left = m0 | m1; left; left &= left - 1u) {
-                const int w = __ffs((int)left) - 1;
-                if (active) {
-                    uint32_t r[32];
-                    tmem_ld_32x32b_x32(tmem + 32u * (uint32_t)w + (((uint32_t)q * 32u) << 16), r);
-                    const bool mine = (lane < 16 ? m0 : m1) >> w & 1u;  // the accumulator's half of the quarter's lanes
+            if (active) {
+#pragma unroll 1
+                for (int h = 0; h < 32; h += 16) {  // 16 stripe rows at a time (registers)
+                    int sum[16];
 #pragma unroll
-                    for (int j = 0; j < 32; j++) sum[j] += mine ? (int)r[j] : 0;
-                    tcgen05_fence_before();
+                    for (int j = 0; j < 16; j++) sum[j] = 0;
+                    for (uint32_t left = m0 | m1; left; left &= left - 1u) {
+                        const int w = __ffs((int)left) - 1;
+                        uint32_t r[16];
+                        tmem_ld_32x32b_x16(tmem + 32u * (uint32_t)w + (uint32_t)h + (((uint32_t)q * 32u) << 16), r);
+                        const bool mine = (lane < 16 ? m0 : m1) >> w & 1u;  // the accumulator's half of the quarter's lanes
+#pragma unroll
+                        for (int j = 0; j < 16; j++) sum[j] += mine ? (int)r[j] : 0;
+                    }
+                    uint32_t base = 0;
+                    if (!m0) base = 16;  // every warp was at its second accumulator
+                    else if (m1)         // some at the first, some at the second: lane l + 16 to lane l
+#pragma unroll
+                        for (int j = 0; j < 16; j++) sum[j] += __shfl_down_sync(0xffffffffu, sum[j], 16);
+                    const int v = 16 * q + lane - (int)base, row0 = I.stripe * 32 + h;
+                    if ((uint32_t)lane >= base && (uint32_t)lane < base + 16u && v < L.batch) {
+                        if (!I.atomic && row0 + 16 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.y & 15) == 0) {
+                            int4 *dst = reinterpret_cast<int4 *>(I.y + (size_t)v * I.rows + row0);
+#pragma unroll
+                            for (int j = 0; j < 4; j++)
+                                dst[j] = make_int4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+                            if (I.ys)
+#pragma unroll
+                                for (int j = 0; j < 16; j++)
+                                    I.ys[(size_t)v * I.rows + row0 + j] = (float)sum[j] * __ldg(I.scales + row0 + j);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                if (row0 + j < I.rows) emit(I, v, row0 + j, sum[j]);
+                        }
+                    }
                 }
-                __syncwarp();
-                if (lane == 0) arrive(B.dempty(w, (int)(m1 >> w & 1u)));
+                tcgen05_fence_before();
             }
-            uint32_t base = 0;
-            if (!m0) base = 16;  // every warp was at its second accumulator
-            else if (m1)         // some at the first, some at the second: lane l + 16 to lane l
-#pragma unroll
-                for (int j = 0; j < 32; j++) sum[j] += __shfl_down_sync(0xffffffffu, sum[j], 16);
-            const int v = 16 * q + lane - (int)base, row0 = I.stripe * 32;
-            if (active && (uint32_t)lane >= base && (uint32_t)lane < base + 16u && v < L.batch) {
-                if (!I.atomic && row0 + 32 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.y & 15) == 0) {
-                    int4 *dst = reinterpret_cast<int4 *>(I.y + (size_t)v * I.rows + row0);
-#pragma unroll
-                    for (int j = 0; j < 8; j++) dst[j] = make_int4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
-                    if (I.ys)
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            I.ys[(size_t)v * I.rows + row0 + j] = (float)sum[j] * __ldg(I.scales + row0 + j);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (row0 + j < I.rows) emit(I, v, row0 + j, sum[j]);
+            __syncwarp();
+            if (lane == 0)
+                for (uint32_t left = m0 | m1; left; left &= left - 1u) {
+                    const int w = __ffs((int)left) - 1;
+                    arrive(B.dempty(w, (int)(m1 >> w & 1u)));
                 }
-            }
             table_vote(true);  // every warp has read the masks
             if (threadIdx.x == 0) st->acc[0] = st->acc[1] = 0;
         }
+    }
+};
+
+// Float forward on the tensor cores, up to 64 bf16 vectors: as MmaCons<false> with kind::f16, bf16 W and x (int8
+// weights are exact in bf16, every product is exact in fp32) and fp32 sums, 8 quads (32 columns, two K steps of 16) at
+// a time: W tile 2 KB, x tile 64 bytes per vector.  Unit u goes to warp u mod W, each warp's MMAs accumulate in order
+// and the warps' sums are added in unit order, so results are reproducible bit for bit.
+struct FwdCons {
+    static constexpr bool kMma = true, kFloat = true, kStatic = true;
+    static constexpr int kRed = 0;
+    static constexpr int kMaxDecode = 16;
+    static constexpr uint32_t kWTile = 2048;
+    static __host__ __device__ constexpr uint32_t tile_bytes(int xrows) { return kWTile + 64u * (uint32_t)xrows; }
+    const uint16_t *x;
+    int cols, seg_quads, qtot;
+    uint32_t wt, xt, d_tmem, lbo, nmma, ndp;
+    uint32_t mbar, dempty;
+    uint64_t a_desc, b_desc;
+    int warp;
+    bool any;
+    __device__ __forceinline__ void init(const Q8WLaunch &L, unsigned char *sm, const Bars &B, uint32_t tmem, int w) {
+        warp = w;
+        wt = smem_u32(sm) + L.lay.tiles + (uint32_t)w * tile_bytes(L.xrows);
+        xt = wt + kWTile;
+        lbo = 16u * (uint32_t)L.xrows;
+        d_tmem = tmem + 32u * (uint32_t)w;
+        a_desc = umma_smem_desc(xt, lbo, 128u);
+        b_desc = umma_smem_desc(wt, 512u, 128u);
+        mbar = B.mma(w);
+        dempty = B.dempty(w, 0);
+        nmma = ndp = 0;
+        any = false;
+    }
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I) {
+        x = reinterpret_cast<const uint16_t *>(I.x);
+        cols = I.cols;
+        seg_quads = I.seg_quads;
+        qtot = cols >> 2;
+    }
+    __device__ __forceinline__ void wait_acc(const Q8WLaunch &L, volatile uint32_t *failed) const {
+        if (ndp >= 2) wait_bar(dempty + 8u * (ndp & 1u), (ndp / 2u - 1u) & 1u, L, failed);
+    }
+    // the previous MMAs are done with both tiles: 32 columns from col on of every vector (see MmaCons::copy_x; columns
+    // past the segment are never multiplied)
+    __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, int lane, volatile uint32_t *failed) const {
+        if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
+        const int r = lane & 7, c = col + 8 * (lane >> 3);
+        const uint16_t *src = x + (size_t)r * cols + c;
+        uint32_t dst = xt + (uint32_t)(lane >> 3) * lbo + (uint32_t)r * 16u;
+        const int n = c < cols ? L.batch - r : 0;
+#pragma unroll 2
+        for (int v = 0; v < n; v += 8) {
+            cp_async_16(dst, src);
+            src += 8 * (size_t)cols;
+            dst += 128u;
+        }
+    }
+    __device__ __forceinline__ void issue(const Q8WLaunch &L, bool two, int lane, volatile uint32_t *failed) {
+        if (!any) wait_acc(L, failed);
+        cp_async_wait_all();
+        fence_proxy_async_smem();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            tcgen05_fence_after();
+            const uint32_t idesc = umma_idesc_bf16(64, 32, 0, 0);
+            const uint32_t d = d_tmem + ((ndp & 1u) << 20);
+            umma_f16_ss(d, a_desc, b_desc, idesc, any ? 1u : 0u);
+            if (two) umma_f16_ss(d, a_desc + (lbo >> 3), b_desc + 64u, idesc, 1u);
+            umma_commit(mbar);
+        }
+        __syncwarp();
+        any = true;
+        nmma++;
+    }
+    // two quads (8 columns) of the lane's row: piece c of the 32-column tile
+    __device__ __forceinline__ void two_quads(Stream &s, const unsigned char *sm, uint32_t lw, uint32_t (&w)[4]) const {
+        s.step_bf16(sm, lw, w[0], w[1]);
+        s.step_bf16(sm, lw, w[2], w[3]);
+    }
+    __device__ __forceinline__ void store_w(uint32_t c, const uint32_t (&w)[4], int lane) const {
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(wt + c * 512u + (uint32_t)lane * 16u), "r"(w[0]),
+                     "r"(w[1]), "r"(w[2]), "r"(w[3])
+                     : "memory");
+    }
+    __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
+                                         uint32_t lw, int lane, volatile uint32_t *failed) {
+        const int q0 = d.seg * seg_quads;
+        const int nq = min(seg_quads, qtot - q0);
+        Stream s(sm, soff, d.rows, lane);
+        uint32_t w[4];
+        int q = 0;
+        for (; q + 8 <= nq; q += 8) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                two_quads(s, sm, lw, w);
+                if (c == 0) refill_tiles(L, 4 * (q0 + q), lane, failed);
+                store_w((uint32_t)c, w, lane);
+                if (c & 1) s.clamp();
+            }
+            issue(L, true, lane, failed);
+        }
+        if (q < nq) {  // the segment's last 4 quads (segments are whole groups of 4: cols % 16 == 0)
+            two_quads(s, sm, lw, w);
+            refill_tiles(L, 4 * (q0 + q), lane, failed);
+            store_w(0, w, lane);
+            two_quads(s, sm, lw, w);
+            store_w(1, w, lane);
+            issue(L, false, lane, failed);
+        }
+        if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
+    }
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool last, unsigned char *sm, const Bars &B,
+                                             int lane, volatile uint32_t *failed) {
+        if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            ItemState *st = reinterpret_cast<ItemState *>(sm + L.lay.cnt) + k % kRing;
+            if (any) atomicOr(&st->acc[ndp & 1u], 1u << warp);
+            arrive(B.tdone(k % kRing));
+        }
+        __syncwarp();
+        if (last) {  // the sums stay where they are until the table warps have read them
+            if (any) ndp++;
+            any = false;
+        }
+    }
+    __device__ __forceinline__ void drain(const Q8WLaunch &L) {
+        cp_async_wait_all();
+        if (nmma)
+            for (uint32_t it = 0; it < L.spin_limit; it++)
+                if (mbar_try_wait(mbar, (nmma - 1) & 1u)) break;
+    }
+    // Table warps: y = s . sums, the warps' sums added in the order of their first units.
+    static __device__ __forceinline__ void epilogue(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm,
+                                                    const Bars &B, uint32_t tmem) {
+        const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        tcgen05_fence_after();
+        ItemState *st = reinterpret_cast<ItemState *>(sm + L.lay.cnt) + k % kRing;
+        const uint32_t m0 = *reinterpret_cast<volatile uint32_t *>(&st->acc[0]);
+        const uint32_t m1 = *reinterpret_cast<volatile uint32_t *>(&st->acc[1]);
+        const bool active = 16 * q < L.batch;
+        const uint32_t W = (uint32_t)L.W, nc = min(I.n, W), first = I.u0 % W;
+        const int v = 16 * q + lane;
+        if (active) {
+#pragma unroll 1
+            for (int h = 0; h < 32; h += 16) {  // 16 stripe rows at a time (registers)
+                float sum[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) sum[j] = 0.f;
+                uint32_t w = first;
+                for (uint32_t i = 0; i < nc; i++, w = w + 1 < W ? w + 1 : 0) {
+                    if (!((m0 | m1) >> w & 1u)) continue;
+                    uint32_t r[16];
+                    tmem_ld_32x32b_x16(tmem + 32u * w + (uint32_t)h + (((uint32_t)q * 32u) << 16), r);
+                    if (m1 >> w & 1u) {  // the second accumulator's sums are 16 lanes further
+#pragma unroll
+                        for (int j = 0; j < 16; j++) r[j] = __shfl_down_sync(0xffffffffu, r[j], 16);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; j++) sum[j] += __uint_as_float(r[j]);
+                }
+                const int row0 = I.stripe * 32 + h;
+                if (lane < 16 && v < L.batch) {
+                    float *dst = I.ys + (size_t)v * I.rows + row0;
+                    if (row0 + 16 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.ys & 15) == 0) {
+#pragma unroll
+                        for (int j = 0; j < 16; j += 4)
+                            *reinterpret_cast<float4 *>(dst + j) = make_float4(
+                                sum[j] * __ldg(I.scales + row0 + j), sum[j + 1] * __ldg(I.scales + row0 + j + 1),
+                                sum[j + 2] * __ldg(I.scales + row0 + j + 2), sum[j + 3] * __ldg(I.scales + row0 + j + 3));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (row0 + j < I.rows) dst[j] = sum[j] * __ldg(I.scales + row0 + j);
+                    }
+                }
+            }
+            tcgen05_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0)
+            for (uint32_t left = m0 | m1; left; left &= left - 1u) {
+                const int w = __ffs((int)left) - 1;
+                arrive(B.dempty(w, (int)(m1 >> w & 1u)));
+            }
+        table_vote(true);  // every warp has read the masks
+        if (threadIdx.x == 0) st->acc[0] = st->acc[1] = 0;
+    }
+};
+
+// Float forward of one bf16 vector on the CUDA cores: fp32 multiply-adds of the table's bf16 symbols, x behind the
+// block in the slot (or read ahead from global memory when the segment is longer than kXQuads).  Unit u goes to warp
+// u mod W, each warp adds its units of an item in order, and the warps' sums are added in the order of their first
+// units: reproducible bit for bit.  (4096x11008: 40 us through the MMAs of FwdCons, whose tiles cost more than one
+// vector's products.)
+struct FwdDot {
+    static constexpr bool kMma = false, kFloat = true, kStatic = true;
+    static constexpr int kMaxDecode = 16;
+    static constexpr int kRed = kMaxDecode * 32;
+    const uint16_t *x;
+    int seg_quads, qtot, warp;
+    bool in_slot;
+    float acc;
+    __device__ __forceinline__ void init(const Q8WLaunch &, unsigned char *, const Bars &, uint32_t, int w) {
+        warp = w;
+        acc = 0.f;
+    }
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I) {
+        in_slot = x_in_slot(L, I.seg_quads);
+        x = reinterpret_cast<const uint16_t *>(I.x);
+        seg_quads = I.seg_quads;
+        qtot = I.cols >> 2;
+    }
+    // one quad: x as two bf16 pairs
+    __device__ __forceinline__ void quad(Stream &s, const unsigned char *sm, uint32_t lw, uint32_t x01, uint32_t x23) {
+        uint32_t e[4];
+        s.step_f(sm, lw, e);
+        acc = fmaf(__uint_as_float(e[0] & 0xFFFF0000u), __uint_as_float(x01 << 16), acc);
+        acc = fmaf(__uint_as_float(e[1] & 0xFFFF0000u), __uint_as_float(x01 & 0xFFFF0000u), acc);
+        acc = fmaf(__uint_as_float(e[2] & 0xFFFF0000u), __uint_as_float(x23 << 16), acc);
+        acc = fmaf(__uint_as_float(e[3] & 0xFFFF0000u), __uint_as_float(x23 & 0xFFFF0000u), acc);
+    }
+    __device__ __forceinline__ void group(Stream &s, const unsigned char *sm, uint32_t lw, const uint4 &a, const uint4 &b) {
+        quad(s, sm, lw, a.x, a.y);
+        quad(s, sm, lw, a.z, a.w);
+        quad(s, sm, lw, b.x, b.y);
+        quad(s, sm, lw, b.z, b.w);
+        s.clamp();
+    }
+    __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
+                                         uint32_t lw, int lane, volatile uint32_t *) {
+        const int q0 = d.seg * seg_quads;
+        const int nq = min(seg_quads, qtot - q0);
+        Stream s(sm, soff, d.rows, lane);
+        if (in_slot) {
+            const unsigned char *xs = sm + soff + L.x_off;
+#pragma unroll 2
+            for (int i = 0; i < nq; i += 4, xs += 32)
+                group(s, sm, lw, *reinterpret_cast<const uint4 *>(xs), *reinterpret_cast<const uint4 *>(xs + 16));
+        } else {
+            const uint4 *xp = reinterpret_cast<const uint4 *>(x + 4 * q0);
+            uint4 a = __ldg(xp), b = __ldg(xp + 1);
+            for (int i = 0; i < nq; i += 4) {
+                xp += i + 4 < nq ? 2 : 0;
+                const uint4 a1 = __ldg(xp), b1 = __ldg(xp + 1);
+                group(s, sm, lw, a, b);
+                a = a1;
+                b = b1;
+            }
+        }
+        if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
+    }
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool last, unsigned char *sm, const Bars &B,
+                                             int lane, volatile uint32_t *) {
+        if (last) {
+            reinterpret_cast<float *>(sm + L.lay.red)[(k % kRing) * kRed + warp * 32 + lane] = acc;
+            acc = 0.f;
+        }
+        __syncwarp();
+        if (lane == 0) arrive(B.tdone(k % kRing));
+    }
+    __device__ __forceinline__ void drain(const Q8WLaunch &) {}
+    static __device__ __forceinline__ void epilogue(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm,
+                                                    const Bars &, uint32_t) {
+        const int lane = threadIdx.x & 31, row = I.stripe * 32 + lane;
+        if (threadIdx.x >= 32) return;
+        const volatile float *red = reinterpret_cast<const volatile float *>(sm + L.lay.red) + (k % kRing) * kRed + lane;
+        const uint32_t W = (uint32_t)L.W, nc = min(I.n, W);
+        uint32_t w = I.u0 % W;
+        float sum = 0.f;
+        for (uint32_t i = 0; i < nc; i++, w = w + 1 < W ? w + 1 : 0) sum += red[w * 32];
+        if (row < I.rows) I.ys[row] = sum * __ldg(I.scales + row);
     }
 };
 
@@ -981,7 +1291,7 @@ __device__ __forceinline__ void serve_tables(const Q8WLaunch &L, unsigned char *
             const uint32_t *so = reinterpret_cast<const uint32_t *>(sm + L.lay.stage_o) + area * kStageOffs;
             const uint16_t *se = reinterpret_cast<const uint16_t *>(
                 sm + L.lay.stage_e + (uint32_t)area * ((uint32_t)L.tbl_stage + kStagePad) * 2u);
-            build_table(L, I.local, sm + 128 * I.tab, so, se + so[37]);
+            build_table<Cons::kFloat>(L, I.local, sm + 128 * I.tab, so, se + so[37]);
         }
         if (L.chain_scales && I.job > 0) {
             for (; done < k; done++)
@@ -1009,11 +1319,12 @@ __device__ __forceinline__ void decode_units(const Q8WLaunch &L, unsigned char *
     uint32_t *unext = reinterpret_cast<uint32_t *>(sm + L.lay.misc) + 2;
     const uint32_t S = (uint32_t)L.S;
     int cur = -1;
-    uint32_t lw = 0, taken = 0;
-    if (lane == 0) taken = atomicAdd(unext, 1u);
+    uint32_t lw = 0, taken = (uint32_t)w, last = 0;
+    if (!Cons::kStatic && lane == 0) taken = atomicAdd(unext, 1u);
     for (;;) {
-        // units are taken as the warps get to them: their pace differs with the other warps of their scheduler
-        const uint32_t u = __shfl_sync(0xffffffffu, taken, 0);
+        // Units are taken as the warps get to them (their pace differs with the other warps of their scheduler), but
+        // for sums whose order counts: there unit u goes to warp u mod W.
+        const uint32_t u = Cons::kStatic ? taken : __shfl_sync(0xffffffffu, taken, 0);
         const uint32_t turn = S == 1u ? u : __umulhi(u, L.S_inv), slot = u - turn * S, ph = turn & 1u;
         // A slot passes from warp to warp, so its barrier may still be a phase behind, where the parity test would
         // pass too early: the unit number in the slot tells, and the copy is waited for again once it is right.
@@ -1030,13 +1341,15 @@ __device__ __forceinline__ void decode_units(const Q8WLaunch &L, unsigned char *
             if (!__all_sync(0xffffffffu, wait_bar(B.tfull(cur % kRing), (uint32_t)(cur / kRing) & 1u, L, failed))) break;
             const ItemRec &I = ring[cur % kRing];
             cons.begin_item(L, I);
+            last = I.u0 + I.n;
             lw = (uint32_t)lane * 4u | (uint32_t)I.tab << 7;
         }
         if (d.rows) cons.unit(L, d, sm, L.lay.slots + slot * L.slot_bytes, lw, lane, failed);
-        if (lane == 0) taken = atomicAdd(unext, 1u);  // (its latency passes while this unit is closed)
+        if (Cons::kStatic) taken += (uint32_t)L.W;
+        else if (lane == 0) taken = atomicAdd(unext, 1u);  // (its latency passes while this unit is closed)
         __syncwarp();
         if (lane == 0) arrive(B.sempty((int)slot));
-        cons.end_unit(L, cur, sm, B, lane, failed);
+        cons.end_unit(L, cur, u + (uint32_t)L.W >= last, sm, B, lane, failed);
     }
     cons.drain(L);
 }
@@ -1127,7 +1440,8 @@ mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
     L.block_bytes = L.slot_bytes;
     if (!Cons::kMma && !L.chain_scales) {
         L.x_off = L.slot_bytes;
-        L.slot_bytes += (uint32_t)(4 * L.batch * kXQuads);
+        L.x_quad = Cons::kFloat ? 8u : 4u;
+        L.slot_bytes += L.x_quad * (uint32_t)(L.batch * kXQuads);
     }
     // Decode warps: as many as asked for (or the consumer's most), no more than a CTA has units for.  The slots
     // beyond one per warp hold the units that the warps take next: without any, a warp would wait for its copy
@@ -1182,6 +1496,13 @@ mv_status q8w_launch_int(const Q8WLaunch &L0, int nv, bool mma, int warps, int u
         case 8: return launch_t<DotCons<8>>(L, warps, units, st);
         default: return launch_t<DotCons<16>>(L, warps, units, st);
     }
+}
+
+mv_status q8w_launch_fwd(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
+    Q8WLaunch L = L0;
+    L.xrows = (L.batch + 7) & ~7;
+    if (L.batch == 1) return launch_t<FwdDot>(L, warps, units, st);
+    return launch_t<FwdCons>(L, warps, units, st);
 }
 
 }  // namespace mv

@@ -33,6 +33,7 @@ struct Q8WLaunch {
     uint32_t S_inv;        // ceil(2^32 / S): unit / S by multiplication
     uint32_t block_bytes;  // of a slot, its block's part
     uint32_t x_off;        // where a slot holds its segment's x (0: nowhere)
+    uint32_t x_quad;       // bytes of a quad of x
     int xrows;  // MMA consumers: rows of the x tile (batch rounded up to 8)
     Q8WLayout lay;
 };
@@ -40,5 +41,7 @@ struct Q8WLaunch {
 // Integer product of L.batch vectors: on the tensor cores (up to 64 vectors) or, with dp4a, nv >= batch vectors
 // (1, 2, 4, 8 or 16).  warps: decode warps per CTA (0: as many as fit); units: the most units a CTA can get.
 mv_status q8w_launch_int(const Q8WLaunch &L, int nv, bool mma, int warps, int units, cudaStream_t st);
+// Float forward of up to 64 vectors (on the tensor cores from 2): job0.x is bf16 [batch][cols], job0.ys fp32 [batch][rows].
+mv_status q8w_launch_fwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st);
 
 }  // namespace mv

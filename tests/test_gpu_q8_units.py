@@ -49,3 +49,24 @@ def test_stack_of_uneven_items_runs_repeatedly(B):
         for W, xd, y in zip(Ws, S.xs, S.ys):
             assert np.array_equal(y.cpu().numpy(), oracle.matvec_i8(W, xd.cpu().numpy())), W.shape
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads,local", [
+    (33, 16, 0, True), (257, 1040, 4, False), (96, 2048, 68, True), (1500, 272, 12, True), (64, 8192, 128, False)])
+def test_float_forward_units(rows, cols, seg_quads, local):
+    # one vector (CUDA cores), the 16-vector lane groups and the 64-vector pass: fp32 sums against 64 bits, relative to
+    # the sum of the magnitudes of a row's terms (a sum of n fp32 terms in any order is within n ulps of it; here a
+    # warp's chain is at most cols / 16 accumulations and the warps' sums are added once), and bit for bit the same twice
+    rng = np.random.default_rng(rows + cols + seg_quads)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, local=local, seg_quads=seg_quads)
+    s = torch.from_numpy(rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)).cuda()
+    W64 = torch.from_numpy(W).cuda().double()
+    for B in (1, 2, 16, 17, 49, 64, 65):
+        x = torch.from_numpy(rng.standard_normal((B, cols)).astype(np.float32)).cuda().to(torch.bfloat16)
+        y = M.matvec_bf16(x, s)
+        ref = (x.double() @ W64.T) * s.double()
+        mag = (x.double().abs() @ W64.abs().T) * s.double()
+        assert ((y.double() - ref).abs() / mag.clamp_min(1e-30)).max().item() < 2.0 ** -24 * (cols / 16 + 20), B
+        assert torch.equal(y, M.matvec_bf16(x, s)), B
+    assert ops.device_status() == 0
