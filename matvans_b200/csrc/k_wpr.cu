@@ -5,12 +5,23 @@
 // own 16-bit word stream (word k at payload[cursor + (k/8)*256 + 8l + k%8],
 // create_matrices_WarpPerRow.py:405-420).  Decode step: q = head & 0xFF,
 // r = ppf[q], w = min + r, head = (head >> 8) * prob(r) + (q - cdf[r]), refill
-// 16 bits when head < 2^16 (kernel.cu:120-157).  B200 changes: the reference's
-// per-lane 16-entry ring queue in local memory (kernel.cu:3-44) becomes one
-// prefetched register word, refilled by selects (no divergent branch);
-// cdf/ppf become one 256 x 32-lane conflict-free shared table of packed
-// (symbol, prob, q - cdf) entries; four decoded symbols go through one dp4a
-// instead of four scalar multiplies; any number of vectors share a decode.
+// 16 bits when head < 2^16 (kernel.cu:120-157).
+//
+// What bounds it: issue.  A step (one symbol per lane) takes ~13 instructions
+// against 34 in the form this replaced, whose refill recomputed a global word
+// index, checked it and reloaded a word at every symbol:
+//   * the lane's stream passes through a ring of its own in shared memory, word k
+//     at byte 64 k + 2 lane, filled 8 words (one 16-byte load, requested a chunk
+//     ahead) at a time between groups of 16 symbols, so that a refill is a merge,
+//     a 16-bit load and an add, all predicated; bounds are checked per chunk, and
+//     an overrun once per row from the number of words taken;
+//   * decode table: one 4-byte entry {prob, 0, symbol, q - cdf} per (quantile,
+//     lane) at byte q*256 + lane*4, one byte permute per address;
+//   * one CTA per SM with as many warps (up to 28) as spread the rows evenly over
+//     the SMs: 4096 rows are 28 warps on each, all in one round.
+// Measured on a B200, 4096x4096, one vector, the kernel alone: 35.1 us before,
+// 20.7 us with the ring and the packed entries.
+// Four decoded symbols go through one dp4a; any number of vectors share a decode.
 #include <algorithm>
 
 #include "mv_device.cuh"
@@ -34,106 +45,126 @@ struct WprLaunch {
     uint32_t *status;
 };
 
+constexpr uint32_t kRingBytes = 32 * 64;               // 32 words of 32 lanes
+constexpr uint32_t kRingAlloc = kRingBytes + 16 * 64;  // the first 16 words again behind the ring: a group of 16
+                                                       // symbols runs past its end without wrapping
 template <int NV>
-__global__ void __launch_bounds__(256) wpr_kernel(const WprLaunch L) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t *lut = reinterpret_cast<uint32_t *>(smem);  // 256 * 32 words
-    uint8_t *xs = reinterpret_cast<uint8_t *>(lut + 256 * 32);  // [NV][cols]
+constexpr int kWprWarps = NV <= 4 ? 28 : NV <= 8 ? 16 : 12;
+
+// Words [ix, ix + 8) of the payload; zeros past its end.
+__device__ __forceinline__ uint4 wpr_chunk(const WprLaunch &L, uint64_t ix) {
+    if (ix + 8 <= L.payload_size && (ix & 7) == 0) return __ldg(reinterpret_cast<const uint4 *>(L.payload + ix));
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint64_t i = ix + 2 * j;
+        w[j] = (i < L.payload_size ? (uint32_t)__ldg(L.payload + i) : 0u) |
+               (i + 1 < L.payload_size ? (uint32_t)__ldg(L.payload + i + 1) << 16 : 0u);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <int NV>
+__global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch L) {
+    extern __shared__ __align__(1024) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
 
-    // one entry per quantile (its three table reads once), written to all 32 lane columns with a rotating
-    // column index so that a warp's stores hit 32 different banks
-    for (uint32_t q = threadIdx.x; q < 256; q += blockDim.x) {
-        const uint32_t r = __ldg(L.ppf + q);
+    // decode table: eight threads per quantile, four lane columns each
+    for (uint32_t i = threadIdx.x; i < 256 * 8; i += blockDim.x) {
+        const uint32_t q = i >> 3, r = __ldg(L.ppf + q);
         uint32_t e = 0;
         if ((int)r + 1 > L.G) {
             atomicOr(L.status, MV_DEV_BAD_TABLE);
         } else {
             const uint32_t c0 = __ldg(L.cdf + r), c1 = __ldg(L.cdf + r + 1);
-            const uint32_t prob = (c1 - c0) & 0xFF;
-            const uint32_t bias = q - c0;  // never negative for a valid table
-            if (c0 > q) atomicOr(L.status, MV_DEV_BAD_TABLE);
-            e = (uint32_t)(uint8_t)(int8_t)(L.min_value + (int)r) | (prob << 8) | ((bias & 0xFFFF) << 16);
+            if (c0 > q) atomicOr(L.status, MV_DEV_BAD_TABLE);  // (q - c0 is never negative for a valid table)
+            e = ((c1 - c0) & 0xFFu) | (uint32_t)(uint8_t)(int8_t)(L.min_value + (int)r) << 16 | (q - c0) << 24;
         }
-#pragma unroll 8
-        for (uint32_t l = 0; l < 32; l++) lut[q * 32 + ((l + q) & 31)] = e;
-    }
-    for (int i = threadIdx.x; i < NV * L.cols / 16; i += blockDim.x) {
-        const int v = i / (L.cols / 16);
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (v < L.batch) val = reinterpret_cast<const uint4 *>(L.x)[i];
-        reinterpret_cast<uint4 *>(xs)[i] = val;
+        const uint4 e4 = make_uint4(e, e, e, e);
+        uint4 *dst = reinterpret_cast<uint4 *>(smem + 256u * q + 16u * (i & 7u));
+        *dst = e4;
     }
     __syncthreads();
 
-    const uint32_t *lut_l = lut + lane;
-    const int steps = L.cols / 32;
-    const uint32_t size = (uint32_t)L.payload_size;  // < 0xF0000000 (checked by the launcher)
+    const uint32_t lane4 = (uint32_t)lane * 4u;
+    const uint32_t ring = smem_u32(smem) + 65536u + (uint32_t)warp * kRingAlloc + (uint32_t)lane * 2u;
+    const int groups = L.cols / 512;
     for (int row = blockIdx.x * W + warp; row < L.rows; row += gridDim.x * W) {
-        // The lane's word k sits at ix = cursor + (k / 8) * 256 + 8 * lane + k % 8: ix advances by 1 inside a
-        // group of 8 words and by 249 from one group to the next.  Reads past the payload return 0 and are
-        // flagged (a cursor past the payload starts the lane at its end; ix then grows by at most 249 per
-        // symbol, far below 2^32 from a payload under 0xF0000000 words).  Two words are in flight ahead of
-        // the state, so a fetch's latency is covered by the symbols of two refills; the refill itself is
-        // selects, not a branch, because the lanes refill at different steps.
         const uint64_t ix0 = (uint64_t)__ldg(L.cursors + row) + 8u * (uint32_t)lane;
-        uint32_t ix = ix0 < size ? (uint32_t)ix0 : size;
-        bool ovf = (uint64_t)ix + 2u > size;
-        const uint32_t w0 = ix < size ? (uint32_t)__ldg(L.payload + ix) : 0u;
-        const uint32_t w1 = ix + 1u < size ? (uint32_t)__ldg(L.payload + ix + 1u) : 0u;
-        uint32_t head = (w0 << 16) | w1;
-        // two words in flight: nw (word k) and nw2 (word k + 1, at ix)
-        ix += 2u;
-        bool nw_oob = ix >= size;
-        uint32_t nw = nw_oob ? 0u : (uint32_t)__ldg(L.payload + ix);
-        ix += 1u;
-        uint32_t j = 3;  // ix's position inside its group of 8
-        bool nw2_oob = ix >= size;
-        uint32_t nw2 = nw2_oob ? 0u : (uint32_t)__ldg(L.payload + ix);
+        uint32_t staged = 0;  // words in the ring so far; the chunk behind them is in `nxt`
+        uint4 nxt = wpr_chunk(L, ix0);
+        const uint4 c0 = nxt;
+        auto stage = [&]() {
+            const uint32_t s = staged & 31u, d = ring + s * 64u;
+            const uint32_t w[4] = {nxt.x, nxt.y, nxt.z, nxt.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint16_t lo = (uint16_t)w[j], hi = (uint16_t)(w[j] >> 16);
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(d + 128u * j), "h"(lo) : "memory");
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(d + 128u * j + 64u), "h"(hi) : "memory");
+                if (s < 16u) {
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(d + 128u * j + kRingBytes), "h"(lo) : "memory");
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(d + 128u * j + 64u + kRingBytes), "h"(hi) : "memory");
+                }
+            }
+            staged += 8u;
+            nxt = wpr_chunk(L, ix0 + 32ull * staged);  // 256 words a chunk of 8
+        };
+        stage();
+        stage();
+        stage();
+        // head from words 0 and 1; nw is the next word, a the place of the one after it
+        uint32_t head = __byte_perm(c0.x, 0u, 0x1032), nw = c0.y & 0xFFFFu, a = ring + 3u * 64u;
+        uint32_t left = staged - 3u;  // staged words from a on
         int acc[NV];
 #pragma unroll
         for (int v = 0; v < NV; v++) acc[v] = 0;
-        for (int j0 = 0; j0 < steps; j0 += 16) {
-            const int colbase = 512 * (j0 >> 4) + 16 * lane;
+        const int8_t *xp = L.x + 16 * lane;
+        for (int g = 0; g < groups; g++, xp += 512) {
             uint4 xv[NV];
 #pragma unroll
-            for (int v = 0; v < NV; v++) xv[v] = *reinterpret_cast<const uint4 *>(xs + (size_t)v * L.cols + colbase);
+            for (int v = 0; v < NV; v++)
+                xv[v] = v < L.batch ? __ldg(reinterpret_cast<const uint4 *>(xp + (size_t)v * L.cols)) : make_uint4(0, 0, 0, 0);
+            const uint32_t a0 = a;
 #pragma unroll
-            for (int g = 0; g < 4; g++) {
+            for (int k = 0; k < 4; k++) {
                 uint32_t e[4];
 #pragma unroll
                 for (int t = 0; t < 4; t++) {
-                    e[t] = lut_l[(head & 0xFFu) << 5];
-                    head = (head >> 8) * __byte_perm(e[t], 0, 0x4441) + (e[t] >> 16);
-                    const bool need = head < (1u << 16);
-                    head = need ? __byte_perm(nw, head, 0x5410) : head;  // (head << 16) | nw
-                    ovf |= need & nw_oob;
-                    // every lane reloads nw2 each symbol, the same word again when it did not refill (an L1
-                    // hit): a conditional reload measured 16% more instructions and 9% more time
-                    nw = need ? nw2 : nw;
-                    nw_oob = need ? nw2_oob : nw_oob;
-                    ix += need ? (j == 7u ? 249u : 1u) : 0u;
-                    j = (j + (need ? 1u : 0u)) & 7u;
-                    nw2_oob = ix >= size;
-                    nw2 = nw2_oob ? 0u : (uint32_t)__ldg(L.payload + ix);
+                    e[t] = *reinterpret_cast<const uint32_t *>(smem + __byte_perm(head, lane4, 0x7604));
+                    // entry bytes (prob, 0, symbol, bias): two of them by dot products, off the permutes' pipe
+                    head = (head >> 8) * (e[t] & 0xFFu) + __dp4a(e[t], 0x01000000u, 0u);
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t.reg .u16 h;\n\t"
+                        "setp.lo.u32 p, %0, 0x10000;\n\t"
+                        "@p prmt.b32 %0, %1, %0, 0x5410;\n\t"  // (head << 16) | nw
+                        "@p ld.shared.u16 %1, [%2];\n\t"
+                        "@p add.u32 %2, %2, 64;\n\t}"
+                        : "+r"(head), "+r"(nw), "+r"(a)::"memory");
                 }
-                // the four symbols (byte 0 of each entry) packed in column order
-                const uint32_t wq = __byte_perm(__byte_perm(e[0], e[1], 0x0040), __byte_perm(e[2], e[3], 0x0040), 0x5410);
+                const uint32_t wq = __byte_perm(__byte_perm(e[0], e[1], 0x0062), __byte_perm(e[2], e[3], 0x0062), 0x5410);
 #pragma unroll
                 for (int v = 0; v < NV; v++) {
-                    const uint32_t xw = g == 0 ? xv[v].x : g == 1 ? xv[v].y : g == 2 ? xv[v].z : xv[v].w;
+                    const uint32_t xw = k == 0 ? xv[v].x : k == 1 ? xv[v].y : k == 2 ? xv[v].z : xv[v].w;
                     acc[v] = __dp4a((int)wq, (int)xw, acc[v]);
+                }
+            }
+            // a group takes at most 16 words; with 18 left the next one cannot run dry
+            left -= (a - a0) >> 6;
+            if (a - ring >= kRingBytes) a -= kRingBytes;
+            if (__any_sync(0xffffffffu, left < 18u)) {
+                if (left < 18u) stage(), left += 8u;
+                if (__any_sync(0xffffffffu, left < 18u)) {
+                    if (left < 18u) stage(), left += 8u;
                 }
             }
         }
         // the coder ends in its initial head 1 << 16 (create_matrices_WarpPerRow.py:271,372)
         if (head != (1u << 16)) atomicOr(L.status, MV_DEV_FINAL_STATE);
-        if (ovf) atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
+        const uint32_t k = staged - left - 2u;  // the last word taken into the head
+        if (ix0 + 256ull * (k >> 3) + (k & 7u) >= L.payload_size) atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
-        }
+        for (int v = 0; v < NV; v++) acc[v] = __reduce_add_sync(0xffffffffu, acc[v]);
         if (lane == 0) {
 #pragma unroll
             for (int v = 0; v < NV; v++)
@@ -170,15 +201,17 @@ namespace {
 
 template <int NV>
 mv_status launch_wpr(const WprLaunch &L, cudaStream_t st) {
-    const int W = 8;
-    const size_t smem = 256 * 32 * 4 + (size_t)NV * L.cols;
-    if (smem > (size_t)max_smem_optin())
+    // (the limit of the form that kept x in shared memory)
+    if (256 * 32 * 4 + (size_t)NV * L.cols > (size_t)max_smem_optin())
         return fail(MV_ERR_UNSUPPORTED, "WPR: %d columns x %d vectors exceed shared memory", L.cols, NV);
+    // rows in even rounds over the SMs
+    const int sms = sm_count(), rounds = (L.rows + sms * kWprWarps<NV> - 1) / (sms * kWprWarps<NV>);
+    const int W = std::max(1, (L.rows + sms * rounds - 1) / (sms * rounds));
+    const size_t smem = 65536 + (size_t)W * kRingAlloc;
     auto kern = wpr_kernel<NV>;
-    int bps = 0;
-    mv_status rc = prepare_kernel((const void *)kern, smem, 32 * W, &bps);
+    mv_status rc = prepare_kernel((const void *)kern, smem, 32 * W, nullptr);
     if (rc) return rc;
-    const int grid = std::max(1, std::min((L.rows + W - 1) / W, std::max(1, bps) * sm_count()));
+    const int grid = std::max(1, std::min((L.rows + W - 1) / W, sms));
     kern<<<grid, 32 * W, smem, st>>>(L);
     MV_CUDA_TRY(cudaGetLastError(), "wpr kernel launch");
     return MV_OK;

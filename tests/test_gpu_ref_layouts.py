@@ -1,0 +1,52 @@
+"""The reference's three stream layouts at the sizes where the kernels' rings, rounds and groups change: one row or
+stripe, more rows than a round of warps, the shortest rows, the densest streams (every refill word of the format's
+worst case), streams that start off the 16-byte grid.  Bit-exact against the CPU oracle's matvec."""
+import numpy as np
+import pytest
+
+from conftest import cuda_ok
+import oracle
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not cuda_ok(), reason="needs a CUDA device")]
+
+if cuda_ok():
+    import torch
+    from matvans_b200 import codec, ops
+
+
+def weights(rng, kind, shape):
+    if kind == "dense":  # nearly uniform: the most words a symbol
+        return rng.integers(-60, 61, size=shape).astype(np.int8)
+    if kind == "tails":  # lanes whose streams run at very different rates
+        W = np.zeros(shape, np.int8)
+        W[:, ::3] = rng.integers(-60, 61, size=W[:, ::3].shape)
+        return W
+    return np.clip(np.round(rng.normal(0, 3.0, size=shape)), -60, 60).astype(np.int8)
+
+
+def check(M, W, rng, batches):
+    for B in batches:
+        x = rng.integers(-128, 128, size=(B, W.shape[1])).astype(np.int8)
+        s = rng.uniform(1e-3, 1e-2, size=W.shape[0]).astype(np.float32)
+        y, ys = M.matvec(torch.from_numpy(x), scales=s)
+        ref = oracle.matvec_i8(W, x)
+        assert np.array_equal(y.cpu().numpy(), ref), B
+        assert np.array_equal(ys.cpu().numpy(), (ref.astype(np.float32) * s[None, :]).astype(np.float32)), B
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["gauss", "dense", "tails"])
+@pytest.mark.parametrize("rows,cols", [(1, 512), (150, 1536), (4200, 512)])
+def test_wpr(kind, rows, cols):
+    rng = np.random.default_rng(rows + cols)
+    W = weights(rng, kind, (rows, cols))
+    check(ops.WprMatrix.encode(W), W, rng, (1, 3, 9, 17))
+
+
+def test_wpr_stream_off_the_grid():
+    rng = np.random.default_rng(3)
+    W = weights(rng, "gauss", (70, 1024))
+    cm = codec.encode_matrix(W)
+    cm.payload = np.concatenate([np.full(3, 0xABCD, np.uint16), cm.payload])
+    cm.cursors = cm.cursors + np.uint32(3)
+    check(ops.WprMatrix(cm), W, rng, (1, 4))
