@@ -8,22 +8,35 @@
 // see ans-warp-rows-kernel.cu:76-139.  That consumption order is part of the
 // format, so this kernel keeps one warp per row and reproduces it exactly.
 // What changes on B200:
-//   * the three 32-entry packed tables are expanded once per CTA into a
-//     128-quantile x 32-lane shared table of 8-byte entries {p | sym << 16,
-//     q - cum} at byte q*256 + l*8, so the four lookups of a quad are four
-//     conflict-free loads instead of twelve warp shuffles
-//     (ans-warp-rows-kernel.cu:147-189), each address is one shift and one
-//     three-input logic op of the state, and q - cum arrives as a clean word;
+//   * the word stream of a row passes through a ring in shared memory, in
+//     consumption order, filled a 128-word block (one 16-byte load per lane) at a
+//     time and requested a block ahead when the stream's length is known; a lane's
+//     word is then one load at cursor + prefix popcount.  (A block is taken only
+//     when a lane actually consumes one of its words: with an unknown length
+//     nothing past the row's words is read.  The reference also reloads when the
+//     cursor lands exactly on a block boundary, which can read past the row.)
+//   * the three 32-entry packed tables become one 4-byte entry {p, 0, symbol,
+//     q - cum} per (quantile, lane) at byte q*128 + lane*4: four conflict-free
+//     loads per quad instead of twelve warp shuffles
+//     (ans-warp-rows-kernel.cu:147-189);
 //   * the state update forms the reference's r0 + p0 r1 + p0p1 r2 + p0p1p2 r3
 //     (ans-warp-rows-kernel.cu:198-202) as (r0 + p0 r1) + (p0 p1)(r2 + p2 r3)
-//     with 16x8-bit dot products: the same integer, fewer instructions;
-//   * the warp cache advances lazily: a block is loaded only when a lane
-//     actually consumes one of its words (the reference also reloads when the
-//     cursor lands exactly on a block boundary, which can read past the row);
-//   * when the stream length is known, the next block is prefetched one block
-//     ahead and every load is bounds-checked;
-//   * any number of vectors per pass (1..16) share one decode, x is staged
-//     once per CTA, and the int32 result is exact (requantisation optional).
+//     with byte dot products: the same integer, fewer instructions;
+//   * one CTA per SM, with as many warps (up to 28) as spread the rows evenly, so
+//     that the table is built and x staged once per SM;
+//   * any number of vectors per pass (1..16) share one decode, and the int32
+//     result is exact (requantisation optional).
+// What bounds it: issue, ~45 instructions a step (98 in the form this replaced,
+// which kept the words in registers and moved them by shuffles).  Measured on a
+// B200, 4096x4096, one vector, the kernel alone: 17.6 us before, 11.5 us now.
+//
+// The "ans-warp-stripes" layout (ans-warp-stripes-kernel.cu:21-227, encoder.py:
+// 323-391) has the same coder and word stream with lane = row of a 32-row stripe:
+// one sequential chain per stripe, bound by the latency of a step.  aws_kernel
+// shortens the chain: what a word decodes to depends on its low 28 bits alone, so
+// helper warps look up every word of the stream ahead of the decode, and a lane
+// that refills takes its four symbols and products from there, in parallel with
+// the lanes that look up their own state.
 #include <algorithm>
 #include <cstdio>
 
@@ -44,178 +57,320 @@ struct AwrLaunch {
     int8_t *out8;  // requantised output (one vector)
     float scale;
     uint32_t *status;
+    uint32_t spin_limit;
 };
 
-// STRIPES: the "ans-warp-stripes" layout (ans-warp-stripes-kernel.cu:21-227, encoder.py:323-391).  The
-// word stream and its cache are the same, but a warp is a stripe of 32 rows: lane l is row 32u + l,
-// decodes its quad j (columns 4j..4j+3) at step j and keeps its own sums (no warp reduction), and
-// there is one offset per stripe.
-template <int NV, bool REQUANT, bool STRIPES>
-__global__ void __launch_bounds__(256) awr_kernel(const AwrLaunch L) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint2 *lut = reinterpret_cast<uint2 *>(smem);        // 128 * 32 entries of 8 bytes
-    uint32_t *xs = reinterpret_cast<uint32_t *>(lut + 128 * 32);  // [cols/4][NV]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
-    const int nq = L.cols >> 2;
+constexpr uint32_t kAwrLut = 128 * 128;    // decode table
+constexpr uint32_t kAwrRing = 512 * 4;     // words in shared memory per warp (at most 31 + 128 are waiting)
+template <int NV>
+constexpr int kAwrWarps = NV <= 4 ? 28 : 20;
 
-    // one entry per quantile (its table reads once), written to all 32 lane columns with a rotating column
-    // index so that a half-warp's 8-byte stores hit distinct banks
-    for (uint32_t q = threadIdx.x; q < 128; q += blockDim.x) {
-        const uint32_t sh = 8 * (q & 3);
+// Decode table by the whole CTA: four threads per quantile, eight lane columns each.
+__device__ __forceinline__ void awr_table(const AwrLaunch &L, unsigned char *lut) {
+    for (uint32_t i = threadIdx.x; i < 128 * 4; i += blockDim.x) {
+        const uint32_t q = i >> 2, sh = 8 * (q & 3);
         const uint32_t sym = (__ldg(L.ppf + (q >> 2)) >> sh) & 0xFF;
         const uint32_t c = (__ldg(L.cum + (q >> 2)) >> sh) & 0xFF;
         const uint32_t p = (__ldg(L.prob + (q >> 2)) >> sh) & 0xFF;
         if (c > q || p == 0) atomicOr(L.status, MV_DEV_BAD_TABLE);
-        const uint2 e = make_uint2(p | (sym << 16), (q - c) & 0xFFFFu);
-#pragma unroll 8
-        for (uint32_t l = 0; l < 32; l++) lut[q * 32 + ((l + q) & 31)] = e;
+        const uint32_t e = p | sym << 16 | ((q - c) & 0xFFu) << 24;
+        uint4 *dst = reinterpret_cast<uint4 *>(lut + q * 128u + (i & 3u) * 32u);
+        dst[0] = dst[1] = make_uint4(e, e, e, e);
     }
+}
+
+// x as quads [cols/4][NV] by the whole CTA
+template <int NV>
+__device__ __forceinline__ void awr_stage_x(const AwrLaunch &L, uint32_t *xs) {
+    const int nq = L.cols >> 2;
     const bool xal = (reinterpret_cast<uintptr_t>(L.x) & 3) == 0;
     for (int i = threadIdx.x; i < nq * NV; i += blockDim.x) {
-        const int c = i / NV, v = i % NV;
+        const int v = i / nq, c = i - v * nq;  // consecutive threads read consecutive quads
         uint32_t val = 0;
         if (v < L.batch) {
             const int8_t *p = L.x + (size_t)v * L.cols + 4 * c;
             if (xal) val = *reinterpret_cast<const uint32_t *>(p);
             else for (int j = 0; j < 4; j++) val |= (uint32_t)(uint8_t)p[j] << (8 * j);
         }
-        xs[i] = val;
+        xs[c * NV + v] = val;
     }
+}
+
+// What the low 28 bits of a state (or of a word) decode to: the packed symbols, the product P of the four
+// probabilities and the mixed-radix remainder t < P.
+__device__ __forceinline__ uint32_t awr_lookup(const unsigned char *lut, uint32_t lane4, uint32_t lo, uint32_t &P, uint32_t &t) {
+    const uint32_t e0 = *reinterpret_cast<const uint32_t *>(lut + (((lo << 7) & 0x3F80u) | lane4));
+    const uint32_t e1 = *reinterpret_cast<const uint32_t *>(lut + ((lo & 0x3F80u) | lane4));
+    const uint32_t e2 = *reinterpret_cast<const uint32_t *>(lut + (((lo >> 7) & 0x3F80u) | lane4));
+    const uint32_t e3 = *reinterpret_cast<const uint32_t *>(lut + (((lo >> 14) & 0x3F80u) | lane4));
+    const uint32_t u01 = __dp4a(e0, __byte_perm(e1, 1u, 0x4553), 0u);  // r0 + p0 r1 = (p0, 0, sym, r0) . (r1, 0, 0, 1)
+    const uint32_t u23 = __dp4a(e2, __byte_perm(e3, 1u, 0x4553), 0u);
+    const uint32_t p01 = __dp2a_lo(e1, e0, 0u), p23 = __dp2a_lo(e3, e2, 0u);
+    P = p01 * p23;
+    t = u01 + p01 * u23;
+    return __byte_perm(__byte_perm(e0, e1, 0x0062), __byte_perm(e2, e3, 0x0062), 0x5410);
+}
+
+// state = (state >> 28) * P + t
+__device__ __forceinline__ void awr_update(uint32_t &lo, uint32_t &hi, uint32_t P, uint32_t t) {
+    const uint32_t a = __funnelshift_r(lo, hi, 28), b = hi >> 28;
+    const unsigned long long s = (unsigned long long)a * P + t;
+    lo = (uint32_t)s;
+    hi = (uint32_t)(s >> 32) + b * P;
+}
+
+template <bool REQUANT, int NV>
+__device__ __forceinline__ void awr_store(const AwrLaunch &L, int r, const int (&acc)[NV]) {
+    if (REQUANT) {
+        const int q = __float2int_rn((float)acc[0] * L.scale);  // ans-warp-rows-kernel.cu:212-220
+        L.out8[r] = (int8_t)max(-128, min(127, q));
+    } else {
+#pragma unroll
+        for (int v = 0; v < NV; v++)
+            if (v < L.batch) {
+                L.y[(size_t)v * L.rows + r] = acc[v];
+                if (L.ys) L.ys[(size_t)v * L.rows + r] = (float)acc[v] * L.scales[r];
+            }
+    }
+}
+
+// STRIPES: lane l is row 32u + l of stripe u, decodes its quad j (columns 4j..4j+3) at step j and keeps its own sums
+// (no warp reduction); one offset per stripe.
+// BOUNDED: the stream's length is known, so words may be staged ahead: the ring is looked after once in four steps
+// (a warp-wide branch costs ~50 cycles of a step's latency).  Otherwise (the reference's launchers do not pass the
+// length) a block is read when a lane takes its first word and not before.
+template <int NV, bool REQUANT, bool STRIPES, bool BOUNDED>
+__global__ void __launch_bounds__(32 * kAwrWarps<NV>) awr_kernel(const AwrLaunch L) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    const int nq = L.cols >> 2;
+    awr_table(L, smem);
+    uint32_t *ring = reinterpret_cast<uint32_t *>(smem + kAwrLut + (uint32_t)warp * kAwrRing);
+    uint32_t *xs = reinterpret_cast<uint32_t *>(smem + kAwrLut + (uint32_t)W * kAwrRing);
+    awr_stage_x<NV>(L, xs);
     __syncthreads();
 
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const unsigned char *lut_b = reinterpret_cast<const unsigned char *>(lut);
-    const uint32_t lane8 = (uint32_t)lane << 3;
-    const bool bounded = L.n_u4 != 0;
-
+    const uint32_t lt_mask = (1u << lane) - 1u, lane4 = (uint32_t)lane << 2;
     const int units = STRIPES ? L.rows / 32 : L.rows;  // warps' work units: rows or 32-row stripes
     for (int row = blockIdx.x * W + warp; row < units; row += gridDim.x * W) {
-        size_t bi = __ldg(L.offs + row);  // uint4 index of the block held in `cache`
-        uint4 cache = make_uint4(0, 0, 0, 0), nxt = make_uint4(0, 0, 0, 0);
-        bool ovf = false;
-        if (!bounded || bi + 32 <= L.n_u4) cache = L.comp[bi + lane];
-        else ovf = true;
-        if (bounded && bi + 64 <= L.n_u4) nxt = L.comp[bi + 32 + lane];
-        unsigned long long state = ((unsigned long long)cache.w << 32) | cache.z;
-        uint32_t wcc = 64;  // reference cursor into the 128-word cache
-        bool lag = false;   // cursor crossed a 32-word boundary without advancing
-
-        auto advance = [&](uint32_t leaving_gen) {
-            if (leaving_gen == 3) {  // next block
-                bi += 32;
-                if (bounded) {
-                    if (bi + 32 > L.n_u4) ovf = true;
-                    cache = nxt;
-                    nxt = (bi + 64 <= L.n_u4) ? L.comp[bi + 32 + lane] : make_uint4(0, 0, 0, 0);
-                } else {
-                    cache = L.comp[bi + lane];
-                }
-            } else {
-                cache.x = cache.y;
-                cache.y = cache.z;
-                cache.z = cache.w;
-            }
+        // The first block holds the initial states (fields z, w) and the first 64 words of the stream (x, y); every
+        // later block 128 words, field by field (ans-warp-rows-kernel.cu:76-139).
+        size_t bi = __ldg(L.offs + row);  // uint4 index of the latest block in the ring
+        auto block = [&](size_t at) {
+            return !BOUNDED || at + 32 <= L.n_u4 ? L.comp[at + lane] : make_uint4(0, 0, 0, 0);
         };
-
+        // words of the stream that can be read (from the first block's x on), for the overrun check
+        const unsigned long long have = BOUNDED ? (bi + 32 <= L.n_u4 ? (L.n_u4 - bi) / 32 * 128 - 64 : 0) : ~0ull;
+        const uint4 first = block(bi);
+        uint4 nxt = BOUNDED ? block(bi + 32) : first;
+        uint32_t lo = first.z, hi = first.w;
+        __syncwarp();
+        ring[lane] = first.x;
+        ring[32 + lane] = first.y;
+        uint32_t cur = 0, staged = 64;  // words consumed, words in the ring
+        auto stage = [&]() {
+            bi += 32;
+            if (!BOUNDED) nxt = block(bi);
+            const uint32_t s = staged + (uint32_t)lane;
+            ring[s & 511u] = nxt.x;
+            ring[(s + 32u) & 511u] = nxt.y;
+            ring[(s + 64u) & 511u] = nxt.z;
+            ring[(s + 96u) & 511u] = nxt.w;
+            staged += 128u;
+            if (BOUNDED) nxt = block(bi + 32);
+            __syncwarp();
+        };
+        __syncwarp();
         int acc[NV];
 #pragma unroll
         for (int v = 0; v < NV; v++) acc[v] = 0;
-
-        for (int j = 0; j < nq; j += STRIPES ? 1 : 32) {
-            const bool need = (state >> 32) == 0;
+        const uint32_t *xq = xs + (STRIPES ? 0 : lane * NV);  // stripes: one x quad for all lanes
+        auto step = [&]() {
+            const bool need = hi == 0;
             const uint32_t ballot = __ballot_sync(0xffffffffu, need);
-            if (ballot) {
-                if (lag) {
-                    advance((wcc >> 5) == 0 ? 3u : 0u);
-                    lag = false;
-                }
-                const uint32_t off = __popc(ballot & lt_mask);
-                const uint32_t num = __popc(ballot);
-                const uint32_t lc = (wcc + off) & 31;
-                const uint32_t gen = wcc >> 5;
-                uint32_t rv = __shfl_sync(0xffffffffu, cache.x, lc);
-                if (((wcc + num - 1) >> 5) != gen) {
-                    advance(gen);
-                    const uint32_t rv2 = __shfl_sync(0xffffffffu, cache.x, lc);
-                    if (((wcc + off) >> 5) != gen) rv = rv2;
-                } else if (((wcc + num) >> 5) != gen) {
-                    lag = true;
-                }
-                if (need) state = (state << 32) | rv;
-                wcc = (wcc + num) & 127;
-            }
-            const uint32_t lo = (uint32_t)state;
-            // quantile k (bits 7k..7k+6) moved to bits 8..14, the lane's byte offset in bits 0..7
-            const uint2 e0 = *reinterpret_cast<const uint2 *>(lut_b + (((lo << 8) & 0x7F00u) | lane8));
-            const uint2 e1 = *reinterpret_cast<const uint2 *>(lut_b + (((lo << 1) & 0x7F00u) | lane8));
-            const uint2 e2 = *reinterpret_cast<const uint2 *>(lut_b + (((lo >> 6) & 0x7F00u) | lane8));
-            const uint2 e3 = *reinterpret_cast<const uint2 *>(lut_b + (((lo >> 13) & 0x7F00u) | lane8));
-            const uint32_t u01 = __dp2a_lo(e1.y, e0.x, e0.y);  // r0 + p0 r1
-            const uint32_t t2 = __dp2a_lo(e3.y, e2.x, e2.y);   // r2 + p2 r3
-            const uint32_t p01 = __dp2a_lo(e1.x, e0.x, 0u);    // p0 p1 (+ sym1 * 0)
-            const uint32_t p23 = __dp2a_lo(e3.x, e2.x, 0u);    // p2 p3
-            state = (state >> 28) * (unsigned long long)(p01 * p23) + (u01 + p01 * t2);
-            const uint32_t wq =
-                __byte_perm(__byte_perm(e0.x, e1.x, 0x0062), __byte_perm(e2.x, e3.x, 0x0062), 0x5410);
-            const uint32_t *xq = xs + (STRIPES ? j : j + lane) * NV;  // stripes: one x quad for all lanes
+            const uint32_t at = cur + __popc(ballot & lt_mask);
+            cur += __popc(ballot);
+            if (!BOUNDED && cur > staged) stage();  // a lane takes a word of the next block (128 > 32: one is enough)
+            const uint32_t w = ring[at & 511u];
+            hi = need ? lo : hi;
+            lo = need ? w : lo;
+            uint32_t P, t;
+            const uint32_t wq = awr_lookup(smem, lane4, lo, P, t);
+            awr_update(lo, hi, P, t);
 #pragma unroll
             for (int v = 0; v < NV; v++) acc[v] = __dp4a((int)wq, (int)xq[v], acc[v]);
+            xq += STRIPES ? NV : 32 * NV;
+        };
+        const int steps = STRIPES ? nq : nq / 32;
+        int j = 0;
+        for (; j + 4 <= steps; j += 4) {
+            if (BOUNDED)
+                while (staged < cur + 128u) stage();  // at most twice: 384 words wait in the ring at most
+            step();
+            step();
+            step();
+            step();
         }
-        if (ovf) atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
+        for (; j < steps; j++) {
+            if (BOUNDED && staged < cur + 32u) stage();
+            step();
+        }
+        if (BOUNDED && (cur > have || have == 0)) atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
         if (STRIPES) {
-            const int r = row * 32 + lane;  // rows % 32 == 0
-            if (REQUANT) {
-                const int q = __float2int_rn((float)acc[0] * L.scale);  // ans-warp-stripes-kernel.cu:220-225
-                L.out8[r] = (int8_t)max(-128, min(127, q));
-            } else {
+            awr_store<REQUANT>(L, row * 32 + lane, acc);  // rows % 32 == 0
+        } else {
 #pragma unroll
-                for (int v = 0; v < NV; v++)
-                    if (v < L.batch) {
-                        L.y[(size_t)v * L.rows + r] = acc[v];
-                        if (L.ys) L.ys[(size_t)v * L.rows + r] = (float)acc[v] * L.scales[r];
-                    }
-            }
-            continue;
-        }
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o);
-        }
-        if (lane == 0) {
-            if (REQUANT) {
-                // ans-warp-rows-kernel.cu:212-220
-                const int r = __float2int_rn((float)acc[0] * L.scale);
-                L.out8[row] = (int8_t)max(-128, min(127, r));
-            } else {
-#pragma unroll
-                for (int v = 0; v < NV; v++)
-                    if (v < L.batch) {
-                        L.y[(size_t)v * L.rows + row] = acc[v];
-                        if (L.ys) L.ys[(size_t)v * L.rows + row] = (float)acc[v] * L.scales[row];
-                    }
-            }
+            for (int v = 0; v < NV; v++) acc[v] = __reduce_add_sync(0xffffffffu, acc[v]);
+            if (lane == 0) awr_store<REQUANT>(L, row, acc);
         }
     }
+}
+
+// Stripes with a stream of known length: one CTA per stripe, warp 0 decodes, kAwsHelpers warps look up the stream's
+// words ahead.  The words go through a ring of kAwsBlocks blocks of 128 entries {P, t, symbols, word} (16 bytes); full
+// and empty mbarriers per block.  A step of the decode is: vote, prefix popcount, one 16-byte load, two selects and the
+// state's multiply-add, beside it the four lookups of the lanes that do not refill.  (Measured on a B200, 4096x4096, one vector: 174.7 us with
+// the words in registers and the lookups behind the refill, 340 cycles a step; 107.2 us now, 204 cycles a step.)
+constexpr int kAwsHelpers = 3, kAwsBlocks = 8;
+constexpr uint32_t kAwsRing = kAwsBlocks * 2048;
+
+template <int NV, bool REQUANT>
+__global__ void __launch_bounds__(32 * (1 + kAwsHelpers)) aws_kernel(const AwrLaunch L) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint64_t full[kAwsBlocks], empty[kAwsBlocks];
+    __shared__ uint32_t stop;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nq = L.cols >> 2;
+    const uint32_t lane4 = (uint32_t)lane << 2;
+    unsigned char *ring = smem + kAwrLut;
+    uint32_t *xs = reinterpret_cast<uint32_t *>(smem + kAwrLut + kAwsRing);
+    if (threadIdx.x < kAwsBlocks) {
+        mbar_init(&full[threadIdx.x], 1);
+        mbar_init(&empty[threadIdx.x], 1);
+    }
+    if (threadIdx.x == 0) stop = 0;
+    fence_mbar_init();
+    awr_table(L, smem);
+    awr_stage_x<NV>(L, xs);
+    __syncthreads();
+
+    const int stripe = blockIdx.x;
+    const size_t b0 = __ldg(L.offs + stripe);  // uint4 index of the stripe's first block
+    const size_t nblk = b0 + 32 <= L.n_u4 ? (L.n_u4 - b0) / 32 : 0;  // whole blocks that can be read
+    volatile uint32_t *done = &stop;
+
+    if (warp > 0) {
+        // helpers: block b (0: the 64 words behind the states) to ring slot b % kAwsBlocks, warp b % kAwsHelpers
+        uint4 v = make_uint4(0, 0, 0, 0);
+        uint32_t b = (uint32_t)warp - 1u;
+        if (b < nblk) v = L.comp[b0 + 32 * (size_t)b + lane];
+        for (; b < nblk; b += kAwsHelpers) {
+            const uint4 c = v;
+            if (b + kAwsHelpers < nblk) v = L.comp[b0 + 32 * (size_t)(b + kAwsHelpers) + lane];
+            const uint32_t slot = b % kAwsBlocks, turn = b / kAwsBlocks;
+            if (turn > 0) {
+                bool ok = false;
+                for (uint32_t it = 0; !ok && it < L.spin_limit; it++) {
+                    ok = mbar_try_wait(&empty[slot], (turn - 1u) & 1u);
+                    if (!ok && *done) break;
+                }
+                if (!__all_sync(0xffffffffu, ok)) return;  // the decode is over (or gave up)
+            }
+            uint4 *dst = reinterpret_cast<uint4 *>(ring + slot * 2048u) + lane;
+            // (block 0: its two fields of words go to the slot's upper half, before block 1)
+            const uint32_t w[4] = {c.x, c.y, b ? c.z : c.x, b ? c.w : c.y};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                uint32_t P, t;
+                const uint32_t wq = awr_lookup(smem, lane4, w[j], P, t);
+                dst[32 * j] = make_uint4(P, t, wq, w[j]);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[slot]);
+        }
+        return;
+    }
+
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint4 first = nblk ? L.comp[b0 + lane] : make_uint4(0, 0, 0, 0);
+    uint32_t lo = first.z, hi = first.w;
+    // words consumed, words in the ring so far, blocks they came from, blocks given back; word w is entry w + 64
+    uint32_t cur = 0, limit = 0, blocks = 0, freed = 0;
+    bool ok = true;
+    int acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) acc[v] = 0;
+    const uint32_t *xq = xs;
+    auto step = [&]() {
+        const bool need = hi == 0;
+        uint32_t P, t;
+        uint32_t wq = awr_lookup(smem, lane4, lo, P, t);  // of the lanes that do not refill
+        const uint32_t ballot = __ballot_sync(0xffffffffu, need);
+        const uint32_t at = cur + __popc(ballot & lt_mask);
+        cur += __popc(ballot);
+        const uint4 e = *reinterpret_cast<const uint4 *>(ring + (((at + 64u) * 16u) & (kAwsRing - 1u)));
+        hi = need ? lo : hi;
+        lo = need ? e.w : lo;
+        P = need ? e.x : P;
+        t = need ? e.y : t;
+        wq = need ? e.z : wq;
+        awr_update(lo, hi, P, t);
+#pragma unroll
+        for (int v = 0; v < NV; v++) acc[v] = __dp4a((int)wq, (int)xq[v], acc[v]);
+        xq += NV;
+    };
+    for (int j = 0; j < nq; j += 8) {
+        // Eight steps take at most 256 words: their blocks are waited for, and the blocks before them given back.  (Once
+        // in eight steps: a warp-wide branch costs ~50 cycles, a step of the chain ~130.)
+        while (limit < cur + 256u && blocks < nblk) {
+            ok &= mbar_wait_bounded(&full[blocks % kAwsBlocks], (blocks / kAwsBlocks) & 1u, L.status, ok ? L.spin_limit : 1u);
+            limit += blocks ? 128u : 64u;
+            blocks++;
+        }
+        const uint32_t over = min((cur + 64u) >> 7, blocks ? blocks - 1u : 0u);  // blocks whose words are all consumed
+        if (freed + (uint32_t)lane < over) mbar_arrive(&empty[(freed + (uint32_t)lane) % kAwsBlocks]);
+        freed = max(freed, over);
+        if (j + 8 <= nq) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) step();
+        } else {
+            for (int i = j; i < nq; i++) step();
+        }
+    }
+    __syncwarp();
+    if (lane == 0) *done = 1u;
+    if (nblk == 0 || cur > 128ull * nblk - 64ull) atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
+    awr_store<REQUANT>(L, stripe * 32 + lane, acc);  // rows % 32 == 0
 }
 
 namespace {
 
 template <int NV, bool REQUANT, bool STRIPES = false>
 mv_status launch_awr(const AwrLaunch &L, cudaStream_t st) {
-    // stripes: few work units (rows / 32, each decoded start to end by one warp), so one-warp CTAs spread
-    // them over all SMs
-    const int W = STRIPES ? 1 : 8;
-    const size_t smem = 128 * 32 * 8 + (size_t)(L.cols / 4) * NV * 4;
-    if (smem > (size_t)max_smem_optin())
+    const size_t xb = (size_t)(L.cols / 4) * NV * 4;
+    if (128 * 32 * 8 + xb > (size_t)max_smem_optin())
         return fail(MV_ERR_UNSUPPORTED, "AWR: %d columns x %d vectors exceed shared memory", L.cols, NV);
-    auto kern = awr_kernel<NV, REQUANT, STRIPES>;
-    int blocks_per_sm = 0;
-    mv_status rc = prepare_kernel((const void *)kern, smem, 32 * W, &blocks_per_sm);
+    if (STRIPES && L.n_u4 && kAwrLut + kAwsRing + xb + 2048 <= (size_t)max_smem_optin()) {  // (2 KB: barriers)
+        const size_t smem = kAwrLut + kAwsRing + xb;
+        auto kern = aws_kernel<NV, REQUANT>;
+        mv_status rc = prepare_kernel((const void *)kern, smem, 32 * (1 + kAwsHelpers), nullptr);
+        if (rc) return rc;
+        kern<<<L.rows / 32, 32 * (1 + kAwsHelpers), smem, st>>>(L);
+        MV_CUDA_TRY(cudaGetLastError(), "aws kernel launch");
+        return MV_OK;
+    }
+    // warps: stripes are few (rows / 32) and long, one to a CTA spreads them over the SMs; rows in even rounds over the
+    // SMs, as many as fit beside x
+    const int units = STRIPES ? L.rows / 32 : L.rows, sms = sm_count();
+    int wmax = STRIPES ? 1 : kAwrWarps<NV>;
+    while (wmax > 1 && kAwrLut + (size_t)wmax * kAwrRing + xb > (size_t)max_smem_optin()) wmax--;
+    const int rounds = (units + sms * wmax - 1) / (sms * wmax);
+    const int W = STRIPES ? 1 : std::max(1, (units + sms * rounds - 1) / (sms * rounds));
+    const size_t smem = kAwrLut + (size_t)W * kAwrRing + xb;
+    auto kern = L.n_u4 ? awr_kernel<NV, REQUANT, STRIPES, true> : awr_kernel<NV, REQUANT, STRIPES, false>;
+    mv_status rc = prepare_kernel((const void *)kern, smem, 32 * W, nullptr);
     if (rc) return rc;
-    const int units = STRIPES ? L.rows / 32 : L.rows;
-    const int want = (units + W - 1) / W;
-    const int grid = std::max(1, std::min(want, std::max(1, blocks_per_sm) * sm_count()));
+    const int grid = STRIPES ? units : std::max(1, std::min((units + W - 1) / W, sms));
     kern<<<grid, 32 * W, smem, st>>>(L);
     MV_CUDA_TRY(cudaGetLastError(), "awr kernel launch");
     return MV_OK;
@@ -238,6 +393,7 @@ mv_status awr_common(const uint32_t *comp, size_t n_words, const uint32_t *offs,
     if (rc) return rc;
     L.comp = reinterpret_cast<const uint4 *>(comp);
     L.n_u4 = n_words / 4;
+    L.spin_limit = wait_spin_limit();
     L.offs = offs;
     L.ppf = ppf;
     L.cum = cum;

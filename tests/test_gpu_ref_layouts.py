@@ -50,3 +50,28 @@ def test_wpr_stream_off_the_grid():
     cm.payload = np.concatenate([np.full(3, 0xABCD, np.uint16), cm.payload])
     cm.cursors = cm.cursors + np.uint32(3)
     check(ops.WprMatrix(cm), W, rng, (1, 4))
+
+
+@pytest.mark.parametrize("kind", ["gauss", "dense", "tails"])
+@pytest.mark.parametrize("rows,cols", [(1, 128), (150, 640), (4200, 256), (33, 4096)])
+def test_awr(kind, rows, cols):
+    rng = np.random.default_rng(rows + cols)
+    W = weights(rng, kind, (rows, cols))
+    check(ops.AwrMatrix.encode(W), W, rng, (1, 3, 9, 17))
+
+
+@pytest.mark.parametrize("kind", ["gauss", "dense", "tails"])
+@pytest.mark.parametrize("rows,cols", [(32, 4), (64, 36), (96, 1000), (4800, 64)])
+def test_aws(kind, rows, cols):
+    rng = np.random.default_rng(rows + cols)
+    W = weights(rng, kind, (rows, cols))
+    M = ops.AwsMatrix.encode(W)
+    check(M, W, rng, (1, 3, 9, 17))
+    # the launcher that does not know the stream's length reads no further than the words it takes
+    x = rng.integers(-128, 128, size=cols).astype(np.int8)
+    out = torch.empty(rows, dtype=torch.int8, device="cuda")
+    assert ops.mat_vec_mul_coalesced_stripes(torch.from_numpy(x).cuda(), out, cols, rows, 2e-3, M.compressed, M.offsets,
+                                             M.ppf, M.ppf_cum, M.ppf_prob) is not None
+    torch.cuda.synchronize()
+    ref = np.clip(np.rint(oracle.matvec_i8(W, x[None, :])[0].astype(np.float32) * np.float32(2e-3)), -128, 127)
+    assert np.array_equal(out.cpu().numpy(), ref.astype(np.int8))
