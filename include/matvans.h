@@ -306,7 +306,7 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
 /* Float form (no reference counterpart): y[b][r] = s[r] * sum_c W[r][c] *
  * x[b][c] with x bf16 [batch][cols] (16-byte aligned), fp32 accumulation in a
  * fixed order (deterministic), fp32 y [batch][rows].  cols % 16 == 0.  Passes
- * of up to 8 vectors share one decode. */
+ * of up to 64 vectors share one decode. */
 mv_status mv_q8_matvec_bf16(const mv_q8_view *m, const uint16_t *x_dev, int batch,
                             const float *row_scales_dev, float *y_dev, const mv_q8_tuning *tuning,
                             void *stream);
@@ -316,7 +316,7 @@ mv_status mv_q8_matvec_bf16(const mv_q8_view *m, const uint16_t *x_dev, int batc
  * (zeroed by the call).  The streams are decoded again (W is never stored);
  * the 32 rows of a stripe are summed per column inside the warp and stripes
  * are combined with fp32 atomics, so the result is reproducible to fp32
- * rounding, not bit for bit. */
+ * rounding, not bit for bit.  Passes of up to 32 vectors share one decode. */
 mv_status mv_q8_matvec_t_bf16(const mv_q8_view *m, const uint16_t *dy_dev, int batch,
                               const float *row_scales_dev, float *dx_dev,
                               const mv_q8_tuning *tuning, void *stream);

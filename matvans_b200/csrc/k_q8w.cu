@@ -646,9 +646,10 @@ __device__ __forceinline__ uint4 ldx_u4(const void *p) { return *reinterpret_cas
 // (exact integer atomics); the warp that counts the item's last part writes the outputs.
 template <int NV>
 struct DotCons {
-    static constexpr bool kMma = false, kFloat = false, kStatic = false;
+    static constexpr bool kMma = false, kFloat = false, kStatic = false, kPrepare = false;
     static constexpr int kRed = NV * 32;  // ints of an item's partial sums
     static constexpr int kMaxDecode = NV <= 2 ? 16 : NV <= 4 ? 14 : NV <= 8 ? 10 : 6;
+    static constexpr uint32_t tile_bytes(int) { return 0; }
     const int8_t *x;
     int cols, seg_quads, qtot;
     bool in_slot;
@@ -658,7 +659,7 @@ struct DotCons {
 #pragma unroll
         for (int v = 0; v < NV; v++) acc[v] = 0;
     }
-    __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I) {
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I, int) {
         in_slot = x_in_slot(L, I.seg_quads);
         x = I.x;
         cols = I.cols;
@@ -750,13 +751,13 @@ struct DotCons {
 // alternate between two accumulators, the second in the 16 lanes of each quarter that M = 64 leaves free.
 template <bool kOwn>
 struct MmaCons {
-    static constexpr bool kMma = true, kFloat = false, kStatic = false;
+    static constexpr bool kMma = true, kFloat = false, kStatic = false, kPrepare = false;
     static constexpr int kPitch = 33;  // words per vector of the item's sums: lanes (vectors) hit distinct banks
     static constexpr int kRed = kOwn ? 16 * kPitch : 0;
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;  // 32 rows x 64 columns
-    static __host__ __device__ constexpr uint32_t x_tile(int xrows) { return 64u * (uint32_t)xrows; }
-    static __host__ __device__ constexpr uint32_t tile_bytes(int xrows) { return kWTile + x_tile(xrows); }
+    static constexpr uint32_t x_tile(int xrows) { return 64u * (uint32_t)xrows; }
+    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + x_tile(xrows); }
     const int8_t *x;
     int cols, seg_quads, qtot;
     uint32_t wt, xt, d_tmem, lbo, nmma, ndp;  // nmma: commits so far, ndp: earlier items this warp has had a part in
@@ -778,7 +779,7 @@ struct MmaCons {
         nmma = ndp = 0;
         any = false;
     }
-    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I) {
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I, int) {
         if (!kOwn) {
             if (any) ndp++;  // the sums of the item before stay where they are until a table warp has read them
             any = false;
@@ -980,11 +981,11 @@ struct MmaCons {
 // a time: W tile 2 KB, x tile 64 bytes per vector.  Unit u goes to warp u mod W, each warp's MMAs accumulate in order
 // and the warps' sums are added in unit order, so results are reproducible bit for bit.
 struct FwdCons {
-    static constexpr bool kMma = true, kFloat = true, kStatic = true;
+    static constexpr bool kMma = true, kFloat = true, kStatic = true, kPrepare = false;
     static constexpr int kRed = 0;
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;
-    static __host__ __device__ constexpr uint32_t tile_bytes(int xrows) { return kWTile + 64u * (uint32_t)xrows; }
+    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + 64u * (uint32_t)xrows; }
     const uint16_t *x;
     int cols, seg_quads, qtot;
     uint32_t wt, xt, d_tmem, lbo, nmma, ndp;
@@ -1005,7 +1006,7 @@ struct FwdCons {
         nmma = ndp = 0;
         any = false;
     }
-    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I) {
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I, int) {
         x = reinterpret_cast<const uint16_t *>(I.x);
         cols = I.cols;
         seg_quads = I.seg_quads;
@@ -1170,9 +1171,10 @@ struct FwdCons {
 // units: reproducible bit for bit.  (4096x11008: 40 us through the MMAs of FwdCons, whose tiles cost more than one
 // vector's products.)
 struct FwdDot {
-    static constexpr bool kMma = false, kFloat = true, kStatic = true;
+    static constexpr bool kMma = false, kFloat = true, kStatic = true, kPrepare = false;
     static constexpr int kMaxDecode = 16;
     static constexpr int kRed = kMaxDecode * 32;
+    static constexpr uint32_t tile_bytes(int) { return 0; }
     const uint16_t *x;
     int seg_quads, qtot, warp;
     bool in_slot;
@@ -1181,7 +1183,7 @@ struct FwdDot {
         warp = w;
         acc = 0.f;
     }
-    __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I) {
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I, int) {
         in_slot = x_in_slot(L, I.seg_quads);
         x = reinterpret_cast<const uint16_t *>(I.x);
         seg_quads = I.seg_quads;
@@ -1249,6 +1251,286 @@ struct FwdDot {
     }
 };
 
+// Float backward on the tensor cores: dX = W^T (s . dY), up to 32 bf16 vectors a pass, added to dX (fp32, zeroed by the
+// launcher) with 16-byte reductions.
+//   A = G = s . dY of the stripe's 32 rows (K), in TMEM: the table warps write it with the item's decode table, vector v
+//       in lane v of every quarter, as bf16 terms hi + lo (g to 2^-17);
+//   B = W: 8 quads at a time, each lane storing its row's four 16-byte pieces (the tile is W^T's transpose as it
+//       stands: MN-major, N = 32 columns, K = 32 rows);
+//   D: 32 TMEM columns per decode warp, vector v in lane v of the warp's own quarter.
+// The sums of a tile are read while the next one decodes.  From 5 vectors on they pass through shared memory so that
+// eight lanes cover the 128 bytes of a vector's row: reductions from one lane per vector ran at 2.6 TB/s, these at 5.4,
+// and they bound the larger batches (4 bytes per vector, column and stripe).
+// Measured on a B200 against the form this replaced (8 vectors a pass, CUDA cores): 11008x4096, 64 vectors 222 -> 145 us,
+// 16 vectors 90 -> 64 us, 2 vectors 76 -> 57 us; 4096x11008, 64 vectors 259 -> 151 us, 16 vectors 106 -> 63 us.
+struct BwdCons {
+    static constexpr bool kMma = true, kFloat = true, kStatic = false, kPrepare = true;
+    static constexpr int kRed = 0;
+    static constexpr int kMaxDecode = 12;
+    static constexpr uint32_t kWTile = 2048, kTr = 4096;
+    static constexpr uint32_t kGCols = 32;  // TMEM columns of an item's G: two terms of two K steps
+    static constexpr uint32_t tile_bytes(int) { return kWTile + kTr; }
+    float *dx;
+    int cols, seg_quads, qtot, batch;
+    uint32_t wt, tr, d_tmem, g_tmem, g_base, nmma, mbar, quarter;
+    int pend_col, pend_n;  // the tile whose sums are still in D: first column, columns
+    __device__ __forceinline__ void init(const Q8WLaunch &L, unsigned char *sm, const Bars &B, uint32_t tmem, int w) {
+        wt = smem_u32(sm) + L.lay.tiles + (uint32_t)w * tile_bytes(0);
+        tr = wt + kWTile;
+        quarter = ((uint32_t)(w + kFirstDecode) & 3u) << 21;
+        g_base = tmem;
+        d_tmem = tmem + 2u * kGCols + 32u * (uint32_t)w;
+        mbar = B.mma(w);
+        nmma = 0;
+        batch = L.batch;
+        pend_n = 0;
+    }
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I, int k) {
+        dx = I.ys;
+        cols = I.cols;
+        seg_quads = I.seg_quads;
+        qtot = cols >> 2;
+        g_tmem = g_base + (uint32_t)(k & 1) * kGCols;
+        tcgen05_fence_after();  // G was written by the table warps
+    }
+    // Table warps: G of item k (into one of two buffers: the item before the previous one is finished).
+    static __device__ __forceinline__ void prepare(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *, uint32_t tmem) {
+        const int q = threadIdx.x >> 5, v = threadIdx.x & 31, row0 = I.stripe * 32;
+        const uint16_t *dy = reinterpret_cast<const uint16_t *>(I.x) + (size_t)v * I.rows + row0;
+        const float sl = row0 + v < I.rows ? __ldg(I.scales + row0 + v) : 0.f;  // lane = row
+        float g[32];
+        if (v < L.batch && row0 + 32 <= I.rows && ((uintptr_t)dy & 15) == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint4 d = __ldg(reinterpret_cast<const uint4 *>(dy) + j);
+                const uint32_t w[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    g[8 * j + 2 * i] = __uint_as_float(w[i] << 16);
+                    g[8 * j + 2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                g[j] = v < L.batch && row0 + j < I.rows ? __uint_as_float((uint32_t)__ldg(dy + j) << 16) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j++) g[j] *= __shfl_sync(0xffffffffu, sl, j);
+        const uint32_t dst = tmem + (uint32_t)(k & 1) * kGCols + ((uint32_t)q << 21);
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            uint32_t r[16];
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+                uint32_t h[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    // term t, and what it leaves (nothing of an infinity or NaN)
+                    const float x = g[j + i];
+                    h[i] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x));
+                    g[j + i] = isfinite(x) ? x - __uint_as_float(h[i] << 16) : 0.f;
+                }
+                r[j >> 1] = h[0] | h[1] << 16;
+            }
+            tmem_st_32x32b_x16_nowait(dst + 16u * (uint32_t)t, r);
+        }
+        tmem_wait_st();
+        tcgen05_fence_before();
+    }
+    // the sums of the pending tile, added to dX
+    __device__ __forceinline__ void flush(const Q8WLaunch &L, int lane, volatile uint32_t *failed) {
+        if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
+        if (!pend_n) return;
+        tcgen05_fence_after();
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(d_tmem + quarter, r);  // lane = vector, r[j] = column pend_col + j
+        tcgen05_fence_before();
+        if (batch <= 4) {
+            float *dst = dx + (size_t)lane * cols + pend_col;
+            if (lane < batch) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                    if (j < pend_n) red4(dst + j, r[j], r[j + 1], r[j + 2], r[j + 3]);
+            }
+        } else {
+            // piece j of vector v at 16 (j ^ v % 8): conflict-free both ways
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(tr + 128u * (uint32_t)lane +
+                                                                           16u * (uint32_t)(j ^ (lane & 7))),
+                             "r"(r[4 * j]), "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3])
+                             : "memory");
+            __syncwarp();
+            const int c = 4 * (lane & 7);
+            float *dst = dx + (size_t)(lane >> 3) * cols + pend_col + c;
+            uint32_t src = tr + 128u * (uint32_t)(lane >> 3);
+            for (int v = lane >> 3; v < batch; v += 4) {
+                uint32_t a0, a1, a2, a3;
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+                             : "r"(src + 16u * (uint32_t)((lane & 7) ^ (v & 7)))
+                             : "memory");
+                if (c < pend_n) red4(dst, a0, a1, a2, a3);
+                dst += 4 * (size_t)cols;
+                src += 512u;
+            }
+            __syncwarp();
+        }
+        pend_n = 0;
+    }
+    static __device__ __forceinline__ void red4(float *p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(__uint_as_float(a)),
+                     "f"(__uint_as_float(b)), "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
+                     : "memory");
+    }
+    __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
+                                         uint32_t lw, int lane, volatile uint32_t *failed) {
+        const int q0 = d.seg * seg_quads;
+        const int nq = min(seg_quads, qtot - q0);
+        Stream s(sm, soff, d.rows, lane);
+        // lane = stripe row r: K step r / 16, K group (r / 8) % 2, row r % 8; N group c (8 columns) at 256 c
+        const uint32_t wdst = wt + (uint32_t)(lane >> 4) * 1024u + (uint32_t)((lane >> 3) & 1) * 128u + (uint32_t)(lane & 7) * 16u;
+#pragma unroll 1
+        for (int q = 0; q < nq; q += 8) {
+            const int n = min(4, (nq - q) >> 1);  // pieces of two quads (segments are whole groups of 4 quads)
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (c < n) {
+                    uint32_t w[4];
+                    s.step_bf16(sm, lw, w[0], w[1]);
+                    s.step_bf16(sm, lw, w[2], w[3]);
+                    if (c & 1) s.clamp();
+                    if (c == 0) flush(L, lane, failed);  // (the W tile is free, too)
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(wdst + 256u * c), "r"(w[0]), "r"(w[1]),
+                                 "r"(w[2]), "r"(w[3])
+                                 : "memory");
+                }
+            }
+            fence_proxy_async_smem();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                tcgen05_fence_after();
+                const uint32_t idesc = umma_idesc_bf16(128, 32, 0, 1);
+#pragma unroll
+                for (int t = 0; t < 2; t++)
+#pragma unroll
+                    for (int kk = 0; kk < 2; kk++)
+                        umma_f16_ts(d_tmem, g_tmem + 16u * (uint32_t)t + 8u * kk, umma_smem_desc(wt + 1024u * kk, 128u, 256u),
+                                    idesc, t || kk ? 1u : 0u);
+                umma_commit(mbar);
+            }
+            __syncwarp();
+            nmma++;
+            pend_col = 4 * (q0 + q);
+            pend_n = 8 * n;
+        }
+        if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
+    }
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool, unsigned char *, const Bars &B, int lane,
+                                             volatile uint32_t *failed) {
+        flush(L, lane, failed);
+        __syncwarp();
+        if (lane == 0) arrive(B.tdone(k % kRing));
+    }
+    __device__ __forceinline__ void drain(const Q8WLaunch &L) {
+        if (nmma)
+            for (uint32_t it = 0; it < L.spin_limit; it++)
+                if (mbar_try_wait(mbar, (nmma - 1) & 1u)) break;
+    }
+    static __device__ __forceinline__ void epilogue(const Q8WLaunch &, const ItemRec &, int, unsigned char *, const Bars &,
+                                                    uint32_t) {}
+};
+
+// Float backward of one vector on the CUDA cores: fp32 products of the table's bf16 symbols with the row's g = s . dy
+// (the tensor cores' sums of 32 rows are less exact than fp32 additions).  The products of 4 quads (16 columns) of the
+// 32 rows change hands in shared memory: a lane stores its row's four 16-byte pieces and reads one piece of four rows,
+// which leaves eight partial sums a column for three shuffle steps.  (All sixteen columns by shuffles alone: 30 selects
+// and 16 shuffles a group against 6 and 4.)  Bound by issue.  Measured on a B200: 4096x11008 52 -> 37 us, 11008x4096
+// 47 -> 41 us (with BwdCons, 55 and 57 us and 2e-6 of error where this form has 2e-7).
+struct BwdDot {
+    static constexpr bool kMma = false, kFloat = true, kStatic = false, kPrepare = true;
+    static constexpr int kMaxDecode = 16;
+    static constexpr int kRed = 32;  // g of the item's rows
+    static constexpr uint32_t tile_bytes(int) { return 2048; }
+    const float *gs;
+    float *dx;
+    float g;
+    int seg_quads, qtot;
+    uint32_t st, ld;  // this lane's row, and its piece of rows lane / 4, + 8, + 16, + 24
+    __device__ __forceinline__ void init(const Q8WLaunch &L, unsigned char *sm, const Bars &, uint32_t, int w) {
+        const uint32_t lane = threadIdx.x & 31u, t = smem_u32(sm) + L.lay.tiles + (uint32_t)w * tile_bytes(0);
+        gs = reinterpret_cast<const float *>(sm + L.lay.red) + lane;
+        // piece j of row r at 64 r + 16 (j ^ r / 2 % 4): conflict-free both ways
+        st = t + 64u * lane + 16u * ((lane >> 1) & 3u);
+        ld = t + 64u * (lane >> 2) + 16u * ((lane & 3u) ^ ((lane >> 3) & 3u));
+    }
+    __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I, int k) {
+        dx = I.ys;
+        seg_quads = I.seg_quads;
+        qtot = I.cols >> 2;
+        g = *reinterpret_cast<const volatile float *>(gs + (k % kRing) * kRed);
+    }
+    static __device__ __forceinline__ void prepare(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm, uint32_t) {
+        if (threadIdx.x >= 32) return;
+        const int row = I.stripe * 32 + (int)threadIdx.x;
+        float v = 0.f;
+        if (row < I.rows)
+            v = __ldg(I.scales + row) * __uint_as_float((uint32_t)__ldg(reinterpret_cast<const uint16_t *>(I.x) + row) << 16);
+        reinterpret_cast<float *>(sm + L.lay.red)[(k % kRing) * kRed + threadIdx.x] = v;
+    }
+    __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
+                                         uint32_t lw, int lane, volatile uint32_t *) {
+        const int q0 = d.seg * seg_quads;
+        const int nq = min(seg_quads, qtot - q0);
+        Stream s(sm, soff, d.rows, lane);
+        const bool b4 = lane & 16, b3 = lane & 8;
+        float *dst = dx + 4 * q0 + 4 * (lane & 3) + (b4 ? 2 : 0) + (b3 ? 1 : 0);
+        for (int i = 0; i < nq; i += 4, dst += 16) {  // segments are whole groups of 4 quads (cols % 16 == 0)
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) {
+                uint32_t e[4];
+                s.step_f(sm, lw, e);
+                asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(st ^ (16u * j)),
+                             "f"(__uint_as_float(e[0] & 0xFFFF0000u) * g), "f"(__uint_as_float(e[1] & 0xFFFF0000u) * g),
+                             "f"(__uint_as_float(e[2] & 0xFFFF0000u) * g), "f"(__uint_as_float(e[3] & 0xFFFF0000u) * g)
+                             : "memory");
+            }
+            s.clamp();
+            __syncwarp();
+            float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (uint32_t r = 0; r < 4; r++) {
+                float v[4];
+                asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                             : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                             : "r"(ld + 512u * r)
+                             : "memory");
+#pragma unroll
+                for (int c = 0; c < 4; c++) a[c] += v[c];
+            }
+            __syncwarp();
+            float k0 = b4 ? a[2] : a[0], k1 = b4 ? a[3] : a[1];
+            k0 += __shfl_xor_sync(0xffffffffu, b4 ? a[0] : a[2], 16);
+            k1 += __shfl_xor_sync(0xffffffffu, b4 ? a[1] : a[3], 16);
+            float c = b3 ? k1 : k0;
+            c += __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+            c += __shfl_xor_sync(0xffffffffu, c, 4);
+            if (!(lane & 4)) atomicAdd(dst, c);
+        }
+        if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
+    }
+    __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool, unsigned char *, const Bars &B, int lane,
+                                             volatile uint32_t *) {
+        __syncwarp();
+        if (lane == 0) arrive(B.tdone(k % kRing));
+    }
+    __device__ __forceinline__ void drain(const Q8WLaunch &) {}
+    static __device__ __forceinline__ void epilogue(const Q8WLaunch &, const ItemRec &, int, unsigned char *, const Bars &,
+                                                    uint32_t) {}
+};
+
 // An item's outputs, once all its units are decoded (table warps).
 template <class Cons>
 __device__ __forceinline__ bool finish_item(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm, const Bars &B,
@@ -1293,6 +1575,7 @@ __device__ __forceinline__ void serve_tables(const Q8WLaunch &L, unsigned char *
                 sm + L.lay.stage_e + (uint32_t)area * ((uint32_t)L.tbl_stage + kStagePad) * 2u);
             build_table<Cons::kFloat>(L, I.local, sm + 128 * I.tab, so, se + so[37]);
         }
+        if constexpr (Cons::kPrepare) Cons::prepare(L, I, k, sm, tmem);
         if (L.chain_scales && I.job > 0) {
             for (; done < k; done++)
                 if (!finish_item<Cons>(L, ring[done % kRing], done, sm, B, tmem, failed)) return;
@@ -1340,7 +1623,7 @@ __device__ __forceinline__ void decode_units(const Q8WLaunch &L, unsigned char *
             cur = d.item;
             if (!__all_sync(0xffffffffu, wait_bar(B.tfull(cur % kRing), (uint32_t)(cur / kRing) & 1u, L, failed))) break;
             const ItemRec &I = ring[cur % kRing];
-            cons.begin_item(L, I);
+            cons.begin_item(L, I, cur);
             last = I.u0 + I.n;
             lw = (uint32_t)lane * 4u | (uint32_t)I.tab << 7;
         }
@@ -1354,7 +1637,12 @@ __device__ __forceinline__ void decode_units(const Q8WLaunch &L, unsigned char *
     cons.drain(L);
 }
 
-__device__ __forceinline__ uint32_t tmem_cols(int W) { return W <= 1 ? 32u : W <= 2 ? 64u : W <= 4 ? 128u : W <= 8 ? 256u : 512u; }
+// TMEM columns: 32 per decode warp, and the backward's G
+template <class Cons>
+__device__ __forceinline__ uint32_t tmem_cols(int W) {
+    if (Cons::kPrepare) W += 2;
+    return W <= 1 ? 32u : W <= 2 ? 64u : W <= 4 ? 128u : W <= 8 ? 256u : 512u;
+}
 
 template <class Cons>
 __global__ void __launch_bounds__(32 * (kFirstDecode + Cons::kMaxDecode), 1) q8w_kernel(const __grid_constant__ Q8WLaunch L) {
@@ -1379,7 +1667,7 @@ __global__ void __launch_bounds__(32 * (kFirstDecode + Cons::kMaxDecode), 1) q8w
     fence_mbar_init();
     uint32_t tmem = 0;
     if (Cons::kMma) {
-        if (warp == 0) tmem_alloc(misc + 1, tmem_cols(L.W));
+        if (warp == 0) tmem_alloc(misc + 1, tmem_cols<Cons>(L.W));
         tcgen05_fence_before();
     }
     __syncthreads();
@@ -1394,7 +1682,7 @@ __global__ void __launch_bounds__(32 * (kFirstDecode + Cons::kMaxDecode), 1) q8w
     if (Cons::kMma) {
         tcgen05_fence_before();
         __syncthreads();
-        if (warp == 0) tmem_dealloc(tmem, tmem_cols(L.W));
+        if (warp == 0) tmem_dealloc(tmem, tmem_cols<Cons>(L.W));
     } else {
         __syncthreads();
     }
@@ -1407,7 +1695,7 @@ Q8WLayout layout(const Q8WLaunch &L, int W, int S) {
     auto up = [](uint32_t p) { return (p + 127u) & ~127u; };
     uint32_t p = kLutBytes;
     o.tiles = p;
-    if constexpr (Cons::kMma) p += (uint32_t)W * Cons::tile_bytes(L.xrows);
+    p += (uint32_t)W * Cons::tile_bytes(L.xrows);
     o.slots = p = up(p);
     p += (uint32_t)S * L.slot_bytes;
     o.red = p;
@@ -1503,6 +1791,11 @@ mv_status q8w_launch_fwd(const Q8WLaunch &L0, int warps, int units, cudaStream_t
     L.xrows = (L.batch + 7) & ~7;
     if (L.batch == 1) return launch_t<FwdDot>(L, warps, units, st);
     return launch_t<FwdCons>(L, warps, units, st);
+}
+
+mv_status q8w_launch_bwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st) {
+    if (L.batch == 1) return launch_t<BwdDot>(L, warps, units, st);
+    return launch_t<BwdCons>(L, warps, units, st);
 }
 
 }  // namespace mv

@@ -70,3 +70,24 @@ def test_float_forward_units(rows, cols, seg_quads, local):
         assert ((y.double() - ref).abs() / mag.clamp_min(1e-30)).max().item() < 2.0 ** -24 * (cols / 16 + 20), B
         assert torch.equal(y, M.matvec_bf16(x, s)), B
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads,local", [
+    (33, 16, 0, True), (257, 1040, 4, False), (96, 2048, 68, True), (1500, 272, 12, True), (64, 8192, 128, False)])
+def test_float_backward_units(rows, cols, seg_quads, local):
+    # one vector (CUDA cores), the sums by vector (to 4) and by row (from 5), the 32-vector pass.  s . dy enters as two
+    # bf16 terms (2^-17 of it, or exactly, at one vector); at most rows + 32 fp32 additions of 2^-23 each, tensor cores
+    # truncating: relative to the sum of the magnitudes of a column's terms
+    rng = np.random.default_rng(rows + cols + seg_quads)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, local=local, seg_quads=seg_quads)
+    s = torch.from_numpy(rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)).cuda()
+    W64 = torch.from_numpy(W).cuda().double()
+    for B in (1, 2, 4, 5, 31, 32, 33):
+        dy = torch.from_numpy(rng.standard_normal((B, rows)).astype(np.float32)).cuda().to(torch.bfloat16)
+        dx = M.matvec_t_bf16(dy, s)
+        ref = (dy.double() * s.double()) @ W64
+        mag = (dy.double() * s.double()).abs() @ W64.abs()
+        bound = (0.0 if B == 1 else 2.0 ** -17) + 2.0 ** -23 * (rows + 32)
+        assert ((dx.double() - ref).abs() / mag.clamp_min(1e-30)).max().item() < bound, B
+    assert ops.device_status() == 0
