@@ -92,25 +92,92 @@ mv_status check_shape(const mv_q8_tuning &t, bool mma, int nv, int max_blk_rows,
     return MV_OK;
 }
 
-// Parts per stripe of a single matrix, from the time of the busiest CTA: its units in rounds of kDecodeWarps (a step
-// of a lone warp takes ~70 cycles, of a full CTA ~9 per warp), no less than its table builds (~2500 cycles each),
-// plus, with more than one part, `split` (for y: its zeroing and the atomics, ~5000 cycles).
-int default_parts(int nseg, int seg_quads, int stripes, long long split) {
-    constexpr long long kDecodeWarps = 15, kBuild = 6000;
+// How one matrix is spread over the CTAs: whole stripes (parts = 1), every stripe in `parts` ranges of its segments, or
+// the units in even shares (parts = 0), which only cuts the stripes at the borders between two CTAs' shares.
+//
+// Chosen by the time of the busiest CTA, in cycles: its units, at `step` a quad with all warps at work and `lone` a
+// quad of a warp's own pace, and no less than its items' service by the table warps (a table build of ~6000 cycles, and
+// the epilogue); to that, what joining cut stripes takes (zeroing launch, scaling launch, atomics).  Measured on a B200,
+// whole stripes | even shares | the best aligned parts, 16 int8 vectors: 11008x4096 (3 items on some CTAs, 2 on others)
+// 38.8 | 38.0 | 40.4 us, 6000x6000 34.9 | 30.1 | 31.4, 2400x11008 32.8 | 25.3 | 29.1, 500x2992 17.5 | 12.5 | 11.9; the
+// same, one vector: 24.8 | 27.0 | 31.4, 24.2 | 23.2 | 24.1, 22.2 | 19.6 | 20.7, 12.0 | 12.0 | 12.2.  The backward adds to
+// dX by atomics in any case: 11008x4096, 64 vectors, 144.6 | 131.5 us.
+struct Cost {
+    int step, lone;
+    int service;     // cycles an item takes the table warps
+    int join_parts;  // every stripe cut; and ~50 of a part's `outputs` a cycle are added
+    long long outputs;
+    int join_even;   // the stripes at the borders of the shares cut
+};
+int choose_parts(int nseg, int seg_quads, int stripes, const Cost &c) {
+    constexpr long long kDecodeWarps = 14, kBuild = 3500;
     const long long G = sm_count();
+    auto time = [&](long long units, long long items) {
+        const long long rounds = (units + kDecodeWarps - 1) / kDecodeWarps;
+        return std::max(seg_quads * std::max(rounds * c.lone, units * c.step) + items * kBuild, items * c.service) + c.service;
+    };
     int best = 1;
     long long best_cost = -1;
     for (int p = 1; p <= 64 && p <= nseg; p++) {
-        const long long items = ((long long)stripes * p + G - 1) / G, units = items * ((nseg + p - 1) / p);
-        const long long rounds = (units + kDecodeWarps - 1) / kDecodeWarps;
-        const long long cost =
-            std::max(seg_quads * std::max(rounds * 70, units * 9), items * kBuild) + (p > 1 ? split : 0);
+        const long long items = ((long long)stripes * p + G - 1) / G;
+        const long long cost = time(items * ((nseg + p - 1) / p), items) + (p > 1 ? c.join_parts + c.outputs * p / 50 : 0);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = p;
         }
     }
+    const long long all = (long long)stripes * nseg;
+    if (all > G && all < 0x7FFFFFFF) {
+        const long long units = (all + G - 1) / G;
+        if (time(units, units / nseg + 2) + c.join_even < best_cost) best = 0;
+    }
     return best;
+}
+
+// The stripes that even shares cut: each border inside a stripe, the first of those in the same stripe.  kScale:
+// the sums are complete, ys = y s (float form: in place); otherwise they are set to zero before the product.
+template <typename T, bool kScale>
+__global__ void __launch_bounds__(256) cut_stripes(T *y, float *ys, const float *scales, int rows, int batch, uint32_t nseg,
+                                                   uint32_t span, uint32_t shares) {
+    const uint32_t b = blockIdx.x + 1, p = (uint32_t)((uint64_t)b * span / shares), stripe = p / nseg;
+    const uint32_t q = (uint32_t)((uint64_t)(b - 1) * span / shares);
+    if (p == stripe * nseg || q > stripe * nseg) return;
+    const int row = (int)stripe * 32 + (int)(threadIdx.x & 31);
+    if (row >= rows) return;
+    const float s = kScale ? scales[row] : 0.f;
+    for (int v = threadIdx.x >> 5; v < batch; v += 8) {
+        const size_t i = (size_t)v * rows + row;
+        if (kScale) ys[i] = (float)y[i] * s;
+        else y[i] = 0;
+    }
+}
+template <typename T, bool kScale>
+mv_status cut_stripes_launch(const Q8WLaunch &L, T *y, float *ys, cudaStream_t st) {
+    const uint32_t shares = std::min<uint32_t>(L.span, (uint32_t)sm_count());
+    cut_stripes<T, kScale><<<shares - 1, 256, 0, st>>>(y, ys, L.job0.scales, L.job0.m.rows, L.batch, (uint32_t)L.job0.m.nseg,
+                                                      L.span, shares);
+    MV_CUDA_TRY(cudaGetLastError(), "cut_stripes launch");
+    return MV_OK;
+}
+
+// Work items of a single-matrix launch: parts as asked for, or as chosen.  Returns the most units a CTA can get.
+int plan_single(Q8WLaunch &L, const mv_q8_tuning &t, const Cost &c) {
+    const mv_q8_view &m = L.job0.m;
+    const int stripes = (m.rows + 31) / 32;
+    const int parts = t.parts > 0 ? t.parts : choose_parts(m.nseg, m.seg_quads, stripes, c);
+    uint32_t items = 0;
+    plan_job(L.job0, t, items, parts > 0 ? parts : 1);
+    L.jobs = nullptr;
+    L.njobs = 1;
+    L.nitems = items;
+    long long units;
+    if (parts == 0) {
+        L.nitems = L.span = (uint32_t)stripes * (uint32_t)m.nseg;
+        units = (L.span + sm_count() - 1) / sm_count();
+    } else {
+        units = ((long long)items + sm_count() - 1) / sm_count() * ((m.nseg + L.job0.ngroups - 1) / L.job0.ngroups);
+    }
+    return (int)std::min<long long>(units, 1 << 20);
 }
 
 // Single matrix through the persistent kernel (one inline job): passes of up to 64 vectors on the tensor cores, of
@@ -133,13 +200,12 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.job0.y = y + (size_t)v0 * m->rows;
         L.job0.scales = scales;
         L.job0.ys = ys ? ys + (size_t)v0 * m->rows : nullptr;
-        uint32_t items = 0;
-        const int stripes = (m->rows + 31) / 32;
-        plan_job(L.job0, t, items, t.parts > 0 ? t.parts : default_parts(m->nseg, m->seg_quads, stripes, 5000));
+        const int nv = nv_round(nb);
+        const Cost cost{mma ? 18 + nb / 4 : 9 + nv, mma ? 220 : 90, 6000 + 100 * nb, 5000 + 60 * nb + (ys ? 3000 : 0),
+                        (long long)nb * m->rows, 9000 + 250 * nb + (ys ? 7000 : 0)};
+        const int units = plan_single(L, t, cost);
+        float *out = L.job0.ys;
         if (L.job0.atomic) L.job0.ys = nullptr;
-        L.jobs = nullptr;
-        L.njobs = 1;
-        L.nitems = items;
         L.batch = nb;
         L.status = status;
         L.spin_limit = wait_spin_limit();
@@ -148,11 +214,16 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
         if (L.job0.atomic)
             MV_CUDA_TRY(cudaMemsetAsync(L.job0.y, 0, sizeof(int32_t) * (size_t)nb * m->rows, st), "cudaMemsetAsync(y)");
-        const int spp = (m->nseg + L.job0.ngroups - 1) / L.job0.ngroups;
-        const long long per_cta = ((long long)items + sm_count() - 1) / sm_count() * spp;
-        rc = q8w_launch_int(L, nv_round(nb), mma, tuning && tuning->warps > 0 ? t.warps : 0,
-                            (int)std::min<long long>(per_cta, 1 << 20), st);
+        if (L.span) {
+            rc = cut_stripes_launch<int32_t, false>(L, L.job0.y, nullptr, st);
+            if (rc) return rc;
+        }
+        rc = q8w_launch_int(L, nv, mma, tuning && tuning->warps > 0 ? t.warps : 0, units, st);
         if (rc) return rc;
+        if (L.span && out) {
+            rc = cut_stripes_launch<int32_t, true>(L, L.job0.y, out, st);
+            if (rc) return rc;
+        }
         if (ys && L.job0.atomic) {
             const int n = nb * m->rows;
             scale_rows_kernel<<<(n + 255) / 256, 256, 0, st>>>(L.job0.y, scales, ys + (size_t)v0 * m->rows, m->rows,
@@ -183,24 +254,36 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
         L.job0.x = reinterpret_cast<const int8_t *>(x + (size_t)v0 * m->cols);
         L.job0.scales = scales;
         L.job0.ys = y + (size_t)v0 * m->rows;
-        uint32_t items = 0;
-        plan_job(L.job0, t, items, 1);
-        L.njobs = 1;
-        L.nitems = items;
         L.batch = std::min(64, batch - v0);
+        // whole stripes, or even shares where no stripe is cut twice: a sum of two parts does not depend on their order
+        // (11008x4096, whole | even: one vector 29.5 | 32.0 us, 16 vectors 48.5 | 52.1, 64 vectors 94.3 | 83.6)
+        constexpr int kNever = 1 << 30;
+        const Cost cost{L.batch == 1 ? 15 : 24 + L.batch / 2, L.batch == 1 ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,
+                        t.parts <= 0 && (m->rows + 31) / 32 >= sm_count() ? 20000 : kNever};
+        mv_q8_tuning by_rule = t;
+        by_rule.parts = 0;
+        const int units = plan_single(L, by_rule, cost);
         L.status = status;
         L.spin_limit = wait_spin_limit();
         L.drop_copy = inject_drop_copy();
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
-        const long long per_cta = ((long long)items + sm_count() - 1) / sm_count() * m->nseg;
-        rc = q8w_launch_fwd(L, asked ? t.warps : 0, (int)std::min<long long>(per_cta, 1 << 20), st);
+        if (L.span) {
+            rc = cut_stripes_launch<float, false>(L, L.job0.ys, nullptr, st);
+            if (rc) return rc;
+        }
+        rc = q8w_launch_fwd(L, asked ? t.warps : 0, units, st);
         if (rc) return rc;
+        if (L.span) {
+            rc = cut_stripes_launch<float, true>(L, L.job0.ys, L.job0.ys, st);
+            if (rc) return rc;
+        }
     }
     return MV_OK;
 }
 
-// Transposed product: passes of 32 vectors, added to dX by atomics, so that stripes may be split.
+// Transposed product: passes of 32 vectors, added to dX by atomics, so that stripes may be split.  The tensor cores'
+// sums leave by 16-byte reductions: a dX off that grid takes the one-vector form, whose reductions are scalars.
 mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float *scales, float *dx,
                  const mv_q8_tuning *tuning, cudaStream_t st) {
     mv_status rc;
@@ -215,27 +298,22 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
     if (need > (size_t)max_smem_optin())
         return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
     MV_CUDA_TRY(cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)batch * m->cols, st), "memset(dx)");
-    const int stripes = (m->rows + 31) / 32;
-    const int parts = t.parts > 0 ? t.parts : default_parts(m->nseg, m->seg_quads, stripes, 0);
-    for (int v0 = 0; v0 < batch; v0 += 32) {
+    const int pass = ((uintptr_t)dx & 15) ? 1 : 32;
+    for (int v0 = 0; v0 < batch; v0 += pass) {
         Q8WLaunch L{};
         L.job0.m = *m;
         L.job0.x = reinterpret_cast<const int8_t *>(dy + (size_t)v0 * m->rows);
         L.job0.scales = scales;
         L.job0.ys = dx + (size_t)v0 * m->cols;
-        uint32_t items = 0;
-        plan_job(L.job0, t, items, parts);
-        L.njobs = 1;
-        L.nitems = items;
-        L.batch = std::min(32, batch - v0);
+        L.batch = std::min(pass, batch - v0);
+        const Cost cost{L.batch == 1 ? 20 : 28 + L.batch / 4, L.batch == 1 ? 90 : 220, 6000, 0, 0, L.batch == 1 ? 8000 : 0};
+        const int units = plan_single(L, t, cost);
         L.status = status;
         L.spin_limit = wait_spin_limit();
         L.drop_copy = inject_drop_copy();
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
-        const int spp = (m->nseg + L.job0.ngroups - 1) / L.job0.ngroups;
-        const long long per_cta = ((long long)items + sm_count() - 1) / sm_count() * spp;
-        rc = q8w_launch_bwd(L, asked ? t.warps : 0, (int)std::min<long long>(per_cta, 1 << 20), st);
+        rc = q8w_launch_bwd(L, asked ? t.warps : 0, units, st);
         if (rc) return rc;
     }
     return MV_OK;

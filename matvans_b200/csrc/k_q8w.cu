@@ -304,7 +304,9 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
     const uint32_t slots = smem_u32(sm) + L.lay.slots;
     const uint32_t S = (uint32_t)L.S, W = (uint32_t)L.W;
     uint32_t u = 0, recorded = 0;  // units published, units of the items recorded
-    uint32_t next = blockIdx.x;  // the CTA's latest item number; its first one is static
+    // the CTA's latest item number (even shares: its first unit); its first one is static
+    uint32_t next = L.span ? (uint32_t)((uint64_t)blockIdx.x * L.span / gridDim.x) : blockIdx.x;
+    const uint32_t limit = L.span ? (uint32_t)((uint64_t)(blockIdx.x + 1) * L.span / gridDim.x) : L.nitems;
     uint32_t grabbed = 0;        // lane 0: the queue's answer for the item after it
     int job = 0, tjob = -1, tstripe = -1, gen = -1;
     int fb1 = -1, fb2 = -1;  // first items of the two latest table builds (fb1 the latest)
@@ -315,14 +317,21 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
     auto record = [&](int k) {
         if (k >= kRing && ok) ok = wait_bar(B.idone(k % kRing), (uint32_t)(k / kRing - 1) & 1u, L, failed);
         ItemRec r{};
-        const bool end = next >= L.nitems;
+        const bool end = next >= limit;
         r.it = end ? -1 : (int32_t)next;
         r.n = W;  // one end mark per decode warp
         r.u0 = recorded;
         r.area_item = -1;
         if (!end) {
             int se = 0;
-            locate(L, next, job, r.stripe, r.sb, se);
+            if (L.span) {
+                const uint32_t nseg = (uint32_t)L.job0.m.nseg;
+                r.stripe = (int)(next / nseg);
+                r.sb = (int)(next - (uint32_t)r.stripe * nseg);
+                se = (int)min(nseg, (uint32_t)r.sb + (limit - next));
+            } else {
+                locate(L, next, job, r.stripe, r.sb, se);
+            }
             if (L.queue && lane == 0) grabbed = atomicAdd(L.queue, 1u);
             r.job = job;
             r.n = (uint32_t)max(0, se - r.sb);
@@ -331,7 +340,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
             r.cols = J.m.cols;
             r.seg_quads = J.m.seg_quads;
             r.local = J.m.local;
-            r.atomic = J.atomic;
+            r.atomic = L.span ? (int)r.n < J.m.nseg : J.atomic;
             r.x = J.x;
             r.y = J.y;
             r.scales = J.scales;
@@ -371,7 +380,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
         ItemRec rn{};
         bool ahead = end;
         auto look_ahead = [&]() {
-            next = L.queue ? __shfl_sync(0xffffffffu, grabbed, 0) + gridDim.x : next + gridDim.x;
+            next = L.queue ? __shfl_sync(0xffffffffu, grabbed, 0) + gridDim.x : next + (L.span ? r.n : gridDim.x);
             // the counter is reset by whoever makes the launch's last grab
             if (L.queue && lane == 0 && next == L.nitems + gridDim.x - 1) atomicExch(L.queue, 0u);
             rn = record(k + 1);
@@ -946,15 +955,20 @@ struct MmaCons {
                         for (int j = 0; j < 16; j++) sum[j] += __shfl_down_sync(0xffffffffu, sum[j], 16);
                     const int v = 16 * q + lane - (int)base, row0 = I.stripe * 32 + h;
                     if ((uint32_t)lane >= base && (uint32_t)lane < base + 16u && v < L.batch) {
-                        if (!I.atomic && row0 + 16 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.y & 15) == 0) {
+                        if (!I.atomic && row0 + 16 <= I.rows && (I.rows & 3) == 0 && (((uintptr_t)I.y | (uintptr_t)I.ys) & 15) == 0) {
                             int4 *dst = reinterpret_cast<int4 *>(I.y + (size_t)v * I.rows + row0);
 #pragma unroll
                             for (int j = 0; j < 4; j++)
                                 dst[j] = make_int4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
-                            if (I.ys)
+                            if (I.ys) {
+                                float4 *ds = reinterpret_cast<float4 *>(I.ys + (size_t)v * I.rows + row0);
 #pragma unroll
-                                for (int j = 0; j < 16; j++)
-                                    I.ys[(size_t)v * I.rows + row0 + j] = (float)sum[j] * __ldg(I.scales + row0 + j);
+                                for (int j = 0; j < 4; j++) {
+                                    const float *sc = I.scales + row0 + 4 * j;
+                                    ds[j] = make_float4((float)sum[4 * j] * __ldg(sc), (float)sum[4 * j + 1] * __ldg(sc + 1),
+                                                        (float)sum[4 * j + 2] * __ldg(sc + 2), (float)sum[4 * j + 3] * __ldg(sc + 3));
+                                }
+                            }
                         } else {
 #pragma unroll
                             for (int j = 0; j < 16; j++)
@@ -1139,7 +1153,11 @@ struct FwdCons {
                 const int row0 = I.stripe * 32 + h;
                 if (lane < 16 && v < L.batch) {
                     float *dst = I.ys + (size_t)v * I.rows + row0;
-                    if (row0 + 16 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.ys & 15) == 0) {
+                    if (I.atomic) {  // even shares: the other CTA's part is added, and scaled with it afterwards
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (row0 + j < I.rows) atomicAdd(dst + j, sum[j]);
+                    } else if (row0 + 16 <= I.rows && (I.rows & 3) == 0 && ((uintptr_t)I.ys & 15) == 0) {
 #pragma unroll
                         for (int j = 0; j < 16; j += 4)
                             *reinterpret_cast<float4 *>(dst + j) = make_float4(
@@ -1247,7 +1265,9 @@ struct FwdDot {
         uint32_t w = I.u0 % W;
         float sum = 0.f;
         for (uint32_t i = 0; i < nc; i++, w = w + 1 < W ? w + 1 : 0) sum += red[w * 32];
-        if (row < I.rows) I.ys[row] = sum * __ldg(I.scales + row);
+        if (row >= I.rows) return;
+        if (I.atomic) atomicAdd(I.ys + row, sum);  // even shares: scaled together with the other CTA's part afterwards
+        else I.ys[row] = sum * __ldg(I.scales + row);
     }
 };
 

@@ -28,6 +28,9 @@ struct Q8WLaunch {
     const float *chain_scales;
     int8_t *chain_out8;
     uint32_t *queue;  // work queue of a stack (jobs[0].pad of the job table), or nullptr: static round robin
+    // One job in even shares (nonzero: its number of units): CTA c of G takes units [c span / G, (c + 1) span / G),
+    // whatever stripes they are of.  Sums of a stripe that several CTAs share are added to y (ys) unscaled.
+    uint32_t span;
     // set by the launcher
     int W, S;              // decode warps, stream slots
     uint32_t S_inv;        // ceil(2^32 / S): unit / S by multiplication

@@ -91,3 +91,33 @@ def test_float_backward_units(rows, cols, seg_quads, local):
         bound = (0.0 if B == 1 else 2.0 ** -17) + 2.0 ** -23 * (rows + 32)
         assert ((dx.double() - ref).abs() / mag.clamp_min(1e-30)).max().item() < bound, B
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads", [(2400, 11008, 0), (4736 + 40, 3104, 64), (7001, 5008, 0)])
+def test_even_shares(rows, cols, seg_quads):
+    # CTAs that share stripes at the borders of their units, whole ranges of stripes in between, the short last segment
+    # and the ragged last stripe; exact sums, their scaled form, and the float form both ways (bounds as above; the
+    # forward is the same bit for bit whatever the order its parts arrive in)
+    rng = np.random.default_rng(rows)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, seg_quads=seg_quads)
+    s = rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)
+    sd, W64 = torch.from_numpy(s).cuda(), torch.from_numpy(W).cuda().double()
+    for B in (1, 5, 16, 64):
+        x = rng.integers(-128, 128, size=(B, cols)).astype(np.int8)
+        y, ys = M.matvec(torch.from_numpy(x), scales=s)
+        ref = torch.from_numpy(x).cuda().double() @ W64.T
+        assert torch.equal(y.double(), ref), B
+        assert torch.equal(ys, ref.float() * sd), B
+        assert torch.equal(M.matvec(torch.from_numpy(x)), y), B
+        xf = torch.from_numpy(rng.standard_normal((B, cols)).astype(np.float32)).cuda().to(torch.bfloat16)
+        yf = M.matvec_bf16(xf, sd)
+        mag = (xf.double().abs() @ W64.abs().T) * sd.double()
+        err = (yf.double() - (xf.double() @ W64.T) * sd.double()).abs() / mag
+        assert err.max().item() < 2.0 ** -24 * (cols / 16 + 20), B
+        assert torch.equal(yf, M.matvec_bf16(xf, sd)), B
+        dy = torch.from_numpy(rng.standard_normal((B, rows)).astype(np.float32)).cuda().to(torch.bfloat16)
+        g = dy.double() * sd.double()
+        err = (M.matvec_t_bf16(dy, sd).double() - g @ W64).abs() / (g.abs() @ W64.abs())
+        assert err.max().item() < (0.0 if B == 1 else 2.0 ** -17) + 2.0 ** -23 * (rows + 32), B
+    assert ops.device_status() == 0
