@@ -11,7 +11,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import Q8Job, Q8StackInfo, Q8Tuning, Q8View, check, lib
+from ._lib import MMA_MIN_BATCH, Q8Job, Q8StackInfo, Q8Tuning, Q8View, check, lib  # noqa: F401 (MMA_MIN_BATCH: ops' users)
 
 _STATUS_BITS = {1: "stream overrun", 2: "final coder state mismatch", 4: "wait timeout", 8: "bad table"}
 
