@@ -213,13 +213,14 @@ mv_status mv_q8_matvec(const mv_q8_view *m, const int8_t *x_dev, int batch, int3
  *   parts        work items per 32-row stripe (its segments split in `parts`
  *                ranges; default: whole stripes in stacks, enough parts to
  *                fill the GPU for a single matrix)
- *   engine       int8 product of 3 or more vectors: 0 = tensor cores
- *                (tcgen05.mma kind::i8, TMEM accumulators, up to 64 vectors
- *                per decode), 1 = CUDA cores (dp4a, up to 16).  One or two
- *                vectors always use dp4a. */
+ *   engine       int8 product: 0 = the library's choice by batch and size:
+ *                from MV_MMA_MIN_VECTORS vectors on it may be the tensor
+ *                cores (tcgen05.mma kind::i8, TMEM accumulators, up to 64
+ *                vectors per decode), below the CUDA cores (dp4a); 1 = CUDA
+ *                cores (up to 16 vectors per decode). */
 #define MV_ENGINE_AUTO 0
 #define MV_ENGINE_DP4A 1
-/* Smallest integer batch that engine 0 (MV_ENGINE_AUTO) runs on the tensor
+/* Smallest integer batch that engine 0 (MV_ENGINE_AUTO) can run on the tensor
  * cores. */
 #define MV_MMA_MIN_VECTORS 3
 typedef struct mv_q8_tuning {

@@ -32,7 +32,7 @@ SINGLE_CANDIDATES = CANDIDATES + [(w, ilp, d, 0, p, 0) for w in (4, 8) for ilp i
 
 def candidates_for(batch, base):
     """Candidates at `batch` vectors: from MMA_MIN_BATCH (3) vectors on they run
-    on the tensor cores (engine 0, where ilp is fixed at 1) or on the CUDA cores
+    on the library's choice (engine 0, with ilp 1) or on the CUDA cores
     (engine 1); fewer vectors always use the CUDA cores."""
     if batch < _lib.MMA_MIN_BATCH:
         return list(base)

@@ -34,11 +34,37 @@ __global__ void q8s_scale_atomic_y(const Q8Job *jobs, int njobs, int batch) {
     }
 }
 
+// n 32-bit zeros.  (A memset between kernels costs more than a small kernel: 500x2992 and 160x4096, one vector, four
+// parts, 12.3 us with cudaMemsetAsync, 9.6 with this.)
+__global__ void __launch_bounds__(256) zero_words(uint32_t *p, size_t n) {
+    const size_t head = min(n, (size_t)((16 - ((uintptr_t)p & 15)) & 15) / 4), n4 = (n - head) / 4;
+    const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    uint4 *q = reinterpret_cast<uint4 *>(p + head);
+    for (size_t i = i0; i < n4; i += step) q[i] = make_uint4(0, 0, 0, 0);
+    if (i0 < head) p[i0] = 0;
+    const size_t t = head + 4 * n4 + i0;
+    if (t < n) p[t] = 0;
+}
+
 namespace {
 
-// Integer batches of at least this many vectors go to the tensor-core consumer (engine 0), whose cost hardly depends
-// on the batch, while the dp4a consumer's grows with it.
-constexpr int kMmaMinVectors = MV_MMA_MIN_VECTORS;
+mv_status zero_launch(void *p, size_t words, cudaStream_t st) {
+    const unsigned grid = (unsigned)std::min<size_t>((words + 1023) / 1024, 4 * (size_t)sm_count());
+    zero_words<<<std::max(1u, grid), 256, 0, st>>>(static_cast<uint32_t *>(p), words);
+    MV_CUDA_TRY(cudaGetLastError(), "zero_words launch");
+    return MV_OK;
+}
+
+// Integer batches of at least this many vectors go to the tensor-core consumer with engine 0, whose cost hardly depends
+// on the batch, while the dp4a consumer's grows with it.  Measured on a B200, dp4a | tensor cores: 11008x4096, 4 vectors
+// 31.0 | 33.0 us, 6 vectors 37.5 | 33.2; 6000x6000, 26.3 | 30.4 and 31.6 | 30.5; a layer of seven matrices, 4 vectors
+// 92.7 | 99.2, 8 vectors 116.6 | 99.3.
+constexpr int kMmaMinVectors = 5;
+// A single matrix that gives no warp a second segment is bound by a lone warp's pace, which the tensor cores' tiles slow
+// down: dp4a up to 8 vectors (500x2992, 8 vectors: 10.5 | 13.0 us; 1024x1024: 9.5 | 10.2).
+constexpr int kMmaMinLone = 9;
+// check_shape: the batch from which a launch shape is taken as a tensor-core one.
+constexpr int kMmaShape = MV_MMA_MIN_VECTORS;
 
 int nv_round(int nb) { return nb <= 2 ? nb : nb <= 4 ? 4 : nb <= 8 ? 8 : 16; }
 
@@ -99,8 +125,8 @@ mv_status check_shape(const mv_q8_tuning &t, bool mma, int nv, int max_blk_rows,
 // quad of a warp's own pace, and no less than its items' service by the table warps (a table build of ~6000 cycles, and
 // the epilogue); to that, what joining cut stripes takes (zeroing launch, scaling launch, atomics).  Measured on a B200,
 // whole stripes | even shares | the best aligned parts, 16 int8 vectors: 11008x4096 (3 items on some CTAs, 2 on others)
-// 38.8 | 38.0 | 40.4 us, 6000x6000 34.9 | 30.1 | 31.4, 2400x11008 32.8 | 25.3 | 29.1, 500x2992 17.5 | 12.5 | 11.9; the
-// same, one vector: 24.8 | 27.0 | 31.4, 24.2 | 23.2 | 24.1, 22.2 | 19.6 | 20.7, 12.0 | 12.0 | 12.2.  The backward adds to
+// 38.8 | 38.0 | 40.4 us, 6000x6000 34.9 | 30.1 | 31.4, 2400x11008 32.8 | 25.3 | 29.1, 500x2992 17.5 | 12.5 | 12.1; the
+// same, one vector: 24.8 | 27.0 | 31.4, 24.2 | 23.2 | 24.1, 22.2 | 19.6 | 21.4, 12.1 | - | 9.3.  The backward adds to
 // dX by atomics in any case: 11008x4096, 64 vectors, 144.6 | 131.5 us.
 struct Cost {
     int step, lone;
@@ -110,7 +136,7 @@ struct Cost {
     int join_even;   // the stripes at the borders of the shares cut
 };
 int choose_parts(int nseg, int seg_quads, int stripes, const Cost &c) {
-    constexpr long long kDecodeWarps = 14, kBuild = 3500;
+    constexpr long long kDecodeWarps = 14, kBuild = 4800;
     const long long G = sm_count();
     auto time = [&](long long units, long long items) {
         const long long rounds = (units + kDecodeWarps - 1) / kDecodeWarps;
@@ -170,6 +196,7 @@ int plan_single(Q8WLaunch &L, const mv_q8_tuning &t, const Cost &c) {
     L.jobs = nullptr;
     L.njobs = 1;
     L.nitems = items;
+    L.span = 0;
     long long units;
     if (parts == 0) {
         L.nitems = L.span = (uint32_t)stripes * (uint32_t)m.nseg;
@@ -191,8 +218,8 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
     const int pass = t.engine == MV_ENGINE_AUTO ? 64 : 16;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         const int nb = std::min(pass, batch - v0);
-        const bool mma = t.engine == MV_ENGINE_AUTO && nb >= kMmaMinVectors;
-        rc = check_shape(t, mma, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
+        bool mma = t.engine == MV_ENGINE_AUTO && nb >= kMmaMinVectors;
+        rc = check_shape(t, t.engine == MV_ENGINE_AUTO && nb >= kMmaShape, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
         if (rc) return rc;
         Q8WLaunch L{};
         L.job0.m = *m;
@@ -201,9 +228,15 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.job0.scales = scales;
         L.job0.ys = ys ? ys + (size_t)v0 * m->rows : nullptr;
         const int nv = nv_round(nb);
-        const Cost cost{mma ? 18 + nb / 4 : 9 + nv, mma ? 220 : 90, 6000 + 100 * nb, 5000 + 60 * nb + (ys ? 3000 : 0),
-                        (long long)nb * m->rows, 9000 + 250 * nb + (ys ? 7000 : 0)};
-        const int units = plan_single(L, t, cost);
+        auto cost = [&](bool mma) {
+            return Cost{mma ? 18 + nb / 4 : 9 + nv, mma ? 220 : 90, 6000 + 100 * nb, 3000 + 60 * nb + (ys ? 1000 : 0),
+                        (long long)nb * m->rows, 6000 + 250 * nb + (ys ? 4000 : 0)};
+        };
+        int units = plan_single(L, t, cost(mma && nb >= kMmaMinLone));
+        if (mma && nb < kMmaMinLone) {
+            mma = units > 10;  // more than a dp4a launch has warps for
+            if (mma) units = plan_single(L, t, cost(true));
+        }
         float *out = L.job0.ys;
         if (L.job0.atomic) L.job0.ys = nullptr;
         L.batch = nb;
@@ -212,8 +245,10 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.drop_copy = inject_drop_copy();
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
-        if (L.job0.atomic)
-            MV_CUDA_TRY(cudaMemsetAsync(L.job0.y, 0, sizeof(int32_t) * (size_t)nb * m->rows, st), "cudaMemsetAsync(y)");
+        if (L.job0.atomic) {
+            rc = zero_launch(L.job0.y, (size_t)nb * m->rows, st);
+            if (rc) return rc;
+        }
         if (L.span) {
             rc = cut_stripes_launch<int32_t, false>(L, L.job0.y, nullptr, st);
             if (rc) return rc;
@@ -297,7 +332,8 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
                         (mma ? 4224 + (size_t)t.warps * 2056 : 0) + 2 * ((size_t)m->tbl_stripe_max + 8) + 1024;
     if (need > (size_t)max_smem_optin())
         return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
-    MV_CUDA_TRY(cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)batch * m->cols, st), "memset(dx)");
+    rc = zero_launch(dx, (size_t)batch * m->cols, st);
+    if (rc) return rc;
     const int pass = ((uintptr_t)dx & 15) ? 1 : 32;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         Q8WLaunch L{};
@@ -306,7 +342,7 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
         L.job0.scales = scales;
         L.job0.ys = dx + (size_t)v0 * m->cols;
         L.batch = std::min(pass, batch - v0);
-        const Cost cost{L.batch == 1 ? 20 : 28 + L.batch / 4, L.batch == 1 ? 90 : 220, 6000, 0, 0, L.batch == 1 ? 8000 : 0};
+        const Cost cost{L.batch == 1 ? 20 : 28 + L.batch / 4, L.batch == 1 ? 90 : 220, 6000, 0, 0, L.batch == 1 ? 10000 : 0};
         const int units = plan_single(L, t, cost);
         L.status = status;
         L.spin_limit = wait_spin_limit();
@@ -436,7 +472,7 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
     L.chain_out8 = out8_dev;
     const int nv = mv::nv_round(batch);
     const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
-    rc = mv::check_shape(t, mma, nv, info->max_blk_rows, info->tbl_stripe_max);
+    rc = mv::check_shape(t, t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaShape, nv, info->max_blk_rows, info->tbl_stripe_max);
     if (rc) return rc;
     mv::q8s_chain_reset<<<(njobs + 255) / 256, 256, 0, st>>>(reinterpret_cast<mv::Q8Job *>(jobs_dev), njobs);
     MV_CUDA_TRY(cudaGetLastError(), "q8s_chain_reset launch");
@@ -467,7 +503,7 @@ mv_status mv_q8_stack_matvec(const mv_q8_job *jobs_dev, int njobs, const mv_q8_s
     if (info->nitems < 0x7FFFFFFFu) L.queue = const_cast<uint32_t *>(&jobs_dev[0].pad);
     const int nv = mv::nv_round(batch);
     const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
-    rc = mv::check_shape(t, mma, nv, info->max_blk_rows, info->tbl_stripe_max);
+    rc = mv::check_shape(t, t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaShape, nv, info->max_blk_rows, info->tbl_stripe_max);
     if (rc) return rc;
     dim3 zg(64, std::min(njobs, 1024));
     if (info->atomic_jobs > 0) {
