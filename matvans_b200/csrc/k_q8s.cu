@@ -229,7 +229,7 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.job0.ys = ys ? ys + (size_t)v0 * m->rows : nullptr;
         const int nv = nv_round(nb);
         auto cost = [&](bool mma) {
-            return Cost{mma ? 18 + nb / 4 : 9 + nv, mma ? 220 : 90, 6000 + 100 * nb, 3000 + 60 * nb + (ys ? 1000 : 0),
+            return Cost{mma ? (nb <= 16 ? 18 + nb / 4 : 23) : 9 + nv, mma ? 220 : 90, 6000 + 100 * nb, 3000 + 60 * nb + (ys ? 1000 : 0),
                         (long long)nb * m->rows, 6000 + 250 * nb + (ys ? 4000 : 0)};
         };
         int units = plan_single(L, t, cost(mma && nb >= kMmaMinLone));
@@ -291,7 +291,8 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
         L.job0.ys = y + (size_t)v0 * m->rows;
         L.batch = std::min(64, batch - v0);
         // whole stripes, or even shares where no stripe is cut twice: a sum of two parts does not depend on their order
-        // (11008x4096, whole | even: one vector 29.5 | 32.0 us, 16 vectors 48.5 | 52.1, 64 vectors 94.3 | 83.6)
+        // (whole | even: 11008x4096, one vector 29.5 | 32.0 us, 16 vectors 48.5 | 52.1, 64 vectors 57.6 | 64.9; 6000x6000, 16
+        // vectors 49.1 | 45.8, 64 vectors 57.8 | 56.5)
         constexpr int kNever = 1 << 30;
         const Cost cost{L.batch == 1 ? 15 : 24 + L.batch / 2, L.batch == 1 ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,
                         t.parts <= 0 && (m->rows + 31) / 32 >= sm_count() ? 20000 : kNever};

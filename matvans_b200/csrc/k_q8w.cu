@@ -23,7 +23,7 @@
 // One CTA-wide barrier per item, a table build and a cross-warp sum between the
 // items of the form this replaced left the SM idle for a third of a launch: the
 // seven matrices of a 7B layer took 139 us there with one vector and take 74 us,
-// with 16 vectors 136 and 109 us; 64 vectors of 11008x4096, 197 and 69 us.
+// with 16 vectors 136 and 109 us; 64 vectors of 11008x4096, 197 and 47 us.
 //
 // Decode table: entry (q, lane) = f | sym << 16 | r << 24 (frequency of the
 // symbol that owns quantile q, the symbol, r = q - cum), 4 bytes at byte
@@ -117,12 +117,13 @@ struct Bars {
     __device__ __forceinline__ uint32_t sempty(int s) const { return at(kFixed + S + s); }
     __device__ __forceinline__ uint32_t mma(int w) const { return at(kFixed + 2 * S + w); }
     __device__ __forceinline__ uint32_t dempty(int w, int b) const { return at(kFixed + 2 * S + W + 2 * w + b); }
-    static __host__ __device__ constexpr int count(int S, int W, bool mma) { return kFixed + 2 * S + (mma ? 3 * W : 0); }
+    __device__ __forceinline__ uint32_t xfull(int w, int b) const { return at(kFixed + 2 * S + 3 * W + 2 * w + b); }  // XTiles
+    static __host__ __device__ constexpr int count(int S, int W, bool mma) { return kFixed + 2 * S + (mma ? 5 * W : 0); }
     // arrivals that complete barrier i's phase
     __device__ __forceinline__ int arrivals(int i) const {
         if (i >= 2 * kRing && i < 3 * kRing) return (int)kTdone;
         if (i >= 4 * kRing && i < kFixed) return 33;  // the stager's lanes, and once for the offsets
-        return i >= kFixed + 2 * S + W ? kTableWarps : 1;  // dempty: every table warp has read the sums
+        return i >= kFixed + 2 * S + W && i < kFixed + 2 * S + 3 * W ? kTableWarps : 1;  // dempty: every table warp has read the sums
     }
 };
 
@@ -746,13 +747,70 @@ struct DotCons {
     __device__ __forceinline__ void drain(const Q8WLaunch &) {}
 };
 
+// x tiles of a decode warp, for consumers of a single matrix with up to 64 vectors: 64 bytes of every vector (a tile row,
+// swizzled), brought in by one tensor copy of lane 0.  (As 16-byte asynchronous copies by all lanes: MmaCons, 64 vectors,
+// 1400 cycles to issue a tile's copies, a quarter of the decode's time.)  With more than 16 vectors two buffers, the next
+// tile's copy a whole tile's decode ahead of its MMAs; a smaller tile comes in while its own weights decode, which leaves
+// the memory to the stream slots and so to more decode warps.  Measured on a B200, 64 vectors, before and after:
+// 11008x4096, int8 58 -> 46 us, bf16 84 -> 58; 4096x11008, 50 -> 40 and 81 -> 51.
+struct XTiles {
+    static __host__ __device__ constexpr uint32_t second(int xrows) { return xrows > 16 ? 1u : 0u; }  // a second buffer?
+    static constexpr uint32_t bytes(int xrows) { return (1u + second(xrows)) * 64u * (uint32_t)xrows; }
+    uint32_t at, bar, n;  // n: copies issued (lane 0)
+    uint64_t a_desc;
+    __device__ __forceinline__ void init(const Bars &B, int w, uint32_t address) {
+        at = address;
+        bar = B.xfull(w, 0);
+        n = 0;
+        a_desc = umma_smem_desc_sw64(address);
+    }
+    // tile i: columns from col on (its buffer's previous MMAs are done).  Once the CTA has failed nothing is copied any
+    // more: the waits for earlier tiles may have given up.
+    __device__ __forceinline__ void load(const Q8WLaunch &L, uint32_t i, int col, int lane, volatile uint32_t *failed) {
+        if (lane != 0 || *failed) return;
+        const uint32_t b = i & second(L.xrows), size = 64u * (uint32_t)L.xrows;
+        arrive_tx(bar + 8u * b, size);
+        asm volatile(
+            "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                at + b * size),
+            "l"(&L.xmap), "r"(col), "r"(0), "r"(bar + 8u * b)
+            : "memory");
+        n = i + 1;
+    }
+    // at a unit's start, and once the MMAs before tile i are done (the unit's tile at col, `next`: with one after it):
+    // `pitch` columns a tile
+    __device__ __forceinline__ void begin(const Q8WLaunch &L, uint32_t i, int col, int lane, volatile uint32_t *failed) {
+        if (second(L.xrows)) load(L, i, col, lane, failed);
+    }
+    __device__ __forceinline__ void refill(const Q8WLaunch &L, uint32_t i, int col, int pitch, bool next, int lane,
+                                           volatile uint32_t *failed) {
+        if (!second(L.xrows)) load(L, i, col, lane, failed);
+        else if (next) load(L, i + 1, col + pitch, lane, failed);
+    }
+    // lane 0: tile i is there; its descriptor
+    __device__ __forceinline__ uint64_t wait(const Q8WLaunch &L, uint32_t i, volatile uint32_t *failed) const {
+        const uint32_t two = second(L.xrows);
+        wait_bar(bar + 8u * (i & two), (i >> two) & 1u, L, failed);
+        return a_desc + (uint64_t)((i & two) * 4u * (uint32_t)L.xrows);
+    }
+    // no copy may be left writing when the CTA exits
+    __device__ __forceinline__ void drain(const Q8WLaunch &L, int lane) const {
+        if (lane != 0) return;
+        const uint32_t two = second(L.xrows);
+        for (uint32_t i = n <= two ? 0u : n - 1u - two; i < n; i++)
+            for (uint32_t it = 0; it < L.spin_limit; it++)
+                if (mbar_try_wait(bar + 8u * (i & two), (i >> two) & 1u)) break;
+    }
+};
+
 // Tensor-core consumer, up to 64 int8 vectors: D[vector][row] += x tile . W tile^T, kind::i8, exact int32.
-//   A = x: M = 64 vectors (rows past xrows read whatever follows and only reach lanes that are never read), K-major
-//       core matrices (8 vectors x 16 bytes), 64 columns at a time, brought in by the warp's own cp.async;
+//   A = x: M = 64 vectors (rows past xrows read whatever follows and only reach lanes that are never read), 64 columns
+//       at a time, K-major: by tensor copies (XTiles), or, kOwn, whose x may be one of many (stacks), as core matrices
+//       (8 vectors x 16 bytes) by the warp's own cp.async;
 //   B = W: the 32 rows of the stripe, each lane storing its row's 16-byte pieces (K-major, conflict-free);
 //   D: 32 TMEM columns per decode warp, vector v in lane 32 (v / 16) + v % 16.
 // Per 16 quads: two MMAs (K = 32) and one commit.  The previous pair's MMAs are waited for after the first 4 quads
-// of the next one are decoded, when W tile and x tile are rewritten; the x copies land during the other 12.
+// of the next one are decoded, when the W tile is rewritten (kOwn: and the x tile, whose copies land during the other 12).
 //
 // kOwn (up to 16 vectors): the A operand starts 16 rows per lane quarter early, so that the vectors land in the warp's
 // own quarter; the warp reads its sums itself after each unit and adds them to the item's in shared memory.  With more
@@ -765,10 +823,10 @@ struct MmaCons {
     static constexpr int kRed = kOwn ? 16 * kPitch : 0;
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;  // 32 rows x 64 columns
-    static constexpr uint32_t x_tile(int xrows) { return 64u * (uint32_t)xrows; }
-    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + x_tile(xrows); }
+    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + (kOwn ? 64u * (uint32_t)xrows : XTiles::bytes(xrows)); }
     const int8_t *x;
     int cols, seg_quads, qtot;
+    XTiles xs;  // !kOwn
     uint32_t wt, xt, d_tmem, lbo, nmma, ndp;  // nmma: commits so far, ndp: earlier items this warp has had a part in
     uint32_t mbar, dempty;                    // dempty: of the first accumulator; the second's follows
     uint64_t a_desc, b_desc;
@@ -781,7 +839,8 @@ struct MmaCons {
         lbo = 16u * (uint32_t)L.xrows;
         const uint32_t quarter = (uint32_t)(w + kFirstDecode) & 3u;  // of TMEM lanes, by the warp's number in the CTA
         d_tmem = tmem + 32u * (uint32_t)w;
-        a_desc = umma_smem_desc(kOwn ? xt - 256u * quarter : xt, lbo, 128u);
+        a_desc = umma_smem_desc(xt - 256u * quarter, lbo, 128u);
+        if (!kOwn) xs.init(B, w, xt);
         b_desc = umma_smem_desc(wt, 512u, 128u);
         mbar = B.mma(w);
         dempty = B.dempty(w, 0);
@@ -802,7 +861,7 @@ struct MmaCons {
     __device__ __forceinline__ void wait_acc(const Q8WLaunch &L, volatile uint32_t *failed) const {
         if (!kOwn && ndp >= 2) wait_bar(dempty + 8u * (ndp & 1u), (ndp / 2u - 1u) & 1u, L, failed);
     }
-    // 64 columns from col on of every vector: lane (r, c) copies chunk c (16 bytes) of vectors r, r + 8, ....  What
+    // kOwn: 64 columns from col on of every vector: lane (r, c) copies chunk c (16 bytes) of vectors r, r + 8.  What
     // is not there (vectors past the batch, columns past the row) is left as it is: it meets zero weights, or ends
     // up in accumulator lanes that are never read.
     __device__ __forceinline__ void copy_x(const Q8WLaunch &L, int col, int lane) const {
@@ -810,17 +869,8 @@ struct MmaCons {
         const int8_t *src = x + (size_t)r * cols + c;
         uint32_t dst = xt + (uint32_t)(lane >> 3) * lbo + (uint32_t)r * 16u;
         const int n = c < cols ? L.batch - r : 0;
-        if constexpr (kOwn) {
-            if (n > 0) cp_async_16(dst, src);
-            if (n > 8) cp_async_16(dst + 128u, src + 8 * (size_t)cols);
-        } else {
-#pragma unroll 2
-            for (int v = 0; v < n; v += 8) {
-                cp_async_16(dst, src);
-                src += 8 * (size_t)cols;
-                dst += 128u;
-            }
-        }
+        if (n > 0) cp_async_16(dst, src);
+        if (n > 8) cp_async_16(dst + 128u, src + 8 * (size_t)cols);
     }
     // four quads (16 columns) of the lane's row: piece c of the 64-column tile
     __device__ __forceinline__ void store_w(uint32_t c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int lane) const {
@@ -828,15 +878,16 @@ struct MmaCons {
                      "r"(w2), "r"(w3)
                      : "memory");
     }
-    // the previous MMAs are done with both tiles; the x copies have the rest of the decode to land in
-    __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, int lane, volatile uint32_t *failed) const {
+    // the previous MMAs are done with the tiles; the x copies have the rest of the decode to land in
+    __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, bool next, int lane, volatile uint32_t *failed) {
         if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
-        copy_x(L, col, lane);
+        if (kOwn) copy_x(L, col, lane);
+        else xs.refill(L, nmma, col, 64, next, lane, failed);
     }
     // the MMAs of a tile: two K steps of 32 columns, or one
     __device__ __forceinline__ void issue(const Q8WLaunch &L, bool two, int lane, volatile uint32_t *failed) {
         if (!any) wait_acc(L, failed);
-        cp_async_wait_all();
+        if (kOwn) cp_async_wait_all();
         fence_proxy_async_smem();  // both tiles are read by the tensor core (async proxy)
         tcgen05_fence_before();
         __syncwarp();
@@ -844,8 +895,9 @@ struct MmaCons {
             tcgen05_fence_after();
             const uint32_t idesc = umma_idesc_i8(64, 32);
             const uint32_t d = kOwn ? d_tmem : d_tmem + ((ndp & 1u) << 20);  // the second accumulator: 16 lanes further
-            umma_i8(d, a_desc, b_desc, idesc, any ? 1u : 0u);
-            if (two) umma_i8(d, a_desc + (lbo >> 3), b_desc + 64u, idesc, 1u);
+            const uint64_t a = kOwn ? a_desc : xs.wait(L, nmma, failed);
+            umma_i8(d, a, b_desc, idesc, any ? 1u : 0u);
+            if (two) umma_i8(d, a + (kOwn ? lbo >> 3 : 2u), b_desc + 64u, idesc, 1u);
             umma_commit(mbar);
         }
         __syncwarp();
@@ -856,6 +908,7 @@ struct MmaCons {
                                          uint32_t lw, int lane, volatile uint32_t *failed) {
         const int q0 = d.seg * seg_quads;
         const int nq = min(seg_quads, qtot - q0);
+        if (!kOwn) xs.begin(L, nmma, 4 * q0, lane, failed);
         Stream s(sm, soff, d.rows, lane);
         int q = 0;
         for (; q + 16 <= nq; q += 16) {
@@ -863,7 +916,7 @@ struct MmaCons {
             for (int c = 0; c < 4; c++) {
                 const uint32_t w0 = s.step_i8(sm, lw), w1 = s.step_i8(sm, lw), w2 = s.step_i8(sm, lw), w3 = s.step_i8(sm, lw);
                 s.clamp();
-                if (c == 0) refill_tiles(L, 4 * (q0 + q), lane, failed);
+                if (c == 0) refill_tiles(L, 4 * (q0 + q), q + 16 < nq, lane, failed);
                 store_w((uint32_t)c, w0, w1, w2, w3, lane);
             }
             issue(L, true, lane, failed);
@@ -874,7 +927,7 @@ struct MmaCons {
             for (int c = 0; c < n; c++) {
                 const uint32_t w0 = s.step_i8(sm, lw), w1 = s.step_i8(sm, lw), w2 = s.step_i8(sm, lw), w3 = s.step_i8(sm, lw);
                 s.clamp();
-                if (c == 0) refill_tiles(L, 4 * (q0 + q), lane, failed);
+                if (c == 0) refill_tiles(L, 4 * (q0 + q), false, lane, failed);
                 store_w((uint32_t)c, w0, w1, w2, w3, lane);
             }
             if (n & 1) store_w((uint32_t)n, 0u, 0u, 0u, 0u, lane);  // a K step is two pieces
@@ -909,7 +962,8 @@ struct MmaCons {
         __syncwarp();
     }
     __device__ __forceinline__ void drain(const Q8WLaunch &L) {
-        cp_async_wait_all();
+        if (kOwn) cp_async_wait_all();
+        else xs.drain(L, threadIdx.x & 31);
         if (nmma)
             for (uint32_t it = 0; it < L.spin_limit; it++)
                 if (mbar_try_wait(mbar, (nmma - 1) & 1u)) break;
@@ -992,28 +1046,26 @@ struct MmaCons {
 
 // Float forward on the tensor cores, up to 64 bf16 vectors: as MmaCons<false> with kind::f16, bf16 W and x (int8
 // weights are exact in bf16, every product is exact in fp32) and fp32 sums, 8 quads (32 columns, two K steps of 16) at
-// a time: W tile 2 KB, x tile 64 bytes per vector.  Unit u goes to warp u mod W, each warp's MMAs accumulate in order
+// a time: W tile 2 KB, x tiles (XTiles) 64 bytes per vector.  Unit u goes to warp u mod W, each warp's MMAs accumulate in order
 // and the warps' sums are added in unit order, so results are reproducible bit for bit.
 struct FwdCons {
     static constexpr bool kMma = true, kFloat = true, kStatic = true, kPrepare = false;
     static constexpr int kRed = 0;
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;
-    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + 64u * (uint32_t)xrows; }
-    const uint16_t *x;
-    int cols, seg_quads, qtot;
-    uint32_t wt, xt, d_tmem, lbo, nmma, ndp;
+    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + XTiles::bytes(xrows); }
+    int seg_quads, qtot;
+    XTiles xs;
+    uint32_t wt, d_tmem, nmma, ndp;
     uint32_t mbar, dempty;
-    uint64_t a_desc, b_desc;
+    uint64_t b_desc;
     int warp;
     bool any;
     __device__ __forceinline__ void init(const Q8WLaunch &L, unsigned char *sm, const Bars &B, uint32_t tmem, int w) {
         warp = w;
         wt = smem_u32(sm) + L.lay.tiles + (uint32_t)w * tile_bytes(L.xrows);
-        xt = wt + kWTile;
-        lbo = 16u * (uint32_t)L.xrows;
+        xs.init(B, w, wt + kWTile);
         d_tmem = tmem + 32u * (uint32_t)w;
-        a_desc = umma_smem_desc(xt, lbo, 128u);
         b_desc = umma_smem_desc(wt, 512u, 128u);
         mbar = B.mma(w);
         dempty = B.dempty(w, 0);
@@ -1021,32 +1073,19 @@ struct FwdCons {
         any = false;
     }
     __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I, int) {
-        x = reinterpret_cast<const uint16_t *>(I.x);
-        cols = I.cols;
         seg_quads = I.seg_quads;
-        qtot = cols >> 2;
+        qtot = I.cols >> 2;
     }
     __device__ __forceinline__ void wait_acc(const Q8WLaunch &L, volatile uint32_t *failed) const {
         if (ndp >= 2) wait_bar(dempty + 8u * (ndp & 1u), (ndp / 2u - 1u) & 1u, L, failed);
     }
-    // the previous MMAs are done with both tiles: 32 columns from col on of every vector (see MmaCons::copy_x; columns
-    // past the segment are never multiplied)
-    __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, int lane, volatile uint32_t *failed) const {
+    // the previous MMAs are done with the tiles (x columns past the segment are never multiplied)
+    __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, bool next, int lane, volatile uint32_t *failed) {
         if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
-        const int r = lane & 7, c = col + 8 * (lane >> 3);
-        const uint16_t *src = x + (size_t)r * cols + c;
-        uint32_t dst = xt + (uint32_t)(lane >> 3) * lbo + (uint32_t)r * 16u;
-        const int n = c < cols ? L.batch - r : 0;
-#pragma unroll 2
-        for (int v = 0; v < n; v += 8) {
-            cp_async_16(dst, src);
-            src += 8 * (size_t)cols;
-            dst += 128u;
-        }
+        xs.refill(L, nmma, col, 32, next, lane, failed);
     }
     __device__ __forceinline__ void issue(const Q8WLaunch &L, bool two, int lane, volatile uint32_t *failed) {
         if (!any) wait_acc(L, failed);
-        cp_async_wait_all();
         fence_proxy_async_smem();
         tcgen05_fence_before();
         __syncwarp();
@@ -1054,8 +1093,9 @@ struct FwdCons {
             tcgen05_fence_after();
             const uint32_t idesc = umma_idesc_bf16(64, 32, 0, 0);
             const uint32_t d = d_tmem + ((ndp & 1u) << 20);
-            umma_f16_ss(d, a_desc, b_desc, idesc, any ? 1u : 0u);
-            if (two) umma_f16_ss(d, a_desc + (lbo >> 3), b_desc + 64u, idesc, 1u);
+            const uint64_t a = xs.wait(L, nmma, failed);
+            umma_f16_ss(d, a, b_desc, idesc, any ? 1u : 0u);
+            if (two) umma_f16_ss(d, a + 2u, b_desc + 64u, idesc, 1u);
             umma_commit(mbar);
         }
         __syncwarp();
@@ -1076,6 +1116,7 @@ struct FwdCons {
                                          uint32_t lw, int lane, volatile uint32_t *failed) {
         const int q0 = d.seg * seg_quads;
         const int nq = min(seg_quads, qtot - q0);
+        xs.begin(L, nmma, 4 * q0, lane, failed);
         Stream s(sm, soff, d.rows, lane);
         uint32_t w[4];
         int q = 0;
@@ -1083,7 +1124,7 @@ struct FwdCons {
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 two_quads(s, sm, lw, w);
-                if (c == 0) refill_tiles(L, 4 * (q0 + q), lane, failed);
+                if (c == 0) refill_tiles(L, 4 * (q0 + q), q + 8 < nq, lane, failed);
                 store_w((uint32_t)c, w, lane);
                 if (c & 1) s.clamp();
             }
@@ -1091,7 +1132,7 @@ struct FwdCons {
         }
         if (q < nq) {  // the segment's last 4 quads (segments are whole groups of 4: cols % 16 == 0)
             two_quads(s, sm, lw, w);
-            refill_tiles(L, 4 * (q0 + q), lane, failed);
+            refill_tiles(L, 4 * (q0 + q), false, lane, failed);
             store_w(0, w, lane);
             two_quads(s, sm, lw, w);
             store_w(1, w, lane);
@@ -1116,7 +1157,7 @@ struct FwdCons {
         }
     }
     __device__ __forceinline__ void drain(const Q8WLaunch &L) {
-        cp_async_wait_all();
+        xs.drain(L, threadIdx.x & 31);
         if (nmma)
             for (uint32_t it = 0; it < L.spin_limit; it++)
                 if (mbar_try_wait(mbar, (nmma - 1) & 1u)) break;
@@ -1735,8 +1776,8 @@ Q8WLayout layout(const Q8WLaunch &L, int W, int S) {
     p += kStages * kStageOffs * 4u;
     o.stage_e = p = (p + 15u) & ~15u;
     p += kStages * ((uint32_t)L.tbl_stage + kStagePad) * 2u;
-    // an x tile is read as 64 vectors, however many it holds: up to 1 KB past the last tile
-    o.total = Cons::kMma ? std::max(p, o.slots + 1024u) : p;
+    // an x tile is read as 64 vectors, however many it holds: up to 4 KB past the last tile
+    o.total = Cons::kMma ? std::max(p, o.slots + 4096u) : p;
     return o;
 }
 
@@ -1791,11 +1832,42 @@ mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
 
 }  // namespace
 
+namespace {
+
+// The tensor map of XTiles: job0.x as batch rows of 64-byte pieces.
+mv_status x_map(Q8WLaunch &L, bool bf16) {
+    typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Encode>(f);
+    }();
+    if (!encode) return fail(MV_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+    const cuuint64_t cols = (cuuint64_t)L.job0.m.cols, row = cols * (bf16 ? 2 : 1);
+    const cuuint64_t dims[2] = {cols, (cuuint64_t)L.batch};
+    const cuuint32_t box[2] = {bf16 ? 32u : 64u, (cuuint32_t)L.xrows}, ones[2] = {1u, 1u};
+    const CUresult r = encode(&L.xmap, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+                              const_cast<int8_t *>(L.job0.x), dims, &row, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(MV_ERR_CUDA, "cuTensorMapEncodeTiled: error %d", (int)r);
+    return MV_OK;
+}
+
+}  // namespace
+
 mv_status q8w_launch_int(const Q8WLaunch &L0, int nv, bool mma, int warps, int units, cudaStream_t st) {
     Q8WLaunch L = L0;
     if (mma) {
         L.xrows = (L.batch + 7) & ~7;
-        return L.batch <= 16 ? launch_t<MmaCons<true>>(L, warps, units, st) : launch_t<MmaCons<false>>(L, warps, units, st);
+        if (L.batch <= 16) return launch_t<MmaCons<true>>(L, warps, units, st);
+        mv_status rc = x_map(L, false);
+        return rc ? rc : launch_t<MmaCons<false>>(L, warps, units, st);
     }
     switch (nv) {
         case 1: return launch_t<DotCons<1>>(L, warps, units, st);
@@ -1810,7 +1882,8 @@ mv_status q8w_launch_fwd(const Q8WLaunch &L0, int warps, int units, cudaStream_t
     Q8WLaunch L = L0;
     L.xrows = (L.batch + 7) & ~7;
     if (L.batch == 1) return launch_t<FwdDot>(L, warps, units, st);
-    return launch_t<FwdCons>(L, warps, units, st);
+    mv_status rc = x_map(L, true);
+    return rc ? rc : launch_t<FwdCons>(L, warps, units, st);
 }
 
 mv_status q8w_launch_bwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st) {

@@ -2,6 +2,8 @@
 // code that plans launches (k_q8s.cu).
 #pragma once
 
+#include <cuda.h>
+
 #include "mv_device.cuh"
 
 namespace mv {
@@ -39,6 +41,7 @@ struct Q8WLaunch {
     uint32_t x_quad;       // bytes of a quad of x
     int xrows;  // MMA consumers: rows of the x tile (batch rounded up to 8)
     Q8WLayout lay;
+    CUtensorMap xmap;  // x of a single matrix as tiles (XTiles)
 };
 
 // Integer product of L.batch vectors: on the tensor cores (up to 64 vectors) or, with dp4a, nv >= batch vectors

@@ -21,6 +21,13 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo,
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
+// The same for rows of 64 bytes in the 64-byte swizzle (16-byte piece c of row r at piece c ^ r / 2 % 4 of the row, as
+// a tensor copy with that swizzle writes them; 512-byte aligned, 8-row groups of 512 bytes): layout type 4.  The next
+// 32 bytes of K are at start address + 32.
+__device__ __forceinline__ uint64_t umma_smem_desc_sw64(uint32_t saddr) {
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(512u >> 4) << 32) | (1ull << 46) | (4ull << 61);
+}
+
 // Instruction descriptor of kind::i8: D s32 (bits [4,6) = 2), A and B signed
 // int8 (bits [7,10) and [10,13) = 1), both K-major, N >> 3 in bits [17,23),
 // M >> 4 in bits [24,29).
