@@ -1,4 +1,5 @@
-// Q8-stripe decode + int8 matvec for sm_100a.
+// Q8-stripe decode (mv_q8_decode) and the int8 matvec of matrices whose blocks
+// are too large for the warp-specialised kernel (k_q8w.cu), for sm_100a.
 //
 // Layout (built by host_q8.cpp): rows are grouped into stripes of 32, lane l
 // of a warp owning row 32*stripe + l; each row is cut into segments of
@@ -304,6 +305,7 @@ int nv_for(int nb) { return nb <= 2 ? nb : nb <= 4 ? 4 : nb <= 8 ? 8 : 16; }
 }  // namespace
 
 bool q8s_supports(const mv_q8_view *m, const int8_t *x);
+bool q8s_takes_ragged(const mv_q8_view *m, int batch);
 mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y, const float *scales, float *ys,
                      const mv_q8_tuning *tuning, cudaStream_t st);
 
@@ -313,7 +315,7 @@ mv_status q8_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y,
     if (rc) return rc;
     if (!x || !y || batch <= 0) return fail(MV_ERR_ARG, "mv_q8_matvec: bad x/y/batch");
     if (ys && !scales) return fail(MV_ERR_ARG, "mv_q8_matvec: y_scaled needs row scales");
-    if (q8s_supports(m, x)) return q8s_matvec(m, x, batch, y, scales, ys, nullptr, st);
+    if (q8s_supports(m, x) || q8s_takes_ragged(m, batch)) return q8s_matvec(m, x, batch, y, scales, ys, nullptr, st);
     uint32_t *status = device_status_word(&rc);
     if (rc) return rc;
     for (int v0 = 0; v0 < batch; v0 += 16) {

@@ -207,21 +207,35 @@ int plan_single(Q8WLaunch &L, const mv_q8_tuning &t, const Cost &c) {
     return (int)std::min<long long>(units, 1 << 20);
 }
 
+// Whether a product that q8s_supports refuses can run there all the same (q8s_matvec then takes it): its blocks must leave
+// room for two decode tables.  The kernel for it is otherwise the CTA-per-stripe one of k_q8.cu.  Measured on a B200,
+// that one | this: 4090x4100, 1, 2, 16 and 64 vectors 17.4 | 13.2, 19.9 | 13.9, 48.7 | 24.7, 193 | 82 us; 10001x5003,
+// 41.8 | 29.3, 48.2 | 30.8, 93 | 61, 371 | 185; 12000x1602, 17.9 | 18.8, 21.0 | 20.0, 45.6 | 34.9, 181 | 78.
+bool q8s_takes_ragged(const mv_q8_view *m, int batch) {
+    Q8WLaunch L{};
+    L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
+    L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
+    L.batch = std::min(batch, 64);
+    return m->max_blk_rows < (1 << 20) && q8w_ragged_fits(L, false) && (L.batch < kMmaMinVectors || q8w_ragged_fits(L, true));
+}
+
 // Single matrix through the persistent kernel (one inline job): passes of up to 64 vectors on the tensor cores, of
-// up to 16 on the CUDA cores.
+// up to 16 on the CUDA cores; ragged ones (see Q8WLaunch) too.
 mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y, const float *scales, float *ys,
                      const mv_q8_tuning *tuning, cudaStream_t st) {
     mv_status rc;
     uint32_t *status = device_status_word(&rc);
     if (rc) return rc;
     const mv_q8_tuning t = resolve(tuning);
+    const bool ragged = !q8s_supports(m, x);
     const int pass = t.engine == MV_ENGINE_AUTO ? 64 : 16;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         const int nb = std::min(pass, batch - v0);
         bool mma = t.engine == MV_ENGINE_AUTO && nb >= kMmaMinVectors;
-        rc = check_shape(t, t.engine == MV_ENGINE_AUTO && nb >= kMmaShape, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
+        if (!ragged) rc = check_shape(t, t.engine == MV_ENGINE_AUTO && nb >= kMmaShape, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
         if (rc) return rc;
         Q8WLaunch L{};
+        L.ragged = ragged;
         L.job0.m = *m;
         L.job0.x = x + (size_t)v0 * m->cols;
         L.job0.y = y + (size_t)v0 * m->rows;

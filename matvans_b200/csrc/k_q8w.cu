@@ -85,7 +85,8 @@ struct alignas(8) ItemState {
 struct alignas(16) ItemRec {
     int32_t it, job, stripe, tab;  // it < 0: no more items; tab: decode table
     int32_t gen;        // number of its table's build in this CTA
-    int32_t build;      // 1: the table is built for this item
+    int32_t build;      // not 0: the table is built for this item; the items before build - 1 are the last to use the
+                        // table that this overwrites
     int32_t area_item;  // the item whose build must be over before this one's data is staged (-1: none)
     int32_t sb;         // first segment
     uint32_t n, u0;     // number of units, and the first one's running number
@@ -189,7 +190,7 @@ __device__ __forceinline__ bool table_vote(bool ok) {
 // CUDA-core consumers: whether the slots hold their segments' x (segments of up to kXQuads quads, not in a chain)
 constexpr int kXQuads = 64;
 __device__ __forceinline__ bool x_in_slot(const Q8WLaunch &L, int seg_quads) {
-    return L.x_off != 0 && seg_quads <= kXQuads;
+    return L.x_off != 0 && !L.ragged && seg_quads <= kXQuads;
 }
 
 // ---------------------------------------------------------------- work items
@@ -355,6 +356,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
                 // two tables and two staging areas: build g overwrites those of build g - 2
                 gen++;
                 r.area_item = gen >= 2 ? fb2 : -1;
+                r.build = 1 + max(fb1, 0);
                 fb2 = fb1;
                 fb1 = k;
                 tjob = job;
@@ -652,12 +654,30 @@ struct Stream {
 // x is read with plain (coherent) loads: in a chain it was written earlier in the same launch.
 __device__ __forceinline__ uint4 ldx_u4(const void *p) { return *reinterpret_cast<const uint4 *>(p); }
 
+// Ragged x: the four bytes at p, of which `valid` belong to the row (the others are zero), from two aligned words; by
+// single bytes where those would leave the launch's x.
+__device__ __forceinline__ uint32_t x_quad_at(const Q8WLaunch &L, const int8_t *p, int valid) {
+    if (valid <= 0) return 0u;
+    const int8_t *x0 = L.job0.x, *xe = x0 + (size_t)L.batch * L.job0.m.cols;
+    const uint32_t *a = reinterpret_cast<const uint32_t *>((uintptr_t)p & ~(uintptr_t)3);
+    uint32_t v = 0;
+    if ((uintptr_t)a >= (uintptr_t)x0 && (uintptr_t)(a + 2) <= (uintptr_t)xe) {
+        v = __funnelshift_r(__ldg(a), __ldg(a + 1), 8u * (uint32_t)((uintptr_t)p & 3));
+        if (valid < 4) v &= (1u << (8 * valid)) - 1u;
+    } else {
+        for (int j = 0; j < min(valid, 4); j++) v |= (uint32_t)(uint8_t)__ldg(p + j) << (8 * j);
+    }
+    return v;
+}
+
 // CUDA-core consumer: NV int8 vectors, dp4a.  The lane's partial sums go to the item's area in shared memory
-// (exact integer atomics); the warp that counts the item's last part writes the outputs.
-template <int NV>
+// (exact integer atomics); the table warps write the outputs.  kRagged: the warp lays out x itself, 64 quads at a time, in
+// the slot's place for it, and the last group of a segment may be of fewer than 4 quads.
+template <int NV, bool kRagged = false>
 struct DotCons {
     static constexpr bool kMma = false, kFloat = false, kStatic = false, kPrepare = false;
     static constexpr int kRed = NV * 32;  // ints of an item's partial sums
+    static constexpr int kLag = NV <= 2 ? 1 : 4;
     static constexpr int kMaxDecode = NV <= 2 ? 16 : NV <= 4 ? 14 : NV <= 8 ? 10 : 6;
     static constexpr uint32_t tile_bytes(int) { return 0; }
     const int8_t *x;
@@ -674,7 +694,7 @@ struct DotCons {
         x = I.x;
         cols = I.cols;
         seg_quads = I.seg_quads;
-        qtot = cols >> 2;
+        qtot = (cols + 3) >> 2;
     }
     __device__ __forceinline__ void group(Stream &s, const unsigned char *sm, uint32_t lw, const uint4 (&xv)[NV]) {
 #pragma unroll
@@ -693,7 +713,35 @@ struct DotCons {
         const int q0 = d.seg * seg_quads;
         const int nq = min(seg_quads, qtot - q0);
         Stream s(sm, soff, d.rows, lane);
-        if (in_slot) {  // x came with the block and lies behind it
+        if constexpr (kRagged) {
+            uint32_t *xs = const_cast<uint32_t *>(reinterpret_cast<const uint32_t *>(sm + soff + L.x_off));
+            for (int q = 0; q < nq; q += kXQuads) {
+                const int n = min(kXQuads, nq - q);
+                for (int v = 0; v < L.batch; v++)
+                    for (int i = lane; i < n; i += 32) {
+                        const int col = 4 * (q0 + q + i);
+                        xs[kXQuads * v + i] = x_quad_at(L, x + (size_t)v * cols + col, cols - col);
+                    }
+                __syncwarp();
+                const uint32_t *xq = xs;
+                int i = 0;
+#pragma unroll 1
+                for (; i + 4 <= n; i += 4, xq += 4) {
+                    uint4 xv[NV];
+#pragma unroll
+                    for (int v = 0; v < NV; v++) xv[v] = *reinterpret_cast<const uint4 *>(xq + kXQuads * v);
+                    group(s, sm, lw, xv);
+                }
+#pragma unroll 1
+                for (; i < n; i++, xq++) {
+                    const uint32_t w = s.step_i8(sm, lw);
+#pragma unroll
+                    for (int v = 0; v < NV; v++) acc[v] = __dp4a((int)w, (int)xq[kXQuads * v], acc[v]);
+                }
+                s.clamp();
+                __syncwarp();
+            }
+        } else if (in_slot) {  // x came with the block and lies behind it
             const unsigned char *xs = sm + soff + L.x_off;
             // unrolled: the loop's back edge costs register moves (4 instructions a step without)
 #pragma unroll kUnroll
@@ -816,17 +864,21 @@ struct XTiles {
 // own quarter; the warp reads its sums itself after each unit and adds them to the item's in shared memory.  With more
 // vectors the sums stay in TMEM for the item, the table warps read every warp's (one lane quarter each), and items
 // alternate between two accumulators, the second in the 16 lanes of each quarter that M = 64 leaves free.
-template <bool kOwn>
+//
+// kRagged: the warp gathers its x tiles by plain loads, and a segment may end within a piece.
+template <bool kOwn, bool kRagged = false>
 struct MmaCons {
     static constexpr bool kMma = true, kFloat = false, kStatic = false, kPrepare = false;
+    static constexpr bool kTma = !kOwn && !kRagged;  // x by XTiles
     static constexpr int kPitch = 33;  // words per vector of the item's sums: lanes (vectors) hit distinct banks
     static constexpr int kRed = kOwn ? 16 * kPitch : 0;
+    static constexpr int kLag = kOwn ? 4 : 2;  // accumulators
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;  // 32 rows x 64 columns
-    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + (kOwn ? 64u * (uint32_t)xrows : XTiles::bytes(xrows)); }
+    static constexpr uint32_t tile_bytes(int xrows) { return kWTile + (kTma ? XTiles::bytes(xrows) : 64u * (uint32_t)xrows); }
     const int8_t *x;
     int cols, seg_quads, qtot;
-    XTiles xs;  // !kOwn
+    XTiles xs;  // kTma
     uint32_t wt, xt, d_tmem, lbo, nmma, ndp;  // nmma: commits so far, ndp: earlier items this warp has had a part in
     uint32_t mbar, dempty;                    // dempty: of the first accumulator; the second's follows
     uint64_t a_desc, b_desc;
@@ -839,8 +891,8 @@ struct MmaCons {
         lbo = 16u * (uint32_t)L.xrows;
         const uint32_t quarter = (uint32_t)(w + kFirstDecode) & 3u;  // of TMEM lanes, by the warp's number in the CTA
         d_tmem = tmem + 32u * (uint32_t)w;
-        a_desc = umma_smem_desc(xt - 256u * quarter, lbo, 128u);
-        if (!kOwn) xs.init(B, w, xt);
+        a_desc = umma_smem_desc(kOwn ? xt - 256u * quarter : xt, lbo, 128u);
+        if (kTma) xs.init(B, w, xt);
         b_desc = umma_smem_desc(wt, 512u, 128u);
         mbar = B.mma(w);
         dempty = B.dempty(w, 0);
@@ -855,7 +907,7 @@ struct MmaCons {
         x = I.x;
         cols = I.cols;
         seg_quads = I.seg_quads;
-        qtot = cols >> 2;
+        qtot = (cols + 3) >> 2;
     }
     // the accumulator of the current item (they alternate) is free: its sums of two items ago are read
     __device__ __forceinline__ void wait_acc(const Q8WLaunch &L, volatile uint32_t *failed) const {
@@ -872,6 +924,17 @@ struct MmaCons {
         if (n > 0) cp_async_16(dst, src);
         if (n > 8) cp_async_16(dst + 128u, src + 8 * (size_t)cols);
     }
+    __device__ __forceinline__ void gather_x(const Q8WLaunch &L, int col, int lane) const {
+        const int r = lane & 7, c = col + 16 * (lane >> 3);
+        uint32_t dst = xt + (uint32_t)(lane >> 3) * lbo + (uint32_t)r * 16u;
+        for (int v = r; v < L.batch; v += 8, dst += 128u) {
+            const int8_t *src = x + (size_t)v * cols + c;
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[j] = x_quad_at(L, src + 4 * j, cols - c - 4 * j);
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+        }
+    }
     // four quads (16 columns) of the lane's row: piece c of the 64-column tile
     __device__ __forceinline__ void store_w(uint32_t c, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3, int lane) const {
         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(wt + c * 512u + (uint32_t)lane * 16u), "r"(w0), "r"(w1),
@@ -881,13 +944,14 @@ struct MmaCons {
     // the previous MMAs are done with the tiles; the x copies have the rest of the decode to land in
     __device__ __forceinline__ void refill_tiles(const Q8WLaunch &L, int col, bool next, int lane, volatile uint32_t *failed) {
         if (nmma) wait_bar(mbar, (nmma - 1) & 1u, L, failed);
-        if (kOwn) copy_x(L, col, lane);
+        if (kRagged) gather_x(L, col, lane);
+        else if (!kTma) copy_x(L, col, lane);
         else xs.refill(L, nmma, col, 64, next, lane, failed);
     }
     // the MMAs of a tile: two K steps of 32 columns, or one
     __device__ __forceinline__ void issue(const Q8WLaunch &L, bool two, int lane, volatile uint32_t *failed) {
         if (!any) wait_acc(L, failed);
-        if (kOwn) cp_async_wait_all();
+        if (!kTma && !kRagged) cp_async_wait_all();
         fence_proxy_async_smem();  // both tiles are read by the tensor core (async proxy)
         tcgen05_fence_before();
         __syncwarp();
@@ -895,9 +959,9 @@ struct MmaCons {
             tcgen05_fence_after();
             const uint32_t idesc = umma_idesc_i8(64, 32);
             const uint32_t d = kOwn ? d_tmem : d_tmem + ((ndp & 1u) << 20);  // the second accumulator: 16 lanes further
-            const uint64_t a = kOwn ? a_desc : xs.wait(L, nmma, failed);
+            const uint64_t a = kTma ? xs.wait(L, nmma, failed) : a_desc;
             umma_i8(d, a, b_desc, idesc, any ? 1u : 0u);
-            if (two) umma_i8(d, a + (kOwn ? lbo >> 3 : 2u), b_desc + 64u, idesc, 1u);
+            if (two) umma_i8(d, a + (kTma ? 2u : lbo >> 3), b_desc + 64u, idesc, 1u);
             umma_commit(mbar);
         }
         __syncwarp();
@@ -908,7 +972,7 @@ struct MmaCons {
                                          uint32_t lw, int lane, volatile uint32_t *failed) {
         const int q0 = d.seg * seg_quads;
         const int nq = min(seg_quads, qtot - q0);
-        if (!kOwn) xs.begin(L, nmma, 4 * q0, lane, failed);
+        if (kTma) xs.begin(L, nmma, 4 * q0, lane, failed);
         Stream s(sm, soff, d.rows, lane);
         int q = 0;
         for (; q + 16 <= nq; q += 16) {
@@ -921,11 +985,13 @@ struct MmaCons {
             }
             issue(L, true, lane, failed);
         }
-        if (q < nq) {  // the segment's last 4, 8 or 12 quads (segments are whole groups of 4: cols % 16 == 0)
-            const int n = (nq - q) >> 2;
+        if (q < nq) {  // the segment's last 4, 8 or 12 quads (segments are whole groups of 4: cols % 16 == 0, or ragged)
+            const int n = (nq - q + 3) >> 2;
 #pragma unroll 1
             for (int c = 0; c < n; c++) {
-                const uint32_t w0 = s.step_i8(sm, lw), w1 = s.step_i8(sm, lw), w2 = s.step_i8(sm, lw), w3 = s.step_i8(sm, lw);
+                const int left = kRagged ? nq - q - 4 * c : 4;
+                const uint32_t w0 = s.step_i8(sm, lw), w1 = left > 1 ? s.step_i8(sm, lw) : 0u,
+                               w2 = left > 2 ? s.step_i8(sm, lw) : 0u, w3 = left > 3 ? s.step_i8(sm, lw) : 0u;
                 s.clamp();
                 if (c == 0) refill_tiles(L, 4 * (q0 + q), false, lane, failed);
                 store_w((uint32_t)c, w0, w1, w2, w3, lane);
@@ -962,7 +1028,7 @@ struct MmaCons {
         __syncwarp();
     }
     __device__ __forceinline__ void drain(const Q8WLaunch &L) {
-        if (kOwn) cp_async_wait_all();
+        if (!kTma) cp_async_wait_all();
         else xs.drain(L, threadIdx.x & 31);
         if (nmma)
             for (uint32_t it = 0; it < L.spin_limit; it++)
@@ -1051,6 +1117,7 @@ struct MmaCons {
 struct FwdCons {
     static constexpr bool kMma = true, kFloat = true, kStatic = true, kPrepare = false;
     static constexpr int kRed = 0;
+    static constexpr int kLag = 2;  // accumulators
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;
     static constexpr uint32_t tile_bytes(int xrows) { return kWTile + XTiles::bytes(xrows); }
@@ -1231,6 +1298,7 @@ struct FwdCons {
 // vector's products.)
 struct FwdDot {
     static constexpr bool kMma = false, kFloat = true, kStatic = true, kPrepare = false;
+    static constexpr int kLag = 1;
     static constexpr int kMaxDecode = 16;
     static constexpr int kRed = kMaxDecode * 32;
     static constexpr uint32_t tile_bytes(int) { return 0; }
@@ -1327,6 +1395,7 @@ struct FwdDot {
 struct BwdCons {
     static constexpr bool kMma = true, kFloat = true, kStatic = false, kPrepare = true;
     static constexpr int kRed = 0;
+    static constexpr int kLag = 1;  // two buffers of G, written with the item's table
     static constexpr int kMaxDecode = 12;
     static constexpr uint32_t kWTile = 2048, kTr = 4096;
     static constexpr uint32_t kGCols = 32;  // TMEM columns of an item's G: two terms of two K steps
@@ -1512,6 +1581,7 @@ struct BwdCons {
 // 47 -> 41 us (with BwdCons, 55 and 57 us and 2e-6 of error where this form has 2e-7).
 struct BwdDot {
     static constexpr bool kMma = false, kFloat = true, kStatic = false, kPrepare = true;
+    static constexpr int kLag = 1;
     static constexpr int kMaxDecode = 16;
     static constexpr int kRed = 32;  // g of the item's rows
     static constexpr uint32_t tile_bytes(int) { return 2048; }
@@ -1628,8 +1698,11 @@ __device__ __forceinline__ void serve_tables(const Q8WLaunch &L, unsigned char *
         }
         if (I.build) {
             const int area = I.gen % kStages;
+            // the table's previous users must be done (with kLag 1 they are among the items finished below)
+            if (Cons::kLag > 1)
+                for (; done < I.build - 1; done++)
+                    if (!finish_item<Cons>(L, ring[done % kRing], done, sm, B, tmem, failed)) return;
             bool ok = !poll || wait_bar(B.staged(area), (uint32_t)(I.gen / kStages) & 1u, L, failed);
-            // (the table's previous users are done: they are among the items finished above)
             if (!table_vote(ok)) return;
             const uint32_t *so = reinterpret_cast<const uint32_t *>(sm + L.lay.stage_o) + area * kStageOffs;
             const uint16_t *se = reinterpret_cast<const uint16_t *>(
@@ -1644,9 +1717,11 @@ __device__ __forceinline__ void serve_tables(const Q8WLaunch &L, unsigned char *
         }
         if (!table_vote(true)) return;
         if (threadIdx.x == 0) arrive(B.tfull(k % kRing));
-        // The previous item's outputs, before the next record is waited for: this item's decode may need its
-        // accumulators and, when it has more units than there are slots, holds that record up.
-        for (; done < k; done++)
+        // Earlier items' outputs, before the next record is waited for: this item's decode may need their accumulators
+        // and, when it has more units than there are slots, holds that record up.  kLag items may be open: small ones
+        // then decode side by side (16000x400, one table for all rows, 16 vectors: 17.3 -> 15.5 us; up to two vectors
+        // gain nothing, and the second copy of the epilogue slowed their decode by 2 %).
+        for (; done + Cons::kLag <= k; done++)
             if (!finish_item<Cons>(L, ring[done % kRing], done, sm, B, tmem, failed)) return;
     }
 }
@@ -1865,10 +1940,19 @@ mv_status q8w_launch_int(const Q8WLaunch &L0, int nv, bool mma, int warps, int u
     Q8WLaunch L = L0;
     if (mma) {
         L.xrows = (L.batch + 7) & ~7;
+        if (L.ragged)
+            return L.batch <= 16 ? launch_t<MmaCons<true, true>>(L, warps, units, st)
+                                 : launch_t<MmaCons<false, true>>(L, warps, units, st);
         if (L.batch <= 16) return launch_t<MmaCons<true>>(L, warps, units, st);
         mv_status rc = x_map(L, false);
         return rc ? rc : launch_t<MmaCons<false>>(L, warps, units, st);
     }
+    if (L.ragged) switch (nv) {
+            case 1: return launch_t<DotCons<1, true>>(L, warps, units, st);
+            case 2: return launch_t<DotCons<2, true>>(L, warps, units, st);
+            case 4: return launch_t<DotCons<4, true>>(L, warps, units, st);
+            default: return launch_t<DotCons<8, true>>(L, warps, units, st);  // (more go to the tensor cores)
+        }
     switch (nv) {
         case 1: return launch_t<DotCons<1>>(L, warps, units, st);
         case 2: return launch_t<DotCons<2>>(L, warps, units, st);
@@ -1876,6 +1960,15 @@ mv_status q8w_launch_int(const Q8WLaunch &L0, int nv, bool mma, int warps, int u
         case 8: return launch_t<DotCons<8>>(L, warps, units, st);
         default: return launch_t<DotCons<16>>(L, warps, units, st);
     }
+}
+
+bool q8w_ragged_fits(const Q8WLaunch &L0, bool mma) {
+    Q8WLaunch L = L0;
+    L.xrows = (L.batch + 7) & ~7;
+    if (!mma) L.slot_bytes += 4u * (uint32_t)(std::min(L.batch, 8) * kXQuads);
+    const uint32_t need = mma ? std::max(layout<MmaCons<true, true>>(L, 1, 1).total, layout<MmaCons<false, true>>(L, 1, 1).total)
+                              : layout<DotCons<8, true>>(L, 1, 1).total;
+    return need <= (uint32_t)max_smem_optin();
 }
 
 mv_status q8w_launch_fwd(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {

@@ -33,6 +33,7 @@ struct Q8WLaunch {
     // One job in even shares (nonzero: its number of units): CTA c of G takes units [c span / G, (c + 1) span / G),
     // whatever stripes they are of.  Sums of a stripe that several CTAs share are added to y (ys) unscaled.
     uint32_t span;
+    int ragged;  // integer products, one job: x off the 16-byte grid, columns or segments not whole groups of 16 columns
     // set by the launcher
     int W, S;              // decode warps, stream slots
     uint32_t S_inv;        // ceil(2^32 / S): unit / S by multiplication
@@ -47,6 +48,8 @@ struct Q8WLaunch {
 // Integer product of L.batch vectors: on the tensor cores (up to 64 vectors) or, with dp4a, nv >= batch vectors
 // (1, 2, 4, 8 or 16).  warps: decode warps per CTA (0: as many as fit); units: the most units a CTA can get.
 mv_status q8w_launch_int(const Q8WLaunch &L, int nv, bool mma, int warps, int units, cudaStream_t st);
+// Whether a ragged one (dp4a: of up to 8 vectors) finds room in shared memory at all.
+bool q8w_ragged_fits(const Q8WLaunch &L, bool mma);
 // Float forward of up to 64 vectors (on the tensor cores from 2): job0.x is bf16 [batch][cols], job0.ys fp32 [batch][rows].
 mv_status q8w_launch_fwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st);
 // Float backward of up to 32 vectors: job0.x is dY, bf16 [batch][rows], added to job0.ys, fp32 [batch][cols].

@@ -121,3 +121,23 @@ def test_even_shares(rows, cols, seg_quads):
         err = (M.matvec_t_bf16(dy, sd).double() - g @ W64).abs() / (g.abs() @ W64.abs())
         assert err.max().item() < (0.0 if B == 1 else 2.0 ** -17) + 2.0 ** -23 * (rows + 32), B
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads,offset", [
+    (33, 1, 0, 0), (100, 15, 0, 0), (257, 1037, 4, 0), (96, 2050, 68, 1), (5000, 275, 0, 0), (64, 8191, 130, 3),
+    (2400, 6001, 0, 0), (64, 1040, 6, 0), (70, 1024, 64, 5)])
+def test_ragged(rows, cols, seg_quads, offset):
+    # rows of x that start anywhere, a last quad of 1 to 3 columns, segments of any number of quads, x off the grid;
+    # dp4a, the small matrices' 8 vectors, the tensor cores' 16, their 64 and the pass after them
+    rng = np.random.default_rng(rows + cols + seg_quads)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, local=rows != 100, seg_quads=seg_quads)
+    s = rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)
+    for B in (1, 2, 3, 5, 8, 9, 16, 19, 64, 70):
+        xf = torch.randint(-128, 128, (offset + B * cols,), dtype=torch.int8, device="cuda")
+        x = xf[offset:].view(B, cols)
+        y, ys = M.matvec(x, scales=s)
+        ref = oracle.matvec_i8(W, x.cpu().numpy())
+        assert np.array_equal(y.cpu().numpy(), ref), B
+        assert np.array_equal(ys.cpu().numpy(), (ref.astype(np.float32) * s[None, :]).astype(np.float32)), B
+    assert ops.device_status() == 0
