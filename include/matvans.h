@@ -143,7 +143,7 @@ mv_status mv_wpr_matvec(const uint16_t *payload_dev, size_t payload_size,
                         float *y_scaled_dev, void *stream);
 
 /* The epilogue of matvansWarpPerRow.cu:51-72,167-172 fused into one kernel
- * without a host round trip: delta = max|y|/127 (fp32), out8[r] =
+ * (n up to 131072; else two) without a host round trip: delta = max|y|/127 (fp32), out8[r] =
  * (int8)round_half_even((float)y[r] / delta), no clamp (as in the reference).
  * `absmax_scratch_dev` is one caller-owned uint32.  Writes delta to
  * *delta_dev. */

@@ -75,3 +75,16 @@ def test_aws(kind, rows, cols):
     torch.cuda.synchronize()
     ref = np.clip(np.rint(oracle.matvec_i8(W, x[None, :])[0].astype(np.float32) * np.float32(2e-3)), -128, 127)
     assert np.array_equal(out.cpu().numpy(), ref.astype(np.int8))
+
+
+@pytest.mark.parametrize("n", [1, 31, 1025, 4096, 4097, 8193, 70000, 8 * 1024 * 16, 8 * 1024 * 16 + 1])
+def test_requant_absmax(n):
+    # one CTA, clusters of 2, 4 and 8, the last element a thread holds, and the three-launch form behind them; fp32
+    # arithmetic of the reference, rounded half to even: equal, not close
+    rng = np.random.default_rng(n)
+    for y in (rng.integers(-5000000, 5000001, size=n).astype(np.int32), np.where(np.arange(n) == n - 1, -127, 3).astype(np.int32)):
+        out8, delta = ops.requant_absmax(torch.from_numpy(y).cuda())
+        d = np.float32(np.abs(y.astype(np.int64)).max()) / np.float32(127.0)
+        assert delta.item() == d
+        assert np.array_equal(out8.cpu().numpy(), np.rint(y.astype(np.float32) / d).astype(np.int8))
+    assert ops.device_status() == 0
