@@ -146,6 +146,7 @@ int choose_parts(int nseg, int seg_quads, int stripes, const Cost &c) {
     long long best_cost = -1;
     for (int p = 1; p <= 64 && p <= nseg; p++) {
         const long long items = ((long long)stripes * p + G - 1) / G;
+        if (best_cost >= 0 && (items + 1) * c.service >= best_cost) break;  // (no larger p is better: time() is at least that)
         const long long cost = time(items * ((nseg + p - 1) / p), items) + (p > 1 ? c.join_parts + c.outputs * p / 50 : 0);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
