@@ -309,7 +309,7 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
         // (whole | even: 11008x4096, one vector 29.5 | 32.0 us, 16 vectors 48.5 | 52.1, 64 vectors 57.6 | 64.9; 6000x6000, 16
         // vectors 49.1 | 45.8, 64 vectors 57.8 | 56.5)
         constexpr int kNever = 1 << 30;
-        const Cost cost{L.batch == 1 ? 15 : 24 + L.batch / 2, L.batch == 1 ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,
+        const Cost cost{L.batch == 1 ? 15 : 26 + L.batch / 16, L.batch == 1 ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,
                         t.parts <= 0 && (m->rows + 31) / 32 >= sm_count() ? 20000 : kNever};
         mv_q8_tuning by_rule = t;
         by_rule.parts = 0;
