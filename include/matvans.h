@@ -199,17 +199,17 @@ typedef struct mv_q8_view {
 mv_status mv_q8_matvec(const mv_q8_view *m, const int8_t *x_dev, int batch, int32_t *y_dev,
                        const float *row_scales_dev, float *y_scaled_dev, void *stream);
 
-/* Launch parameters of the persistent Q8 kernel (0 = library default).
- * The integer product runs one CTA per SM: `warps` is the number of its decode
- * warps (default: as many as fit, up to 16), `parts` as below, and the others
- * only have to fit shared memory (MV_ERR_UNSUPPORTED if they do not).
- *   warps        float form: warps per CTA (default 8; 16 for the forward on the
- *                CUDA cores): up to 16, except 8 for the backward and for
- *                the tensor cores
- *   ilp          independent segments decoded per warp (1 or 2, default 2;
- *                1 for the float form)
- *   depth        shared-memory stream buffers per warp (1 or 2, default 1)
- *   ctas_per_sm  cap on resident CTAs per SM (default: occupancy limit)
+/* Launch parameters of the persistent Q8 kernel (0 = library default).  It
+ * runs one CTA per SM.
+ *   warps        decode warps: 1..8 stand for twice as many per SM (two CTAs'
+ *                worth), 9..16 for themselves; default as many as fit.  The
+ *                float backward, and the float forward of 2 or more vectors on
+ *                engine 0, take at most 8
+ *   ilp, depth, ctas_per_sm
+ *                not used by the kernel; a launch shape of `warps` x ilp x
+ *                depth stream buffers (defaults 8, 2, 1; ilp 1 on the tensor
+ *                cores and in the float form) still has to fit shared memory
+ *                (MV_ERR_UNSUPPORTED if it does not)
  *   parts        work items per 32-row stripe (its segments split in `parts`
  *                ranges; default: whole stripes in stacks, enough parts to
  *                fill the GPU for a single matrix)
