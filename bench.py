@@ -37,7 +37,7 @@ METRIC = "us/matvec & int8-equiv GB/s vs dense dp4a int8 on B200, bit-exact int3
 UNIT = "GB/s"
 L2_BYTES = 126 * 2 ** 20
 # DRAM traffic of one launch of the step's kernel, as the latest committed ncu summary of it records
-PROFILE_RECORD = os.path.join(ROOT, "profiles", "q8s_kernel_stack12_b1.json")
+PROFILE_RECORD = os.path.join(ROOT, "profiles", "q8w_kernel_stack12_b1.json")
 
 
 def profiled_traffic():
@@ -920,7 +920,7 @@ def run_ours(args):
                          "frac": achieved / peak, "traffic": traffic, "traffic_unit": "bytes per launch",
                          "traffic_source": traffic_src,
                          "algorithmic_bytes": alg, "peak_kind": peak_kind,
-                         "kernel": "q8s_kernel<1,ILP,DEPTH> (mv_q8_stack_matvec)",
+                         "kernel": "q8w_kernel<DotCons<1>> (mv_q8_stack_matvec)",
                          "note": "algorithmic bytes = compressed streams + tables + offsets + x + int32 y"},
             "gpu_launches": args.steps * S.launches_per_run,
             "clocks": sampler.summary(),

@@ -1,5 +1,5 @@
 // Encoder for the Q8-stripe layout (this library's own layout; the kernel is
-// k_q8.cu, the layout is documented on mv_q8_view in include/matvans.h).
+// k_q8w.cu, the layout is documented on mv_q8_view in include/matvans.h).
 //
 // Coder: per lane, rANS with 8-bit probabilities, a 64-bit state and 32-bit
 // refill words, four symbols per step (the quad coder of
