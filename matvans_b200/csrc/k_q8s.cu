@@ -37,6 +37,7 @@ __global__ void q8s_scale_atomic_y(const Q8Job *jobs, int njobs, int batch) {
 // n 32-bit zeros.  (A memset between kernels costs more than a small kernel: 500x2992 and 160x4096, one vector, four
 // parts, 12.3 us with cudaMemsetAsync, 9.6 with this.)
 __global__ void __launch_bounds__(256) zero_words(uint32_t *p, size_t n) {
+    grid_launch_dependents();  // (the product behind it waits for these zeros before its first sum)
     const size_t head = min(n, (size_t)((16 - ((uintptr_t)p & 15)) & 15) / 4), n4 = (n - head) / 4;
     const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
     uint4 *q = reinterpret_cast<uint4 *>(p + head);
@@ -174,6 +175,7 @@ int choose_parts(int nseg, int seg_quads, int stripes, const Cost &c) {
 template <typename T, bool kScale>
 __global__ void __launch_bounds__(256) cut_stripes(T *y, float *ys, const float *scales, int rows, int batch, uint32_t nseg,
                                                    uint32_t span, uint32_t shares) {
+    if (!kScale) grid_launch_dependents();
     const uint32_t b = blockIdx.x + 1, p = (uint32_t)((uint64_t)b * span / shares), stripe = p / nseg;
     const uint32_t q = (uint32_t)((uint64_t)(b - 1) * span / shares);
     if (p == stripe * nseg || q > stripe * nseg) return;

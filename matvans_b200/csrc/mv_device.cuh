@@ -106,6 +106,11 @@ __device__ __forceinline__ uint4 ldg_nc_u4(const uint4 *p) {
     return v;
 }
 
+// Programmatic dependent launch: wait until the grids this one depends on are complete and their writes visible (at once
+// when it was launched without the attribute), and let the grid behind this one in the stream be scheduled.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Host side: per-device status word, lazily allocated once per device.
 uint32_t *device_status_word(mv_status *st);
 uint32_t wait_spin_limit();   // kWaitSpinLimit unless MV_INJECT_WAIT_LIMIT set another bound
