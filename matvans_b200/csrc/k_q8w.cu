@@ -1913,17 +1913,7 @@ mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
     // builds its first table meanwhile (5 to 7 us); see produce() for what waits.  Measured on a B200, launches back to back
     // without and with it: a layer of seven matrices, one vector 73.7 -> 71.0 us, 16 vectors 108.6 -> 104.9; of hidden size
     // 512, 13.4 -> 10.4; 11008x4096, 64 int8 vectors 44.5 -> 40.3, bf16 56.0 -> 51.6.
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = L.lay.total;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    MV_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, L), "q8 kernel launch");
+    MV_CUDA_TRY(launch_dependent(kern, dim3(grid), block, L.lay.total, st, L), "q8 kernel launch");
     return MV_OK;
 }
 

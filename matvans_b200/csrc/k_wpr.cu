@@ -70,8 +70,6 @@ template <int NV>
 __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch L) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
-    grid_launch_dependents();  // (the requantisation's launch latency passes meanwhile)
-
     // decode table: eight threads per quantile, four lane columns each
     for (uint32_t i = threadIdx.x; i < 256 * 8; i += blockDim.x) {
         const uint32_t q = i >> 3, r = __ldg(L.ppf + q);
@@ -87,6 +85,9 @@ __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch
         uint4 *dst = reinterpret_cast<uint4 *>(smem + 256u * q + 16u * (i & 7u));
         *dst = e4;
     }
+    // (the table is built while the launch before this one ends; x and the outputs are not touched earlier)
+    grid_dependency_wait();
+    grid_launch_dependents();
     __syncthreads();
 
     const uint32_t lane4 = (uint32_t)lane * 4u;
@@ -258,8 +259,7 @@ mv_status launch_wpr(const WprLaunch &L, cudaStream_t st) {
     mv_status rc = prepare_kernel((const void *)kern, smem, 32 * W, nullptr);
     if (rc) return rc;
     const int grid = std::max(1, std::min((L.rows + W - 1) / W, sms));
-    kern<<<grid, 32 * W, smem, st>>>(L);
-    MV_CUDA_TRY(cudaGetLastError(), "wpr kernel launch");
+    MV_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(32 * W), smem, st, L), "wpr kernel launch");
     return MV_OK;
 }
 

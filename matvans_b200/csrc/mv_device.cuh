@@ -111,6 +111,23 @@ __device__ __forceinline__ uint4 ldg_nc_u4(const uint4 *p) {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Launch that may begin while the kernel before it in the stream ends: the kernel reads nothing that launches write (and
+// writes nothing but status bits) ahead of grid_dependency_wait.
+template <typename Arg>
+inline cudaError_t launch_dependent(void (*kern)(Arg), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Arg &arg) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, arg);
+}
+
 // Host side: per-device status word, lazily allocated once per device.
 uint32_t *device_status_word(mv_status *st);
 uint32_t wait_spin_limit();   // kWaitSpinLimit unless MV_INJECT_WAIT_LIMIT set another bound
