@@ -76,14 +76,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return mbar_wait_bounded(smem_u32(bar), parity, status, limit);
 }
 
-// 4-byte asynchronous copy global -> shared (cp.async, no registers): src_bytes (0, 2 or 4) are read, the
-// rest of the 4 bytes is zero-filled.  dst and src 4-byte aligned.  Completion: cp_async_commit, then
-// cp_async_wait_all in the issuing thread (and a barrier for other threads).
-__device__ __forceinline__ void cp_async_4(void *dst, const void *src, uint32_t src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits for the issuing thread's asynchronous copies.
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // 16-byte asynchronous copy global -> shared (dst a shared-memory address), cached in L2 only; dst and src
@@ -134,7 +127,6 @@ uint32_t wait_spin_limit();   // kWaitSpinLimit unless MV_INJECT_WAIT_LIMIT set 
 int inject_drop_copy();
 int sm_count();
 int max_smem_optin();
-int max_smem_per_sm();
 // Raise the kernel's dynamic shared-memory limit to `smem` (once per kernel
 // and device) and, if blocks_per_sm is non-NULL, return its occupancy for
 // `threads` threads (cached).  Safe to call while a stream is being captured.
