@@ -715,6 +715,14 @@ struct DotCons {
         }
         s.clamp();
     }
+    // 16 bytes of every vector at p (NV is the batch rounded up, so that one or two vectors are all there)
+    __device__ __forceinline__ void load_x(const int8_t *p, int batch, uint4 (&xv)[NV]) const {
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            xv[v] = ldx_u4(p);
+            if (NV <= 2 || v + 1 < batch) p += cols;
+        }
+    }
     __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
                                          uint32_t lw, int lane, volatile uint32_t *) {
         const int q0 = d.seg * seg_quads;
@@ -759,18 +767,16 @@ struct DotCons {
                 group(s, sm, lw, xv);
             }
         } else {  // x from global memory, one group ahead: long segments, and chains, whose x is not there any earlier
+            // (the vectors past the batch, whose sums nobody reads, read its last row: x ends there)
             const int8_t *xp = x + 4 * q0;
             uint4 xn[NV];
-#pragma unroll
-            for (int v = 0; v < NV; v++) xn[v] = ldx_u4(xp + (size_t)v * cols);
+            load_x(xp, L.batch, xn);
             for (int i = 0; i < nq; i += 4) {
                 uint4 xv[NV];
                 xp += i + 4 < nq ? 16 : 0;
 #pragma unroll
-                for (int v = 0; v < NV; v++) {
-                    xv[v] = xn[v];
-                    xn[v] = ldx_u4(xp + (size_t)v * cols);
-                }
+                for (int v = 0; v < NV; v++) xv[v] = xn[v];
+                load_x(xp, L.batch, xn);
                 group(s, sm, lw, xv);
             }
         }

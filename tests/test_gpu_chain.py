@@ -105,3 +105,24 @@ def test_chain_rejects_mismatched_shapes():
     Ms = [ops.Q8Matrix.encode(np.ones((64, 128), np.int8)), ops.Q8Matrix.encode(np.ones((64, 128), np.int8))]
     with pytest.raises(_lib.MatvansError):
         ops.Q8Chain(Ms, [1.0, 1.0])
+
+
+@pytest.mark.parametrize("B,engine", [(3, 0), (3, 1), (5, 1), (7, 1), (9, 1), (15, 1)])
+def test_chain_odd_batches(B, engine):
+    # a chain's x comes from global memory: no row past the batch's last is read (x0 is the head of a larger buffer,
+    # whose other rows change)
+    rng = np.random.default_rng(B)
+    dims = [512, 1008, 256]
+    Ws = [gauss(rng, 4.0, (dims[i + 1], dims[i])) for i in range(2)]
+    Ms = [ops.Q8Matrix.encode(W) for W in Ws]
+    buf = torch.from_numpy(rng.integers(-127, 128, size=(16, dims[0])).astype(np.int8)).cuda()
+    x = buf[:B].cpu().numpy()
+    scales = busy_scales(Ws, x)
+    ref = host_chain(Ws, scales, x)
+    C = ops.Q8Chain(Ms, scales, batch=B, tuning=(16, 1, 1, 0, 0, engine), x0=buf[:B])
+    for fill in (None, -128):
+        if fill is not None:
+            buf[B:] = fill
+        C.run()
+        assert np.array_equal(C.xs[1].cpu().numpy(), ref[1]) and np.array_equal(C.out8.cpu().numpy(), ref[2])
+    assert ops.device_status() == 0

@@ -141,3 +141,25 @@ def test_ragged(rows, cols, seg_quads, offset):
         assert np.array_equal(y.cpu().numpy(), ref), B
         assert np.array_equal(ys.cpu().numpy(), (ref.astype(np.float32) * s[None, :]).astype(np.float32)), B
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads", [(96, 2048, 68), (64, 8192, 128), (500, 1040, 260)])
+def test_x_from_global_memory_odd_batches(rows, cols, seg_quads):
+    # segments of more than 64 quads read x from global memory; batches below the 4, 8 or 16 vectors that the consumer
+    # holds (3 vectors, 5 to 7 of a small matrix, and with engine 1 up to 15) take no row past the batch's last.  x is the
+    # head of a larger buffer; the rows behind it change and the outputs do not
+    rng = np.random.default_rng(seg_quads)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, seg_quads=seg_quads)
+    for B, engine in [(3, 0), (5, 0), (6, 0), (7, 0), (3, 1), (6, 1), (9, 1), (13, 1), (15, 1)]:
+        buf = torch.randint(-128, 128, (16, cols), dtype=torch.int8, device="cuda")
+        x = buf[:B]
+        ref = oracle.matvec_i8(W, x.cpu().numpy())
+        tuning = (4, 1, 1, 0, 0, engine)  # (a launch shape that these blocks fit)
+        S = ops.Q8Stack([M], batch=B, xs=[x], tuning=tuning)
+        for fill in (None, 127):
+            if fill is not None:
+                buf[B:] = fill
+            for y in (M.matvec(x, tuning=tuning), S.run()[0]):
+                assert np.array_equal(y.cpu().numpy(), ref), (B, engine)
+    assert ops.device_status() == 0
