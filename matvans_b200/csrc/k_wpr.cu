@@ -212,7 +212,8 @@ __global__ void __launch_bounds__(1024) requant_cluster_kernel(const int32_t *y,
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ uint32_t warp_max[32], cta_max[8];
     const int step = (int)gridDim.x * 1024, i0 = (int)(blockIdx.x * 1024 + threadIdx.x);
-    grid_dependency_wait();  // y may be the launch before's
+    cluster_arrive_relaxed();  // (this CTA runs; waited for before the others' shared memory is written)
+    grid_dependency_wait();    // y may be the launch before's
     int v[kRequantEach];
     uint32_t local = 0;
 #pragma unroll
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(1024) requant_cluster_kernel(const int32_t *y,
     local = __reduce_max_sync(0xffffffffu, local);
     if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = local;
     __syncthreads();
+    cluster_wait();
     if (threadIdx.x < 32) {
         const uint32_t mine = __reduce_max_sync(0xffffffffu, warp_max[threadIdx.x]);
         if (threadIdx.x < gridDim.x) *cluster.map_shared_rank(&cta_max[blockIdx.x], threadIdx.x) = mine;

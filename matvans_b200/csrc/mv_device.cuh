@@ -99,6 +99,11 @@ __device__ __forceinline__ uint4 ldg_nc_u4(const uint4 *p) {
     return v;
 }
 
+// Cluster barrier in two halves, for every thread of the cluster.  Shared memory of another CTA may be touched only once
+// that CTA is known to run: arrive first thing, wait before the first access.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // Programmatic dependent launch: wait until the grids this one depends on are complete and their writes visible (at once
 // when it was launched without the attribute), and let the grid behind this one in the stream be scheduled.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -88,3 +88,20 @@ def test_requant_absmax(n):
         assert delta.item() == d
         assert np.array_equal(out8.cpu().numpy(), np.rint(y.astype(np.float32) / d).astype(np.int8))
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [4097, 9000, 8 * 1024 * 16])
+def test_requant_absmax_every_cta_counts(n):
+    # clusters of 2, 4 and 8 whose CTAs write their maxima to each other: the maximum moves over all of them, many launches
+    # behind one another
+    rng = np.random.default_rng(n)
+    base = rng.integers(-1000, 1001, size=n).astype(np.int32)
+    got, want = [], []
+    for i in range(64):
+        y = base.copy()
+        y[(i * 1024 + 7 * i) % n] = 5000 + i
+        got.append(ops.requant_absmax(torch.from_numpy(y).cuda()))
+        d = np.float32(5000 + i) / np.float32(127.0)
+        want.append((np.rint(y.astype(np.float32) / d).astype(np.int8), d))
+    for (out8, delta), (ref, d) in zip(got, want):
+        assert delta.item() == d and np.array_equal(out8.cpu().numpy(), ref)
