@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(32 * (1 + kAwsHelpers)) aws_kernel(const AwrLa
             blocks++;
         }
         const uint32_t over = min((cur + 64u) >> 7, blocks ? blocks - 1u : 0u);  // blocks whose words are all consumed
+        __syncwarp();  // (every lane has loaded its words of the steps before: one lane's arrival gives a block back)
         if (freed + (uint32_t)lane < over) mbar_arrive(&empty[(freed + (uint32_t)lane) % kAwsBlocks]);
         freed = max(freed, over);
         if (j + 8 <= nq) {

@@ -105,3 +105,18 @@ def test_requant_absmax_every_cta_counts(n):
         want.append((np.rint(y.astype(np.float32) / d).astype(np.int8), d))
     for (out8, delta), (ref, d) in zip(got, want):
         assert delta.item() == d and np.array_equal(out8.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("batch", [1, 16])
+def test_aws_blocks_come_round(batch):
+    # dense streams of many more blocks than the ring holds, so that each is overwritten while the decode runs on; the
+    # same sums every time
+    rng = np.random.default_rng(batch)
+    W = weights(rng, "dense", (160, 4096))
+    M = ops.AwsMatrix.encode(W)
+    x = torch.from_numpy(rng.integers(-128, 128, size=(batch, 4096)).astype(np.int8)).cuda()
+    ref = oracle.matvec_i8(W, x.cpu().numpy())
+    ys = [M.matvec(x) for _ in range(50)]
+    for y in ys:
+        assert np.array_equal(y.cpu().numpy(), ref)
+    assert ops.device_status() == 0
