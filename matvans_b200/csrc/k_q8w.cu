@@ -404,7 +404,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
                 o0 = __ldg(m.blk_off + b);
                 const uint32_t o1 = __ldg(m.blk_off + b + 1);
                 rows = o1 - o0;
-                if (o1 < o0 || o1 > m.blocks_rows || rows < 2 || (rows + 1) * 128u > L.block_bytes) {
+                if (o1 < o0 || o1 > m.blocks_rows || rows < 2 || rows >= L.block_bytes / 128u) {
                     atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
                     rows = 0;
                 }

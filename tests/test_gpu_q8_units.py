@@ -163,3 +163,19 @@ def test_x_from_global_memory_odd_batches(rows, cols, seg_quads):
             for y in (M.matvec(x, tuning=tuning), S.run()[0]):
                 assert np.array_equal(y.cpu().numpy(), ref), (B, engine)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [2 ** 25 - 1, 2 ** 25 + 3])
+def test_block_of_four_gigabytes_is_rejected(rows):
+    # offsets that claim a block of 2^32 bytes and more, all of it readable: no 32-bit size may wrap round to a small one
+    W = np.ones((32, 64), np.int8)
+    M = ops.Q8Matrix.encode(W)
+    M.blocks = torch.zeros(32 * (rows + 8), dtype=torch.int32, device="cuda")
+    M.blk_off = torch.tensor([0, rows], dtype=torch.int32, device="cuda")
+    M._view = M.view()
+    x = torch.ones((1, 64), dtype=torch.int8, device="cuda")
+    M.matvec(x)
+    assert ops.device_status(raise_on_error=False) == 1  # MV_DEV_STREAM_OVERRUN: nothing was decoded
+    G = ops.Q8Matrix.encode(W)
+    assert np.array_equal(G.matvec(x).cpu().numpy(), oracle.matvec_i8(W, x.cpu().numpy()))
+    assert ops.device_status() == 0
