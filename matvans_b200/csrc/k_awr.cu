@@ -29,7 +29,7 @@
 // What bounds it: issue, ~45 instructions a step (98 in the form this replaced,
 // which kept the words in registers and moved them by shuffles).  Measured on a
 // B200, 4096x4096, one vector: 17.6 us before, 11.5 us now; calls back to back,
-// the table built while the launch before ends, 13.4 -> 11.1 us.
+// each launched while the one before it ends, 13.3 -> 11.4 us.
 //
 // The "ans-warp-stripes" layout (ans-warp-stripes-kernel.cu:21-227, encoder.py:
 // 323-391) has the same coder and word stream with lane = row of a 32-row stripe:
@@ -145,12 +145,11 @@ __global__ void __launch_bounds__(32 * kAwrWarps<NV>) awr_kernel(const AwrLaunch
     extern __shared__ __align__(1024) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
     const int nq = L.cols >> 2;
-    awr_table(L, smem);
     uint32_t *ring = reinterpret_cast<uint32_t *>(smem + kAwrLut + (uint32_t)warp * kAwrRing);
     uint32_t *xs = reinterpret_cast<uint32_t *>(smem + kAwrLut + (uint32_t)W * kAwrRing);
-    // (the table is built while the launch before this one ends; x and the outputs are not touched earlier)
-    grid_dependency_wait();
+    grid_dependency_wait();  // (the launch before this one may have written the tables, the stream or x)
     grid_launch_dependents();
+    awr_table(L, smem);
     awr_stage_x<NV>(L, xs);
     __syncthreads();
 
@@ -254,9 +253,9 @@ __global__ void __launch_bounds__(32 * (1 + kAwsHelpers)) aws_kernel(const AwrLa
     }
     if (threadIdx.x == 0) stop = 0;
     fence_mbar_init();
-    awr_table(L, smem);
     grid_dependency_wait();  // (as in awr_kernel)
     grid_launch_dependents();
+    awr_table(L, smem);
     awr_stage_x<NV>(L, xs);
     __syncthreads();
 

@@ -270,6 +270,7 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.drop_copy = inject_drop_copy();
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
+        L.early = v0 > 0 || L.job0.atomic || L.span;
         if (L.job0.atomic) {
             rc = zero_launch(L.job0.y, (size_t)nb * m->rows, st);
             if (rc) return rc;
@@ -329,6 +330,7 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
         L.drop_copy = inject_drop_copy();
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
+        L.early = v0 > 0 || L.span;
         if (L.span) {
             rc = cut_stripes_launch<float, false>(L, L.job0.ys, nullptr, st);
             if (rc) return rc;
@@ -375,6 +377,7 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
         L.drop_copy = inject_drop_copy();
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
+        L.early = 1;  // (dX has been zeroed)
         rc = q8w_launch_bwd(L, decode_warps(tuning, t), units, st);
         if (rc) return rc;
     }
@@ -532,6 +535,7 @@ mv_status mv_q8_stack_matvec(const mv_q8_job *jobs_dev, int njobs, const mv_q8_s
     rc = mv::check_shape(t, t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaShape, nv, info->max_blk_rows, info->tbl_stripe_max);
     if (rc) return rc;
     dim3 zg(64, std::min(njobs, 1024));
+    L.early = info->atomic_jobs > 0;
     if (info->atomic_jobs > 0) {
         mv::q8s_zero_atomic_y<<<zg, 256, 0, st>>>(jobs_dev, njobs, batch);
         MV_CUDA_TRY(cudaGetLastError(), "q8s_zero_atomic_y launch");

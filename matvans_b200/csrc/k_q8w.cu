@@ -376,9 +376,8 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
         return r;
     };
     ItemRec r = record(0);
-    // Up to here, and in the first table's staging and build, only matrices and job descriptions were read, which no
-    // launch of this library writes: the launch before this one may still be running (see launch_t).  Inputs, outputs and
-    // the queue come after it.
+    // Up to here, and in the first table's staging and build, only the matrix was read (L.early: see q8w_kernel).  Inputs,
+    // outputs and the queue come after the launch before this one.
     grid_dependency_wait();
     grid_launch_dependents();
     if (L.queue && r.it >= 0 && lane == 0) grabbed = atomicAdd(L.queue, 1u);
@@ -1821,6 +1820,11 @@ __global__ void __launch_bounds__(32 * (kFirstDecode + Cons::kMaxDecode), 1) q8w
         if (warp == 0) tmem_alloc(misc + 1, tmem_cols<Cons>(L.W));
         tcgen05_fence_before();
     }
+    // The launch before this one may still be running (see launch_t).  Whatever the caller passes, matrices and job tables
+    // too, may be what it writes, so nothing of that is read before it is complete and its writes are visible.  Where the
+    // launch before is this library's own, made in the same call after everything the caller's memory depends on (a zeroing
+    // launch, an earlier pass), the first item's record and table go ahead of it.
+    if (!L.early) grid_dependency_wait();
     __syncthreads();
     if (Cons::kMma) {
         tcgen05_fence_after();
@@ -1915,10 +1919,11 @@ mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
                     "q8 chain cooperative launch");
         return MV_OK;
     }
-    // Programmatic dependent launch: a CTA takes over an SM as soon as the launch before it has left it, and fetches and
-    // builds its first table meanwhile (5 to 7 us); see produce() for what waits.  Measured on a B200, launches back to back
-    // without and with it: a layer of seven matrices, one vector 73.7 -> 71.0 us, 16 vectors 108.6 -> 104.9; of hidden size
-    // 512, 13.4 -> 10.4; 11008x4096, 64 int8 vectors 44.5 -> 40.3, bf16 56.0 -> 51.6.
+    // Programmatic dependent launch: a CTA takes over an SM as soon as the launch before it has left it, and sets up its
+    // barriers and tensor memory meanwhile; see q8w_kernel for what waits.  Measured on a B200, calls back to back without and
+    // with it: a layer of seven matrices, one vector 77.3 -> 74.7 us, 16 vectors 110.3 -> 107.5; 4090x4100, 2 vectors
+    // 15.3 -> 13.0; 11008x4096, 64 vectors 47.8 -> 46.4.  (With the first table fetched and built ahead of the wait, 72, 104,
+    // 12.1 and 42.6 us; but then a matrix that the launch before writes would be read too early.)
     MV_CUDA_TRY(launch_dependent(kern, dim3(grid), block, L.lay.total, st, L), "q8 kernel launch");
     return MV_OK;
 }

@@ -70,6 +70,8 @@ template <int NV>
 __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch L) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    grid_dependency_wait();  // (the launch before this one may have written the tables, the payload or x)
+    grid_launch_dependents();
     // decode table: eight threads per quantile, four lane columns each
     for (uint32_t i = threadIdx.x; i < 256 * 8; i += blockDim.x) {
         const uint32_t q = i >> 3, r = __ldg(L.ppf + q);
@@ -85,9 +87,6 @@ __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch
         uint4 *dst = reinterpret_cast<uint4 *>(smem + 256u * q + 16u * (i & 7u));
         *dst = e4;
     }
-    // (the table is built while the launch before this one ends; x and the outputs are not touched earlier)
-    grid_dependency_wait();
-    grid_launch_dependents();
     __syncthreads();
 
     const uint32_t lane4 = (uint32_t)lane * 4u;
@@ -204,7 +203,7 @@ __global__ void requant_kernel(const int32_t *y, int n, const uint32_t *m, int8_
 // The same in one launch for n up to kRequantMax: one cluster of up to 8 CTAs holds y in registers, exchanges the CTAs'
 // maxima through their shared memory and quantises.  Bound by launch latency, which a memset and two kernels pay three
 // times: on a B200, 4096 elements 6.4 -> 3.7 us, 131072 9.3 -> 5.1 us.  Launched while the kernel before it ends (it waits
-// for it before it reads): WPR 4096x4096 and this, the calls, 22.4 -> 19.8 us.
+// for it before it reads): WPR 4096x4096 and this, the calls, 22.5 -> 20.3 us.
 constexpr int kRequantEach = 16, kRequantMax = 8 * 1024 * kRequantEach;
 
 __global__ void __launch_bounds__(1024) requant_cluster_kernel(const int32_t *y, int n, uint32_t *m, int8_t *out8, float *delta) {

@@ -109,8 +109,9 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Launch that may begin while the kernel before it in the stream ends: the kernel reads nothing that launches write (and
-// writes nothing but status bits) ahead of grid_dependency_wait.
+// Launch that may begin while the kernel before it in the stream ends.  That kernel may be the caller's, and may write
+// anything that this one is given: ahead of grid_dependency_wait the kernel reads none of the caller's memory (and writes
+// nothing but status bits).
 template <typename Arg>
 inline cudaError_t launch_dependent(void (*kern)(Arg), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Arg &arg) {
     cudaLaunchAttribute attr[1];

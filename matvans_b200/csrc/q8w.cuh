@@ -33,6 +33,7 @@ struct Q8WLaunch {
     // One job in even shares (nonzero: its number of units): CTA c of G takes units [c span / G, (c + 1) span / G),
     // whatever stripes they are of.  Sums of a stripe that several CTAs share are added to y (ys) unscaled.
     uint32_t span;
+    int early;  // the launch before this one is this library's own, made in the same call (see q8w_kernel)
     int ragged;  // integer products, one job: x off the 16-byte grid, columns or segments not whole groups of 16 columns
     // set by the launcher
     int W, S;              // decode warps, stream slots
