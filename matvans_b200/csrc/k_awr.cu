@@ -70,9 +70,9 @@ constexpr int kAwrWarps = NV <= 4 ? 28 : 20;
 __device__ __forceinline__ void awr_table(const AwrLaunch &L, unsigned char *lut) {
     for (uint32_t i = threadIdx.x; i < 128 * 4; i += blockDim.x) {
         const uint32_t q = i >> 2, sh = 8 * (q & 3);
-        const uint32_t sym = (__ldg(L.ppf + (q >> 2)) >> sh) & 0xFF;
-        const uint32_t c = (__ldg(L.cum + (q >> 2)) >> sh) & 0xFF;
-        const uint32_t p = (__ldg(L.prob + (q >> 2)) >> sh) & 0xFF;
+        const uint32_t sym = (ldp(L.ppf + (q >> 2)) >> sh) & 0xFF;
+        const uint32_t c = (ldp(L.cum + (q >> 2)) >> sh) & 0xFF;
+        const uint32_t p = (ldp(L.prob + (q >> 2)) >> sh) & 0xFF;
         if (c > q || p == 0) atomicOr(L.status, MV_DEV_BAD_TABLE);
         const uint32_t e = p | sym << 16 | ((q - c) & 0xFFu) << 24;
         uint4 *dst = reinterpret_cast<uint4 *>(lut + q * 128u + (i & 3u) * 32u);
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(32 * kAwrWarps<NV>) awr_kernel(const AwrLaunch
     for (int row = blockIdx.x * W + warp; row < units; row += gridDim.x * W) {
         // The first block holds the initial states (fields z, w) and the first 64 words of the stream (x, y); every
         // later block 128 words, field by field (ans-warp-rows-kernel.cu:76-139).
-        size_t bi = __ldg(L.offs + row);  // uint4 index of the latest block in the ring
+        size_t bi = ldp(L.offs + row);  // uint4 index of the latest block in the ring
         auto block = [&](size_t at) {
             return !BOUNDED || at + 32 <= L.n_u4 ? L.comp[at + lane] : make_uint4(0, 0, 0, 0);
         };
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(32 * (1 + kAwsHelpers)) aws_kernel(const AwrLa
     __syncthreads();
 
     const int stripe = blockIdx.x;
-    const size_t b0 = __ldg(L.offs + stripe);  // uint4 index of the stripe's first block
+    const size_t b0 = ldp(L.offs + stripe);  // uint4 index of the stripe's first block
     const size_t nblk = b0 + 32 <= L.n_u4 ? (L.n_u4 - b0) / 32 : 0;  // whole blocks that can be read
     volatile uint32_t *done = &stop;
 

@@ -207,17 +207,17 @@ __device__ __forceinline__ void locate(const Q8WLaunch &L, uint32_t it, int &job
     uint32_t rel = it;
     int ng = L.job0.ngroups;
     if (L.jobs) {
-        if (job + 1 < L.njobs && __ldg(&L.jobs[job + 1].item0) <= it) {
+        if (job + 1 < L.njobs && ldp(&L.jobs[job + 1].item0) <= it) {
             int lo = job + 1, hi = L.njobs - 1;
             while (lo < hi) {  // last job with item0 <= it
                 const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(&L.jobs[mid].item0) <= it) lo = mid;
+                if (ldp(&L.jobs[mid].item0) <= it) lo = mid;
                 else hi = mid - 1;
             }
             job = lo;
         }
-        rel = it - __ldg(&L.jobs[job].item0);
-        ng = __ldg(&L.jobs[job].ngroups);
+        rel = it - ldp(&L.jobs[job].item0);
+        ng = ldp(&L.jobs[job].ngroups);
     }
     stripe = (int)(rel / (uint32_t)ng);
     item_segs(job_at(L, job).m, ng, (int)(rel % (uint32_t)ng), sb, se);
@@ -228,15 +228,20 @@ __device__ __forceinline__ int8_t chain_q(const ItemRec &I, int sum) {
     return (int8_t)max(-128, min(127, __float2int_rn((float)sum * I.chain_scale)));
 }
 
+// The scale of a row's outputs (loaded ahead of the stores, which a plain load would not pass).
+__device__ __forceinline__ float row_scale(const ItemRec &I, int row) {
+    return I.ys && row < I.rows ? ldp(I.scales + row) : 0.f;
+}
+
 // One output: y (exact int32), its scaled form, and the chain's int8.
-__device__ __forceinline__ void emit(const ItemRec &I, int v, int row, int sum) {
+__device__ __forceinline__ void emit(const ItemRec &I, int v, int row, int sum, float scale) {
     const size_t i = (size_t)v * I.rows + row;
     if (I.atomic) {
         atomicAdd(I.y + i, sum);
         return;
     }
     I.y[i] = sum;
-    if (I.ys) I.ys[i] = (float)sum * __ldg(I.scales + row);
+    if (I.ys) I.ys[i] = (float)sum * scale;
     if (I.chain_out) I.chain_out[i] = chain_q(I, sum);
 }
 
@@ -250,10 +255,13 @@ __device__ __forceinline__ void stage_table(const Q8WLaunch &L, const ItemRec &r
     uint32_t *so = reinterpret_cast<uint32_t *>(sm + L.lay.stage_o) + area * kStageOffs;
     const uint32_t r0 = m.local ? (uint32_t)r.stripe * 32u : 0u;
     const uint32_t nt = m.local ? 32u : 1u;
-    const uint32_t o = (uint32_t)lane <= nt ? __ldg(m.tbl_off + r0 + lane) : 0u;
-    const uint32_t te = __ldg(m.tbl_off + r0 + nt);
+    const uint32_t *toff = m.tbl_off + r0;  // (the job's fields once, ahead of the stores: a plain load passes none)
+    const uint16_t *tbl = m.tbl;
+    const uint32_t tbl_len = m.tbl_len;
+    const uint32_t o = ldp(toff + min((uint32_t)lane, nt));
+    const uint32_t te = ldp(toff + nt);
     const uint32_t tb = __shfl_sync(0xffffffffu, o, 0);
-    const bool ok = te >= tb && te <= m.tbl_len && te - tb <= (uint32_t)L.tbl_stage;
+    const bool ok = te >= tb && te <= tbl_len && te - tb <= (uint32_t)L.tbl_stage;
     if ((uint32_t)lane <= nt) so[lane] = (ok && o >= tb && o <= te) ? o - tb : 0u;
     if (lane == 0) {
         if (nt == 32u) so[32] = ok ? te - tb : 0u;
@@ -263,17 +271,17 @@ __device__ __forceinline__ void stage_table(const Q8WLaunch &L, const ItemRec &r
     if (ok) {
         const uint32_t a = tb & ~7u, n = te - a;
         unsigned char *se = sm + L.lay.stage_e + (uint32_t)area * ((uint32_t)L.tbl_stage + kStagePad) * 2u;
-        if (((uintptr_t)m.tbl & 15) == 0) {
+        if (((uintptr_t)tbl & 15) == 0) {
             const uint32_t dst = smem_u32(se);
             for (uint32_t c = lane; 8 * c < n; c += 32) {
-                const uint32_t avail = min(8u, m.tbl_len - (a + 8 * c));
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16u * c), "l"(m.tbl + a + 8 * c),
+                const uint32_t avail = min(8u, tbl_len - (a + 8 * c));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 16u * c), "l"(tbl + a + 8 * c),
                              "r"(2u * avail)
                              : "memory");
             }
         } else {
             uint16_t *d = reinterpret_cast<uint16_t *>(se);
-            for (uint32_t e = lane; e < n; e += 32) d[e] = __ldg(m.tbl + a + e);
+            for (uint32_t e = lane; e < n; e += 32) d[e] = ldp(tbl + a + e);
         }
     }
     cp_async_mbar_arrive_noinc(B.staged(area));
@@ -349,7 +357,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
             r.scales = J.scales;
             r.ys = J.ys;
             if (L.chain_scales) {
-                r.chain_scale = __ldg(L.chain_scales + job);
+                r.chain_scale = ldp(L.chain_scales + job);
                 r.chain_out = job + 1 < L.njobs ? const_cast<int8_t *>(L.jobs[job + 1].x) : L.chain_out8;
             }
             r.build = job != tjob || (r.local && r.stripe != tstripe);
@@ -400,8 +408,8 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
             uint32_t o0 = 0, rows = 0;
             if (!end && i < r.n) {
                 const int b = r.stripe * m.nseg + r.sb + (int)i;
-                o0 = __ldg(m.blk_off + b);
-                const uint32_t o1 = __ldg(m.blk_off + b + 1);
+                o0 = ldp(m.blk_off + b);
+                const uint32_t o1 = ldp(m.blk_off + b + 1);
                 rows = o1 - o0;
                 if (o1 < o0 || o1 > m.blocks_rows || rows < 2 || rows >= L.block_bytes / 128u) {
                     atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
@@ -668,10 +676,10 @@ __device__ __forceinline__ uint32_t x_quad_at(const Q8WLaunch &L, const int8_t *
     const uint32_t *a = reinterpret_cast<const uint32_t *>((uintptr_t)p & ~(uintptr_t)3);
     uint32_t v = 0;
     if ((uintptr_t)a >= (uintptr_t)x0 && (uintptr_t)(a + 2) <= (uintptr_t)xe) {
-        v = __funnelshift_r(__ldg(a), __ldg(a + 1), 8u * (uint32_t)((uintptr_t)p & 3));
+        v = __funnelshift_r(ldp(a), ldp(a + 1), 8u * (uint32_t)((uintptr_t)p & 3));
         if (valid < 4) v &= (1u << (8 * valid)) - 1u;
     } else {
-        for (int j = 0; j < min(valid, 4); j++) v |= (uint32_t)(uint8_t)__ldg(p + j) << (8 * j);
+        for (int j = 0; j < min(valid, 4); j++) v |= (uint32_t)(uint8_t)ldp(p + j) << (8 * j);
     }
     return v;
 }
@@ -798,10 +806,11 @@ struct DotCons {
         const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
         volatile int *red = reinterpret_cast<volatile int *>(sm + L.lay.red) + (size_t)(k % kRing) * NV * 32 + lane;
         const int row = I.stripe * 32 + lane;
+        const float scale = row_scale(I, row);
         for (int v = q; v < NV; v += kTableWarps) {
             const int sum = red[v * 32];
             red[v * 32] = 0;
-            if (row < I.rows && v < L.batch) emit(I, v, row, sum);
+            if (row < I.rows && v < L.batch) emit(I, v, row, sum, scale);
         }
     }
     __device__ __forceinline__ void drain(const Q8WLaunch &) {}
@@ -1055,10 +1064,11 @@ struct MmaCons {
         if constexpr (kOwn) {
             volatile int *red = reinterpret_cast<volatile int *>(sm + L.lay.red) + (size_t)(k % kRing) * kRed + lane;
             const int row = I.stripe * 32 + lane;
+            const float scale = row_scale(I, row);
             for (int v = q; v < L.batch; v += kTableWarps) {
                 const int sum = red[v * kPitch];
                 red[v * kPitch] = 0;
-                if (row < I.rows) emit(I, v, row, sum);
+                if (row < I.rows) emit(I, v, row, sum, scale);
             }
         } else {
             tcgen05_fence_after();
@@ -1087,6 +1097,9 @@ struct MmaCons {
                         for (int j = 0; j < 16; j++) sum[j] += __shfl_down_sync(0xffffffffu, sum[j], 16);
                     const int v = 16 * q + lane - (int)base, row0 = I.stripe * 32 + h;
                     if ((uint32_t)lane >= base && (uint32_t)lane < base + 16u && v < L.batch) {
+                        float sc[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j++) sc[j] = row_scale(I, row0 + j);
                         if (!I.atomic && row0 + 16 <= I.rows && (I.rows & 3) == 0 && (((uintptr_t)I.y | (uintptr_t)I.ys) & 15) == 0) {
                             int4 *dst = reinterpret_cast<int4 *>(I.y + (size_t)v * I.rows + row0);
 #pragma unroll
@@ -1095,16 +1108,14 @@ struct MmaCons {
                             if (I.ys) {
                                 float4 *ds = reinterpret_cast<float4 *>(I.ys + (size_t)v * I.rows + row0);
 #pragma unroll
-                                for (int j = 0; j < 4; j++) {
-                                    const float *sc = I.scales + row0 + 4 * j;
-                                    ds[j] = make_float4((float)sum[4 * j] * __ldg(sc), (float)sum[4 * j + 1] * __ldg(sc + 1),
-                                                        (float)sum[4 * j + 2] * __ldg(sc + 2), (float)sum[4 * j + 3] * __ldg(sc + 3));
-                                }
+                                for (int j = 0; j < 4; j++)
+                                    ds[j] = make_float4((float)sum[4 * j] * sc[4 * j], (float)sum[4 * j + 1] * sc[4 * j + 1],
+                                                        (float)sum[4 * j + 2] * sc[4 * j + 2], (float)sum[4 * j + 3] * sc[4 * j + 3]);
                             }
                         } else {
 #pragma unroll
                             for (int j = 0; j < 16; j++)
-                                if (row0 + j < I.rows) emit(I, v, row0 + j, sum[j]);
+                                if (row0 + j < I.rows) emit(I, v, row0 + j, sum[j], sc[j]);
                         }
                     }
                 }
@@ -1273,6 +1284,9 @@ struct FwdCons {
                 const int row0 = I.stripe * 32 + h;
                 if (lane < 16 && v < L.batch) {
                     float *dst = I.ys + (size_t)v * I.rows + row0;
+                    float sc[16];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) sc[j] = row_scale(I, row0 + j);
                     if (I.atomic) {  // even shares: the other CTA's part is added, and scaled with it afterwards
 #pragma unroll
                         for (int j = 0; j < 16; j++)
@@ -1281,12 +1295,11 @@ struct FwdCons {
 #pragma unroll
                         for (int j = 0; j < 16; j += 4)
                             *reinterpret_cast<float4 *>(dst + j) = make_float4(
-                                sum[j] * __ldg(I.scales + row0 + j), sum[j + 1] * __ldg(I.scales + row0 + j + 1),
-                                sum[j + 2] * __ldg(I.scales + row0 + j + 2), sum[j + 3] * __ldg(I.scales + row0 + j + 3));
+                                sum[j] * sc[j], sum[j + 1] * sc[j + 1], sum[j + 2] * sc[j + 2], sum[j + 3] * sc[j + 3]);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 16; j++)
-                            if (row0 + j < I.rows) dst[j] = sum[j] * __ldg(I.scales + row0 + j);
+                            if (row0 + j < I.rows) dst[j] = sum[j] * sc[j];
                     }
                 }
             }
@@ -1356,10 +1369,10 @@ struct FwdDot {
                 group(s, sm, lw, *reinterpret_cast<const uint4 *>(xs), *reinterpret_cast<const uint4 *>(xs + 16));
         } else {
             const uint4 *xp = reinterpret_cast<const uint4 *>(x + 4 * q0);
-            uint4 a = __ldg(xp), b = __ldg(xp + 1);
+            uint4 a = ldp(xp), b = ldp(xp + 1);
             for (int i = 0; i < nq; i += 4) {
                 xp += i + 4 < nq ? 2 : 0;
-                const uint4 a1 = __ldg(xp), b1 = __ldg(xp + 1);
+                const uint4 a1 = ldp(xp), b1 = ldp(xp + 1);
                 group(s, sm, lw, a, b);
                 a = a1;
                 b = b1;
@@ -1388,7 +1401,7 @@ struct FwdDot {
         for (uint32_t i = 0; i < nc; i++, w = w + 1 < W ? w + 1 : 0) sum += red[w * 32];
         if (row >= I.rows) return;
         if (I.atomic) atomicAdd(I.ys + row, sum);  // even shares: scaled together with the other CTA's part afterwards
-        else I.ys[row] = sum * __ldg(I.scales + row);
+        else I.ys[row] = sum * ldp(I.scales + row);
     }
 };
 
@@ -1439,12 +1452,12 @@ struct BwdCons {
     static __device__ __forceinline__ void prepare(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *, uint32_t tmem) {
         const int q = threadIdx.x >> 5, v = threadIdx.x & 31, row0 = I.stripe * 32;
         const uint16_t *dy = reinterpret_cast<const uint16_t *>(I.x) + (size_t)v * I.rows + row0;
-        const float sl = row0 + v < I.rows ? __ldg(I.scales + row0 + v) : 0.f;  // lane = row
+        const float sl = row0 + v < I.rows ? ldp(I.scales + row0 + v) : 0.f;  // lane = row
         float g[32];
         if (v < L.batch && row0 + 32 <= I.rows && ((uintptr_t)dy & 15) == 0) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const uint4 d = __ldg(reinterpret_cast<const uint4 *>(dy) + j);
+                const uint4 d = ldp(reinterpret_cast<const uint4 *>(dy) + j);
                 const uint32_t w[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -1455,7 +1468,7 @@ struct BwdCons {
         } else {
 #pragma unroll
             for (int j = 0; j < 32; j++)
-                g[j] = v < L.batch && row0 + j < I.rows ? __uint_as_float((uint32_t)__ldg(dy + j) << 16) : 0.f;
+                g[j] = v < L.batch && row0 + j < I.rows ? __uint_as_float((uint32_t)ldp(dy + j) << 16) : 0.f;
         }
 #pragma unroll
         for (int j = 0; j < 32; j++) g[j] *= __shfl_sync(0xffffffffu, sl, j);
@@ -1620,7 +1633,7 @@ struct BwdDot {
         const int row = I.stripe * 32 + (int)threadIdx.x;
         float v = 0.f;
         if (row < I.rows)
-            v = __ldg(I.scales + row) * __uint_as_float((uint32_t)__ldg(reinterpret_cast<const uint16_t *>(I.x) + row) << 16);
+            v = ldp(I.scales + row) * __uint_as_float((uint32_t)ldp(reinterpret_cast<const uint16_t *>(I.x) + row) << 16);
         reinterpret_cast<float *>(sm + L.lay.red)[(k % kRing) * kRed + threadIdx.x] = v;
     }
     __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,

@@ -55,13 +55,13 @@ constexpr int kWprWarps = NV <= 4 ? 28 : NV <= 8 ? 16 : 12;
 
 // Words [ix, ix + 8) of the payload; zeros past its end.
 __device__ __forceinline__ uint4 wpr_chunk(const WprLaunch &L, uint64_t ix) {
-    if (ix + 8 <= L.payload_size && (ix & 7) == 0) return __ldg(reinterpret_cast<const uint4 *>(L.payload + ix));
+    if (ix + 8 <= L.payload_size && (ix & 7) == 0) return ldp(reinterpret_cast<const uint4 *>(L.payload + ix));
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const uint64_t i = ix + 2 * j;
-        w[j] = (i < L.payload_size ? (uint32_t)__ldg(L.payload + i) : 0u) |
-               (i + 1 < L.payload_size ? (uint32_t)__ldg(L.payload + i + 1) << 16 : 0u);
+        w[j] = (i < L.payload_size ? (uint32_t)ldp(L.payload + i) : 0u) |
+               (i + 1 < L.payload_size ? (uint32_t)ldp(L.payload + i + 1) << 16 : 0u);
     }
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
@@ -74,12 +74,12 @@ __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch
     grid_launch_dependents();
     // decode table: eight threads per quantile, four lane columns each
     for (uint32_t i = threadIdx.x; i < 256 * 8; i += blockDim.x) {
-        const uint32_t q = i >> 3, r = __ldg(L.ppf + q);
+        const uint32_t q = i >> 3, r = ldp(L.ppf + q);
         uint32_t e = 0;
         if ((int)r + 1 > L.G) {
             atomicOr(L.status, MV_DEV_BAD_TABLE);
         } else {
-            const uint32_t c0 = __ldg(L.cdf + r), c1 = __ldg(L.cdf + r + 1);
+            const uint32_t c0 = ldp(L.cdf + r), c1 = ldp(L.cdf + r + 1);
             if (c0 > q) atomicOr(L.status, MV_DEV_BAD_TABLE);  // (q - c0 is never negative for a valid table)
             e = ((c1 - c0) & 0xFFu) | (uint32_t)(uint8_t)(int8_t)(L.min_value + (int)r) << 16 | (q - c0) << 24;
         }
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch
     const uint32_t ring = smem_u32(smem) + 65536u + (uint32_t)warp * kRingAlloc + (uint32_t)lane * 2u;
     const int groups = L.cols / 512;
     for (int row = blockIdx.x * W + warp; row < L.rows; row += gridDim.x * W) {
-        const uint64_t ix0 = (uint64_t)__ldg(L.cursors + row) + 8u * (uint32_t)lane;
+        const uint64_t ix0 = (uint64_t)ldp(L.cursors + row) + 8u * (uint32_t)lane;
         uint32_t staged = 0;  // words in the ring so far; the chunk behind them is in `nxt`
         uint4 nxt = wpr_chunk(L, ix0);
         const uint4 c0 = nxt;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(32 * kWprWarps<NV>) wpr_kernel(const WprLaunch
             uint4 xv[NV];
 #pragma unroll
             for (int v = 0; v < NV; v++)
-                xv[v] = v < L.batch ? __ldg(reinterpret_cast<const uint4 *>(xp + (size_t)v * L.cols)) : make_uint4(0, 0, 0, 0);
+                xv[v] = v < L.batch ? ldp(reinterpret_cast<const uint4 *>(xp + (size_t)v * L.cols)) : make_uint4(0, 0, 0, 0);
             const uint32_t a0 = a;
 #pragma unroll
             for (int k = 0; k < 4; k++) {

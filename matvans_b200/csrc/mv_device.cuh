@@ -109,6 +109,13 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Plain load.  The kernels that launch_dependent starts read global memory this way and not by the read-only path (__ldg),
+// which wants memory that does not change in the kernel's life: theirs begins before the launch before them has written.
+template <typename T>
+__device__ __forceinline__ T ldp(const T *p) {
+    return *p;
+}
+
 // Launch that may begin while the kernel before it in the stream ends.  That kernel may be the caller's, and may write
 // anything that this one is given: ahead of grid_dependency_wait the kernel reads none of the caller's memory (and writes
 // nothing but status bits).
