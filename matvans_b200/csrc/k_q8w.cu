@@ -1892,9 +1892,9 @@ template <class Cons>
 mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
     Q8WLaunch L = L0;
     const uint32_t limit = (uint32_t)max_smem_optin();
-    // CUDA-core consumers: x of a segment behind its block, but for chains
+    // CUDA-core consumers: x of a segment behind its block, but for chains, and for the backward, whose job0.x is dY
     L.block_bytes = L.slot_bytes;
-    if (!Cons::kMma && !L.chain_scales) {
+    if (!Cons::kMma && !Cons::kPrepare && !L.chain_scales) {
         L.x_off = L.slot_bytes;
         L.x_quad = Cons::kFloat ? 8u : 4u;
         L.slot_bytes += L.x_quad * (uint32_t)(L.batch * kXQuads);

@@ -179,3 +179,29 @@ def test_block_of_four_gigabytes_is_rejected(rows):
     G = ops.Q8Matrix.encode(W)
     assert np.array_equal(G.matvec(x).cpu().numpy(), oracle.matvec_i8(W, x.cpu().numpy()))
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,seg_quads", [(32, 4096, 64), (100, 1520, 36), (257, 8192, 0)])
+def test_float_backward_reads_dy_alone(rows, cols, seg_quads):
+    # many more columns than rows, dY off the 16-byte grid, a dX off it too, each in the middle of a larger buffer that is
+    # all NaN or a sign value around it: dY is read within its rows, dX written within its columns (bounds as above; a dX off
+    # the grid, and one vector, have no split of s . dy)
+    rng = np.random.default_rng(rows + cols)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -127, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, seg_quads=seg_quads)
+    s = torch.from_numpy(rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)).cuda()
+    W64 = torch.from_numpy(W).cuda().double()
+    for B in (1, 2, 5, 33):
+        for dy_off, dx_off in [(0, 0), (1, 0), (5, 1), (8, 3)]:
+            dyb = torch.full((B * rows + 4096,), float("nan"), dtype=torch.bfloat16, device="cuda")
+            dy = dyb[dy_off:dy_off + B * rows].view(B, rows)
+            dy.copy_(torch.from_numpy(rng.standard_normal((B, rows)).astype(np.float32)))
+            dxb = torch.full((B * cols + 64,), -7.0, device="cuda")
+            dx = dxb[dx_off:dx_off + B * cols].view(B, cols)
+            M.matvec_t_bf16(dy, s, out=dx)
+            g = dy.double() * s.double()
+            err = (dx.double() - g @ W64).abs() / (g.abs() @ W64.abs()).clamp_min(1e-30)
+            bound = (0.0 if B == 1 or dx_off % 4 else 2.0 ** -17) + 2.0 ** -23 * (rows + 32)
+            assert err.max().item() < bound, (B, dy_off, dx_off)
+            assert (dxb[:dx_off] == -7).all() and (dxb[dx_off + B * cols:] == -7).all(), (B, dy_off, dx_off)
+    assert ops.device_status() == 0
