@@ -217,7 +217,12 @@ mv_status mv_q8_matvec(const mv_q8_view *m, const int8_t *x_dev, int batch, int3
  *                from MV_MMA_MIN_VECTORS vectors on it may be the tensor
  *                cores (tcgen05.mma kind::i8, TMEM accumulators, up to 64
  *                vectors per decode), below the CUDA cores (dp4a); 1 = CUDA
- *                cores (up to 16 vectors per decode). */
+ *                cores (up to 16 vectors per decode).  The sums are exact
+ *                either way.
+ *                float form: 0 = one vector on the CUDA cores, more on the
+ *                tensor cores (fp32 accumulation; backward: s . dy as two
+ *                bf16 terms, 2^-17 of it); 1 = CUDA cores, fp32 throughout,
+ *                for any number of vectors (up to 8 per decode). */
 #define MV_ENGINE_AUTO 0
 #define MV_ENGINE_DP4A 1
 /* Smallest integer batch that engine 0 (MV_ENGINE_AUTO) can run on the tensor
@@ -307,7 +312,7 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
 /* Float form (no reference counterpart): y[b][r] = s[r] * sum_c W[r][c] *
  * x[b][c] with x bf16 [batch][cols] (16-byte aligned), fp32 accumulation in a
  * fixed order (deterministic), fp32 y [batch][rows].  cols % 16 == 0.  Passes
- * of up to 64 vectors share one decode. */
+ * of up to 64 vectors (8 with engine 1) share one decode. */
 mv_status mv_q8_matvec_bf16(const mv_q8_view *m, const uint16_t *x_dev, int batch,
                             const float *row_scales_dev, float *y_dev, const mv_q8_tuning *tuning,
                             void *stream);
@@ -317,7 +322,8 @@ mv_status mv_q8_matvec_bf16(const mv_q8_view *m, const uint16_t *x_dev, int batc
  * (zeroed by the call).  The streams are decoded again (W is never stored);
  * the 32 rows of a stripe are summed per column inside the warp and stripes
  * are combined with fp32 atomics, so the result is reproducible to fp32
- * rounding, not bit for bit.  Passes of up to 32 vectors share one decode. */
+ * rounding, not bit for bit.  Passes of up to 32 vectors (8 with engine 1)
+ * share one decode. */
 mv_status mv_q8_matvec_t_bf16(const mv_q8_view *m, const uint16_t *dy_dev, int batch,
                               const float *row_scales_dev, float *dx_dev,
                               const mv_q8_tuning *tuning, void *stream);

@@ -295,7 +295,7 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
     return MV_OK;
 }
 
-// Float forward: passes of up to 64 vectors through the warp-specialised kernel, whole stripes per work item.
+// Float forward: passes of up to 64 vectors (8 with engine 1, on the CUDA cores) through the warp-specialised kernel.
 mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float *scales, float *y,
                  const mv_q8_tuning *tuning, cudaStream_t st) {
     mv_status rc;
@@ -309,18 +309,21 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
                         2 * ((size_t)m->tbl_stripe_max + 8) + 1024;
     if (need > (size_t)max_smem_optin())
         return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
-    for (int v0 = 0; v0 < batch; v0 += 64) {
+    const bool dot = t.engine == MV_ENGINE_DP4A;
+    const int pass = dot ? 8 : 64;
+    for (int v0 = 0; v0 < batch; v0 += pass) {
         Q8WLaunch L{};
         L.job0.m = *m;
         L.job0.x = reinterpret_cast<const int8_t *>(x + (size_t)v0 * m->cols);
         L.job0.scales = scales;
         L.job0.ys = y + (size_t)v0 * m->rows;
-        L.batch = std::min(64, batch - v0);
+        L.batch = std::min(pass, batch - v0);
         // whole stripes, or even shares where no stripe is cut twice: a sum of two parts does not depend on their order
         // (whole | even: 11008x4096, one vector 29.5 | 32.0 us, 16 vectors 48.5 | 52.1, 64 vectors 57.6 | 64.9; 6000x6000, 16
         // vectors 49.1 | 45.8, 64 vectors 57.8 | 56.5)
         constexpr int kNever = 1 << 30;
-        const Cost cost{L.batch == 1 ? 15 : 26 + L.batch / 16, L.batch == 1 ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,
+        const bool cuda = dot || L.batch == 1;
+        const Cost cost{cuda ? 11 + 4 * nv_round(L.batch) : 26 + L.batch / 16, cuda ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,
                         t.parts <= 0 && (m->rows + 31) / 32 >= sm_count() ? 20000 : kNever};
         mv_q8_tuning by_rule = t;
         by_rule.parts = 0;
@@ -335,7 +338,7 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
             rc = cut_stripes_launch<float, false>(L, L.job0.ys, nullptr, st);
             if (rc) return rc;
         }
-        rc = q8w_launch_fwd(L, decode_warps(tuning, t), units, st);
+        rc = q8w_launch_fwd(L, dot, decode_warps(tuning, t), units, st);
         if (rc) return rc;
         if (L.span) {
             rc = cut_stripes_launch<float, true>(L, L.job0.ys, L.job0.ys, st);
@@ -345,7 +348,7 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
     return MV_OK;
 }
 
-// Transposed product: passes of 32 vectors, added to dX by atomics, so that stripes may be split.  The tensor cores'
+// Transposed product: passes of 32 vectors (8 with engine 1, on the CUDA cores), added to dX by atomics, so that stripes may be split.  The tensor cores'
 // sums leave by 16-byte reductions: a dX off that grid takes the one-vector form, whose reductions are scalars.
 mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float *scales, float *dx,
                  const mv_q8_tuning *tuning, cudaStream_t st) {
@@ -362,7 +365,8 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
         return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
     rc = zero_launch(dx, (size_t)batch * m->cols, st);
     if (rc) return rc;
-    const int pass = ((uintptr_t)dx & 15) ? 1 : 32;
+    const bool dot = t.engine == MV_ENGINE_DP4A;
+    const int pass = dot ? 8 : ((uintptr_t)dx & 15) ? 1 : 32;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         Q8WLaunch L{};
         L.job0.m = *m;
@@ -370,7 +374,8 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
         L.job0.scales = scales;
         L.job0.ys = dx + (size_t)v0 * m->cols;
         L.batch = std::min(pass, batch - v0);
-        const Cost cost{L.batch == 1 ? 20 : 28 + L.batch / 4, L.batch == 1 ? 90 : 220, 6000, 0, 0, L.batch == 1 ? 10000 : 0};
+        const bool cuda = dot || L.batch == 1;
+        const Cost cost{cuda ? 10 + 10 * nv_round(L.batch) : 28 + L.batch / 4, cuda ? 90 : 220, 6000, 0, 0, L.batch == 1 ? 10000 : 0};
         const int units = plan_single(L, t, cost);
         L.status = status;
         L.spin_limit = wait_spin_limit();
@@ -378,7 +383,7 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
         L.slot_bytes = (uint32_t)(m->max_blk_rows + 1) * 128u;
         L.tbl_stage = (int)((m->tbl_stripe_max + 7) & ~7u);
         L.early = 1;  // (dX has been zeroed)
-        rc = q8w_launch_bwd(L, decode_warps(tuning, t), units, st);
+        rc = q8w_launch_bwd(L, dot, decode_warps(tuning, t), units, st);
         if (rc) return rc;
     }
     return MV_OK;

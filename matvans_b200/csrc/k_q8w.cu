@@ -444,7 +444,7 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
                             const int8_t *x = r.x + (size_t)L.x_quad * q;
                             if (xb)
                                 for (int v = 0; v < L.batch; v++)
-                                    bulk_in(dst + L.x_off + 4u * (uint32_t)(v * m.seg_quads), x + (size_t)v * m.cols, xb, bar);  // (float: one vector)
+                                    bulk_in(dst + L.x_off + L.x_quad * (uint32_t)(v * m.seg_quads), x + (size_t)v * (m.cols >> 2) * L.x_quad, xb, bar);
                         }
                     }
                     __syncwarp();
@@ -691,6 +691,7 @@ template <int NV, bool kRagged = false>
 struct DotCons {
     static constexpr bool kMma = false, kFloat = false, kStatic = false, kPrepare = false;
     static constexpr int kRed = NV * 32;  // ints of an item's partial sums
+    static constexpr int kAreas = kRing;  // of them, in turn
     static constexpr int kLag = NV <= 2 ? 1 : 4;
     static constexpr int kMaxDecode = NV <= 2 ? 16 : NV <= 4 ? 14 : NV <= 8 ? 10 : 6;
     static constexpr uint32_t tile_bytes(int) { return 0; }
@@ -893,6 +894,7 @@ struct MmaCons {
     static constexpr bool kTma = !kOwn && !kRagged;  // x by XTiles
     static constexpr int kPitch = 33;  // words per vector of the item's sums: lanes (vectors) hit distinct banks
     static constexpr int kRed = kOwn ? 16 * kPitch : 0;
+    static constexpr int kAreas = kRing;
     static constexpr int kLag = kOwn ? 4 : 2;  // accumulators
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;  // 32 rows x 64 columns
@@ -1139,7 +1141,7 @@ struct MmaCons {
 // and the warps' sums are added in unit order, so results are reproducible bit for bit.
 struct FwdCons {
     static constexpr bool kMma = true, kFloat = true, kStatic = true, kPrepare = false;
-    static constexpr int kRed = 0;
+    static constexpr int kRed = 0, kAreas = 0;
     static constexpr int kLag = 2;  // accumulators
     static constexpr int kMaxDecode = 16;
     static constexpr uint32_t kWTile = 2048;
@@ -1316,46 +1318,60 @@ struct FwdCons {
     }
 };
 
-// Float forward of one bf16 vector on the CUDA cores: fp32 multiply-adds of the table's bf16 symbols, x behind the
-// block in the slot (or read ahead from global memory when the segment is longer than kXQuads).  Unit u goes to warp
-// u mod W, each warp adds its units of an item in order, and the warps' sums are added in the order of their first
-// units: reproducible bit for bit.  (4096x11008: 40 us through the MMAs of FwdCons, whose tiles cost more than one
-// vector's products.)
+// Float forward on the CUDA cores, one bf16 vector, or (engine 1) up to 8 of them: fp32 multiply-adds of the table's bf16
+// symbols, x behind the block in the slot (or from global memory when the segment is longer than kXQuads).  Unit u goes to
+// warp u mod W, each warp adds its units of an item in order, and the warps' sums are added in the order of their first
+// units: reproducible bit for bit, and for each vector what it is alone.  Measured on a B200, 1, 2, 4 and 8 vectors:
+// 11008x4096 28, 33, 43 and 60 us; 4096x11008 26, 29, 41 and 63 (one vector through the MMAs of FwdCons, whose tiles cost
+// more than its products: 40).
+template <int NV>
 struct FwdDot {
     static constexpr bool kMma = false, kFloat = true, kStatic = true, kPrepare = false;
     static constexpr int kLag = 1;
-    static constexpr int kMaxDecode = 16;
-    static constexpr int kRed = kMaxDecode * 32;
+    static constexpr int kMaxDecode = NV <= 4 ? 16 : 12;  // (registers, and the slots' x)
+    static constexpr int kRed = kMaxDecode * NV * 32;
+    static constexpr int kAreas = 2;  // (with kLag 1 two items are open)
     static constexpr uint32_t tile_bytes(int) { return 0; }
     const uint16_t *x;
-    int seg_quads, qtot, warp;
+    int cols, seg_quads, qtot, warp;
     bool in_slot;
-    float acc;
+    float acc[NV];
     __device__ __forceinline__ void init(const Q8WLaunch &, unsigned char *, const Bars &, uint32_t, int w) {
         warp = w;
-        acc = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; v++) acc[v] = 0.f;
     }
     __device__ __forceinline__ void begin_item(const Q8WLaunch &L, const ItemRec &I, int) {
         in_slot = x_in_slot(L, I.seg_quads);
         x = reinterpret_cast<const uint16_t *>(I.x);
+        cols = I.cols;
         seg_quads = I.seg_quads;
-        qtot = I.cols >> 2;
+        qtot = cols >> 2;
     }
-    // one quad: x as two bf16 pairs
-    __device__ __forceinline__ void quad(Stream &s, const unsigned char *sm, uint32_t lw, uint32_t x01, uint32_t x23) {
+    // one quad of one vector: x as two bf16 pairs
+    static __device__ __forceinline__ void fma4(float &a, const uint32_t (&e)[4], uint32_t x01, uint32_t x23) {
+        a = fmaf(__uint_as_float(e[0] & 0xFFFF0000u), __uint_as_float(x01 << 16), a);
+        a = fmaf(__uint_as_float(e[1] & 0xFFFF0000u), __uint_as_float(x01 & 0xFFFF0000u), a);
+        a = fmaf(__uint_as_float(e[2] & 0xFFFF0000u), __uint_as_float(x23 << 16), a);
+        a = fmaf(__uint_as_float(e[3] & 0xFFFF0000u), __uint_as_float(x23 & 0xFFFF0000u), a);
+    }
+    // two quads of every vector
+    __device__ __forceinline__ void pair(Stream &s, const unsigned char *sm, uint32_t lw, const uint4 (&xv)[NV]) {
         uint32_t e[4];
         s.step_f(sm, lw, e);
-        acc = fmaf(__uint_as_float(e[0] & 0xFFFF0000u), __uint_as_float(x01 << 16), acc);
-        acc = fmaf(__uint_as_float(e[1] & 0xFFFF0000u), __uint_as_float(x01 & 0xFFFF0000u), acc);
-        acc = fmaf(__uint_as_float(e[2] & 0xFFFF0000u), __uint_as_float(x23 << 16), acc);
-        acc = fmaf(__uint_as_float(e[3] & 0xFFFF0000u), __uint_as_float(x23 & 0xFFFF0000u), acc);
+#pragma unroll
+        for (int v = 0; v < NV; v++) fma4(acc[v], e, xv[v].x, xv[v].y);
+        s.step_f(sm, lw, e);
+#pragma unroll
+        for (int v = 0; v < NV; v++) fma4(acc[v], e, xv[v].z, xv[v].w);
     }
-    __device__ __forceinline__ void group(Stream &s, const unsigned char *sm, uint32_t lw, const uint4 &a, const uint4 &b) {
-        quad(s, sm, lw, a.x, a.y);
-        quad(s, sm, lw, a.z, a.w);
-        quad(s, sm, lw, b.x, b.y);
-        quad(s, sm, lw, b.z, b.w);
-        s.clamp();
+    // eight columns of every vector at p (past the batch: its last vector again)
+    __device__ __forceinline__ void load_x(const uint16_t *p, int batch, uint4 (&xv)[NV]) const {
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            xv[v] = ldx_u4(p);
+            if (NV <= 2 || v + 1 < batch) p += cols;
+        }
     }
     __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
                                          uint32_t lw, int lane, volatile uint32_t *) {
@@ -1364,18 +1380,30 @@ struct FwdDot {
         Stream s(sm, soff, d.rows, lane);
         if (in_slot) {
             const unsigned char *xs = sm + soff + L.x_off;
-#pragma unroll 2
-            for (int i = 0; i < nq; i += 4, xs += 32)
-                group(s, sm, lw, *reinterpret_cast<const uint4 *>(xs), *reinterpret_cast<const uint4 *>(xs + 16));
+            constexpr int kUnroll = NV == 1 ? 2 : 1;
+#pragma unroll kUnroll
+            for (int i = 0; i < nq; i += 4, xs += 32) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    uint4 xv[NV];
+#pragma unroll
+                    for (int v = 0; v < NV; v++) xv[v] = *reinterpret_cast<const uint4 *>(xs + 8 * v * seg_quads + 16 * h);
+                    pair(s, sm, lw, xv);
+                }
+                s.clamp();
+            }
         } else {
-            const uint4 *xp = reinterpret_cast<const uint4 *>(x + 4 * q0);
-            uint4 a = ldp(xp), b = ldp(xp + 1);
-            for (int i = 0; i < nq; i += 4) {
-                xp += i + 4 < nq ? 2 : 0;
-                const uint4 a1 = ldp(xp), b1 = ldp(xp + 1);
-                group(s, sm, lw, a, b);
-                a = a1;
-                b = b1;
+            const uint16_t *xp = x + 4 * q0;
+            uint4 xn[NV];
+            load_x(xp, L.batch, xn);
+            for (int i = 0; i < nq; i += 2) {
+                uint4 xv[NV];
+#pragma unroll
+                for (int v = 0; v < NV; v++) xv[v] = xn[v];
+                xp += i + 2 < nq ? 8 : 0;
+                load_x(xp, L.batch, xn);
+                pair(s, sm, lw, xv);
+                if (i & 2) s.clamp();
             }
         }
         if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
@@ -1383,25 +1411,33 @@ struct FwdDot {
     __device__ __forceinline__ void end_unit(const Q8WLaunch &L, int k, bool last, unsigned char *sm, const Bars &B,
                                              int lane, volatile uint32_t *) {
         if (last) {
-            reinterpret_cast<float *>(sm + L.lay.red)[(k % kRing) * kRed + warp * 32 + lane] = acc;
-            acc = 0.f;
+            float *red = reinterpret_cast<float *>(sm + L.lay.red) + (k % kAreas) * kRed + warp * NV * 32 + lane;
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                red[v * 32] = acc[v];
+                acc[v] = 0.f;
+            }
         }
         __syncwarp();
         if (lane == 0) arrive(B.tdone(k % kRing));
     }
     __device__ __forceinline__ void drain(const Q8WLaunch &) {}
+    // Table warps: one vector per warp at a time, lane = stripe row.
     static __device__ __forceinline__ void epilogue(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm,
                                                     const Bars &, uint32_t) {
         const int lane = threadIdx.x & 31, row = I.stripe * 32 + lane;
-        if (threadIdx.x >= 32) return;
-        const volatile float *red = reinterpret_cast<const volatile float *>(sm + L.lay.red) + (k % kRing) * kRed + lane;
-        const uint32_t W = (uint32_t)L.W, nc = min(I.n, W);
-        uint32_t w = I.u0 % W;
-        float sum = 0.f;
-        for (uint32_t i = 0; i < nc; i++, w = w + 1 < W ? w + 1 : 0) sum += red[w * 32];
-        if (row >= I.rows) return;
-        if (I.atomic) atomicAdd(I.ys + row, sum);  // even shares: scaled together with the other CTA's part afterwards
-        else I.ys[row] = sum * ldp(I.scales + row);
+        const float scale = row_scale(I, row);
+        const uint32_t W = (uint32_t)L.W, nc = min(I.n, W), first = I.u0 % W;
+        for (int v = threadIdx.x >> 5; v < min(NV, L.batch); v += kTableWarps) {
+            const volatile float *red = reinterpret_cast<const volatile float *>(sm + L.lay.red) + (k % kAreas) * kRed + v * 32 + lane;
+            uint32_t w = first;
+            float sum = 0.f;
+            for (uint32_t i = 0; i < nc; i++, w = w + 1 < W ? w + 1 : 0) sum += red[w * NV * 32];
+            if (row >= I.rows) continue;
+            float *dst = I.ys + (size_t)v * I.rows + row;
+            if (I.atomic) atomicAdd(dst, sum);  // even shares: scaled together with the other CTA's part afterwards
+            else *dst = sum * scale;
+        }
     }
 };
 
@@ -1419,7 +1455,7 @@ struct FwdDot {
 // 16 vectors 90 -> 64 us, 2 vectors 76 -> 57 us; 4096x11008, 64 vectors 259 -> 151 us, 16 vectors 106 -> 63 us.
 struct BwdCons {
     static constexpr bool kMma = true, kFloat = true, kStatic = false, kPrepare = true;
-    static constexpr int kRed = 0;
+    static constexpr int kRed = 0, kAreas = 0;
     static constexpr int kLag = 1;  // two buffers of G, written with the item's table
     static constexpr int kMaxDecode = 12;
     static constexpr uint32_t kWTile = 2048, kTr = 4096;
@@ -1598,22 +1634,25 @@ struct BwdCons {
                                                     uint32_t) {}
 };
 
-// Float backward of one vector on the CUDA cores: fp32 products of the table's bf16 symbols with the row's g = s . dy
-// (the tensor cores' sums of 32 rows are less exact than fp32 additions).  The products of 4 quads (16 columns) of the
-// 32 rows change hands in shared memory: a lane stores its row's four 16-byte pieces and reads one piece of four rows,
-// which leaves eight partial sums a column for three shuffle steps.  (All sixteen columns by shuffles alone: 30 selects
-// and 16 shuffles a group against 6 and 4.)  Bound by issue.  Measured on a B200: 4096x11008 52 -> 37 us, 11008x4096
-// 47 -> 41 us (with BwdCons, 55 and 57 us and 2e-6 of error where this form has 2e-7).
+// Float backward on the CUDA cores, one vector, or (engine 1) up to 8 of them: fp32 products of the table's bf16 symbols
+// with the row's g = s . dy (the tensor cores' sums of 32 rows are less exact than fp32 additions).  The products of 4 quads
+// (16 columns) of the 32 rows change hands in shared memory, a vector at a time: a lane stores its row's four 16-byte pieces
+// and reads one piece of four rows, which leaves eight partial sums a column for three shuffle steps.  (All sixteen columns
+// by shuffles alone: 30 selects and 16 shuffles a group against 6 and 4.)  Bound by issue.  Measured on a B200, one vector:
+// 4096x11008 52 -> 37 us, 11008x4096 47 -> 41 us (with BwdCons, 55 and 57 us and 2e-6 of error where this form has 2e-7); 8 vectors
+// 141 and 150 us.
+template <int NV>
 struct BwdDot {
     static constexpr bool kMma = false, kFloat = true, kStatic = false, kPrepare = true;
     static constexpr int kLag = 1;
     static constexpr int kMaxDecode = 16;
-    static constexpr int kRed = 32;  // g of the item's rows
+    static constexpr int kRed = NV * 32;  // g of the item's rows
+    static constexpr int kAreas = kRing;
     static constexpr uint32_t tile_bytes(int) { return 2048; }
     const float *gs;
     float *dx;
-    float g;
-    int seg_quads, qtot;
+    float g[NV];
+    int cols, seg_quads, qtot;
     uint32_t st, ld;  // this lane's row, and its piece of rows lane / 4, + 8, + 16, + 24
     __device__ __forceinline__ void init(const Q8WLaunch &L, unsigned char *sm, const Bars &, uint32_t, int w) {
         const uint32_t lane = threadIdx.x & 31u, t = smem_u32(sm) + L.lay.tiles + (uint32_t)w * tile_bytes(0);
@@ -1624,56 +1663,82 @@ struct BwdDot {
     }
     __device__ __forceinline__ void begin_item(const Q8WLaunch &, const ItemRec &I, int k) {
         dx = I.ys;
+        cols = I.cols;
         seg_quads = I.seg_quads;
         qtot = I.cols >> 2;
-        g = *reinterpret_cast<const volatile float *>(gs + (k % kRing) * kRed);
+#pragma unroll
+        for (int v = 0; v < NV; v++) g[v] = *reinterpret_cast<const volatile float *>(gs + (k % kAreas) * kRed + v * 32);
     }
     static __device__ __forceinline__ void prepare(const Q8WLaunch &L, const ItemRec &I, int k, unsigned char *sm, uint32_t) {
-        if (threadIdx.x >= 32) return;
-        const int row = I.stripe * 32 + (int)threadIdx.x;
-        float v = 0.f;
-        if (row < I.rows)
-            v = ldp(I.scales + row) * __uint_as_float((uint32_t)ldp(reinterpret_cast<const uint16_t *>(I.x) + row) << 16);
-        reinterpret_cast<float *>(sm + L.lay.red)[(k % kRing) * kRed + threadIdx.x] = v;
+        const int lane = threadIdx.x & 31, row = I.stripe * 32 + lane;
+        const float scale = row_scale(I, row);
+        for (int v = threadIdx.x >> 5; v < NV; v += kTableWarps) {
+            float gv = 0.f;
+            if (row < I.rows && v < L.batch)
+                gv = scale * __uint_as_float((uint32_t)ldp(reinterpret_cast<const uint16_t *>(I.x) + (size_t)v * I.rows + row) << 16);
+            reinterpret_cast<float *>(sm + L.lay.red)[(k % kAreas) * kRed + v * 32 + lane] = gv;
+        }
+    }
+    // the lane's products of quad j with its row's g
+    __device__ __forceinline__ void store4(uint32_t j, const uint32_t (&e)[4], float gv) const {
+        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(st ^ (16u * j)), "f"(__uint_as_float(e[0] & 0xFFFF0000u) * gv),
+                     "f"(__uint_as_float(e[1] & 0xFFFF0000u) * gv), "f"(__uint_as_float(e[2] & 0xFFFF0000u) * gv),
+                     "f"(__uint_as_float(e[3] & 0xFFFF0000u) * gv)
+                     : "memory");
+    }
+    // the 32 rows' products of 16 columns, summed and added to dst (which is this lane's column)
+    __device__ __forceinline__ void reduce(float *dst, int lane) const {
+        const bool b4 = lane & 16, b3 = lane & 8;
+        __syncwarp();
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (uint32_t r = 0; r < 4; r++) {
+            float v[4];
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                         : "r"(ld + 512u * r)
+                         : "memory");
+#pragma unroll
+            for (int c = 0; c < 4; c++) a[c] += v[c];
+        }
+        __syncwarp();
+        float k0 = b4 ? a[2] : a[0], k1 = b4 ? a[3] : a[1];
+        k0 += __shfl_xor_sync(0xffffffffu, b4 ? a[0] : a[2], 16);
+        k1 += __shfl_xor_sync(0xffffffffu, b4 ? a[1] : a[3], 16);
+        float c = b3 ? k1 : k0;
+        c += __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+        c += __shfl_xor_sync(0xffffffffu, c, 4);
+        if (!(lane & 4)) atomicAdd(dst, c);
     }
     __device__ __forceinline__ void unit(const Q8WLaunch &L, const UnitDesc &d, const unsigned char *sm, uint32_t soff,
                                          uint32_t lw, int lane, volatile uint32_t *) {
         const int q0 = d.seg * seg_quads;
         const int nq = min(seg_quads, qtot - q0);
         Stream s(sm, soff, d.rows, lane);
-        const bool b4 = lane & 16, b3 = lane & 8;
-        float *dst = dx + 4 * q0 + 4 * (lane & 3) + (b4 ? 2 : 0) + (b3 ? 1 : 0);
+        float *dst = dx + 4 * q0 + 4 * (lane & 3) + (lane & 16 ? 2 : 0) + (lane & 8 ? 1 : 0);
         for (int i = 0; i < nq; i += 4, dst += 16) {  // segments are whole groups of 4 quads (cols % 16 == 0)
+            if constexpr (NV == 1) {
 #pragma unroll
-            for (uint32_t j = 0; j < 4; j++) {
-                uint32_t e[4];
-                s.step_f(sm, lw, e);
-                asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(st ^ (16u * j)),
-                             "f"(__uint_as_float(e[0] & 0xFFFF0000u) * g), "f"(__uint_as_float(e[1] & 0xFFFF0000u) * g),
-                             "f"(__uint_as_float(e[2] & 0xFFFF0000u) * g), "f"(__uint_as_float(e[3] & 0xFFFF0000u) * g)
-                             : "memory");
+                for (uint32_t j = 0; j < 4; j++) {
+                    uint32_t e[4];
+                    s.step_f(sm, lw, e);
+                    store4(j, e, g[0]);
+                }
+                s.clamp();
+                reduce(dst, lane);
+            } else {
+                uint32_t e[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) s.step_f(sm, lw, e[j]);
+                s.clamp();
+#pragma unroll
+                for (int v = 0; v < NV; v++)
+                    if (v < L.batch) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++) store4(j, e[j], g[v]);
+                        reduce(dst + (size_t)v * cols, lane);
+                    }
             }
-            s.clamp();
-            __syncwarp();
-            float a[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (uint32_t r = 0; r < 4; r++) {
-                float v[4];
-                asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
-                             : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                             : "r"(ld + 512u * r)
-                             : "memory");
-#pragma unroll
-                for (int c = 0; c < 4; c++) a[c] += v[c];
-            }
-            __syncwarp();
-            float k0 = b4 ? a[2] : a[0], k1 = b4 ? a[3] : a[1];
-            k0 += __shfl_xor_sync(0xffffffffu, b4 ? a[0] : a[2], 16);
-            k1 += __shfl_xor_sync(0xffffffffu, b4 ? a[1] : a[3], 16);
-            float c = b3 ? k1 : k0;
-            c += __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
-            c += __shfl_xor_sync(0xffffffffu, c, 4);
-            if (!(lane & 4)) atomicAdd(dst, c);
         }
         if (!s.ok()) atomicOr(L.status, MV_DEV_FINAL_STATE);
     }
@@ -1825,7 +1890,7 @@ __global__ void __launch_bounds__(32 * (kFirstDecode + Cons::kMaxDecode), 1) q8w
         UnitDesc *desc = reinterpret_cast<UnitDesc *>(smem + L.lay.desc);
         for (int i = threadIdx.x; i < L.S; i += blockDim.x) desc[i].unit = 0xFFFFFFFFu;
         uint32_t *red = reinterpret_cast<uint32_t *>(smem + L.lay.red);
-        for (int i = threadIdx.x; i < kRing * Cons::kRed; i += blockDim.x) red[i] = 0;
+        for (int i = threadIdx.x; i < Cons::kAreas * Cons::kRed; i += blockDim.x) red[i] = 0;
     }
     fence_mbar_init();
     uint32_t tmem = 0;
@@ -1867,7 +1932,7 @@ Q8WLayout layout(const Q8WLaunch &L, int W, int S) {
     o.slots = p = up(p);
     p += (uint32_t)S * L.slot_bytes;
     o.red = p;
-    p += (uint32_t)(kRing * Cons::kRed) * 4u;
+    p += (uint32_t)(Cons::kAreas * Cons::kRed) * 4u;
     o.bars = p;
     p += 8u * (uint32_t)Bars::count(S, W, Cons::kMma);
     p = (p + 15u) & ~15u;
@@ -2007,16 +2072,24 @@ bool q8w_ragged_fits(const Q8WLaunch &L0, bool mma) {
     return need <= (uint32_t)max_smem_optin();
 }
 
-mv_status q8w_launch_fwd(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
+mv_status q8w_launch_fwd(const Q8WLaunch &L0, bool dot, int warps, int units, cudaStream_t st) {
     Q8WLaunch L = L0;
+    if (L.batch == 1) return launch_t<FwdDot<1>>(L, warps, units, st);
+    if (dot)
+        return L.batch == 2  ? launch_t<FwdDot<2>>(L, warps, units, st)
+               : L.batch <= 4 ? launch_t<FwdDot<4>>(L, warps, units, st)
+                              : launch_t<FwdDot<8>>(L, warps, units, st);
     L.xrows = (L.batch + 7) & ~7;
-    if (L.batch == 1) return launch_t<FwdDot>(L, warps, units, st);
     mv_status rc = x_map(L, true);
     return rc ? rc : launch_t<FwdCons>(L, warps, units, st);
 }
 
-mv_status q8w_launch_bwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st) {
-    if (L.batch == 1) return launch_t<BwdDot>(L, warps, units, st);
+mv_status q8w_launch_bwd(const Q8WLaunch &L, bool dot, int warps, int units, cudaStream_t st) {
+    if (L.batch == 1) return launch_t<BwdDot<1>>(L, warps, units, st);
+    if (dot)
+        return L.batch == 2  ? launch_t<BwdDot<2>>(L, warps, units, st)
+               : L.batch <= 4 ? launch_t<BwdDot<4>>(L, warps, units, st)
+                              : launch_t<BwdDot<8>>(L, warps, units, st);
     return launch_t<BwdCons>(L, warps, units, st);
 }
 

@@ -51,9 +51,11 @@ struct Q8WLaunch {
 mv_status q8w_launch_int(const Q8WLaunch &L, int nv, bool mma, int warps, int units, cudaStream_t st);
 // Whether a ragged one (dp4a: of up to 8 vectors) finds room in shared memory at all.
 bool q8w_ragged_fits(const Q8WLaunch &L, bool mma);
-// Float forward of up to 64 vectors (on the tensor cores from 2): job0.x is bf16 [batch][cols], job0.ys fp32 [batch][rows].
-mv_status q8w_launch_fwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st);
-// Float backward of up to 32 vectors: job0.x is dY, bf16 [batch][rows], added to job0.ys, fp32 [batch][cols].
-mv_status q8w_launch_bwd(const Q8WLaunch &L, int warps, int units, cudaStream_t st);
+// Float forward: job0.x is bf16 [batch][cols], job0.ys fp32 [batch][rows].  On the tensor cores up to 64 vectors, on the CUDA
+// cores (dot; one vector always) up to 8.
+mv_status q8w_launch_fwd(const Q8WLaunch &L, bool dot, int warps, int units, cudaStream_t st);
+// Float backward: job0.x is dY, bf16 [batch][rows], added to job0.ys, fp32 [batch][cols].  On the tensor cores up to 32
+// vectors, on the CUDA cores (as above) up to 8.
+mv_status q8w_launch_bwd(const Q8WLaunch &L, bool dot, int warps, int units, cudaStream_t st);
 
 }  // namespace mv
