@@ -237,9 +237,9 @@ __global__ void __launch_bounds__(512) q8_kernel(const Q8Launch L) {
 
 __global__ void scale_rows_kernel(const int32_t *y, const float *s, float *ys, int rows, int batch,
                                   int ldy) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < rows * batch) {
-        const int r = i % rows, v = i / rows;
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i < (size_t)rows * batch) {
+        const int r = (int)(i % rows), v = (int)(i / rows);
         ys[(size_t)v * ldy + r] = (float)y[(size_t)v * ldy + r] * s[r];
     }
 }
@@ -345,8 +345,8 @@ mv_status q8_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y,
         else rc = launch_q8<16, false>(L, W, ngroups, st);
         if (rc) return rc;
         if (ys && atomic) {
-            const int n = nb * m->rows;
-            scale_rows_kernel<<<(n + 255) / 256, 256, 0, st>>>(L.y, scales, ys + (size_t)v0 * m->rows,
+            const size_t n = (size_t)nb * m->rows;
+            scale_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(L.y, scales, ys + (size_t)v0 * m->rows,
                                                                m->rows, nb, m->rows);
             MV_CUDA_TRY(cudaGetLastError(), "scale_rows_kernel launch");
         }

@@ -286,8 +286,8 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
             if (rc) return rc;
         }
         if (ys && L.job0.atomic) {
-            const int n = nb * m->rows;
-            scale_rows_kernel<<<(n + 255) / 256, 256, 0, st>>>(L.job0.y, scales, ys + (size_t)v0 * m->rows, m->rows,
+            const size_t n = (size_t)nb * m->rows;
+            scale_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(L.job0.y, scales, ys + (size_t)v0 * m->rows, m->rows,
                                                                nb, m->rows);
             MV_CUDA_TRY(cudaGetLastError(), "scale_rows_kernel launch");
         }

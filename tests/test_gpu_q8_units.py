@@ -205,3 +205,25 @@ def test_float_backward_reads_dy_alone(rows, cols, seg_quads):
             assert err.max().item() < bound, (B, dy_off, dx_off)
             assert (dxb[:dx_off] == -7).all() and (dxb[dx_off + B * cols:] == -7).all(), (B, dy_off, dx_off)
     assert ops.device_status() == 0
+
+
+def test_scaled_outputs_of_more_than_two_billion_elements():
+    # 64 vectors of 2^25 + 32 rows in two parts a stripe: sums joined by atomics, then scaled, element numbers past 31 bits.
+    # The matrix is one stripe's block over and over
+    stripes, B = 2 ** 20 + 1, 64
+    E = ops.Q8Matrix.encode(np.ones((32, 32), np.int8), local=False, seg_quads=4)
+    off = E.blk_off.view(torch.int32)
+    per = int(off[2])
+    assert E.nseg == 2
+    E.blocks = E.blocks.view(torch.int32)[:32 * per].repeat(stripes)
+    E.blk_off = torch.cat([(torch.arange(stripes, dtype=torch.int32, device="cuda")[:, None] * per + off[None, :2]).reshape(-1),
+                           torch.tensor([stripes * per], dtype=torch.int32, device="cuda")])
+    E.rows = 32 * stripes
+    E._view = E.view()
+    x = torch.randint(-128, 128, (B, 32), dtype=torch.int8, device="cuda")
+    s = torch.rand(E.rows, device="cuda")
+    y, ys = E.matvec(x, scales=s, tuning=(8, 1, 1, 0, 2, 0))
+    sums = x.sum(1, dtype=torch.int32)
+    for b in range(B):
+        assert bool((y[b] == sums[b]).all()) and torch.equal(ys[b], sums[b].float() * s), b
+    assert ops.device_status() == 0
