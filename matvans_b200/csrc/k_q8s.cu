@@ -113,18 +113,20 @@ bool q8s_supports(const mv_q8_view *m, const int8_t *x) {
     return (m->cols & 15) == 0 && ((uintptr_t)x & 15) == 0 && (m->seg_quads & 3) == 0;
 }
 
-// The launch shape a caller asks for (or the default one) has to fit shared memory with a decode table of 64 KB and
-// `warps` x ilp x depth stream slots, whatever shape the kernel then runs in.
-mv_status check_shape(const mv_q8_tuning &t, bool mma, int nv, int max_blk_rows, uint32_t tbl_stripe_max) {
-    const int ilp = mma ? 1 : t.ilp;
-    const size_t slots = (size_t)t.warps * ilp * t.depth;
-    const size_t need = 65536 + slots * (size_t)(max_blk_rows + 1) * 128 + 2 * ((size_t)tbl_stripe_max + 8) +
-                        (mma ? (size_t)std::max(0, t.warps - 8) * 4096 + (size_t)t.warps * 24 + 128
-                             : (size_t)2 * t.warps * nv * 128) + 1024;
+// The launch shape a caller asks for (or the default one) has to fit shared memory: a decode table, `warps` x ilp x depth
+// stream buffers and the tiles or sums of `warps`, whatever shape the kernel then runs in.  (Callers that try shapes count on
+// the refusal; where a shape passes, the kernel finds one of its own.)
+mv_status check_shape(const mv_q8_tuning &t, int ilp, int max_blk_rows, size_t table, size_t warp_bytes) {
+    const size_t need = table + (size_t)t.warps * ilp * t.depth * (size_t)(max_blk_rows + 1) * 128 + warp_bytes;
     if (need > (size_t)max_smem_optin())
         return fail(MV_ERR_UNSUPPORTED, "Q8 launch: %d warps x %d segments x %d buffers need %zu B of shared memory (max %d)",
                     t.warps, ilp, t.depth, need, max_smem_optin());
     return MV_OK;
+}
+mv_status check_shape_int(const mv_q8_tuning &t, int nv, int max_blk_rows, uint32_t tbl_stripe_max) {
+    const bool mma = t.engine == MV_ENGINE_AUTO && nv >= kMmaShape;
+    return check_shape(t, mma ? 1 : t.ilp, max_blk_rows, 65536 + 2 * (size_t)tbl_stripe_max,
+                       mma ? (size_t)std::max(0, t.warps - 8) * 4096 : (size_t)2 * t.warps * nv * 128);
 }
 
 // How one matrix is spread over the CTAs: whole stripes (parts = 1), every stripe in `parts` ranges of its segments, or
@@ -243,7 +245,7 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
     for (int v0 = 0; v0 < batch; v0 += pass) {
         const int nb = std::min(pass, batch - v0);
         bool mma = t.engine == MV_ENGINE_AUTO && nb >= kMmaMinVectors;
-        if (!ragged) rc = check_shape(t, t.engine == MV_ENGINE_AUTO && nb >= kMmaShape, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
+        if (!ragged) rc = check_shape_int(t, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
         if (rc) return rc;
         Q8WLaunch L{};
         L.ragged = ragged;
@@ -305,11 +307,9 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
     const bool asked = tuning && tuning->warps > 0;
     if (asked && t.warps > 8 && t.engine == MV_ENGINE_AUTO && batch >= 2)
         return fail(MV_ERR_ARG, "Q8 launch: %d warps per CTA; the float form on the tensor cores takes at most 8", t.warps);
-    const size_t need = 32768 + (size_t)t.warps * t.depth * ((size_t)(m->max_blk_rows + 1) * 128 + 2056) +
-                        2 * ((size_t)m->tbl_stripe_max + 8) + 1024;
-    if (need > (size_t)max_smem_optin())
-        return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
     const bool dot = t.engine == MV_ENGINE_DP4A;
+    rc = check_shape(t, 1, m->max_blk_rows, 32768, dot || batch == 1 ? 0 : (size_t)t.warps * 2048);
+    if (rc) return rc;
     const int pass = dot ? 8 : 64;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         Q8WLaunch L{};
@@ -359,10 +359,8 @@ mv_status q8_bwd(const mv_q8_view *m, const uint16_t *dy, int batch, const float
     if (!tuning || (tuning->ilp != 1 && tuning->ilp != 2)) t.ilp = 1;  // the float form's default
     const bool mma = t.engine == MV_ENGINE_AUTO && batch >= 2;
     if (t.warps > 8) return fail(MV_ERR_ARG, "Q8 launch: %d warps per CTA; the float backward takes at most 8", t.warps);
-    const size_t need = 32768 + (size_t)t.warps * (mma ? 1 : t.ilp) * t.depth * (size_t)(m->max_blk_rows + 1) * 128 +
-                        (mma ? 4224 + (size_t)t.warps * 2056 : 0) + 2 * ((size_t)m->tbl_stripe_max + 8) + 1024;
-    if (need > (size_t)max_smem_optin())
-        return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", need, max_smem_optin());
+    rc = check_shape(t, mma ? 1 : t.ilp, m->max_blk_rows, 32768, mma ? 4096 + (size_t)t.warps * 2048 : 0);
+    if (rc) return rc;
     rc = zero_launch(dx, (size_t)batch * m->cols, st);
     if (rc) return rc;
     const bool dot = t.engine == MV_ENGINE_DP4A;
@@ -506,7 +504,7 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
     L.chain_out8 = out8_dev;
     const int nv = mv::nv_round(batch);
     const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
-    rc = mv::check_shape(t, t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaShape, nv, info->max_blk_rows, info->tbl_stripe_max);
+    rc = mv::check_shape_int(t, nv, info->max_blk_rows, info->tbl_stripe_max);
     if (rc) return rc;
     mv::q8s_chain_reset<<<(njobs + 255) / 256, 256, 0, st>>>(reinterpret_cast<mv::Q8Job *>(jobs_dev), njobs);
     MV_CUDA_TRY(cudaGetLastError(), "q8s_chain_reset launch");
@@ -537,7 +535,7 @@ mv_status mv_q8_stack_matvec(const mv_q8_job *jobs_dev, int njobs, const mv_q8_s
     if (info->nitems < 0x7FFFFFFFu) L.queue = const_cast<uint32_t *>(&jobs_dev[0].pad);
     const int nv = mv::nv_round(batch);
     const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
-    rc = mv::check_shape(t, t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaShape, nv, info->max_blk_rows, info->tbl_stripe_max);
+    rc = mv::check_shape_int(t, nv, info->max_blk_rows, info->tbl_stripe_max);
     if (rc) return rc;
     dim3 zg(64, std::min(njobs, 1024));
     L.early = info->atomic_jobs > 0;

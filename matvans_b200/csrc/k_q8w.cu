@@ -223,6 +223,36 @@ __device__ __forceinline__ void locate(const Q8WLaunch &L, uint32_t it, int &job
     item_segs(job_at(L, job).m, ng, (int)(rel % (uint32_t)ng), sb, se);
 }
 
+// Item `next` (even shares: the units from `next` to the stripe's end or `limit`): what its record says of the matrix, the
+// stripe and the buffers.
+__device__ __forceinline__ void fill_item(const Q8WLaunch &L, uint32_t next, uint32_t limit, int &job, ItemRec &r) {
+    int se = 0;
+    if (L.span) {
+        const uint32_t nseg = (uint32_t)L.job0.m.nseg;
+        r.stripe = (int)(next / nseg);
+        r.sb = (int)(next - (uint32_t)r.stripe * nseg);
+        se = (int)min(nseg, (uint32_t)r.sb + (limit - next));
+    } else {
+        locate(L, next, job, r.stripe, r.sb, se);
+    }
+    r.job = job;
+    r.n = (uint32_t)max(0, se - r.sb);
+    const Q8Job &J = job_at(L, job);
+    r.rows = J.m.rows;
+    r.cols = J.m.cols;
+    r.seg_quads = J.m.seg_quads;
+    r.local = J.m.local;
+    r.atomic = L.span ? (int)r.n < J.m.nseg : J.atomic;
+    r.x = J.x;
+    r.y = J.y;
+    r.scales = J.scales;
+    r.ys = J.ys;
+    if (L.chain_scales) {
+        r.chain_scale = ldp(L.chain_scales + job);
+        r.chain_out = job + 1 < L.njobs ? const_cast<int8_t *>(L.jobs[job + 1].x) : L.chain_out8;
+    }
+}
+
 // The chained pipeline's int8 output: the reference's fp32 requantisation (ans-warp-rows-kernel.cu:212-220).
 __device__ __forceinline__ int8_t chain_q(const ItemRec &I, int sum) {
     return (int8_t)max(-128, min(127, __float2int_rn((float)sum * I.chain_scale)));
@@ -334,32 +364,8 @@ __device__ __forceinline__ void produce(const Q8WLaunch &L, unsigned char *sm, c
         r.u0 = recorded;
         r.area_item = -1;
         if (!end) {
-            int se = 0;
-            if (L.span) {
-                const uint32_t nseg = (uint32_t)L.job0.m.nseg;
-                r.stripe = (int)(next / nseg);
-                r.sb = (int)(next - (uint32_t)r.stripe * nseg);
-                se = (int)min(nseg, (uint32_t)r.sb + (limit - next));
-            } else {
-                locate(L, next, job, r.stripe, r.sb, se);
-            }
+            fill_item(L, next, limit, job, r);
             if (L.queue && k > 0 && lane == 0) grabbed = atomicAdd(L.queue, 1u);
-            r.job = job;
-            r.n = (uint32_t)max(0, se - r.sb);
-            const Q8Job &J = job_at(L, job);
-            r.rows = J.m.rows;
-            r.cols = J.m.cols;
-            r.seg_quads = J.m.seg_quads;
-            r.local = J.m.local;
-            r.atomic = L.span ? (int)r.n < J.m.nseg : J.atomic;
-            r.x = J.x;
-            r.y = J.y;
-            r.scales = J.scales;
-            r.ys = J.ys;
-            if (L.chain_scales) {
-                r.chain_scale = ldp(L.chain_scales + job);
-                r.chain_out = job + 1 < L.njobs ? const_cast<int8_t *>(L.jobs[job + 1].x) : L.chain_out8;
-            }
             r.build = job != tjob || (r.local && r.stripe != tstripe);
             if (r.build) {
                 // two tables and two staging areas: build g overwrites those of build g - 2
@@ -1953,6 +1959,207 @@ Q8WLayout layout(const Q8WLaunch &L, int W, int S) {
     return o;
 }
 
+// The 32 rows' products of 16 columns (w: the lane's row of them, g its s . dy) summed over the lanes and added to dst: over
+// lane bits 16, 8, 4 and 2 each half keeps half of the columns, then lanes 2 c and 2 c + 1 hold column c.
+__device__ __forceinline__ void wide_reduce(const float (&w)[16], float g, float *dst, int lane) {
+    float a[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) a[j] = w[j] * g;
+#pragma unroll
+    for (int n = 8; n > 0; n >>= 1) {
+        const bool up = lane & (2 * n);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (j < n) {
+                const float give = up ? a[j] : a[j + n], keep = up ? a[j + n] : a[j];
+                a[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * n);
+            }
+    }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    if (!(lane & 1)) atomicAdd(dst + (lane >> 1), a[0]);
+}
+
+// The same products where one block leaves no room for q8w_kernel's two decode tables and staging areas (segments of some
+// 900 quads and more at 8 bits a weight): a CTA is one warp with one table of 32 KB and one block at a time, no copy under
+// way while it decodes.  A block of up to 195 KB fits, more than any launch shape asks for.  kMode 0: integer product, 1:
+// float forward, 2: float backward; NV vectors a decode.  Items are q8w_kernel's, each CTA taking every G-th one (even
+// shares: its share); of a chain, those of job `only`.  Bound by the lone warp's chain of steps, its x a group of 4 quads
+// ahead.
+template <int kMode, int NV>
+__global__ void __launch_bounds__(32) q8_wide_kernel(const __grid_constant__ Q8WLaunch L, int only) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint64_t bar;
+    const int lane = threadIdx.x;
+    uint32_t *lut = reinterpret_cast<uint32_t *>(smem) + lane;
+    const uint32_t *buf = reinterpret_cast<const uint32_t *>(smem + 32768);
+    if (lane == 0) mbar_init(&bar, 1);
+    fence_mbar_init();
+    __syncwarp();
+    uint32_t phase = 0;
+    int job = only >= 0 ? only : 0, tjob = -1, tstripe = -1;
+    uint32_t next = only >= 0 ? L.jobs[job].item0 + blockIdx.x : blockIdx.x, limit = L.nitems;
+    if (only >= 0 && job + 1 < L.njobs) limit = L.jobs[job + 1].item0;
+    if (L.span) {
+        next = (uint32_t)((uint64_t)blockIdx.x * L.span / gridDim.x);
+        limit = (uint32_t)((uint64_t)(blockIdx.x + 1) * L.span / gridDim.x);
+    }
+    ItemRec r{};
+    for (; next < limit; next += L.span ? r.n : gridDim.x) {
+        r = ItemRec{};
+        fill_item(L, next, limit, job, r);
+        const mv_q8_view &m = job_at(L, job).m;
+        if (job != tjob || (r.local && r.stripe != tstripe)) {  // the lane's column of the decode table
+            tjob = job;
+            tstripe = r.stripe;
+            const uint32_t t = r.local ? (uint32_t)r.stripe * 32u + (uint32_t)lane : 0u;
+            const uint32_t o0 = ldp(m.tbl_off + t), o1 = min(ldp(m.tbl_off + t + 1), m.tbl_len);
+            uint32_t q = 0;
+            for (uint32_t k = o0; k < o1 && q < 256u; k++) {
+                const uint32_t ent = ldp(m.tbl + k), f = ent >> 8;
+                for (uint32_t i = 0; i < f && q < 256u; i++, q++) lut[q * 32u] = f | (ent & 0xFFu) << 16 | i << 24;
+            }
+            if (q < 256u) atomicOr(L.status, MV_DEV_BAD_TABLE);
+            for (; q < 256u; q++) lut[q * 32u] = 1u;
+        }
+        const int row = r.stripe * 32 + lane;
+        const float scale = row_scale(r, row);
+        for (int v0 = 0; v0 < L.batch; v0 += NV) {
+            const int nb = min(NV, L.batch - v0);
+            int sum[NV];
+            float fs[NV];  // sums, or g = s . dy
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                sum[v] = 0;
+                fs[v] = 0.f;
+                if (kMode == 2 && row < r.rows && v < nb)
+                    fs[v] = scale * __uint_as_float((uint32_t)ldp(reinterpret_cast<const uint16_t *>(r.x) + (size_t)(v0 + v) * r.rows + row) << 16);
+            }
+            for (int seg = r.sb; seg < r.sb + (int)r.n; seg++) {
+                const int b = r.stripe * m.nseg + seg;
+                const uint32_t o0 = ldp(m.blk_off + b), o1 = ldp(m.blk_off + b + 1), rows = o1 - o0;
+                if (o1 < o0 || o1 > m.blocks_rows || rows < 2 || rows >= L.block_bytes / 128u) {
+                    if (lane == 0) atomicOr(L.status, MV_DEV_STREAM_OVERRUN);
+                    continue;
+                }
+                __syncwarp();  // (the block before is decoded)
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(&bar, rows * 128u);
+                    if (!L.drop_copy) bulk_g2s(smem + 32768, m.blocks + (size_t)o0 * 32, rows * 128u, &bar);
+                }
+                const int q0 = seg * r.seg_quads, nq = min(r.seg_quads, (r.cols >> 2) - q0);
+                // four quads of every vector (past the batch: its last vector again)
+                constexpr int kX = kMode == 0 ? 1 : kMode == 1 ? 2 : 0;  // 16-byte pieces of them
+                uint4 xn[NV][kX ? kX : 1];
+                const int8_t *xp = r.x + ((size_t)v0 * r.cols + 4 * (size_t)q0) * kX;
+                auto load_x = [&]() {
+                    const int8_t *p = xp;
+#pragma unroll
+                    for (int v = 0; v < (kX ? NV : 0); v++) {
+#pragma unroll
+                        for (int h = 0; h < kX; h++) xn[v][h] = ldx_u4(p + 16 * h);
+                        if (v + 1 < nb) p += (size_t)r.cols * kX;
+                    }
+                };
+                load_x();
+                const bool ok = mbar_wait_bounded(&bar, phase, L.status, L.spin_limit);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    mbar_wait_bounded(&bar, phase, nullptr, L.spin_limit);  // let a late copy land before the exit
+                    return;
+                }
+                phase ^= 1u;
+                uint32_t lo = buf[lane], hi = buf[32 + lane], at = 64u + (uint32_t)lane, P = 0;
+                const uint32_t end = rows * 32u + (uint32_t)lane;
+                for (int q = 0; q < nq; q += 4) {  // segments are whole groups of 4 quads (cols % 16 == 0)
+                    uint4 xv[NV][kX ? kX : 1];
+#pragma unroll
+                    for (int v = 0; v < (kX ? NV : 0); v++)
+#pragma unroll
+                        for (int h = 0; h < kX; h++) xv[v][h] = xn[v][h];
+                    xp += q + 4 < nq ? 16 * kX : 0;
+                    load_x();
+                    float w[16];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const uint32_t word = buf[at];
+                        if (hi == 0) {
+                            hi = lo;
+                            lo = word;
+                            at = min(at + 32u, end);
+                        }
+                        uint32_t e[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) e[j] = lut[((lo >> (8 * j)) & 0xFFu) * 32u];
+                        const uint32_t f0 = e[0] & 0xFFu, f1 = e[1] & 0xFFu, f2 = e[2] & 0xFFu;
+                        P = f0 * f1 * (f2 * (e[3] & 0xFFu));
+                        const unsigned long long st = (unsigned long long)hi * P +
+                                                      ((e[0] >> 24) + f0 * ((e[1] >> 24) + f1 * ((e[2] >> 24) + f2 * (e[3] >> 24))));
+                        lo = (uint32_t)st;
+                        hi = (uint32_t)(st >> 32);
+                        const uint32_t wq = __byte_perm(__byte_perm(e[0], e[1], 0x0062), __byte_perm(e[2], e[3], 0x0062), 0x5410);
+                        if constexpr (kMode == 0) {
+#pragma unroll
+                            for (int v = 0; v < NV; v++) {
+                                const uint4 &x = xv[v][0];
+                                sum[v] = __dp4a((int)wq, (int)(i == 0 ? x.x : i == 1 ? x.y : i == 2 ? x.z : x.w), sum[v]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 4; j++) w[4 * i + j] = (float)(int8_t)(wq >> (8 * j));
+                        }
+                        if constexpr (kMode == 1) {
+#pragma unroll
+                            for (int v = 0; v < NV; v++) {
+                                const uint4 &x = xv[v][i >> 1];
+                                const uint32_t x01 = i & 1 ? x.z : x.x, x23 = i & 1 ? x.w : x.y;
+                                fs[v] = fmaf(w[4 * i], __uint_as_float(x01 << 16), fs[v]);
+                                fs[v] = fmaf(w[4 * i + 1], __uint_as_float(x01 & 0xFFFF0000u), fs[v]);
+                                fs[v] = fmaf(w[4 * i + 2], __uint_as_float(x23 << 16), fs[v]);
+                                fs[v] = fmaf(w[4 * i + 3], __uint_as_float(x23 & 0xFFFF0000u), fs[v]);
+                            }
+                        }
+                    }
+                    if constexpr (kMode == 2) {
+#pragma unroll
+                        for (int v = 0; v < NV; v++)
+                            if (v < nb) wide_reduce(w, fs[v], r.ys + (size_t)(v0 + v) * r.cols + 4 * (q0 + q), lane);
+                    }
+                }
+                if (nq > 0 && (hi != 0 || lo != P)) atomicOr(L.status, MV_DEV_FINAL_STATE);
+            }
+            if (kMode == 2 || row >= r.rows) continue;
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                if (v >= nb) break;
+                if (kMode == 0) {
+                    emit(r, v0 + v, row, sum[v], scale);
+                } else {
+                    float *dst = r.ys + (size_t)(v0 + v) * r.rows + row;
+                    if (r.atomic) atomicAdd(dst, fs[v]);
+                    else *dst = fs[v] * scale;
+                }
+            }
+        }
+    }
+}
+
+template <int kMode>
+mv_status launch_wide(const Q8WLaunch &L0, cudaStream_t st) {
+    Q8WLaunch L = L0;
+    L.block_bytes = L.slot_bytes;
+    const size_t smem = 32768 + (size_t)L.block_bytes;
+    if (L.ragged || smem + 64 > (size_t)max_smem_optin())
+        return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %zu B of shared memory (max %d)", smem + 64, max_smem_optin());
+    auto kern = L.batch == 1 ? q8_wide_kernel<kMode, 1> : q8_wide_kernel<kMode, kMode == 0 ? 16 : 8>;
+    mv_status rc = prepare_kernel((const void *)kern, smem, 32, nullptr);
+    if (rc) return rc;
+    const unsigned grid = (unsigned)std::max(1LL, std::min<long long>(L.nitems, sm_count()));
+    for (int job = L.chain_scales ? 0 : -1; job < (L.chain_scales ? L.njobs : 0); job++) {  // a chain: job after job
+        kern<<<grid, 32, smem, st>>>(L, job);
+        MV_CUDA_TRY(cudaGetLastError(), "q8 wide kernel launch");
+    }
+    return MV_OK;
+}
+
 template <class Cons>
 mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
     Q8WLaunch L = L0;
@@ -1977,10 +2184,7 @@ mv_status launch_t(const Q8WLaunch &L0, int warps, int units, cudaStream_t st) {
         if (S >= W + spare || (S >= W && (W == 1 || S >= units))) break;
         S = 0;
     }
-    if (!S) {
-        const uint32_t need = layout<Cons>(L, 1, 1).total;
-        return fail(MV_ERR_UNSUPPORTED, "Q8 launch needs %u B of shared memory (max %u)", need, limit);
-    }
+    if (!S) return launch_wide<Cons::kPrepare ? 2 : Cons::kFloat ? 1 : 0>(L0, st);
     L.W = W;
     L.S = S;
     L.S_inv = (uint32_t)((0x100000000ull + (uint32_t)S - 1) / (uint32_t)S);

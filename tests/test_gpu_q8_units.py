@@ -227,3 +227,75 @@ def test_scaled_outputs_of_more_than_two_billion_elements():
     for b in range(B):
         assert bool((y[b] == sums[b]).all()) and torch.equal(ys[b], sums[b].float() * s), b
     assert ops.device_status() == 0
+
+
+def wide(rng, rows, cols, seg_quads, local=True):
+    W = rng.integers(-128, 128, size=(rows, cols)).astype(np.int8)  # 8 bits a weight, tables of 256 symbols
+    return W, ops.Q8Matrix.encode(W, local=local, seg_quads=seg_quads)
+
+
+@pytest.mark.parametrize("rows,seg_quads,local", [(40, 880, True), (96, 1132, True), (4768, 1132, True), (96, 1236, False)])
+def test_blocks_that_fill_shared_memory(rows, seg_quads, local):
+    # the largest blocks that a launch shape of one warp, one segment and one buffer lets through: more than the kernel's
+    # tables and staging leave room for.  Single matrices in whole stripes, parts and even shares, stacks, with and without
+    # scales, both engines
+    rng = np.random.default_rng(rows + seg_quads)
+    cols = 4 * (2 * seg_quads + 36)
+    W, M = wide(rng, rows, cols, seg_quads, local)
+    assert M.max_blk_rows >= seg_quads
+    s = rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)
+    for B in (1, 3, 16, 35) if rows < 1000 else (2,):
+        x = rng.integers(-128, 128, size=(B, cols)).astype(np.int8)
+        xd = torch.from_numpy(x).cuda()
+        ref = oracle.matvec_i8(W, x)
+        for parts, engine in ((0, 0), (2, 0), (0, 1)):
+            y, ys = M.matvec(xd, scales=s, tuning=(1, 1, 1, 0, parts, engine))
+            assert np.array_equal(y.cpu().numpy(), ref), (B, parts, engine)
+            assert np.array_equal(ys.cpu().numpy(), (ref.astype(np.float32) * s[None, :]).astype(np.float32)), (B, parts, engine)
+            if B <= 16:
+                S = ops.Q8Stack([M, M], batch=B, xs=[xd, xd], tuning=(1, 1, 1, 0, parts, engine))
+                for _ in range(2):
+                    S.y_flat.fill_(-1)
+                    assert all(np.array_equal(y.cpu().numpy(), ref) for y in S.run()), (B, parts, engine)
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("B", [1, 3, 16])
+def test_chain_of_blocks_that_fill_shared_memory(B):
+    rng = np.random.default_rng(B)
+    W0, M0 = wide(rng, 4720, 128, 32)
+    W1, M1 = wide(rng, 64, 4720, 1132)
+    x = torch.from_numpy(rng.integers(-128, 128, size=(B, 128)).astype(np.int8)).cuda()
+    C = ops.Q8Chain([M0, M1], [2e-4, 2e-5], batch=B, tuning=(1, 1, 1, 0), x0=x)
+    for _ in range(2):
+        C.run()
+        xh = x.cpu().numpy()
+        for W, scale, out, y in ((W0, 2e-4, C.xs[1], C.ys[0]), (W1, 2e-5, C.out8, C.ys[1])):
+            yh = oracle.matvec_i8(W, xh)
+            xh = np.clip(np.rint(yh.astype(np.float32) * np.float32(scale)), -128, 127).astype(np.int8)
+            assert np.array_equal(y.cpu().numpy(), yh) and np.array_equal(out.cpu().numpy(), xh)
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,seg_quads", [(40, 1148), (96, 1400), (4768, 1160)])
+def test_float_blocks_that_fill_shared_memory(rows, seg_quads):
+    # bounds as above (these sums are fp32 throughout: a lane's chain of all columns forward, no split of s . dy backward)
+    rng = np.random.default_rng(rows + seg_quads)
+    cols = 4 * (2 * seg_quads + 36)
+    W, M = wide(rng, rows, cols, seg_quads)
+    s = torch.from_numpy(rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)).cuda()
+    W64 = torch.from_numpy(W).cuda().double()
+    for B in (1, 2, 9, 40) if rows < 1000 else (3,):
+        for engine in (0, 1):
+            t = (1, 1, 1, 0, 0, engine)
+            x = torch.from_numpy(rng.standard_normal((B, cols)).astype(np.float32)).cuda().to(torch.bfloat16)
+            dy = torch.from_numpy(rng.standard_normal((B, rows)).astype(np.float32)).cuda().to(torch.bfloat16)
+            if seg_quads <= 1160:
+                y = M.matvec_bf16(x, s, tuning=t)
+                mag = (x.double().abs() @ W64.abs().T) * s.double()
+                assert ((y.double() - (x.double() @ W64.T) * s.double()).abs() / mag).max().item() < 2.0 ** -24 * (cols + 20)
+                assert torch.equal(y, M.matvec_bf16(x, s, tuning=t)), B
+            dx = M.matvec_t_bf16(dy, s, tuning=t)
+            g = dy.double() * s.double()
+            assert ((dx.double() - g @ W64).abs() / (g.abs() @ W64.abs())).max().item() < 2.0 ** -24 * (12 + rows / 32 + 1)
+    assert ops.device_status() == 0
