@@ -61,6 +61,10 @@ mv_status zero_launch(void *p, size_t words, cudaStream_t st) {
 // 31.0 | 33.0 us, 6 vectors 37.5 | 33.2; 6000x6000, 26.3 | 30.4 and 31.6 | 30.5; a layer of seven matrices, 4 vectors
 // 92.7 | 99.2, 8 vectors 116.6 | 99.3.
 constexpr int kMmaMinVectors = 5;
+// Where the dp4a consumer reads x from global memory, a load per vector and group in its loop (chains, whose x is not there
+// any earlier, and segments of more than kXQuads quads), from 3 vectors: a chain of 7B matrices, 3 vectors 94.6 | 73.5 us,
+// of hidden size 512 22.3 | 21.9; 4096x4096 in segments of 128 quads 17.3 | 15.9, of 256 25.3 | 20.7.
+constexpr int kMmaMinGlobalX = 3;
 // A single matrix that gives no warp a second segment is bound by a lone warp's pace, which the tensor cores' tiles slow
 // down: dp4a up to 8 vectors (500x2992, 8 vectors: 10.5 | 13.0 us; 1024x1024: 9.5 | 10.2).
 constexpr int kMmaMinLone = 9;
@@ -244,7 +248,8 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
     const int pass = t.engine == MV_ENGINE_AUTO ? 64 : 16;
     for (int v0 = 0; v0 < batch; v0 += pass) {
         const int nb = std::min(pass, batch - v0);
-        bool mma = t.engine == MV_ENGINE_AUTO && nb >= kMmaMinVectors;
+        const bool global_x = !ragged && m->seg_quads > kXQuads;
+        bool mma = t.engine == MV_ENGINE_AUTO && nb >= (global_x ? kMmaMinGlobalX : kMmaMinVectors);
         if (!ragged) rc = check_shape_int(t, nv_round(nb), m->max_blk_rows, m->tbl_stripe_max);
         if (rc) return rc;
         Q8WLaunch L{};
@@ -256,11 +261,13 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         L.job0.ys = ys ? ys + (size_t)v0 * m->rows : nullptr;
         const int nv = nv_round(nb);
         auto cost = [&](bool mma) {
-            return Cost{mma ? (nb <= 16 ? 18 + nb / 4 : 23) : 9 + nv, mma ? 220 : 90, 6000 + 100 * nb, 3000 + 60 * nb + (ys ? 1000 : 0),
-                        (long long)nb * m->rows, 6000 + 250 * nb + (ys ? 4000 : 0)};
+            const int n = mma ? std::max(nb, kMmaMinVectors) : nb;  // (tuned from there on)
+            return Cost{mma ? (n <= 16 ? 18 + n / 4 : 23) : 9 + nv, mma ? 220 : 90, 6000 + 100 * n, 3000 + 60 * n + (ys ? 1000 : 0),
+                        (long long)n * m->rows, 6000 + 250 * n + (ys ? 4000 : 0)};
         };
-        int units = plan_single(L, t, cost(mma && nb >= kMmaMinLone));
-        if (mma && nb < kMmaMinLone) {
+        const bool choose = mma && nb < kMmaMinLone && !global_x;
+        int units = plan_single(L, t, cost(mma && !choose));
+        if (choose) {
             mma = units > 10;  // more than a dp4a launch has warps for
             if (mma) units = plan_single(L, t, cost(true));
         }
@@ -503,7 +510,7 @@ mv_status mv_q8_chain_matvec(mv_q8_job *jobs_dev, int njobs, const mv_q8_stack_i
     L.chain_scales = chain_scales_dev;
     L.chain_out8 = out8_dev;
     const int nv = mv::nv_round(batch);
-    const bool mma = t.engine == MV_ENGINE_AUTO && nv >= mv::kMmaMinVectors;
+    const bool mma = t.engine == MV_ENGINE_AUTO && batch >= mv::kMmaMinGlobalX;
     rc = mv::check_shape_int(t, nv, info->max_blk_rows, info->tbl_stripe_max);
     if (rc) return rc;
     mv::q8s_chain_reset<<<(njobs + 255) / 256, 256, 0, st>>>(reinterpret_cast<mv::Q8Job *>(jobs_dev), njobs);

@@ -188,7 +188,6 @@ __device__ __forceinline__ bool table_vote(bool ok) {
 }
 
 // CUDA-core consumers: whether the slots hold their segments' x (segments of up to kXQuads quads, not in a chain)
-constexpr int kXQuads = 64;
 __device__ __forceinline__ bool x_in_slot(const Q8WLaunch &L, int seg_quads) {
     return L.x_off != 0 && !L.ragged && seg_quads <= kXQuads;
 }

@@ -10,6 +10,8 @@ namespace mv {
 
 typedef mv_q8_job Q8Job;
 
+constexpr int kXQuads = 64;  // the longest segments, in quads, whose x the CUDA-core consumers' slots hold
+
 struct Q8WLayout {  // byte offsets in shared memory
     uint32_t tiles, slots, red, bars, desc, ring, cnt, stage_o, stage_e, misc, total;
 };
