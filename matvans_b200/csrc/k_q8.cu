@@ -1,5 +1,6 @@
-// Q8-stripe decode (mv_q8_decode) and the int8 matvec of matrices whose blocks
-// are too large for the warp-specialised kernel (k_q8w.cu), for sm_100a.
+// Q8-stripe decode (mv_q8_decode) and the int8 matvec of ragged matrices with
+// short rows (q8_by_stripe) or with blocks that are too large for the warp-
+// specialised kernel (k_q8w.cu), for sm_100a.
 //
 // Layout (built by host_q8.cpp): rows are grouped into stripes of 32, lane l
 // of a warp owning row 32*stripe + l; each row is cut into segments of
@@ -302,6 +303,41 @@ int pick_warps(const mv_q8_view &m, int nv, bool decode) {
 
 int nv_for(int nb) { return nb <= 2 ? nb : nb <= 4 ? 4 : nb <= 8 ? 8 : 16; }
 
+template <int NV>
+int resident(const mv_q8_view &m, int W) {  // CTAs an SM holds (0: unknown)
+    int n = 0;
+    return prepare_kernel((const void *)q8_kernel<NV, false>, q8_smem_bytes(m, W, NV, false), 32 * W, &n) ? 0 : n;
+}
+
+// Whether a ragged product is this kernel's and not the warp-specialised one's (q8s_takes_ragged).  With short rows and
+// several stripes an SM a launch is little more than table builds, which that one does one after another on an SM, and this
+// one in as many CTAs as the SM holds.  So: where the whole grid is resident at once and an SM of the other kernel has 3
+// stripes or more (one table for all rows: more, since it is built once there); beyond that, where it is many rounds on
+// both, for the sizes and batches it still gains at.  Measured on a B200, this | that: 16000x401, a table per row, 1, 2, 8
+// and 16 vectors 11.7 | 15.3, 13.7 | 15.6, 14.6 | 19.5 and 28.8 | 24.7 us (not resident at 16); 9600x401 10.9 | 11.7,
+// 12.9 | 12.4, 13.8 | 15.8 and 17.6 | 19.0; 6000x401 10.2 | 9.5, 12.2 | 9.7, 12.7 | 10.9 and 16.3 | 12.8; one table,
+// 16000x401 10.3 | 12.1, 11.9 | 12.7, 13.3 | 14.2 and 26.4 | 17.2; 50000x401, a table per row 29.6 | 33.4, 34.9 | 34.2,
+// 38.7 | 44.0 and 59.5 | 56.7; 50000x17, 24 | 36 with 16 vectors.
+bool q8_by_stripe(const mv_q8_view &m, int batch) {
+    if (batch > 16 || m.cols > 1024 || m.nseg > 8) return false;
+    const int stripes = (m.rows + 31) / 32, sms = sm_count(), items = (stripes + sms - 1) / sms;
+    if (items < 3) return false;
+    const int nv = nv_for(batch), W = pick_warps(m, nv, false);
+    const int n = nv == 1   ? resident<1>(m, W)
+                  : nv == 2 ? resident<2>(m, W)
+                  : nv == 4 ? resident<4>(m, W)
+                  : nv == 8 ? resident<8>(m, W)
+                            : resident<16>(m, W);
+    if (W == m.nseg && stripes <= n * sms) {
+        if (!m.local) return items >= (batch == 1 ? 3 : batch == 2 ? 4 : 5);
+        return items >= (batch >= 2 && batch <= 4 ? 4 : 3) + (m.nseg == 1 || m.cols > 832 ? 1 : 0);
+    }
+    if (items < 7 || m.cols > 640) return false;
+    if (m.cols <= (m.local ? 80 : 48)) return true;
+    if (batch == 1) return m.local || m.nseg == 1;
+    return m.local && m.nseg >= 3 && batch > 4 && batch <= 8;
+}
+
 }  // namespace
 
 bool q8s_supports(const mv_q8_view *m, const int8_t *x);
@@ -315,7 +351,8 @@ mv_status q8_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y,
     if (rc) return rc;
     if (!x || !y || batch <= 0) return fail(MV_ERR_ARG, "mv_q8_matvec: bad x/y/batch");
     if (ys && !scales) return fail(MV_ERR_ARG, "mv_q8_matvec: y_scaled needs row scales");
-    if (q8s_supports(m, x) || q8s_takes_ragged(m, batch)) return q8s_matvec(m, x, batch, y, scales, ys, nullptr, st);
+    if (q8s_supports(m, x) || (q8s_takes_ragged(m, batch) && !q8_by_stripe(*m, batch)))
+        return q8s_matvec(m, x, batch, y, scales, ys, nullptr, st);
     uint32_t *status = device_status_word(&rc);
     if (rc) return rc;
     for (int v0 = 0; v0 < batch; v0 += 16) {

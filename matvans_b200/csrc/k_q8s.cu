@@ -268,7 +268,10 @@ mv_status q8s_matvec(const mv_q8_view *m, const int8_t *x, int batch, int32_t *y
         const bool choose = mma && nb < kMmaMinLone && !global_x;
         int units = plan_single(L, t, cost(mma && !choose));
         if (choose) {
-            mma = units > 10;  // more than a dp4a launch has warps for
+            // More than a dp4a launch has warps for.  Not for ragged short rows, bound by their tables and outputs: dp4a |
+            // tensor cores, 8 vectors, 16000x401 19.5 | 21.8 us, one table for all 14.2 | 15.3; 50000x129 42.6 | 45.8, one
+            // table 22.9 | 29.9; 30000x803 33.8 | 36.9, one table 27.7 | 25.1.
+            mma = units > 10 && !(ragged && m->cols <= (m->local ? 832 : 480));
             if (mma) units = plan_single(L, t, cost(true));
         }
         float *out = L.job0.ys;

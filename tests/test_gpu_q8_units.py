@@ -299,3 +299,23 @@ def test_float_blocks_that_fill_shared_memory(rows, seg_quads):
             g = dy.double() * s.double()
             assert ((dx.double() - g @ W64).abs() / (g.abs() @ W64.abs())).max().item() < 2.0 ** -24 * (12 + rows / 32 + 1)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,cols,local", [(9600, 301, True), (16000, 401, True), (16001, 129, False), (33200, 65, True),
+                                             (35000, 17, False), (34000, 303, True), (14000, 1021, True)])
+def test_ragged_short_rows(rows, cols, local):
+    # around the line between the two kernels for ragged products (grids that are resident at once, and of several rounds),
+    # plain and scaled, on rows of x that start anywhere
+    rng = np.random.default_rng(rows + cols)
+    W = np.clip(np.round(rng.normal(0, 4.0, size=(rows, cols))), -128, 127).astype(np.int8)
+    M = ops.Q8Matrix.encode(W, local=local)
+    W64 = torch.from_numpy(W).cuda().double()
+    s = torch.from_numpy(rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)).cuda()
+    for B in (1, 2, 4, 7, 8, 16, 17):
+        x = torch.randint(-128, 128, (3 + B * cols,), dtype=torch.int8, device="cuda")[3:].view(B, cols)
+        ref = x.double() @ W64.T
+        y, ys = M.matvec(x, scales=s)
+        assert torch.equal(y.double(), ref), B
+        assert torch.equal(ys, ref.float() * s), B
+        assert torch.equal(M.matvec(x), y), B
+    assert ops.device_status() == 0
