@@ -112,7 +112,7 @@ struct Bars {
     __device__ __forceinline__ uint32_t rfull(int k) const { return at(k); }              // item record written
     __device__ __forceinline__ uint32_t tfull(int k) const { return at(kRing + k); }      // decode table ready
     __device__ __forceinline__ uint32_t tdone(int k) const { return at(2 * kRing + k); }  // item decoded
-    __device__ __forceinline__ uint32_t idone(int k) const { return at(3 * kRing + k); }  // item's outputs written
+    __device__ __forceinline__ uint32_t idone(int k) const { return at(3 * kRing + k); }  // item's outputs written, record read
     __device__ __forceinline__ uint32_t staged(int g) const { return at(4 * kRing + g); } // table data in shared memory
     __device__ __forceinline__ uint32_t sfull(int s) const { return at(kFixed + s); }
     __device__ __forceinline__ uint32_t sempty(int s) const { return at(kFixed + S + s); }
@@ -123,6 +123,7 @@ struct Bars {
     // arrivals that complete barrier i's phase
     __device__ __forceinline__ int arrivals(int i) const {
         if (i >= 2 * kRing && i < 3 * kRing) return (int)kTdone;
+        if (i >= 3 * kRing && i < 4 * kRing) return 2;  // the table warps, and the stager, which reads every record too
         if (i >= 4 * kRing && i < kFixed) return 33;  // the stager's lanes, and once for the offsets
         return i >= kFixed + 2 * S + W && i < kFixed + 2 * S + 3 * W ? kTableWarps : 1;  // dempty: every table warp has read the sums
     }
@@ -326,13 +327,16 @@ __device__ __forceinline__ void stage_tables(const Q8WLaunch &L, unsigned char *
         if (!__all_sync(0xffffffffu, wait_bar(B.rfull(k % kRing), (uint32_t)(k / kRing) & 1u, L, failed))) break;
         const ItemRec &r = ring[k % kRing];
         if (r.it < 0) break;
-        if (!r.build) continue;
-        if (r.area_item >= 0 && r.area_item > k - kRing) {  // (earlier items are done)
-            const bool built = wait_bar(B.tfull(r.area_item % kRing), (uint32_t)(r.area_item / kRing) & 1u, L, failed);
-            if (!__all_sync(0xffffffffu, built)) break;
+        if (r.build) {
+            if (r.area_item >= 0 && r.area_item > k - kRing) {  // (earlier items are done)
+                const bool built = wait_bar(B.tfull(r.area_item % kRing), (uint32_t)(r.area_item / kRing) & 1u, L, failed);
+                if (!__all_sync(0xffffffffu, built)) break;
+            }
+            stage_table(L, r, sm, B, lane);
+            if (k == 0) grid_dependency_wait();  // (see produce)
         }
-        stage_table(L, r, sm, B, lane);
-        if (k == 0) grid_dependency_wait();  // (see produce)
+        __syncwarp();
+        if (lane == 0) arrive(B.idone(k % kRing));  // the record may be overwritten
     }
     cp_async_wait_all();
 }

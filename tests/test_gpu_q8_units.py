@@ -319,3 +319,23 @@ def test_ragged_short_rows(rows, cols, local):
         assert torch.equal(ys, ref.float() * s), B
         assert torch.equal(M.matvec(x), y), B
     assert ops.device_status() == 0
+
+
+def test_many_items_share_one_table():
+    # one table for all rows and items of a single short unit: records pass through their ring as fast as they can, most of
+    # them with no table to stage, between them in a stack the few that have one
+    rng = np.random.default_rng(5)
+    shapes = [(60000, 16), (64, 512), (40000, 32), (30000, 16)]
+    Ws = [np.clip(np.round(rng.normal(0, 3.0, size=sh)), -127, 127).astype(np.int8) for sh in shapes]
+    Ms = [ops.Q8Matrix.encode(W, local=i == 1) for i, W in enumerate(Ws)]
+    for B in (1, 3, 16):
+        xs = [torch.from_numpy(rng.integers(-128, 128, size=(B, M.cols)).astype(np.int8)).cuda() for M in Ms]
+        S = ops.Q8Stack(Ms, batch=B, xs=xs)
+        for _ in range(10):
+            S.y_flat.fill_(-1)
+            S.run()
+            for W, x, y in zip(Ws, xs, S.ys):
+                assert np.array_equal(y.cpu().numpy(), oracle.matvec_i8(W, x.cpu().numpy())), (B, W.shape)
+        for M, W, x in zip(Ms, Ws, xs):
+            assert np.array_equal(M.matvec(x).cpu().numpy(), oracle.matvec_i8(W, x.cpu().numpy())), (B, W.shape)
+    assert ops.device_status() == 0
