@@ -24,6 +24,9 @@
  *     library does not allocate on the launch paths except one lazily created
  *     per-device status word (see mv_device_status).
  *   - `stream` is a cudaStream_t passed as void* (NULL = legacy default).
+ *     Stream order holds for all that a call is given: a launch may start
+ *     while the one before it ends, but reads inputs, matrices, tables and job
+ *     tables only once that one is complete.
  *   - x is [batch][cols] int8 row-major; y is [batch][rows] int32.  y is
  *     exact: decoded weights times x accumulated in int32.  y_scaled, when
  *     non-NULL, is [batch][rows] float with y_scaled = (float)y * scale[row].
@@ -226,27 +229,24 @@ mv_status mv_q8_matvec(const mv_q8_view *m, const int8_t *x_dev, int batch, int3
 #define MV_ENGINE_AUTO 0
 #define MV_ENGINE_DP4A 1
 /* Smallest integer batch that engine 0 (MV_ENGINE_AUTO) can run on the tensor
- * cores. */
+ * cores (chains and segments of more than 64 quads do from here on, stacks from
+ * 5 vectors, single matrices from 5 or 9 by size). */
 #define MV_MMA_MIN_VECTORS 3
 typedef struct mv_q8_tuning {
     int32_t warps, ilp, depth, ctas_per_sm, parts, engine;
 } mv_q8_tuning;
 
 /* mv_q8_matvec with explicit launch parameters (needs cols % 16 == 0,
- * seg_quads % 4 == 0 and a 16-byte aligned x; mv_q8_matvec itself falls back
- * to a non-persistent kernel otherwise). */
+ * seg_quads % 4 == 0 and a 16-byte aligned x; mv_q8_matvec itself takes any). */
 mv_status mv_q8_matvec_tuned(const mv_q8_view *m, const int8_t *x_dev, int batch, int32_t *y_dev,
                              const float *row_scales_dev, float *y_scaled_dev,
                              const mv_q8_tuning *tuning, void *stream);
 
 /* One matrix of a batched launch: the matrix, its input x [batch][cols] and
  * outputs y [batch][rows] (+ optional scaled output).  ngroups, atomic and
- * item0 are filled in by mv_q8_stack_plan.  x_tiles (optional, NULL for none)
- * is device scratch of mv_q8_x_tiles_bytes(&m) bytes, 16-byte aligned: with
- * 3..16 vectors on the tensor cores, mv_q8_stack_matvec first lays x out there
- * in the MMA operand layout, and each warp then brings its x windows in with
- * asynchronous copies (four 16-byte cp.async per lane per window, completing
- * on an mbarrier) instead of loads and stores through registers. */
+ * item0 are filled in by mv_q8_stack_plan.  x_tiles is accepted and not used:
+ * callers may leave it NULL or keep giving it the scratch of
+ * mv_q8_x_tiles_bytes(&m) bytes that it once named. */
 typedef struct mv_q8_job {
     mv_q8_view m;
     const int8_t *x;

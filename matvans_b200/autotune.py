@@ -1,9 +1,11 @@
 """Per-shape launch-parameter autotuner for the persistent Q8 kernel, with a JSON cache.
 
-The tunables are the ones the kernel exposes through mv_q8_tuning: warps per
-CTA, independent streams decoded per warp (ilp) and shared-memory stream buffer
-depth (depth).  Stream interleave inside a row (segment length) is fixed when a
-matrix is encoded (q8_encode's seg_quads), so it is part of the cache key.
+The tunables are mv_q8_tuning's: the decode warps (up to 8 stand for twice as
+many), the parts a single matrix's stripes are split into, and the engine.  ilp
+and depth only decide whether a launch shape is accepted; shapes that differ in
+nothing else run the same launch and are timed as often as they are listed.  The
+segment length is fixed when a matrix is encoded (q8_encode's seg_quads), so it
+is part of the cache key.
 
 Each candidate is timed as a CUDA graph of R launches over R copies of the
 matrix, enough copies that their compressed bytes exceed twice the L2, so every

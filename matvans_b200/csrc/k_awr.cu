@@ -28,8 +28,8 @@
 //     result is exact (requantisation optional).
 // What bounds it: issue, ~45 instructions a step (98 in the form this replaced,
 // which kept the words in registers and moved them by shuffles).  Measured on a
-// B200, 4096x4096, one vector: 17.6 us before, 11.5 us now; calls back to back,
-// each launched while the one before it ends, 13.3 -> 11.4 us.
+// B200, 4096x4096, one vector: 19.4 us before, 12.0 us now; calls back to back,
+// launched after one another and while the one before ends, 13.3 and 11.4 us.
 //
 // The "ans-warp-stripes" layout (ans-warp-stripes-kernel.cu:21-227, encoder.py:
 // 323-391) has the same coder and word stream with lane = row of a 32-row stripe:

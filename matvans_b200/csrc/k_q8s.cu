@@ -1,6 +1,6 @@
 // Planning and launching of the Q8-stripe products: single matrices, stacks (many
 // matrices in one launch), the chained pipeline and the float form, all through
-// the warp-specialised kernel of k_q8w.cu.
+// the kernels of k_q8w.cu.
 #include <algorithm>
 
 #include "mv_device.cuh"
@@ -58,15 +58,15 @@ mv_status zero_launch(void *p, size_t words, cudaStream_t st) {
 
 // Integer batches of at least this many vectors go to the tensor-core consumer with engine 0, whose cost hardly depends
 // on the batch, while the dp4a consumer's grows with it.  Measured on a B200, dp4a | tensor cores: 11008x4096, 4 vectors
-// 31.0 | 33.0 us, 6 vectors 37.5 | 33.2; 6000x6000, 26.3 | 30.4 and 31.6 | 30.5; a layer of seven matrices, 4 vectors
-// 92.7 | 99.2, 8 vectors 116.6 | 99.3.
+// 30.2 | 32.6 us, 6 vectors 36.4 | 31.4; 6000x6000, 25.5 | 29.5 and 30.8 | 29.5; a layer of seven matrices, 4 vectors
+// 92.7 | 97.1, 8 vectors 115.4 | 97.5.
 constexpr int kMmaMinVectors = 5;
 // Where the dp4a consumer reads x from global memory, a load per vector and group in its loop (chains, whose x is not there
 // any earlier, and segments of more than kXQuads quads), from 3 vectors: a chain of 7B matrices, 3 vectors 94.6 | 73.5 us,
 // of hidden size 512 22.3 | 21.9; 4096x4096 in segments of 128 quads 17.3 | 15.9, of 256 25.3 | 20.7.
 constexpr int kMmaMinGlobalX = 3;
 // A single matrix that gives no warp a second segment is bound by a lone warp's pace, which the tensor cores' tiles slow
-// down: dp4a up to 8 vectors (500x2992, 8 vectors: 10.5 | 13.0 us; 1024x1024: 9.5 | 10.2).
+// down: dp4a up to 8 vectors (500x2992, 8 vectors: 10.0 | 12.4 us; 1024x1024: 8.8 | 9.0).
 constexpr int kMmaMinLone = 9;
 // check_shape: the batch from which a launch shape is taken as a tensor-core one.
 constexpr int kMmaShape = MV_MMA_MIN_VECTORS;
@@ -140,9 +140,9 @@ mv_status check_shape_int(const mv_q8_tuning &t, int nv, int max_blk_rows, uint3
 // quad of a warp's own pace, and no less than its items' service by the table warps (a table build of ~6000 cycles, and
 // the epilogue); to that, what joining cut stripes takes (zeroing launch, scaling launch, atomics).  Measured on a B200,
 // whole stripes | even shares | the best aligned parts, 16 int8 vectors: 11008x4096 (3 items on some CTAs, 2 on others)
-// 38.8 | 38.0 | 40.4 us, 6000x6000 34.9 | 30.1 | 31.4, 2400x11008 32.8 | 25.3 | 29.1, 500x2992 17.5 | 12.5 | 12.1; the
-// same, one vector: 24.8 | 27.0 | 31.4, 24.2 | 23.2 | 24.1, 22.2 | 19.6 | 21.4, 12.1 | - | 9.3.  The backward adds to
-// dX by atomics in any case: 11008x4096, 64 vectors, 144.6 | 131.5 us.
+// 36.7 | 36.1 | 39.4 us, 6000x6000 33.1 | 28.8 | 30.6, 2400x11008 31.3 | 24.5 | 27.3, 500x2992 16.2 | 14.0 | 11.7; the
+// same, one vector: 23.7 | 26.4 | 30.0, 23.0 | 22.3 | 23.4, 21.3 | 19.1 | 19.7, 11.2 | 11.6 | 9.3.  The backward adds to
+// dX by atomics in any case: 11008x4096, 64 vectors, 132.8 | 121.9 us.
 struct Cost {
     int step, lone;
     int service;     // cycles an item takes the table warps
@@ -329,8 +329,8 @@ mv_status q8_fwd(const mv_q8_view *m, const uint16_t *x, int batch, const float 
         L.job0.ys = y + (size_t)v0 * m->rows;
         L.batch = std::min(pass, batch - v0);
         // whole stripes, or even shares where no stripe is cut twice: a sum of two parts does not depend on their order
-        // (whole | even: 11008x4096, one vector 29.5 | 32.0 us, 16 vectors 48.5 | 52.1, 64 vectors 57.6 | 64.9; 6000x6000, 16
-        // vectors 49.1 | 45.8, 64 vectors 57.8 | 56.5)
+        // (whole | even: 11008x4096, one vector 28.3 | 31.4 us, 16 vectors 46.7 | 51.6, 64 vectors 54.5 | 63.1; 6000x6000, 16
+        // vectors 46.7 | 45.1, 64 vectors 54.3 | 55.2)
         constexpr int kNever = 1 << 30;
         const bool cuda = dot || L.batch == 1;
         const Cost cost{cuda ? 11 + 4 * nv_round(L.batch) : 26 + L.batch / 16, cuda ? 90 : 220, 6000 + 100 * L.batch, kNever, 0,

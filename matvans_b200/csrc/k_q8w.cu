@@ -23,7 +23,7 @@
 // One CTA-wide barrier per item, a table build and a cross-warp sum between the
 // items of the form this replaced left the SM idle for a third of a launch: the
 // seven matrices of a 7B layer took 139 us there with one vector and take 74 us,
-// with 16 vectors 136 and 109 us; 64 vectors of 11008x4096, 197 and 47 us.
+// with 16 vectors 136 and 107 us; 64 vectors of 11008x4096, 198 and 46 us.
 //
 // Decode table: entry (q, lane) = f | sym << 16 | r << 24 (frequency of the
 // symbol that owns quantile q, the symbol, r = q - cum), 4 bytes at byte
@@ -43,7 +43,8 @@
 //             multiply-add
 //
 // What bounds it: issue and the ALU pipe.  A step takes 29 instructions (9 byte
-// permutes at half rate) and 5 shared-memory wavefronts; a loop of steps alone
+// permutes at half rate; 35 with all that a launch does around it) and 5
+// shared-memory wavefronts; a loop of steps alone
 // runs at 9.2 SM cycles a step with 16 warps (a single warp's step takes 80), and
 // the kernel at 11 on a 7B layer (one vector).
 #include <algorithm>
@@ -1460,8 +1461,9 @@ struct FwdDot {
 // The sums of a tile are read while the next one decodes.  From 5 vectors on they pass through shared memory so that
 // eight lanes cover the 128 bytes of a vector's row: reductions from one lane per vector ran at 2.6 TB/s, these at 5.4,
 // and they bound the larger batches (4 bytes per vector, column and stripe).
-// Measured on a B200 against the form this replaced (8 vectors a pass, CUDA cores): 11008x4096, 64 vectors 222 -> 145 us,
-// 16 vectors 90 -> 64 us, 2 vectors 76 -> 57 us; 4096x11008, 64 vectors 259 -> 151 us, 16 vectors 106 -> 63 us.
+// Measured on a B200 against the form this replaced (the same passes, terms and MMAs in a CTA with barriers between its
+// items): 11008x4096, 64 vectors 219 -> 120 us, 16 vectors 87 -> 52 us, 2 vectors 75 -> 45 us; 4096x11008, 64 vectors
+// 251 -> 120 us, 16 vectors 104 -> 52 us.
 struct BwdCons {
     static constexpr bool kMma = true, kFloat = true, kStatic = false, kPrepare = true;
     static constexpr int kRed = 0, kAreas = 0;
@@ -1647,9 +1649,9 @@ struct BwdCons {
 // with the row's g = s . dy (the tensor cores' sums of 32 rows are less exact than fp32 additions).  The products of 4 quads
 // (16 columns) of the 32 rows change hands in shared memory, a vector at a time: a lane stores its row's four 16-byte pieces
 // and reads one piece of four rows, which leaves eight partial sums a column for three shuffle steps.  (All sixteen columns
-// by shuffles alone: 30 selects and 16 shuffles a group against 6 and 4.)  Bound by issue.  Measured on a B200, one vector:
-// 4096x11008 52 -> 37 us, 11008x4096 47 -> 41 us (with BwdCons, 55 and 57 us and 2e-6 of error where this form has 2e-7); 8 vectors
-// 141 and 150 us.
+// by shuffles alone: 30 selects and 16 shuffles a group against 6 and 4.)  Bound by issue.  Measured on a B200, one vector,
+// by shuffles between barriers and now: 4096x11008 47 -> 37 us, 11008x4096 50 -> 41 us (with BwdCons, 45 us and 2e-6 of
+// error where this form has 2e-7); 8 vectors 141 and 150 us.
 template <int NV>
 struct BwdDot {
     static constexpr bool kMma = false, kFloat = true, kStatic = false, kPrepare = true;
