@@ -265,3 +265,40 @@ def test_tables_written_late_by_a_launch_that_lets_the_next_begin_early(kind):
         for i, y in enumerate(ys):
             assert np.array_equal(y.cpu().numpy(), refs[i % 2]), i
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("B", [1, 2, 40, 70])
+def test_float_form_and_scales_written_by_the_launch_before(B):
+    # x, dY, row scales and the matrix by kernels right before each product, the float form both ways and the scaled integer
+    # product: what an undisturbed call gives (dX to the order of its additions: two stripes' parts add up the same either way)
+    rng = np.random.default_rng(B)
+    rows, cols = 64, 2048
+    M, Ws, src, dst = two_q8(rng, rows, cols, True)
+    fs = [torch.from_numpy(rng.uniform(1e-3, 1e-2, size=rows).astype(np.float32)).cuda() for _ in range(2)]
+    xf = [torch.randn((B, cols), device="cuda").bfloat16() for _ in range(2)]
+    dy = [torch.randn((B, rows), device="cuda").bfloat16() for _ in range(2)]
+    x8 = [torch.randint(-128, 128, (B, cols), dtype=torch.int8, device="cuda") for _ in range(2)]
+    s, x, d, q = (torch.empty_like(v[0]) for v in (fs, xf, dy, x8))
+
+    def calls():
+        return [M.matvec_bf16(x, s), M.matvec_t_bf16(d, s), *M.matvec(q, scales=s)]
+    want = []
+    for i in range(2):
+        for t, v in zip(dst + [s, x, d, q], src[i] + [fs[i], xf[i], dy[i], x8[i]]):
+            put(t, v)
+        torch.cuda.synchronize()
+        want.append(calls())
+        assert np.array_equal(want[i][2].cpu().numpy(), oracle.matvec_i8(Ws[i], x8[i].cpu().numpy()))
+    torch.cuda.synchronize()
+
+    def body():
+        out = []
+        for i in range(RUNS):
+            for t, v in zip(dst + [s, x, d, q], src[i % 2] + [fs[i % 2], xf[i % 2], dy[i % 2], x8[i % 2]]):
+                put(t, v)
+            out.append(calls())
+        return out
+    for out in eager_and_graph(body):
+        for i, got in enumerate(out):
+            assert all(torch.equal(a, b) for a, b in zip(got, want[i % 2])), i
+    assert ops.device_status() == 0
